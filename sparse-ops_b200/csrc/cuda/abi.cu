@@ -44,7 +44,7 @@ int sm_count(int device)
 
 // The zero fill of the slabs is enqueued on `s`, the stream the caller fills them on afterwards:
 // a non-blocking stream is not ordered behind work on the default stream.
-int alloc_ell(uint32_t m, uint32_t n, uint32_t r, spx_ell** out, cudaStream_t s)
+int alloc_ell(uint32_t m, uint32_t n, uint32_t r, spx_ell** out, cudaStream_t s, bool zero_fill)
 {
     spx_ell* e = new (std::nothrow) spx_ell();
     if (!e) return fail(SPX_ERR_OOM, "out of host memory");
@@ -58,42 +58,48 @@ int alloc_ell(uint32_t m, uint32_t n, uint32_t r, spx_ell** out, cudaStream_t s)
     e->m = m; e->n = n; e->r = r;
     e->pitch = r ? round_up<uint32_t>(r, 32u) : 0u;
     const size_t slots = (size_t)m * e->pitch;
+    int rc = SPX_OK;
     cudaError_t err = cudaSuccess;
     if (slots) {
-        err = cudaMalloc(&e->Wd, slots * sizeof(float));
-        if (err == cudaSuccess) err = cudaMalloc(&e->idx, slots * sizeof(uint32_t));
+        rc = pool_alloc(reinterpret_cast<void**>(&e->Wd), slots * sizeof(float), e->device, s);
+        if (rc == SPX_OK) rc = pool_alloc(reinterpret_cast<void**>(&e->idx), slots * sizeof(uint32_t), e->device, s);
         // padding slots hold Wd = 0.0f, idx = 0 like the reference's (src/ellpack_encoder.cpp:25)
-        if (err == cudaSuccess) err = cudaMemsetAsync(e->Wd, 0, slots * sizeof(float), s);
-        if (err == cudaSuccess) err = cudaMemsetAsync(e->idx, 0, slots * sizeof(uint32_t), s);
+        if (rc == SPX_OK && zero_fill) err = cudaMemsetAsync(e->Wd, 0, slots * sizeof(float), s);
+        if (rc == SPX_OK && zero_fill && err == cudaSuccess) err = cudaMemsetAsync(e->idx, 0, slots * sizeof(uint32_t), s);
     }
-    if (err == cudaSuccess && m) err = cudaMalloc(&e->nnz, (size_t)m * sizeof(uint32_t));
-    if (err == cudaSuccess && m) err = cudaMemsetAsync(e->nnz, 0, (size_t)m * sizeof(uint32_t), s);
-    if (err != cudaSuccess) {
-        cudaFree(e->Wd); cudaFree(e->idx); cudaFree(e->nnz);
+    if (rc == SPX_OK && m) rc = pool_alloc(reinterpret_cast<void**>(&e->nnz), (size_t)m * sizeof(uint32_t), e->device, s);
+    if (rc == SPX_OK && m && zero_fill && err == cudaSuccess) err = cudaMemsetAsync(e->nnz, 0, (size_t)m * sizeof(uint32_t), s);
+    if (rc != SPX_OK || err != cudaSuccess) {
+        pool_free(e->Wd, slots * sizeof(float), s); pool_free(e->idx, slots * sizeof(uint32_t), s); pool_free(e->nnz, (size_t)m * sizeof(uint32_t), s);
         delete e;
-        return fail(err == cudaErrorMemoryAllocation ? SPX_ERR_OOM : SPX_ERR_CUDA,
-                    "ELLPACK device allocation (%zu slots) failed: %s", slots, cudaGetErrorString(err));
+        return rc != SPX_OK ? rc : fail(SPX_ERR_CUDA, "ELLPACK zero fill (%zu slots) failed: %s", slots, cudaGetErrorString(err));
     }
     *out = e;
+    return SPX_OK;
+}
+
+int sort_rows(spx_ell* e, const uint32_t* host_nnz, uint32_t* order, cudaStream_t s)
+{
+    // counting sort by row length, longest first; stable, so ties keep ascending row id
+    std::vector<uint32_t> start((size_t)e->r + 2, 0);
+    e->long_rows = 0;
+    e->min_nnz = host_nnz[0];
+    for (uint32_t i = 0; i < e->m; ++i) {
+        start[e->r - host_nnz[i] + 1]++;
+        e->long_rows += host_nnz[i] >= 512 ? 1u : 0u;
+        e->min_nnz = std::min(e->min_nnz, host_nnz[i]);
+    }
+    for (size_t k = 1; k < start.size(); ++k) start[k] += start[k - 1];
+    for (uint32_t i = 0; i < e->m; ++i) order[start[e->r - host_nnz[i]]++] = i;
+    if (!e->row_order) return pool_alloc(reinterpret_cast<void**>(&e->row_order), (size_t)e->m * sizeof(uint32_t), e->device, s);
     return SPX_OK;
 }
 
 int set_row_order(spx_ell* e, const uint32_t* host_nnz)
 {
     if (e->m == 0) return SPX_OK;
-    // counting sort by row length, longest first; stable, so ties keep ascending row id
-    std::vector<uint64_t> start((size_t)e->r + 2, 0);
-    for (uint32_t i = 0; i < e->m; ++i) start[e->r - host_nnz[i] + 1]++;
-    for (size_t k = 1; k < start.size(); ++k) start[k] += start[k - 1];
     std::vector<uint32_t> order(e->m);
-    for (uint32_t i = 0; i < e->m; ++i) order[start[e->r - host_nnz[i]]++] = i;
-    e->long_rows = 0;
-    e->min_nnz = host_nnz[0];
-    for (uint32_t i = 0; i < e->m; ++i) {
-        e->long_rows += host_nnz[i] >= 512 ? 1u : 0u;
-        e->min_nnz = std::min(e->min_nnz, host_nnz[i]);
-    }
-    if (!e->row_order) SPX_CUDA(cudaMalloc(&e->row_order, (size_t)e->m * sizeof(uint32_t)));
+    if (int rc = sort_rows(e, host_nnz, order.data(), nullptr)) return rc;
     SPX_CUDA(cudaMemcpy(e->row_order, order.data(), (size_t)e->m * sizeof(uint32_t), cudaMemcpyHostToDevice));
     return SPX_OK;
 }
@@ -323,6 +329,8 @@ int spx_ell_create(uint32_t m, uint32_t n, uint32_t r, const float* Wd, const ui
         return fail(SPX_ERR_CUDA, "ELLPACK upload failed: %s", cudaGetErrorString(err));
     }
     rc = set_row_order(e, nnz);
+    // copies from pageable memory may still be on their way: the handle is complete for every stream
+    if (rc == SPX_OK && cudaStreamSynchronize(nullptr) != cudaSuccess) rc = fail(SPX_ERR_CUDA, "ELLPACK upload failed");
     if (rc != SPX_OK) { spx_ell_destroy(e); return rc; }
     *out = e;
     return SPX_OK;
@@ -376,6 +384,7 @@ int spx_ell_create_csr(uint32_t m, uint32_t n, const uint64_t* rowptr, const uin
         std::vector<uint32_t> counts(m);
         for (uint32_t i = 0; i < m; ++i) counts[i] = (uint32_t)(rowptr[i + 1] - rowptr[i]);
         rc = set_row_order(e, counts.data());
+        if (rc == SPX_OK && cudaStreamSynchronize(nullptr) != cudaSuccess) rc = fail(SPX_ERR_CUDA, "CSR upload failed");
         if (rc != SPX_OK) { spx_ell_destroy(e); return rc; }
     }
     *out = e;
@@ -399,7 +408,16 @@ int spx_ell_destroy(spx_ell* e)
     if (e->view) e->Wd = nullptr, e->idx = nullptr, e->nnz = nullptr;      // the parent's arrays
     for (cudaStream_t st : e->xchg_streams) if (st) cudaStreamDestroy(st);
     for (cudaEvent_t ev : e->xchg_events) if (ev) cudaEventDestroy(ev);
-    cudaFree(e->Wd); cudaFree(e->idx); cudaFree(e->nnz); cudaFree(e->row_order); cudaFree(e->taps); cudaFree(e->spmv_split); cudaFree(e->rbm_hdr); cudaFree(e->rbm_w); cudaFree(e->rbm_ncols); cudaFree(e->stage_dev); cudaFree(e->conv_scratch); cudaFree(e->fm_scratch);
+    // Kernels that read the handle may still run, on any stream: one wait for the device, after which
+    // its arrays go back to the pool without another one.
+    (void)cudaDeviceSynchronize();
+    pool_free(e->Wd, (size_t)e->m * e->pitch * 4, nullptr);
+    pool_free(e->idx, (size_t)e->m * e->pitch * 4, nullptr);
+    pool_free(e->nnz, (size_t)e->m * 4, nullptr);
+    pool_free(e->row_order, (size_t)e->m * 4, nullptr);
+    for (void* p : {(void*)e->taps, (void*)e->spmv_split, (void*)e->rbm_hdr, (void*)e->rbm_w, (void*)e->rbm_ncols, e->stage_dev,
+                    e->conv_scratch, e->fm_scratch})
+        if (p) cudaFree(p);
     if (e->tma_failed_host) cudaFreeHost(e->tma_failed_host);
     if (e->tma_failed_dev) cudaFree(e->tma_failed_dev);
     for (cudaStream_t st : e->pipe_streams) if (st) cudaStreamDestroy(st);

@@ -146,8 +146,25 @@ int encode_device(const float* dW, uint32_t m, uint32_t n, cudaStream_t s, spx_e
 int decode_device(const spx_ell* e, float* dW, cudaStream_t s);
 int csr_to_ell_device(spx_ell* e, const uint64_t* d_rowptr, const uint32_t* d_col, const float* d_val,
                       cudaStream_t s);
-int alloc_ell(uint32_t m, uint32_t n, uint32_t r, spx_ell** out, cudaStream_t s);
+// zero_fill: whether the slabs and counts are cleared on s (a caller that writes every slot passes false).
+int alloc_ell(uint32_t m, uint32_t n, uint32_t r, spx_ell** out, cudaStream_t s, bool zero_fill = true);
 int check_current_device(const spx_ell* e, const char* what);
 // Builds e->row_order from host row counts (counting sort by length) and uploads it.
 int set_row_order(spx_ell* e, const uint32_t* host_nnz);
+// The sort behind it: fills order[m], and the handle's long_rows / min_nnz; e->row_order is allocated.
+int sort_rows(spx_ell* e, const uint32_t* host_nnz, uint32_t* order, cudaStream_t s);
+
+// Device memory from the library's pool of the given device, stream-ordered (mem.cu).
+int pool_alloc(void** p, size_t bytes, int device, cudaStream_t s);
+void pool_free(void* p, size_t bytes, cudaStream_t s);      // bytes as allocated; p may be null
+void pool_trim(int device);                     // waits for the device, then gives all free memory back
+// A non-blocking stream per device for small transfers beside the caller's stream, created once (mem.cu).
+int side_stream(int device, cudaStream_t* out);
+// Pinned host memory from a bounded free list (mem.cu).
+struct PinnedBlock {
+    void* host = nullptr;
+    size_t bytes = 0;
+};
+int pinned_acquire(size_t bytes, PinnedBlock* out);
+void pinned_release(const PinnedBlock& b);
 }  // namespace spx

@@ -1,0 +1,140 @@
+// mem.cu -- device and pinned-host memory that outlives a single call.
+//
+// Device: the arrays of an ELLPACK handle come from one CUDA memory pool per device.  cudaMalloc and
+// cudaFree cost 50 us to several milliseconds each here (page mapping, and an implicit wait for the
+// whole device in every free); a program that re-encodes a weight each step paid that a dozen times
+// per handle (encode + decode + destroy of an 8192 x 8192 matrix: 2.4 ms, of which the kernels were
+// 0.2 ms).  The pool keeps at most kPoolKeep bytes of freed memory per device, gives everything above
+// that back at the next synchronisation, and all of it when an allocation of this library fails.
+// The driver's pool is safe to use from several threads and streams.
+//
+// Pinned host: staging blocks for transfers, kept on a free list of at most kPinnedKeep bytes.
+#include "common.cuh"
+
+#include <cstdlib>
+#include <mutex>
+#include <vector>
+
+namespace spx {
+
+namespace {
+
+constexpr uint64_t kPoolKeep = 1ull << 30;          // of about 180 GB
+// A block that would take a large part of that is mapped and unmapped directly: the pool would not
+// keep it, and growing it by such a block took twice as long as cudaMalloc (slabs of 2 x 0.9 GB).
+constexpr size_t kPoolBlock = kPoolKeep / 4;
+constexpr size_t kPinnedKeep = 64u << 20;
+constexpr int kMaxDevices = 64;
+
+std::mutex g_pool_mu;
+cudaMemPool_t g_pools[kMaxDevices] = {};
+
+int device_pool(int device, cudaMemPool_t* out)
+{
+    if (device < 0 || device >= kMaxDevices) return fail(SPX_ERR_LIMIT, "device ordinal %d not supported", device);
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    if (!g_pools[device]) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaMemPool_t p = nullptr;
+        SPX_CUDA(cudaMemPoolCreate(&p, &props));
+        uint64_t keep = kPoolKeep;
+        SPX_CUDA(cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep));
+        g_pools[device] = p;
+    }
+    *out = g_pools[device];
+    return SPX_OK;
+}
+
+std::mutex g_pinned_mu;
+std::vector<PinnedBlock> g_pinned;                  // free blocks
+size_t g_pinned_bytes = 0;
+
+}  // namespace
+
+int pool_alloc(void** p, size_t bytes, int device, cudaStream_t s)
+{
+    *p = nullptr;
+    if (bytes == 0) return SPX_OK;
+    cudaMemPool_t pool = nullptr;
+    if (int rc = device_pool(device, &pool)) return rc;
+    auto get = [&] { return bytes > kPoolBlock ? cudaMalloc(p, bytes) : cudaMallocFromPoolAsync(p, bytes, pool, s); };
+    cudaError_t err = get();
+    if (err == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        pool_trim(device);
+        err = get();
+    }
+    if (err != cudaSuccess) {
+        (void)cudaGetLastError();
+        *p = nullptr;
+        return fail(err == cudaErrorMemoryAllocation ? SPX_ERR_OOM : SPX_ERR_CUDA, "device allocation of %zu bytes failed: %s",
+                    bytes, cudaGetErrorString(err));
+    }
+    return SPX_OK;
+}
+
+void pool_free(void* p, size_t bytes, cudaStream_t s)
+{
+    if (p) (void)(bytes > kPoolBlock ? cudaFree(p) : cudaFreeAsync(p, s));
+}
+
+void pool_trim(int device)
+{
+    if (device < 0 || device >= kMaxDevices) return;
+    (void)cudaDeviceSynchronize();
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    if (g_pools[device]) (void)cudaMemPoolTrimTo(g_pools[device], 0);
+}
+
+int side_stream(int device, cudaStream_t* out)
+{
+    static cudaStream_t streams[kMaxDevices] = {};
+    if (device < 0 || device >= kMaxDevices) return fail(SPX_ERR_LIMIT, "device ordinal %d not supported", device);
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    if (!streams[device]) SPX_CUDA(cudaStreamCreateWithFlags(&streams[device], cudaStreamNonBlocking));
+    *out = streams[device];
+    return SPX_OK;
+}
+
+int pinned_acquire(size_t bytes, PinnedBlock* out)
+{
+    *out = PinnedBlock{};
+    const size_t want = round_up<size_t>(bytes ? bytes : 1, 64 * 1024);
+    {
+        std::lock_guard<std::mutex> lk(g_pinned_mu);
+        size_t best = SIZE_MAX;
+        for (size_t i = 0; i < g_pinned.size(); ++i)        // smallest that fits and is not four times too large
+            if (g_pinned[i].bytes >= want && g_pinned[i].bytes / 4 <= want && (best == SIZE_MAX || g_pinned[i].bytes < g_pinned[best].bytes))
+                best = i;
+        if (best != SIZE_MAX) {
+            *out = g_pinned[best];
+            g_pinned_bytes -= out->bytes;
+            g_pinned[best] = g_pinned.back();
+            g_pinned.pop_back();
+            return SPX_OK;
+        }
+    }
+    // portable: usable from every device's context; mapped: kernels may store small results into it
+    SPX_CUDA(cudaHostAlloc(&out->host, want, cudaHostAllocPortable | cudaHostAllocMapped));
+    out->bytes = want;
+    return SPX_OK;
+}
+
+void pinned_release(const PinnedBlock& b)
+{
+    if (!b.host) return;
+    {
+        std::lock_guard<std::mutex> lk(g_pinned_mu);
+        if (g_pinned_bytes + b.bytes <= kPinnedKeep) {
+            g_pinned.push_back(b);
+            g_pinned_bytes += b.bytes;
+            return;
+        }
+    }
+    (void)cudaFreeHost(b.host);
+}
+
+}  // namespace spx

@@ -350,6 +350,30 @@ def test_csr_and_device_encoder(lib, orc, cuda):
     assert_bit_equal(out.cpu().numpy(), orc.decode(E), "device decode")
 
 
+@pytest.mark.parametrize("m,n,offset", [(1, 1, 0), (1, 5000, 0), (3, 2049, 1), (5, 1023, 3), (700, 1025, 2), (64, 4096, 0),
+                                        (2500, 130, 0), (10001, 33, 1)])
+def test_device_codec_edges(lib, orc, cuda, m, n, offset):
+    """Row lengths that are no multiple of a 16-byte vector, rows split into segments, a matrix that
+    starts `offset` elements after an aligned address: the encoding and its decoding are the same bytes."""
+    rng = np.random.default_rng([m, n, offset])
+    W = sparse(rng, m, n, 0.2)
+    W[m // 2, :] = 0
+    W[0, n - 1] = np.float32(np.nan) if n > 1 else 1.0
+    flat = torch.full((offset + m * n,), 7.0, device=cuda, dtype=torch.float32)
+    flat[offset:] = dev(W, cuda).reshape(-1)
+    h = lib.ell_encode_device(flat.data_ptr() + 4 * offset, m, n)
+    E = orc.encode(W)
+    Wd, idx, nnz = h.download()
+    assert h.r == E.r and np.array_equal(nnz, E.nnz) and np.array_equal(idx, E.idx)
+    assert_bit_equal(Wd, E.Wd, "Wd")
+    out = torch.full((offset + m * n + 4,), 7.0, device=cuda, dtype=torch.float32)
+    lib.spx_ell_decode_device(h.h, out.data_ptr() + 4 * offset, 0)
+    torch.cuda.synchronize()
+    got = out.cpu().numpy()
+    assert_bit_equal(got[offset:offset + m * n].reshape(m, n), orc.decode(E), "decode")
+    assert (got[:offset] == 7.0).all() and (got[offset + m * n:] == 7.0).all()
+
+
 def test_device_encoder_on_a_non_blocking_stream(lib, orc, cuda):
     """spx_ell_encode_device on a stream made by spx_stream_create (non-blocking: not ordered behind
     the default stream): the zero fill of the slabs must be ordered before the pack on that same
