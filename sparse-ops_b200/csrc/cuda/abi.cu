@@ -78,7 +78,7 @@ int alloc_ell(uint32_t m, uint32_t n, uint32_t r, spx_ell** out, cudaStream_t s,
     return SPX_OK;
 }
 
-int sort_rows(spx_ell* e, const uint32_t* host_nnz, uint32_t* order, cudaStream_t s)
+int sort_rows(spx_ell* e, const uint32_t* host_nnz, uint2* order, cudaStream_t s)
 {
     // counting sort by row length, longest first; stable, so ties keep ascending row id
     std::vector<uint32_t> start((size_t)e->r + 2, 0);
@@ -90,17 +90,17 @@ int sort_rows(spx_ell* e, const uint32_t* host_nnz, uint32_t* order, cudaStream_
         e->min_nnz = std::min(e->min_nnz, host_nnz[i]);
     }
     for (size_t k = 1; k < start.size(); ++k) start[k] += start[k - 1];
-    for (uint32_t i = 0; i < e->m; ++i) order[start[e->r - host_nnz[i]]++] = i;
-    if (!e->row_order) return pool_alloc(reinterpret_cast<void**>(&e->row_order), (size_t)e->m * sizeof(uint32_t), e->device, s);
+    for (uint32_t i = 0; i < e->m; ++i) order[start[e->r - host_nnz[i]]++] = make_uint2(i, host_nnz[i]);
+    if (!e->rows) return pool_alloc(reinterpret_cast<void**>(&e->rows), (size_t)e->m * sizeof(uint2), e->device, s);
     return SPX_OK;
 }
 
 int set_row_order(spx_ell* e, const uint32_t* host_nnz)
 {
     if (e->m == 0) return SPX_OK;
-    std::vector<uint32_t> order(e->m);
+    std::vector<uint2> order(e->m);
     if (int rc = sort_rows(e, host_nnz, order.data(), nullptr)) return rc;
-    SPX_CUDA(cudaMemcpy(e->row_order, order.data(), (size_t)e->m * sizeof(uint32_t), cudaMemcpyHostToDevice));
+    SPX_CUDA(cudaMemcpy(e->rows, order.data(), (size_t)e->m * sizeof(uint2), cudaMemcpyHostToDevice));
     return SPX_OK;
 }
 
@@ -414,7 +414,7 @@ int spx_ell_destroy(spx_ell* e)
     pool_free(e->Wd, (size_t)e->m * e->pitch * 4, nullptr);
     pool_free(e->idx, (size_t)e->m * e->pitch * 4, nullptr);
     pool_free(e->nnz, (size_t)e->m * 4, nullptr);
-    pool_free(e->row_order, (size_t)e->m * 4, nullptr);
+    pool_free(e->rows, (size_t)e->m * 8, nullptr);
     for (void* p : {(void*)e->taps, (void*)e->spmv_split, (void*)e->rbm_hdr, (void*)e->rbm_w, (void*)e->rbm_ncols, e->stage_dev,
                     e->conv_scratch, e->fm_scratch})
         if (p) cudaFree(p);

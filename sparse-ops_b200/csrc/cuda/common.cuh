@@ -23,11 +23,12 @@ struct spx_ell {
     float* Wd = nullptr;         // m * pitch floats
     uint32_t* idx = nullptr;     // m * pitch column ids
     uint32_t* nnz = nullptr;     // m counts
-    // Row schedule: row ids sorted by descending nnz (ties by ascending id).  Kernels that give a
-    // warp one row take rows in this order, so the warps of a CTA get rows of equal length
-    // (no warp idles behind a long row) and the longest rows start first.
-    uint32_t* row_order = nullptr;   // m row ids
-    uint32_t long_rows = 0;          // rows with at least 512 stored entries (a prefix of row_order)
+    // Row schedule: (row id, nnz) sorted by descending nnz (ties by ascending id).  Kernels that give
+    // a warp one row take rows in this order, so the warps of a CTA get rows of equal length
+    // (no warp idles behind a long row) and the longest rows start first.  The length sits beside the
+    // id so that a warp needs one load, not two dependent ones, before it can ask for its slab.
+    uint2* rows = nullptr;           // m entries
+    uint32_t long_rows = 0;          // rows with at least 512 stored entries (a prefix of rows)
     // Lazily built, cached conv tap table: idx decoded to packed (cin, kh, kw) for one
     // kernel shape (conv.cu); keyed by (kH, kW).
     uint32_t* taps = nullptr;
@@ -101,6 +102,30 @@ __device__ __forceinline__ float apply_act(float v, int act) {
     }
 }
 
+// Programmatic dependent launch: a kernel launched with launch_pdl() may start while its predecessor
+// in the stream is still draining.  Before pdl_wait() it may only touch what no kernel of the stream
+// writes -- the arrays of a finished handle; after it everything the predecessors wrote is visible.
+// pdl_launch() lets the successor in as soon as every CTA of this grid has reached it.  Every thread
+// calls pdl_wait() before it leaves.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... KArgs, class... Args>
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args)
+{
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 // (a0, a1) += w * (x0, x1) with ONE instruction: sm_100a's packed fma.rn.f32x2.  Each half is an
 // IEEE fused multiply-add rounded to nearest -- exactly fmaf -- so chains stay bit-identical while
 // the FMA instruction count halves.  The 64-bit pairs are formed inside the block, which leaves
@@ -149,10 +174,10 @@ int csr_to_ell_device(spx_ell* e, const uint64_t* d_rowptr, const uint32_t* d_co
 // zero_fill: whether the slabs and counts are cleared on s (a caller that writes every slot passes false).
 int alloc_ell(uint32_t m, uint32_t n, uint32_t r, spx_ell** out, cudaStream_t s, bool zero_fill = true);
 int check_current_device(const spx_ell* e, const char* what);
-// Builds e->row_order from host row counts (counting sort by length) and uploads it.
+// Builds e->rows from host row counts (counting sort by length) and uploads it.
 int set_row_order(spx_ell* e, const uint32_t* host_nnz);
-// The sort behind it: fills order[m], and the handle's long_rows / min_nnz; e->row_order is allocated.
-int sort_rows(spx_ell* e, const uint32_t* host_nnz, uint32_t* order, cudaStream_t s);
+// The sort behind it: fills order[m], and the handle's long_rows / min_nnz; e->rows is allocated.
+int sort_rows(spx_ell* e, const uint32_t* host_nnz, uint2* order, cudaStream_t s);
 
 // Device memory from the library's pool of the given device, stream-ordered (mem.cu).
 int pool_alloc(void** p, size_t bytes, int device, cudaStream_t s);

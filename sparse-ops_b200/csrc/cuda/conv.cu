@@ -13,9 +13,7 @@
 // reference for stride 1 (the reference mis-indexes stride_w > 1, :305-306 and :438-439; this
 // kernel implements the mathematically correct stride).
 #include "common.cuh"
-
-#include <cuda.h>            // CUtensorMap and its enums only; the encoder is looked up at run time
-#include <cudaTypedefs.h>
+#include "tma.cuh"
 
 #include <algorithm>
 #include <climits>
@@ -25,6 +23,11 @@
 #include <cstring>
 
 namespace {
+
+using spx::mbar_init;
+using spx::mbar_expect_tx;
+using spx::mbar_wait;
+using spx::tma_load_4d;
 
 // Per-nonzero tap table: idx k decoded once per kernel shape to cin<<16 | kh<<8 | kw.
 __global__ void build_taps_kernel(const uint32_t* __restrict__ idx, const uint32_t* __restrict__ nnz,
@@ -206,41 +209,6 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-
-// ---- bulk tensor copies (TMA) for the staged input patch -----------------------------------------
-// One thread asks the copy unit for the whole [channels][rows][columns][batch] box of a chunk; the
-// unit writes it into shared memory (zeros where the box leaves the image) and signals an mbarrier
-// with the byte count.  No multicast, the tensor map covers this GPU's own input tensor only.
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(bar)), "r"(count) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void tma_load_4d(void* smem, const CUtensorMap* map, int c0, int c1, int c2, int c3, uint64_t* bar) {
-    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
-                 ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3),
-                   "r"((uint32_t)__cvta_generic_to_shared(bar)) : "memory");
-}
-// Waits for the phase with the given parity; gives up one second (of the GPU's wall clock) after
-// its 256th unsuccessful poll and returns false, so a copy that never completes cannot hang the GPU.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-    const uint32_t a = (uint32_t)__cvta_generic_to_shared(bar);
-    uint64_t t0 = 0;
-    for (uint32_t i = 1;; ++i) {
-        uint32_t done;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(done) : "r"(a), "r"(parity) : "memory");
-        if (done) return true;
-        if ((i & 255u) == 0) {
-            uint64_t now;
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-            if (t0 == 0) t0 = now;
-            else if (now - t0 > 1000000000ull) return false;
-        }
-    }
-}
 
 // Stages input channels [c0, c1) of a CTA's receptive field in shared memory as
 // [channel][row][column][BT batch entries]: one warp per (channel, row), 16-byte cp.async copies,
@@ -752,20 +720,7 @@ static int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s)
             return -1;
         }
         e->rbm_cap = cap;
-        // Two words for a kernel whose bounded wait for a bulk tensor copy runs out: one in device
-        // memory, which CTAs that start later read and leave on, and one in pinned host memory
-        // (only ever written by the kernel: a read of host memory costs an SM about a microsecond),
-        // which the next convolution call on the handle reports.
-        if (!e->tma_failed_host && cudaHostAlloc(reinterpret_cast<void**>(&e->tma_failed_host), sizeof(int), cudaHostAllocMapped) == cudaSuccess) {
-            *e->tma_failed_host = 0;
-            if (cudaHostGetDevicePointer(reinterpret_cast<void**>(&e->tma_failed_mapped), e->tma_failed_host, 0) != cudaSuccess ||
-                cudaMalloc(reinterpret_cast<void**>(&e->tma_failed_dev), sizeof(int)) != cudaSuccess ||
-                cudaMemset(e->tma_failed_dev, 0, sizeof(int)) != cudaSuccess) {
-                e->tma_failed_mapped = nullptr;
-                if (e->tma_failed_dev) cudaFree(e->tma_failed_dev);
-                e->tma_failed_dev = nullptr;
-            }
-        }
+        ensure_tma_words(e);
         (void)cudaGetLastError();
     }
     const size_t smem = (size_t)((e->n + 31) / 32) * 2 * sizeof(uint32_t);
@@ -775,22 +730,6 @@ static int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s)
     e->rbm_kH = kH;
     e->rbm_kW = kW;
     return SPX_OK;
-}
-
-// cuTensorMapEncodeTiled, looked up through the runtime (the library does not link libcuda).
-static PFN_cuTensorMapEncodeTiled tensor_map_encoder()
-{
-    static const PFN_cuTensorMapEncodeTiled fn = [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess) {
-            (void)cudaGetLastError();
-            p = nullptr;
-        }
-        return reinterpret_cast<PFN_cuTensorMapEncodeTiled>(p);
-    }();
-    return fn;
 }
 
 template <int QB, int G>
@@ -901,12 +840,7 @@ static int launch_conv_rbm_tile(spx_ell* e, const ConvParams& p, uint32_t BT, co
 {
     static const int enabled = [] { const char* v = getenv("SPX_CONV_RBM"); return v ? atoi(v) : 1; }();
     static const double share_env = [] { const char* v = getenv("SPX_CONV_RBM_MIN_SHARE"); return v ? atof(v) : -1.0; }();
-    if (e->tma_failed_host && *e->tma_failed_host) {
-        // reported once; the handle stages with per-thread copies from here on
-        *e->tma_failed_host = 0;
-        e->tma_off = true;
-        return fail(SPX_ERR_CUDA, "conv2d: a bulk tensor copy of an earlier call on this handle did not complete; its output is invalid");
-    }
+    if (int rc = check_tma_words(e, "conv2d")) return rc;     // the handle stages with per-thread copies from then on
     // fewer than 8 row blocks would leave most of the CTA's 16 warps without work
     if (!enabled || e->n > kRbmMaxK || e->m < 8 * kRbmRows - 3 || e->max_nnz == 0) return -1;
     (void)BT;

@@ -280,7 +280,7 @@ static int encode_rows(const float* dW, uint32_t m, uint32_t n, cudaStream_t s, 
                        uint32_t* d_counts, spx_ell** out)
 {
     const uint32_t mis = misalignment(dW);
-    uint32_t* h_counts = static_cast<uint32_t*>(stage.host);    // m * segs counts, then m row ids
+    uint32_t* h_counts = static_cast<uint32_t*>(stage.host);    // m * segs counts, then the schedule
     const size_t units = (size_t)m * sp.segs;
     count_kernel<<<sp.blocks, kWarps * 32, 0, s>>>(dW, mis, m, n, sp.segs, sp.seg, d_counts);
     SPX_LAUNCH_CHECK("count_kernel");
@@ -306,13 +306,13 @@ static int encode_rows(const float* dW, uint32_t m, uint32_t n, cudaStream_t s, 
         pack_kernel<<<sp.blocks, kWarps * 32, 0, s>>>(dW, mis, m, n, sp.segs, sp.seg, d_counts, e->pitch, e->Wd, e->idx, e->nnz);
         SPX_LAUNCH_CHECK("pack_kernel");
     }
-    uint32_t* h_order = h_counts + units;
+    uint2* h_order = reinterpret_cast<uint2*>(h_counts + round_up<size_t>(units, 2));
     if (int rc = sort_rows(e, h_counts, h_order, s)) return rc;
     // on a stream of its own, beside the packer (nothing on s uses that block: blocks return to the
     // pool only after the work on them has been waited for)
     cudaStream_t side = nullptr;
     if (int rc = side_stream(e->device, &side)) return rc;
-    SPX_CUDA(cudaMemcpyAsync(e->row_order, h_order, (size_t)m * sizeof(uint32_t), cudaMemcpyHostToDevice, side));
+    SPX_CUDA(cudaMemcpyAsync(e->rows, h_order, (size_t)m * sizeof(uint2), cudaMemcpyHostToDevice, side));
     SPX_CUDA(cudaStreamSynchronize(side));
     SPX_CUDA(cudaStreamSynchronize(s));         // the handle may be used on any stream from here on
     return SPX_OK;
@@ -331,7 +331,7 @@ int encode_device(const float* dW, uint32_t m, uint32_t n, cudaStream_t s, spx_e
     const Split sp = split_rows(m, n, sm_count(device));
     const size_t units = (size_t)m * sp.segs;
     PinnedBlock stage;
-    if (int rc = pinned_acquire((units + m) * sizeof(uint32_t), &stage)) return rc;
+    if (int rc = pinned_acquire((units + 1) * sizeof(uint32_t) + m * sizeof(uint2), &stage)) return rc;
     void* d_counts = nullptr;
     int rc = pool_alloc(&d_counts, units * sizeof(uint32_t), device, s);
     if (rc == SPX_OK) rc = encode_rows(dW, m, n, s, stage, sp, static_cast<uint32_t*>(d_counts), out);

@@ -10,6 +10,7 @@
 //
 // Pinned host: staging blocks for transfers, kept on a free list of at most kPinnedKeep bytes.
 #include "common.cuh"
+#include "tma.cuh"
 
 #include <cstdlib>
 #include <mutex>
@@ -135,6 +136,46 @@ void pinned_release(const PinnedBlock& b)
         }
     }
     (void)cudaFreeHost(b.host);
+}
+
+void ensure_tma_words(spx_ell* e)
+{
+    if (e->tma_failed_host || cudaHostAlloc(reinterpret_cast<void**>(&e->tma_failed_host), sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return;
+    }
+    *e->tma_failed_host = 0;
+    if (cudaHostGetDevicePointer(reinterpret_cast<void**>(&e->tma_failed_mapped), e->tma_failed_host, 0) != cudaSuccess ||
+        cudaMalloc(reinterpret_cast<void**>(&e->tma_failed_dev), sizeof(int)) != cudaSuccess ||
+        cudaMemset(e->tma_failed_dev, 0, sizeof(int)) != cudaSuccess) {
+        e->tma_failed_mapped = nullptr;
+        if (e->tma_failed_dev) cudaFree(e->tma_failed_dev);
+        e->tma_failed_dev = nullptr;
+        (void)cudaGetLastError();
+    }
+}
+
+int check_tma_words(spx_ell* e, const char* what)
+{
+    if (!e->tma_failed_host || !*e->tma_failed_host) return SPX_OK;
+    *e->tma_failed_host = 0;
+    e->tma_off = true;
+    return fail(SPX_ERR_CUDA, "%s: a bulk tensor copy of an earlier call on this handle did not complete; its output is invalid", what);
+}
+
+PFN_cuTensorMapEncodeTiled tensor_map_encoder()
+{
+    static const PFN_cuTensorMapEncodeTiled fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            (void)cudaGetLastError();
+            p = nullptr;
+        }
+        return reinterpret_cast<PFN_cuTensorMapEncodeTiled>(p);
+    }();
+    return fn;
 }
 
 }  // namespace spx

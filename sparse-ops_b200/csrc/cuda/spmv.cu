@@ -30,7 +30,7 @@ __device__ __forceinline__ float group_sum(float v) {
 template <int LPR, bool SMEM>
 __global__ void __launch_bounds__(1024)
 spmv_ell_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ idx,
-                const uint32_t* __restrict__ nnz, const uint32_t* __restrict__ row_order,
+                const uint32_t* __restrict__ nnz, const uint2* __restrict__ rows,
                 uint32_t m, uint32_t n, uint32_t pitch,
                 const float* __restrict__ x, const float* __restrict__ bias, float* __restrict__ y)
 {
@@ -57,8 +57,8 @@ spmv_ell_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ idx,
         // slots of the sorted row schedule are dealt round-robin: every group gets long and short rows
         const uint32_t slot = group + it * stride;
         const bool live = slot < m;
-        const uint32_t row = live ? __ldg(row_order + slot) : 0u;
-        const uint32_t nn = live ? __ldg(nnz + row) : 0u;
+        const uint2 ri = live ? __ldg(rows + slot) : make_uint2(0u, 0u);
+        const uint32_t row = ri.x, nn = ri.y;
         const float4* __restrict__ w4 = reinterpret_cast<const float4*>(Wd + (size_t)row * pitch);
         const uint4* __restrict__ k4 = reinterpret_cast<const uint4*>(idx + (size_t)row * pitch);
         float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
@@ -99,12 +99,12 @@ spmv_ell_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ idx,
 // round trips in a row.  So this kernel is software-pipelined: a group asks
 // for its first row's id and length and for that row's first slab vectors BEFORE x is staged (none
 // of them depends on x), and while a row is summed the next row's id, length and first vectors
-// are already in flight.  row_order may be null (rows of near-equal length): slot == row then, and
+// are already in flight.  rows may be null (rows of near-equal length): slot == row then, and
 // one dependent load goes away.
 template <int LPR>
 __global__ void __launch_bounds__(1024)
 spmv_ell_small_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ idx,
-                const uint32_t* __restrict__ nnz, const uint32_t* __restrict__ row_order,
+                const uint32_t* __restrict__ nnz, const uint2* __restrict__ rows,
                 uint32_t m, uint32_t n, uint32_t pitch,
                 const float* __restrict__ x, const float* __restrict__ bias, float* __restrict__ y)
 {
@@ -140,8 +140,10 @@ spmv_ell_small_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__
     // slots of the sorted row schedule are dealt round-robin: every group gets long and short rows
     uint32_t slot = group;
     bool live = slot < m;
-    uint32_t row = live ? (row_order ? __ldg(row_order + slot) : slot) : 0u;
-    uint32_t nn = live ? __ldg(nnz + row) : 0u;
+    // rows may be null: slot == row then
+    auto row_info = [&](uint32_t sl) { return rows ? __ldg(rows + sl) : make_uint2(sl, __ldg(nnz + sl)); };
+    uint2 ri = live ? row_info(slot) : make_uint2(0u, 0u);
+    uint32_t row = ri.x, nn = ri.y;
     load_chunk(row, nn, lane * 4);
 
     {
@@ -158,8 +160,8 @@ spmv_ell_small_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__
         // the next row's id and length travel while this row is summed
         const uint32_t slot_n = slot + stride;
         const bool live_n = (it + 1 < iters) && slot_n < m;
-        const uint32_t row_n = live_n ? (row_order ? __ldg(row_order + slot_n) : slot_n) : 0u;
-        const uint32_t nn_n = live_n ? __ldg(nnz + row_n) : 0u;
+        ri = live_n ? row_info(slot_n) : make_uint2(0u, 0u);
+        const uint32_t row_n = ri.x, nn_n = ri.y;
         const float b = (live && bias) ? __ldg(bias + row) : 0.0f;
 
         float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
@@ -211,7 +213,7 @@ spmv_splits_kernel(const uint32_t* __restrict__ idx, const uint32_t* __restrict_
 template <int LPR>
 __global__ void __launch_bounds__(1024)
 spmv_ell_windowed_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ idx,
-                         const uint32_t* __restrict__ nnz, const uint32_t* __restrict__ row_order,
+                         const uint32_t* __restrict__ nnz, const uint2* __restrict__ rows,
                          const uint32_t* __restrict__ split, uint32_t m, uint32_t n, uint32_t win, uint32_t pitch,
                          const float* __restrict__ x, const float* __restrict__ bias, float* __restrict__ y)
 {
@@ -238,11 +240,14 @@ spmv_ell_windowed_kernel(const float* __restrict__ Wd, const uint32_t* __restric
             b0 = p ? __ldg(split + (size_t)(p - 1) * m + r) : 0u;
             b1 = (p + 1 < phases) ? __ldg(split + (size_t)p * m + r) : __ldg(nnz + r);
         };
+        // ids only: carrying the lengths along costs the registers of a vector in flight (313 -> 332 us at
+        // 65536 x 65536, 95 % sparse)
+        auto id_of = [&](uint64_t slot) { return __ldg(&rows[slot].x); };
         // the next row's run and the id of the row after it are fetched while the current row streams
-        uint32_t row = group < m ? __ldg(row_order + group) : 0u;
+        uint32_t row = group < m ? id_of(group) : 0u;
         uint32_t j0_next = 0, j1_next = 0;
         if (group < m) run_of(row, j0_next, j1_next);
-        uint32_t row_next = (uint64_t)group + stride < m ? __ldg(row_order + group + stride) : 0u;
+        uint32_t row_next = (uint64_t)group + stride < m ? id_of((uint64_t)group + stride) : 0u;
         for (uint32_t it = 0; it < iters; ++it) {
             const uint32_t slot = group + it * stride;
             const bool live = slot < m;
@@ -252,7 +257,7 @@ spmv_ell_windowed_kernel(const float* __restrict__ Wd, const uint32_t* __restric
                 const uint64_t s1 = (uint64_t)slot + stride, s2 = s1 + stride;
                 j0_next = j1_next = 0;
                 if (s1 < m) run_of(row_after, j0_next, j1_next);
-                row_next = s2 < m ? __ldg(row_order + s2) : 0u;
+                row_next = s2 < m ? id_of(s2) : 0u;
             }
             const float4* __restrict__ w4 = reinterpret_cast<const float4*>(Wd + (size_t)row * pitch);
             const uint4* __restrict__ k4 = reinterpret_cast<const uint4*>(idx + (size_t)row * pitch);
@@ -329,7 +334,7 @@ int launch_one(const spx_ell* e, const float* x, const float* bias, float* y, cu
         cudaError_t err = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (err != cudaSuccess) return spx::fail(SPX_ERR_CUDA, "spmv: shared memory opt-in failed: %s", cudaGetErrorString(err));
     }
-    kfn<<<blocks, threads, smem, s>>>(e->Wd, e->idx, e->nnz, e->row_order, e->m, e->n, e->pitch, x, bias, y);
+    kfn<<<blocks, threads, smem, s>>>(e->Wd, e->idx, e->nnz, e->rows, e->m, e->n, e->pitch, x, bias, y);
     SPX_LAUNCH_CHECK("spmv_ell_kernel");
     return SPX_OK;
 }
@@ -352,7 +357,7 @@ int launch_small(const spx_ell* e, const float* x, const float* bias, float* y, 
     const size_t xbytes = (size_t)e->n * sizeof(float);
     const uint64_t groups_needed = e->m;
     // Rows of near-equal length need no schedule: slot == row saves one dependent load per row.
-    const uint32_t* order = (e->max_nnz - e->min_nnz) * 8u <= e->max_nnz ? nullptr : e->row_order;
+    const uint2* order = (e->max_nnz - e->min_nnz) * 8u <= e->max_nnz ? nullptr : e->rows;
     // Rows per group (iters) as if every SM held 4 CTAs of 512 threads; then the same number of CTAs
     // on every SM -- as few as carry the rows in that many iterations (x is staged once per CTA) --
     // each with equally many groups.  A grid that is not a multiple of the SM count leaves some SMs
@@ -404,7 +409,7 @@ int launch_lpr(const spx_ell* e, const float* x, const float* bias, float* y, cu
         auto kfn = spmv_ell_windowed_kernel<LPR>;
         cudaError_t err = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (err != cudaSuccess) return spx::fail(SPX_ERR_CUDA, "spmv: shared memory opt-in failed: %s", cudaGetErrorString(err));
-        kfn<<<blocks, 1024, smem, s>>>(e->Wd, e->idx, e->nnz, e->row_order, e->spmv_split, e->m, e->n, e->spmv_win,
+        kfn<<<blocks, 1024, smem, s>>>(e->Wd, e->idx, e->nnz, e->rows, e->spmv_split, e->m, e->n, e->spmv_win,
                                        e->pitch, x, bias, y);
         SPX_LAUNCH_CHECK("spmv_ell_windowed_kernel");
         return SPX_OK;

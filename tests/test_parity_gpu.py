@@ -260,6 +260,44 @@ def test_spmm_each_wide_kernel_forced(env):
     assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-2000:]
 
 
+SPMM_EDGE_CASES = [
+    # X staged whole, up to 8 columns: a row per CTA, several, rows shorter and longer than a batch, no entries
+    (1, 4096, 1, 0.1), (700, 4096, 1, 0.1), (300, 2000, 2, 0.3), (130, 1000, 3, 0.5), (260, 900, 7, 0.2), (9, 31, 8, 1.0),
+    (3000, 40, 4, 0.9), (40, 50, 3, 0.0),
+    # X staged whole, wider
+    (512, 512, 64, 0.2), (333, 300, 12, 0.3), (40, 100, 20, 1.0),
+    # gathered: single columns, pairs, quads; one panel and several; a last panel with few columns
+    (50, 40000, 1, 0.01), (90, 3000, 37, 0.2), (300, 900, 139, 0.1), (257, 1200, 258, 0.1), (65, 700, 1007, 0.05), (2, 5000, 132, 0.3),
+    # X staged block by block from the second call on: aligned, a last group of 1 row, C not a multiple of 4
+    (1312, 2080, 160, 0.27), (601, 1537, 100, 0.5), (1201, 1100, 77, 0.5),
+]
+
+
+@pytest.mark.parametrize("pad", [0, 3], ids=["dense", "padded"])
+@pytest.mark.parametrize("m,n,C,p", SPMM_EDGE_CASES)
+def test_spmm_edges_repeated_calls(lib, orc, cuda, m, n, C, p, pad):
+    """Edges of each SpMM kernel's range, three calls in a row on one handle (a later call may use another
+    form of the matrix), operands with contiguous rows and as an unaligned window of a wider buffer."""
+    rng = np.random.default_rng([m, n, C, pad])
+    W = sparse(rng, m, n, p)
+    W[m // 3, :] = 0
+    E = orc.encode(W)
+    h = gpu_ell(lib, E)
+    X = rng.uniform(-1, 1, (n, C)).astype(np.float32)
+    b = rng.standard_normal(m).astype(np.float32)
+    dX = torch.full((n, C + pad), float("nan"), device=cuda, dtype=torch.float32)
+    dX[:, pad // 2:pad // 2 + C] = dev(X, cuda)
+    dB = dev(b, cuda)
+    want = orc.spmm(E, X, b, act=1)
+    for call in range(3):
+        dY = torch.full((m, C + pad), 7.0, device=cuda, dtype=torch.float32)
+        h.spmm(dX.data_ptr() + 4 * (pad // 2), C, C + pad, dB.data_ptr(), sx.ACT_RELU, dY.data_ptr() + 4 * (pad // 2), C + pad)
+        torch.cuda.synchronize()
+        got = dY.cpu().numpy()
+        assert_bit_equal(np.ascontiguousarray(got[:, pad // 2:pad // 2 + C]), want, f"call {call}")
+        assert (got[:, :pad // 2] == 7.0).all() and (got[:, pad // 2 + C:] == 7.0).all()
+
+
 @pytest.mark.parametrize("act", [sx.ACT_SIGMOID, sx.ACT_TANH])
 def test_spmm_sigmoid_tanh_epilogue(lib, orc, cuda, act):
     rng = np.random.default_rng(act)
