@@ -131,7 +131,11 @@ int spx_ell_decode_device(const spx_ell* e, float* dW, void* stream);
 /* Y[i,c] = act(bias[i] + sum_j Wd[i,j] * X[idx[i,j], c]), j in storage order, one FMA each.
  * Replaces ellpack_matmul (include/ellpack_matmul.hpp:23-43) and
  * ellpack_matmul_fused<USE_MASK,FUSE_RELU> (src/ellpack_matmul.cpp:11-92).
- * X: n rows of ldx floats (C used), Y: m rows of ldy floats.  bias may be NULL (= 0). */
+ * X: n rows of ldx floats (C used), Y: m rows of ldy floats.  bias may be NULL (= 0).
+ * Where staging X block by block is the faster way (columns used several times by a CTA's rows), the
+ * second such call on a handle builds and keeps another form of the matrix (about the size of its
+ * entries; that call waits for the stream, other threads' calls on the handle wait for it) and later
+ * calls use it; a call inside a stream capture never builds it.  Results are the same either way. */
 int spx_spmm(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const float* bias,
              int act, float* Y, uint64_t ldy, void* stream);
 /* y[i] = bias[i] + sum_j Wd[i,j] * x[idx[i,j]].  Replaces ellpack_matvec

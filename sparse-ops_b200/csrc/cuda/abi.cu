@@ -56,6 +56,7 @@ int alloc_ell(uint32_t m, uint32_t n, uint32_t r, spx_ell** out, cudaStream_t s,
         }
     }
     e->m = m; e->n = n; e->r = r;
+    e->tiles = new_tiles();
     e->pitch = r ? round_up<uint32_t>(r, 32u) : 0u;
     const size_t slots = (size_t)m * e->pitch;
     int rc = SPX_OK;
@@ -71,6 +72,7 @@ int alloc_ell(uint32_t m, uint32_t n, uint32_t r, spx_ell** out, cudaStream_t s,
     if (rc == SPX_OK && m && zero_fill && err == cudaSuccess) err = cudaMemsetAsync(e->nnz, 0, (size_t)m * sizeof(uint32_t), s);
     if (rc != SPX_OK || err != cudaSuccess) {
         pool_free(e->Wd, slots * sizeof(float), s); pool_free(e->idx, slots * sizeof(uint32_t), s); pool_free(e->nnz, (size_t)m * sizeof(uint32_t), s);
+        free_tiles(e);
         delete e;
         return rc != SPX_OK ? rc : fail(SPX_ERR_CUDA, "ELLPACK zero fill (%zu slots) failed: %s", slots, cudaGetErrorString(err));
     }
@@ -411,6 +413,7 @@ int spx_ell_destroy(spx_ell* e)
     // Kernels that read the handle may still run, on any stream: one wait for the device, after which
     // its arrays go back to the pool without another one.
     (void)cudaDeviceSynchronize();
+    free_tiles(e);
     pool_free(e->Wd, (size_t)e->m * e->pitch * 4, nullptr);
     pool_free(e->idx, (size_t)e->m * e->pitch * 4, nullptr);
     pool_free(e->nnz, (size_t)e->m * 4, nullptr);

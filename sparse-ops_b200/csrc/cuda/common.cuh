@@ -52,6 +52,8 @@ struct spx_ell {
     int* tma_failed_mapped = nullptr;
     int* tma_failed_dev = nullptr;
     bool tma_off = false;
+    // Tiled form of the matrix for spmm_tile.cu, built on the second SpMM call that can use it.
+    void* tiles = nullptr;
     // SpMV with x larger than shared memory (spmv.cu): column window width and the per-row split
     // table, built on the first spx_spmv of such a handle.  spmv_win == UINT32_MAX: not applicable.
     uint32_t* spmv_split = nullptr;
@@ -162,6 +164,8 @@ int launch_spmm(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx, cons
                 int act, float* Y, uint64_t ldy, cudaStream_t s);
 int launch_spmm_bcast(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const float* bias, int act,
                       float* const* Ys, uint32_t npeers, uint64_t row0, uint64_t ldy, cudaStream_t s, bool mcast = false);
+void* new_tiles();
+void free_tiles(spx_ell* e);
 int launch_spmv(spx_ell* e, const float* x, const float* bias, float* y, cudaStream_t s);
 int launch_spmv_reforder(const spx_ell* e, const float* x, const float* bias, float* y, cudaStream_t s);
 int launch_conv2d(spx_ell* e, const spx_conv_geom* g, int layout, const float* in, uint32_t B,

@@ -9,6 +9,8 @@
 //
 // Kernels (launch_spmm_bcast chooses):
 //   spmm_chain, spmm_direct   X fits in shared memory: staged whole, chains fed from there
+//   spmm_tile_kernel          (spmm_tile.cu) columns are used often enough by the rows of a CTA to stage X
+//                             block by block
 //   spmm_rows                 everything else: rows of X gathered through L1 / L2
 //   spmm_gather_half          64 < C <= 128 and very many short rows
 //   spmm_gather_staged        a few long rows decide the duration (row shard of a skewed matrix)
@@ -1041,6 +1043,9 @@ static int launch_rows(const spx_ell* e, RowsArgs a, cudaStream_t s)
     return fail(SPX_ERR_LIMIT, "spmm: no kernel");
 }
 
+int launch_spmm_tile(spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const float* bias, int act, const PeerOut& out,
+                     uint64_t ldy, bool vec_x, bool vec_out, cudaStream_t s);
+
 int launch_spmm(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const float* bias,
                 int act, float* Y, uint64_t ldy, cudaStream_t s)
 {
@@ -1076,6 +1081,11 @@ int launch_spmm_bcast(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx
     if (staged && (C <= 4 || (C <= 8 && x_bytes <= 32 * 1024))) return launch_chain(e, a, s);
     if (staged && vec_ok && C <= 64 && e->m <= (uint64_t)sm_count(e->device) * (kChainConsumers / (C / 4)))
         return launch_direct(e, a, true, s);
+    {
+        const bool vec_x = C % 4 == 0 && ldx % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+        const int rc = launch_spmm_tile(const_cast<spx_ell*>(e), X, C, ldx, bias, act, out, ldy, vec_x, C % 4 == 0 && ldy % 4 == 0 && aligned, s);
+        if (rc != -1) return rc;
+    }
     if (ldx >= (1ull << 30)) {
         const uint64_t blocks = ((uint64_t)e->m * C + 255) / 256;
         if (blocks > 0x7fffffffull) return fail(SPX_ERR_LIMIT, "spmm: grid too large");

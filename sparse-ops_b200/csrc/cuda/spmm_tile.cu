@@ -1,0 +1,529 @@
+// spmm_tile.cu -- SpMM with the dense operand staged in shared memory block by block, for matrices whose
+// columns are used several times by the rows of one CTA (iid-sparse weights of a few thousand columns).
+//
+// The gather kernels of spmm.cu fetch 4*C bytes of X per stored entry through L1 / L2, and L2 -> SM
+// bandwidth (64 B/clk/SM) and L1 wavefronts bound them.  Here a CTA owns a slice of 32 * NV columns of X
+// and up to 28 groups of 4 rows, walks the columns of E in chunks of 384, and brings a chunk's
+// 384 x (32 * NV) block of X into shared memory with bulk tensor copies, 4 / NV blocks deep: X crosses
+// L2 -> SM once per CTA instead of once per entry, and every gather is a conflict-free 16-byte
+// shared-memory read (8 lanes cover 128 contiguous bytes).  A warp owns one group: 8 lanes per row, NV
+// float4 accumulators per lane for the whole kernel.  Per output element the entries still come in
+// storage order, one FMA each: bit-identical to the other kernels.
+//
+// The entries come in a form of their own, built once per handle: per group and chunk a run of 128-byte
+// steps, each 4 entries of each of the 4 rows, which a warp streams through a private ring in shared
+// memory with cp.async.  So the hand-off of 16 entries costs 2 broadcast reads, and no search, no shuffle.
+//
+// Bound by shared-memory wavefronts (16 NV + 4 per step and warp) with many warps per SM, by the latency
+// of a warp's steps (82 ns each) with few.  Measured against gathering: 1312 x 2080, 27 %, C = 160
+// 27 us against 54; 2433 x 6496, 33 %, C = 320 257 against 541; 8192 x 8192, 10 %, C = 64 79 against 106;
+// 4096 x 4096, 10 %, C = 64 / 128 25 / 41 against 28.5 / 43 (ncu at C = 256: shared-memory pipe 81 %).
+#include "common.cuh"
+#include "tma.cuh"
+#include "peer_out.cuh"
+
+#include <algorithm>
+#include <atomic>
+#include <cmath>
+#include <cstdlib>
+#include <cstring>
+#include <mutex>
+#include <vector>
+
+namespace {
+
+using spx::PeerOut;
+using spx::store_out;
+
+constexpr uint32_t kChunk = 384;        // columns of E per chunk
+constexpr uint32_t kBoxRows = 192;      // rows of X per bulk copy (a box extent is at most 256)
+constexpr uint32_t kGroupRows = 4;
+constexpr uint32_t kStepWords = 32;     // 128 bytes: 16 weights, 16 local column ids ([row][4 entries] each)
+// A slot without an entry holds the weight -0.0f and the id of a row of zeros behind the chunk: -0 * 0
+// is -0, and adding -0 leaves every accumulator as it is, -0 and NaN included.
+constexpr uint32_t kNone = kChunk;
+constexpr uint32_t kNoWeight = 0x80000000u;
+constexpr uint32_t kMaxWarps = 28;      // per CTA: leaves 72 registers a thread
+
+// First entry of a row whose column is at least c.
+__device__ __forceinline__ uint32_t lower_bound(const uint32_t* __restrict__ k, uint32_t n, uint32_t c)
+{
+    uint32_t lo = 0, hi = n;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (__ldg(k + mid) < c) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+}
+
+// Warp per group.  cnt[group][chunk] = its steps; pos[group][chunk][row] = the row's first entry in the
+// chunk; total[group] = all its steps.
+__global__ void __launch_bounds__(256)
+tile_count_kernel(const uint32_t* __restrict__ idx, const uint2* __restrict__ rows, uint32_t m, uint32_t pitch, uint32_t groups,
+                  uint32_t chunks, uint32_t* __restrict__ cnt, uint4* __restrict__ pos, uint32_t* __restrict__ total)
+{
+    const uint32_t lane = threadIdx.x & 31, g = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (g >= groups) return;
+    uint2 ri[kGroupRows];
+#pragma unroll
+    for (uint32_t r = 0; r < kGroupRows; ++r) ri[r] = g * kGroupRows + r < m ? __ldg(rows + g * kGroupRows + r) : make_uint2(0u, 0u);
+    uint32_t sum = 0;
+    for (uint32_t c = lane; c < chunks; c += 32) {
+        uint32_t lo[kGroupRows], most = 0;
+#pragma unroll
+        for (uint32_t r = 0; r < kGroupRows; ++r) {
+            const uint32_t* __restrict__ k = idx + (size_t)ri[r].x * pitch;
+            lo[r] = lower_bound(k, ri[r].y, c * kChunk);
+            const uint32_t len = lower_bound(k, ri[r].y, (c + 1) * kChunk) - lo[r];
+            most = max(most, len);
+        }
+        cnt[(size_t)g * chunks + c] = (most + 3) / 4;
+        pos[(size_t)g * chunks + c] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        sum += (most + 3) / 4;
+    }
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0) total[g] = sum;
+}
+
+// Warp per group: its steps, chunk after chunk.
+__global__ void __launch_bounds__(256)
+tile_fill_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ idx, const uint2* __restrict__ rows, uint32_t m, uint32_t pitch,
+                 uint32_t groups, uint32_t chunks, const uint32_t* __restrict__ cnt, const uint4* __restrict__ pos,
+                 const uint32_t* __restrict__ off, uint32_t* __restrict__ steps)
+{
+    const uint32_t lane = threadIdx.x & 31, g = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (g >= groups) return;
+    const uint32_t r = (lane / 4) % kGroupRows, e = lane % 4;       // this lane's slot; lanes 16.. write the ids
+    const uint2 ri = g * kGroupRows + r < m ? __ldg(rows + g * kGroupRows + r) : make_uint2(0u, 0u);
+    const size_t base = (size_t)ri.x * pitch;
+    size_t at = (size_t)off[g] * kStepWords;
+    for (uint32_t c = 0; c < chunks; ++c) {
+        const uint4 p4 = pos[(size_t)g * chunks + c];
+        const uint32_t lo = r == 0 ? p4.x : r == 1 ? p4.y : r == 2 ? p4.z : p4.w;
+        const uint32_t n_steps = cnt[(size_t)g * chunks + c];
+        for (uint32_t s = 0; s < n_steps; ++s, at += kStepWords) {
+            const uint32_t j = lo + 4 * s + e;
+            const uint32_t k = j < ri.y ? __ldg(idx + base + j) : 0xffffffffu;
+            const bool have = k < (c + 1) * kChunk;                 // ids ascend: beyond the chunk is beyond the run
+            steps[at + lane] = lane < 16 ? (have ? __float_as_uint(__ldg(Wd + base + j)) : kNoWeight) : (have ? k - c * kChunk : kNone);
+        }
+    }
+}
+
+struct TileArgs {
+    const uint32_t* steps;
+    const uint32_t* off;
+    const uint32_t* cnt;
+    const uint2* rows;
+    uint32_t m, groups, chunks, row_blocks, C, ring_blocks;
+    int vec_out;                // 16-byte stores: C % 4 == 0 and aligned destinations
+    const float* bias;
+    int act;
+    uint64_t ldy;
+    int* failed;
+    int* failed_host;
+    PeerOut out;
+};
+
+__device__ __forceinline__ void cp_async16(uint32_t smem, const void* gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ float4 lds128(uint32_t at) {
+    float4 d;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(d.x), "=f"(d.y), "=f"(d.z), "=f"(d.w) : "r"(at) : "memory");
+    return d;
+}
+__device__ __forceinline__ void fma_vec(float4& a, float w, const float4& x) {
+    spx::fma_pair(a.x, a.y, w, x.x, x.y);
+    spx::fma_pair(a.z, a.w, w, x.z, x.w);
+}
+
+// N consecutive steps: entry u of a step of this lane's row is at `at` (weights) and `at` + 64 (ids).
+template <int NV, int N>
+__device__ __forceinline__ void tile_steps(float4 (&acc)[NV], uint32_t at, uint32_t xs)
+{
+    constexpr int kAhead = NV == 1 ? 2 : 1;     // steps of gathered operands held in registers
+    float4 w[N], k[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        w[i] = lds128(at + i * 128);
+        k[i] = lds128(at + i * 128 + 64);
+    }
+    float4 x[kAhead][4][NV];
+    auto gather = [&](int i) {
+        const uint32_t id[4] = {__float_as_uint(k[i].x), __float_as_uint(k[i].y), __float_as_uint(k[i].z), __float_as_uint(k[i].w)};
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int v = 0; v < NV; ++v) x[i % kAhead][u][v] = lds128(xs + id[u] * (NV * 128u) + v * 128u);
+    };
+    if (kAhead == 2) gather(0);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        if (kAhead == 1) gather(i);
+        else if (i + 1 < N) gather(i + 1);
+        const float wv[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int v = 0; v < NV; ++v) fma_vec(acc[v], wv[u], x[i % kAhead][u][v]);
+    }
+}
+
+// X with rows of C floats at any alignment into rows of Cp floats (a multiple of 4), zeros behind.
+__global__ void __launch_bounds__(256)
+align_rows_kernel(const float* __restrict__ X, uint64_t ldx, uint32_t n, uint32_t C, uint32_t Cp, float* __restrict__ dst)
+{
+    spx::pdl_launch();
+    spx::pdl_wait();
+    const uint32_t quads = Cp / 4;
+    const uint64_t total = (uint64_t)n * quads;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t k = (uint32_t)(i / quads), c = (uint32_t)(i - (uint64_t)k * quads) * 4;
+        const float* __restrict__ p = X + (size_t)k * ldx + c;
+        float4 v = make_float4(__ldg(p), 0.f, 0.f, 0.f);
+        if (c + 1 < C) v.y = __ldg(p + 1);
+        if (c + 2 < C) v.z = __ldg(p + 2);
+        if (c + 3 < C) v.w = __ldg(p + 3);
+        reinterpret_cast<float4*>(dst)[i] = v;
+    }
+}
+
+template <int NV>
+__global__ void __launch_bounds__(kMaxWarps * 32, 1)
+spmm_tile_kernel(const __grid_constant__ TileArgs a, const __grid_constant__ CUtensorMap tmap)
+{
+    constexpr uint32_t kPitch = NV * 128u;                  // bytes of a staged row of X
+    constexpr uint32_t kBox = kChunk * kPitch;              // bytes of a staged chunk
+    constexpr uint32_t kStage = kBox + kPitch;              // and a row of zeros
+    constexpr uint32_t kStages = 4 / NV;
+    extern __shared__ __align__(128) unsigned char s_mem[]; // [kStages] chunks of X, then a ring per warp
+    __shared__ __align__(8) uint64_t s_bar[kStages];
+    __shared__ __align__(8) uint64_t s_free[kStages];       // arrivals of the warps that are out of the chunk in stage s
+    __shared__ uint32_t s_asked;                            // copies asked for
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const uint32_t slice = blockIdx.x / a.row_blocks, rb = blockIdx.x % a.row_blocks;
+    const uint32_t group = rb * warps + warp;
+    const bool active = group < a.groups;
+    const uint32_t nactive = min(warps, a.groups - rb * warps);
+    spx::pdl_launch();
+
+    // the warp's steps and counts do not depend on the predecessor kernel
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(s_mem) + kStages * kStage + warp * (a.ring_blocks * 512u);
+    const uint32_t ring_mask = a.ring_blocks - 1;          // a power of two
+    const uint32_t first = active ? __ldg(a.off + group) : 0u, n_steps = active ? __ldg(a.off + group + 1) - first : 0u;
+    const unsigned char* src = reinterpret_cast<const unsigned char*>(a.steps) + (size_t)first * 128 + lane * 16;
+    auto fill = [&](uint32_t blk) {             // block blk of 4 steps; the array ends with room for a whole block
+        if (blk < (n_steps + 3) / 4) cp_async16(ring + (blk & ring_mask) * 512u + lane * 16, src + (size_t)blk * 512);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (uint32_t b = 0; b < 3; ++b) fill(b < ring_mask ? b : 0xffffffu);     // three groups, whatever the ring holds
+    const uint32_t slot = group * kGroupRows + lane / 8;
+    const uint2 ri = active && slot < a.m ? __ldg(a.rows + slot) : make_uint2(0u, 0u);
+    uint32_t my_cnt = active && lane < a.chunks ? __ldg(a.cnt + (size_t)group * a.chunks + lane) : 0u;
+
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (uint32_t s = 0; s < kStages; ++s) {
+            spx::mbar_init(&s_bar[s], 1);
+            spx::mbar_init(&s_free[s], nactive);
+        }
+        s_asked = min(kStages, a.chunks);
+    }
+    if (threadIdx.x < kStages * kPitch / 16)    // 32 threads: the rows of zeros
+        *reinterpret_cast<float4*>(s_mem + threadIdx.x / (kPitch / 16) * kStage + kBox + threadIdx.x % (kPitch / 16) * 16) = make_float4(0.f, 0.f, 0.f, 0.f);
+    // an earlier CTA's (or call's) wait ran out: leave at once
+    const bool bad = __syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile int*>(a.failed) != 0);
+    spx::pdl_wait();
+    if (bad) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        return;
+    }
+    auto ask = [&](uint32_t c) {                // by one thread: chunk c into stage c % kStages
+        const uint32_t st = c % kStages;
+        spx::mbar_expect_tx(&s_bar[st], kBox);
+        for (uint32_t h = 0; h < kChunk; h += kBoxRows)
+            spx::tma_load_2d(s_mem + st * kStage + h * kPitch, &tmap, (int)(slice * 32u * NV), (int)(c * kChunk + h), &s_bar[st]);
+    };
+    if (threadIdx.x == 0)
+        for (uint32_t c = 0; c < min(kStages, a.chunks); ++c) ask(c);
+    if (!active) return;
+
+    const uint32_t r = lane / 8, l = lane & 7;
+    const float b = (slot < a.m && a.bias) ? __ldg(a.bias + ri.x) : 0.0f;
+    float4 acc[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) acc[v] = make_float4(b, b, b, b);
+    const uint32_t xbase = (uint32_t)__cvta_generic_to_shared(s_mem) + l * 16;
+    uint32_t step = 0;                          // of the group's stream
+    bool landed = true;
+    for (uint32_t c = 0; c < a.chunks; ++c) {
+        if (c && (c & 31u) == 0) my_cnt = c + lane < a.chunks ? __ldg(a.cnt + (size_t)group * a.chunks + c + lane) : 0u;
+        const uint32_t all = __shfl_sync(0xffffffffu, my_cnt, c & 31u);
+        const uint32_t st = c % kStages;
+        if (landed) landed = spx::mbar_wait(&s_bar[st], (c / kStages) & 1u);
+        const uint32_t xs = xbase + st * kStage;
+        for (uint32_t s = 0; s < all;) {
+            const uint32_t in_block = step & 3u, n = min(4u - in_block, all - s);
+            if (in_block == 0) {                // entering a block of the ring: it has landed, and the one before is free
+                if (ring_mask == 1) asm volatile("cp.async.wait_group 0;" ::: "memory");
+                else asm volatile("cp.async.wait_group 2;" ::: "memory");
+                __syncwarp();
+                fill(step / 4 + ring_mask);
+            }
+            const uint32_t at = ring + ((step & (4 * ring_mask + 3)) * 128u) + r * 16;
+            switch (n) {                        // unrolled: the hand-off and the gathers of a step run ahead of its FMAs
+            case 1: tile_steps<NV, 1>(acc, at, xs); break;
+            case 2: tile_steps<NV, 2>(acc, at, xs); break;
+            case 3: tile_steps<NV, 3>(acc, at, xs); break;
+            default: tile_steps<NV, 4>(acc, at, xs);
+            }
+            s += n;
+            step += n;
+        }
+        __syncwarp();
+        // The last warp out of the chunk asks for the one that takes its place.  The arrival tells whether
+        // it is the last (one pending before it); a fence and an atomic instead would wait for the
+        // warp's cp.async in flight, 1500 cycles per chunk.
+        if (lane == 0 && spx::mbar_arrive_pending(&s_free[st]) == 1u && landed && c + kStages < a.chunks) {
+            ask(c + kStages);
+            atomicAdd(&s_asked, 1u);
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (!landed) {
+        *a.failed = 1;
+        *a.failed_host = 1;
+        // copies still in flight write this CTA's shared memory: one more bounded wait for each
+        if (lane == 0) {
+            const uint32_t asked = *reinterpret_cast<volatile uint32_t*>(&s_asked);
+            for (uint32_t j = asked > kStages ? asked - kStages : 0; j < asked; ++j) (void)spx::mbar_wait(&s_bar[j % kStages], (j / kStages) & 1u);
+        }
+    }
+    if (slot >= a.m) return;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        const uint32_t col = slice * 32u * NV + v * 32u + l * 4u;
+        if (col < a.C) {
+            float4 o = acc[v];
+            if (a.act != SPX_ACT_NONE) {
+                o.x = spx::apply_act(o.x, a.act); o.y = spx::apply_act(o.y, a.act);
+                o.z = spx::apply_act(o.z, a.act); o.w = spx::apply_act(o.w, a.act);
+            }
+            const size_t at = (size_t)(a.out.row0 + ri.x) * a.ldy + col;
+            if (a.vec_out) {
+                store_out(a.out, at, o);
+            } else {
+                store_out(a.out, at, o.x);
+                if (col + 1 < a.C) store_out(a.out, at + 1, o.y);
+                if (col + 2 < a.C) store_out(a.out, at + 2, o.z);
+                if (col + 3 < a.C) store_out(a.out, at + 3, o.w);
+            }
+        }
+    }
+}
+
+}  // namespace
+
+namespace spx {
+
+// The tiled form of a handle's matrix.  A group's steps are contiguous, chunk after chunk.
+struct spx_tiles_impl {
+    std::mutex mu;
+    int calls = 0;              // SpMM calls that could have used the form
+    std::atomic<int> state{0};  // 0: not built, 1: ready, 2: cannot be built
+    uint32_t groups = 0, chunks = 0;
+    uint64_t steps_bytes = 0;
+    uint32_t* steps = nullptr;
+    uint32_t* off = nullptr;
+    uint32_t* cnt = nullptr;
+};
+
+void free_tiles(spx_ell* e)
+{
+    spx_tiles_impl* t = static_cast<spx_tiles_impl*>(e->tiles);
+    if (!t) return;
+    pool_free(t->steps, t->steps_bytes, nullptr);
+    pool_free(t->off, (size_t)(t->groups + 1) * 4, nullptr);
+    pool_free(t->cnt, (size_t)t->groups * t->chunks * 4, nullptr);
+    delete t;
+    e->tiles = nullptr;
+}
+
+void* new_tiles() { return new (std::nothrow) spx_tiles_impl(); }
+
+static int build_tiles(spx_ell* e, spx_tiles_impl* t, cudaStream_t s)
+{
+    t->state = 2;
+    t->groups = (e->m + kGroupRows - 1) / kGroupRows;
+    t->chunks = (e->n + kChunk - 1) / kChunk;
+    const size_t cells = (size_t)t->groups * t->chunks;
+    ensure_tma_words(e);
+    if (!e->tma_failed_dev || !e->tma_failed_mapped) return SPX_OK;
+    void *pos = nullptr, *total = nullptr, *cnt = nullptr, *off = nullptr, *steps = nullptr;
+    PinnedBlock stage;
+    std::vector<uint32_t> host(t->groups + 1);
+    auto body = [&]() -> int {
+        if (int rc = pool_alloc(&pos, cells * sizeof(uint4), e->device, s)) return rc;
+        if (int rc = pool_alloc(&cnt, cells * 4, e->device, s)) return rc;
+        if (int rc = pool_alloc(&total, (size_t)t->groups * 4, e->device, s)) return rc;
+        if (int rc = pool_alloc(&off, (size_t)(t->groups + 1) * 4, e->device, s)) return rc;
+        if (int rc = pinned_acquire((size_t)(t->groups + 1) * 4, &stage)) return rc;
+        uint32_t* h = static_cast<uint32_t*>(stage.host);
+        tile_count_kernel<<<(t->groups + 7) / 8, 256, 0, s>>>(e->idx, e->rows, e->m, e->pitch, t->groups, t->chunks,
+                                                             static_cast<uint32_t*>(cnt), static_cast<uint4*>(pos), static_cast<uint32_t*>(total));
+        SPX_LAUNCH_CHECK("tile_count_kernel");
+        SPX_CUDA(cudaMemcpyAsync(h, total, (size_t)t->groups * 4, cudaMemcpyDeviceToHost, s));
+        SPX_CUDA(cudaStreamSynchronize(s));
+        uint64_t run = 0;
+        for (uint32_t g = 0; g < t->groups; ++g) {
+            const uint32_t n = h[g];
+            h[g] = (uint32_t)run;
+            run += n;
+        }
+        h[t->groups] = (uint32_t)run;
+        if (run >= (1ull << 31)) return SPX_OK;
+        t->steps_bytes = (run + 4) * kStepWords * 4;        // the ring copies whole blocks of 4 steps
+        if (int rc = pool_alloc(&steps, t->steps_bytes, e->device, s)) return rc;
+        SPX_CUDA(cudaMemcpyAsync(off, h, (size_t)(t->groups + 1) * 4, cudaMemcpyHostToDevice, s));
+        tile_fill_kernel<<<(t->groups + 7) / 8, 256, 0, s>>>(e->Wd, e->idx, e->rows, e->m, e->pitch, t->groups, t->chunks,
+                                                            static_cast<uint32_t*>(cnt), static_cast<uint4*>(pos), static_cast<uint32_t*>(off),
+                                                            static_cast<uint32_t*>(steps));
+        SPX_LAUNCH_CHECK("tile_fill_kernel");
+        return SPX_OK;
+    };
+    const int rc = body();
+    const cudaError_t err = cudaStreamSynchronize(s);       // complete for every stream, and for the blocks given back
+    pool_free(pos, cells * sizeof(uint4), s);
+    pool_free(total, (size_t)t->groups * 4, s);
+    pinned_release(stage);
+    if (rc != SPX_OK || err != cudaSuccess || !steps) {
+        pool_free(cnt, cells * 4, s);
+        pool_free(off, (size_t)(t->groups + 1) * 4, s);
+        pool_free(steps, t->steps_bytes, s);
+        if (err != cudaSuccess) return fail(SPX_ERR_CUDA, "spmm: building the tiled form failed: %s", cudaGetErrorString(err));
+        return rc == SPX_ERR_OOM ? SPX_OK : rc;             // no room: the gather kernels need none
+    }
+    t->steps = static_cast<uint32_t*>(steps);
+    t->off = static_cast<uint32_t*>(off);
+    t->cnt = static_cast<uint32_t*>(cnt);
+    t->state = 1;
+    return SPX_OK;
+}
+
+template <int NV>
+static int launch_tile_nv(const spx_ell* e, TileArgs a, const CUtensorMap& map, uint32_t warps, uint32_t slices, cudaStream_t s)
+{
+    a.row_blocks = (a.groups + warps - 1) / warps;
+    a.ring_blocks = warps > 14 ? 2 : 4;
+    const size_t smem = (4 / NV) * (size_t)(kChunk + 1) * NV * 128 + (size_t)warps * a.ring_blocks * 512;
+    auto kfn = spmm_tile_kernel<NV>;
+    SPX_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SPX_CUDA(launch_pdl(kfn, dim3(a.row_blocks * slices), dim3(warps * 32), smem, s, a, map));
+    count_launch();
+    return SPX_OK;
+}
+
+namespace {
+
+struct Plan {
+    uint32_t slices, warps;
+    uint64_t waves;
+    double us;
+};
+
+// Launch shape and expected time.  As few waves of CTAs as kMaxWarps warps each allow, and then equally
+// many warps in every CTA.  Time: about 1.4 / 1.7 ns per row of X to stage it (NV = 1 / 2), and per step
+// of a warp the larger of its latency (82 ns) and the shared-memory wavefronts of all the SM's warps
+// (16 NV gathers + 4 of hand-off, one per cycle); a group's steps in a chunk are those of its
+// longest row of four.  Fits 4096 x 4096, 10 %: C = 32 / 64 / 128 / 256 in 17.7 / 25 / 41 / 76 us.
+Plan plan_tiles(const spx_ell* e, uint32_t C, uint32_t NV, uint32_t sms)
+{
+    Plan p;
+    const uint32_t groups = (e->m + kGroupRows - 1) / kGroupRows, chunks = (e->n + kChunk - 1) / kChunk;
+    p.slices = (C + 32 * NV - 1) / (32 * NV);
+    const uint64_t units = (uint64_t)groups * p.slices;
+    p.waves = (units + (uint64_t)sms * kMaxWarps - 1) / ((uint64_t)sms * kMaxWarps);
+    p.warps = (uint32_t)std::min<uint64_t>(kMaxWarps, (units + sms * p.waves - 1) / (sms * p.waves));
+    while (p.warps < kMaxWarps && (uint64_t)((groups + p.warps - 1) / p.warps) * p.slices > p.waves * sms) ++p.warps;
+    const double per_chunk = (double)e->nnz_total / e->m / chunks;
+    const double steps = chunks * (per_chunk + std::sqrt(per_chunk) + 2.0) / 4.0;
+    p.us = 1.5 + p.waves * (e->n * (NV == 1 ? 1.4e-3 : 1.7e-3) + steps * std::max(0.082, p.warps * (16.0 * NV + 4.0) / 1900.0));
+    return p;
+}
+
+// Expected time of the gather kernel (spmm_rows): bytes of gathered operands over the rate it reaches, which
+// grows with the width and falls with idle lanes (C = 160: 20 of 32 lanes), or the rounds of its longest row.
+double gather_us(const spx_ell* e, uint32_t C, bool aligned)
+{
+    const double density = (double)e->nnz_total / ((double)e->m * e->n);
+    const uint32_t V = aligned ? 4 : 1, q = (C + V - 1) / V, nv_max = aligned ? 2 : 3;
+    const uint32_t NV = std::min(nv_max, (q + 31) / 32), panels = (q + 32 * NV - 1) / (32 * NV);
+    const uint32_t per = (q + panels - 1) / panels, G = (per + NV - 1) / NV, RW = std::min(32 / G, 16u);
+    const double lanes = (double)q * RW / (32.0 * NV * panels);
+    double rate = density < 0.04 ? 26e6 : C <= 64 ? 16e6 : C <= 128 ? 20e6 : 23e6;     // bytes per us, measured
+    if (!aligned) rate *= 0.6;
+    return 2.0 + std::max((double)e->nnz_total * C * 4.0 / (rate * lanes), e->max_nnz / (NV == 1 ? 32.0 : 16.0) * 0.85);
+}
+
+}  // namespace
+
+// Returns -1 when the shape or the handle is not for this kernel.
+int launch_spmm_tile(spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const float* bias, int act, const PeerOut& out,
+                     uint64_t ldy, bool vec_x, bool vec_out, cudaStream_t s)
+{
+    static const int env = [] { const char* v = getenv("SPX_SPMM_TILE"); return v ? atoi(v) : 1; }();
+    if (!env || !e->tiles || !e->cols_ascending || e->tma_off || e->max_nnz == 0) return -1;
+    const PFN_cuTensorMapEncodeTiled encode = tensor_map_encoder();
+    if (!encode || ldx > 0xffffffffull || e->n > 65536 || C > 65536) return -1;
+    const uint32_t NV = C <= 32 ? 1 : 2;
+    const Plan p = plan_tiles(e, C, NV, sm_count(e->device));
+    if ((uint64_t)p.slices * e->m > 0x7fffffffull) return -1;
+    if (env != 2 && (e->n < kChunk || p.us + (vec_x ? 0.0 : 4.0) > 0.95 * gather_us(e, C, vec_x))) return -1;
+    spx_tiles_impl* t = static_cast<spx_tiles_impl*>(e->tiles);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (t->state != 1 || !vec_x) {              // building and the scratch below allocate: not while a graph is captured
+        if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) { (void)cudaGetLastError(); return -1; }
+    }
+    if (t->state != 1) {
+        std::lock_guard<std::mutex> lk(t->mu);
+        if (t->state == 0) {
+            if (++t->calls < 2) return -1;      // a matrix that is multiplied once is not worth the second form
+            if (int rc = build_tiles(e, t, s)) return rc;
+        }
+        if (t->state != 1) return -1;
+    }
+    if (int rc = check_tma_words(e, "spmm")) return rc;
+    void* aligned = nullptr;
+    const uint32_t Cp = round_up(C, 4u);
+    const size_t aligned_bytes = (size_t)e->n * Cp * 4;
+    if (!vec_x) {                               // bulk copies need 16-byte rows: X moves into scratch that has them
+        if (int rc = pool_alloc(&aligned, aligned_bytes, e->device, s)) return rc == SPX_ERR_OOM ? -1 : rc;
+        const uint64_t quads = (uint64_t)e->n * (Cp / 4);
+        const unsigned blocks = (unsigned)std::min<uint64_t>((quads + 255) / 256, (uint64_t)sm_count(e->device) * 16);
+        const cudaError_t err = launch_pdl(align_rows_kernel, dim3(blocks), dim3(256), 0, s, X, ldx, e->n, C, Cp, static_cast<float*>(aligned));
+        if (err != cudaSuccess) { pool_free(aligned, aligned_bytes, s); return fail(SPX_ERR_CUDA, "launch of align_rows_kernel failed: %s", cudaGetErrorString(err)); }
+        count_launch();
+        X = static_cast<const float*>(aligned);
+        ldx = Cp;
+    }
+    CUtensorMap map;
+    const cuuint64_t gdim[2] = {vec_x ? C : Cp, e->n};
+    const cuuint64_t gstr[1] = {ldx * 4};
+    const cuuint32_t box[2] = {32 * NV, kBoxRows};
+    const cuuint32_t estr[2] = {1, 1};
+    int rc = -1;
+    if (encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(X), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS) {
+        TileArgs a{};
+        a.steps = t->steps; a.off = t->off; a.cnt = t->cnt; a.rows = e->rows;
+        a.m = e->m; a.groups = t->groups; a.chunks = t->chunks; a.C = C; a.vec_out = vec_out;
+        a.bias = bias; a.act = act; a.ldy = ldy; a.out = out;
+        a.failed = e->tma_failed_dev; a.failed_host = e->tma_failed_mapped;
+        rc = NV == 1 ? launch_tile_nv<1>(e, a, map, p.warps, p.slices, s) : launch_tile_nv<2>(e, a, map, p.warps, p.slices, s);
+    }
+    pool_free(aligned, aligned_bytes, s);
+    return rc;
+}
+
+}  // namespace spx

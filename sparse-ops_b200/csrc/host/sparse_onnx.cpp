@@ -473,12 +473,12 @@ void SparseOnnxModel::build_exec(uint32_t B) const
     }
     exec_ = std::move(ex);
 
-    // One eager pass (lets kernels make their lazy, per-handle allocations outside a capture),
-    // then capture the same launches as a graph for the host-buffer run().
+    // Two eager passes (let kernels make their lazy, per-handle allocations and second forms of the
+    // weights outside a capture; a matrix gets its second form when it is multiplied again), then capture the same launches as a graph for the host-buffer run().
     float* d_in = exec_->buf.at(input_name_);
     float* d_out = exec_->buf.at(output_name_);
     check(spx_memset(d_in, 0, size_t(in_features_) * B * sizeof(float), exec_->stream), "memset");
-    launch_layers(d_in, d_out, B, exec_->stream);
+    for (int pass = 0; pass < 2; ++pass) launch_layers(d_in, d_out, B, exec_->stream);
     check(spx_stream_sync(exec_->stream), "warm-up pass");
     const char* no_graph = std::getenv("SPX_NO_GRAPH");
     if (!(no_graph && no_graph[0] == '1')) {

@@ -298,6 +298,17 @@ def test_spmm_edges_repeated_calls(lib, orc, cuda, m, n, C, p, pad):
         assert (got[:, :pad // 2] == 7.0).all() and (got[:, pad // 2 + C:] == 7.0).all()
 
 
+def test_spmm_edges_with_the_block_kernel_forced():
+    import os
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    cmd = [sys.executable, "-m", "pytest", "-q", "-x", "-m", "gpu", "-p", "no:cacheprovider",
+           os.path.join(here, "test_parity_gpu.py"), "-k", "edges_repeated"]
+    r = subprocess.run(cmd, env={**os.environ, "SPX_SPMM_TILE": "2"}, capture_output=True, text=True, timeout=900)
+    assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-2000:]
+
+
 @pytest.mark.parametrize("act", [sx.ACT_SIGMOID, sx.ACT_TANH])
 def test_spmm_sigmoid_tanh_epilogue(lib, orc, cuda, act):
     rng = np.random.default_rng(act)
