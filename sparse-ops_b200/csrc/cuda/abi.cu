@@ -109,13 +109,7 @@ int set_row_order(spx_ell* e, const uint32_t* host_nnz)
 // Device scratch owned by a handle for the host-buffer entry points.
 static int ensure_stage(spx_ell* e, size_t bytes)
 {
-    if (e->stage_dev_bytes >= bytes) return SPX_OK;
-    if (e->stage_dev) cudaFree(e->stage_dev);
-    e->stage_dev = nullptr;
-    e->stage_dev_bytes = 0;
-    SPX_CUDA(cudaMalloc(&e->stage_dev, bytes));
-    e->stage_dev_bytes = bytes;
-    return SPX_OK;
+    return e->stage_dev_bytes >= bytes ? SPX_OK : grow_scratch(e, &e->stage_dev, &e->stage_dev_bytes, bytes);
 }
 
 // Kernel entry points launch on the current device: a handle made on another GPU would hand the
@@ -184,8 +178,7 @@ int spx_host_alloc(void** hptr, size_t bytes)
 int spx_host_free(void* hptr) { if (hptr) SPX_CUDA(cudaFreeHost(hptr)); return SPX_OK; }
 int spx_memcpy_h2d(void* dst, const void* src, size_t bytes, void* stream)
 {
-    if (bytes) SPX_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, (cudaStream_t)stream));
-    return SPX_OK;
+    return copy_h2d(dst, src, bytes, (cudaStream_t)stream);
 }
 int spx_memcpy_d2h(void* dst, const void* src, size_t bytes, void* stream)
 {
@@ -418,11 +411,17 @@ int spx_ell_destroy(spx_ell* e)
     pool_free(e->idx, (size_t)e->m * e->pitch * 4, nullptr);
     pool_free(e->nnz, (size_t)e->m * 4, nullptr);
     pool_free(e->rows, (size_t)e->m * 8, nullptr);
-    for (void* p : {(void*)e->taps, (void*)e->spmv_split, (void*)e->rbm_hdr, (void*)e->rbm_w, (void*)e->rbm_ncols, e->stage_dev,
-                    e->conv_scratch, e->fm_scratch})
-        if (p) cudaFree(p);
-    if (e->tma_failed_host) cudaFreeHost(e->tma_failed_host);
-    if (e->tma_failed_dev) cudaFree(e->tma_failed_dev);
+    pool_free(e->taps, (size_t)e->m * e->pitch * 4, nullptr);
+    pool_free(e->spmv_split, e->spmv_split_bytes, nullptr);
+    const size_t blocks4 = (e->m + 3) / 4, slots4 = blocks4 * e->rbm_cap;       // rbm_cap means nothing without the arrays
+    pool_free(e->rbm_ncols, blocks4 * 4, nullptr);
+    pool_free(e->rbm_w, slots4 * 16, nullptr);
+    pool_free(e->rbm_hdr, slots4 * sizeof(uint2), nullptr);
+    pool_free(e->stage_dev, e->stage_dev_bytes, nullptr);
+    pool_free(e->conv_scratch, e->conv_scratch_bytes, nullptr);
+    pool_free(e->fm_scratch, e->fm_scratch_bytes, nullptr);
+    pool_free(e->tma_failed_dev, sizeof(int), nullptr);
+    pinned_release(e->tma_failed_block);
     for (cudaStream_t st : e->pipe_streams) if (st) cudaStreamDestroy(st);
     for (cudaEvent_t ev : e->pipe_events) if (ev) cudaEventDestroy(ev);
     delete e;
@@ -684,6 +683,81 @@ static inline uint32_t host_panel_width(uint32_t c0, uint32_t C)
     return std::min<uint32_t>(256, C - c0);
 }
 
+// One host-buffer call: a stream, and where the operands are small a pinned block through which they travel.
+// Small means that latency is all there is to it: inputs are packed and sent as one copy, and the kernel
+// stores its result straight into the pinned block, so the call is one copy, one kernel and one wait
+// (2048 x 2048 SpMV: 26 us with two pageable copies in and one out).
+struct HostCall {
+    static constexpr size_t kSmall = 64 * 1024;         // bytes of inputs, and of the result
+    cudaStream_t stream = nullptr;
+    PinnedBlock block;                                  // [inputs | result], kSmall each
+    bool open = false;
+
+    int begin(int device) {
+        if (int rc = host_stream(device, 0, &stream)) return rc;
+        open = true;
+        return SPX_OK;
+    }
+    int stage(size_t bytes) { return block.host ? SPX_OK : pinned_acquire(bytes, &block); }
+    char* host() const { return static_cast<char*>(block.host); }
+    // The result half of the block as the device sees it; null when that is not to be had.
+    float* mapped_result() {
+        void* p = nullptr;
+        if (stage(2 * kSmall) != SPX_OK || cudaHostGetDevicePointer(&p, host() + kSmall, 0) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return nullptr;
+        }
+        return static_cast<float*>(p);
+    }
+    // Waits for the result and hands it over: from device memory, or (from == null) from the pinned block.
+    int finish(float* to, const float* from, size_t bytes) {
+        if (from) SPX_CUDA(cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, stream));
+        open = false;
+        SPX_CUDA(cudaStreamSynchronize(stream));
+        if (!from) std::memcpy(to, host() + kSmall, bytes);
+        return SPX_OK;
+    }
+    ~HostCall() {
+        if (open && stream) (void)cudaStreamSynchronize(stream);   // an error on the way: nothing may still use the block
+        pinned_release(block);
+    }
+};
+
+constexpr size_t kPanelBytes = 1u << 20;
+
+static int spmm_host_panels(spx_ell* e, const float* X, uint32_t C, const float* bias, int act, float* Y, float* dX, float* dB, float* dY)
+{
+    struct Events {
+        cudaEvent_t ev[4] = {};
+        ~Events() { for (cudaEvent_t v : ev) if (v) (void)cudaEventDestroy(v); }
+    } done;
+    struct Drain {                              // also after an error: the buffers are reused by the next call
+        cudaStream_t s[3] = {};
+        ~Drain() { for (cudaStream_t st : s) if (st) (void)cudaStreamSynchronize(st); }
+    } st;
+    for (int i = 0; i < 3; ++i)
+        if (int rc = host_stream(e->device, i, &st.s[i])) return rc;
+    for (cudaEvent_t& v : done.ev) SPX_CUDA(cudaEventCreateWithFlags(&v, cudaEventDisableTiming));
+    if (bias) SPX_CUDA(cudaMemcpyAsync(dB, bias, (size_t)e->m * 4, cudaMemcpyHostToDevice, st.s[0]));
+    const uint32_t w = C / 2;                   // a multiple of 4
+    for (int p = 0; p < 2; ++p) {
+        float* dXp = dX + (size_t)p * e->n * w;
+        if (int rc = copy_h2d_rows(dXp, X + (size_t)p * w, e->n, (size_t)w * 4, (size_t)C * 4, st.s[0])) return rc;
+        SPX_CUDA(cudaEventRecord(done.ev[2 * p], st.s[0]));
+        SPX_CUDA(cudaStreamWaitEvent(st.s[1], done.ev[2 * p], 0));
+        if (int rc = spx_spmm(e, dXp, w, w, bias ? dB : nullptr, act, dY + (size_t)p * w, C, st.s[1])) return rc;
+        SPX_CUDA(cudaEventRecord(done.ev[2 * p + 1], st.s[1]));
+        SPX_CUDA(cudaStreamWaitEvent(st.s[2], done.ev[2 * p + 1], 0));
+        // the copy of panel 0 to pageable memory would hold up the calling thread: both panels last, then
+        if (p == 1 || !pageable_memory(Y))
+            for (int q = (p == 1 && pageable_memory(Y)) ? 0 : p; q <= p; ++q)
+                SPX_CUDA(cudaMemcpy2DAsync(Y + (size_t)q * w, (size_t)C * 4, dY + (size_t)q * w, (size_t)C * 4, (size_t)w * 4, e->m,
+                                           cudaMemcpyDeviceToHost, st.s[2]));
+    }
+    SPX_CUDA(cudaStreamSynchronize(st.s[2]));
+    return SPX_OK;
+}
+
 // ---- host-buffer entry points ----------------------------------------------------------------
 // Pageable host buffers are copied by the driver through its own pinned bounce buffers; callers
 // that pass pinned memory (spx_host_alloc) get direct DMA.  Layout of the staging block:
@@ -738,13 +812,33 @@ int spx_spmm_host(const spx_ell* ce, const float* X, uint32_t C, const float* bi
         if (err != cudaSuccess) return fail(SPX_ERR_CUDA, "spmm_host: pipelined copy failed: %s", cudaGetErrorString(err));
         return SPX_OK;
     }
-    if (e->n) SPX_CUDA(cudaMemcpyAsync(dX, X, (size_t)e->n * C * 4, cudaMemcpyHostToDevice, nullptr));
-    if (bias) SPX_CUDA(cudaMemcpyAsync(dB, bias, (size_t)e->m * 4, cudaMemcpyHostToDevice, nullptr));
-    rc = spx_spmm(e, dX, C, C, bias ? dB : nullptr, act, dY, C, nullptr);
+    // Medium operands: two column panels, so that the copy in of one runs beside the multiply and the copy out
+    // of the other (4096 x 4096, C = 256: 305 -> 260 us).  A panel of X is packed on its way in.
+    // Panel rows of whole 128-byte lines only: the copy unit moved 4096 rows of 272 bytes in 600 us.
+    if (C % 64 == 0 && (size_t)e->n * C * 4 >= kPanelBytes && (size_t)e->m * C * 4 >= kPanelBytes) {
+        rc = spmm_host_panels(e, X, C, bias, act, Y, dX, dB, dY);
+        return rc;
+    }
+    HostCall call;
+    rc = call.begin(e->device);
     if (rc != SPX_OK) return rc;
-    SPX_CUDA(cudaMemcpyAsync(Y, dY, (size_t)e->m * C * 4, cudaMemcpyDeviceToHost, nullptr));
-    SPX_CUDA(cudaStreamSynchronize(nullptr));
-    return SPX_OK;
+    const size_t x_bytes = (size_t)e->n * C * 4, bias_bytes = bias ? (size_t)e->m * 4 : 0, y_bytes = (size_t)e->m * C * 4;
+    // X and the bias are neighbours on the device: where both are small they go over in one copy
+    if (xb + bb <= HostCall::kSmall) {
+        rc = call.stage(2 * HostCall::kSmall);
+        if (rc != SPX_OK) return rc;
+        if (x_bytes) std::memcpy(call.host(), X, x_bytes);
+        if (bias) std::memcpy(call.host() + xb, bias, bias_bytes);
+        const size_t both = bias ? xb + bias_bytes : x_bytes;
+        if (both) SPX_CUDA(cudaMemcpyAsync(dX, call.host(), both, cudaMemcpyHostToDevice, call.stream));
+    } else {
+        if (bias) SPX_CUDA(cudaMemcpyAsync(dB, bias, bias_bytes, cudaMemcpyHostToDevice, call.stream));
+        if (int rx = copy_h2d(dX, X, x_bytes, call.stream)) return rx;
+    }
+    float* direct = y_bytes <= HostCall::kSmall ? call.mapped_result() : nullptr;
+    rc = spx_spmm(e, dX, C, C, bias ? dB : nullptr, act, direct ? direct : dY, C, call.stream);
+    if (rc != SPX_OK) return rc;
+    return call.finish(Y, direct ? nullptr : dY, y_bytes);
 }
 
 // Row-sharded SpMM on host buffers, one process per GPU.  Every rank holds the same host X but
@@ -856,13 +950,25 @@ int spx_spmv_host(const spx_ell* ce, const float* x, const float* bias, float* y
     float* dx = reinterpret_cast<float*>(base);
     float* dB = reinterpret_cast<float*>(base + xb);
     float* dy = reinterpret_cast<float*>(base + xb + bb);
-    if (e->n) SPX_CUDA(cudaMemcpyAsync(dx, x, (size_t)e->n * 4, cudaMemcpyHostToDevice, nullptr));
-    if (bias) SPX_CUDA(cudaMemcpyAsync(dB, bias, (size_t)e->m * 4, cudaMemcpyHostToDevice, nullptr));
-    rc = spx_spmv(e, dx, bias ? dB : nullptr, dy, nullptr);
+    HostCall call;
+    rc = call.begin(e->device);
     if (rc != SPX_OK) return rc;
-    SPX_CUDA(cudaMemcpyAsync(y, dy, (size_t)e->m * 4, cudaMemcpyDeviceToHost, nullptr));
-    SPX_CUDA(cudaStreamSynchronize(nullptr));
-    return SPX_OK;
+    const size_t x_bytes = (size_t)e->n * 4, y_bytes = (size_t)e->m * 4;
+    if (xb + y_bytes <= HostCall::kSmall) {     // x and the bias in one copy
+        rc = call.stage(2 * HostCall::kSmall);
+        if (rc != SPX_OK) return rc;
+        if (x_bytes) std::memcpy(call.host(), x, x_bytes);
+        if (bias) std::memcpy(call.host() + xb, bias, y_bytes);
+        const size_t both = bias ? xb + y_bytes : x_bytes;
+        if (both) SPX_CUDA(cudaMemcpyAsync(dx, call.host(), both, cudaMemcpyHostToDevice, call.stream));
+    } else {
+        if (bias) SPX_CUDA(cudaMemcpyAsync(dB, bias, y_bytes, cudaMemcpyHostToDevice, call.stream));
+        if (int rx = copy_h2d(dx, x, x_bytes, call.stream)) return rx;
+    }
+    float* direct = y_bytes <= HostCall::kSmall ? call.mapped_result() : nullptr;
+    rc = spx_spmv(e, dx, bias ? dB : nullptr, direct ? direct : dy, call.stream);
+    if (rc != SPX_OK) return rc;
+    return call.finish(y, direct ? nullptr : dy, y_bytes);
 }
 
 }  // extern "C"

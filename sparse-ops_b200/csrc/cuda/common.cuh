@@ -10,6 +10,13 @@
 
 #include "spx_b200.h"
 
+namespace spx {
+struct PinnedBlock {
+    void* host = nullptr;
+    size_t bytes = 0;
+};
+}  // namespace spx
+
 // Device-resident ELLPACK (see include/spx_b200.h).  Row i occupies entries
 // [i*pitch, i*pitch + nnz[i]) of Wd / idx; pitch is a multiple of 32 entries so that
 // every row starts on a 128-byte boundary and float4 / uint4 loads are aligned.
@@ -49,6 +56,7 @@ struct spx_ell {
     // device memory (read by the kernel's later CTAs) and a word in pinned host memory (its device
     // alias is tma_failed_mapped; read by the next convolution call on the handle).
     int* tma_failed_host = nullptr;
+    spx::PinnedBlock tma_failed_block;
     int* tma_failed_mapped = nullptr;
     int* tma_failed_dev = nullptr;
     bool tma_off = false;
@@ -57,6 +65,7 @@ struct spx_ell {
     // SpMV with x larger than shared memory (spmv.cu): column window width and the per-row split
     // table, built on the first spx_spmv of such a handle.  spmv_win == UINT32_MAX: not applicable.
     uint32_t* spmv_split = nullptr;
+    size_t spmv_split_bytes = 0;
     uint32_t spmv_win = 0;
     // Pinned + device staging for the host-buffer entry points (abi.cu), grown on demand.
     void* stage_dev = nullptr;
@@ -186,14 +195,21 @@ int sort_rows(spx_ell* e, const uint32_t* host_nnz, uint2* order, cudaStream_t s
 // Device memory from the library's pool of the given device, stream-ordered (mem.cu).
 int pool_alloc(void** p, size_t bytes, int device, cudaStream_t s);
 void pool_free(void* p, size_t bytes, cudaStream_t s);      // bytes as allocated; p may be null
+int pool_alloc_now(void** p, size_t bytes, int device);     // usable on every stream at once
+// Host -> device copy in stream order; pageable sources are staged by several threads (hostcopy.cu).
+int copy_h2d(void* dst, const void* src, size_t bytes, cudaStream_t s);
+// The same for rows of `row` bytes, `stride` bytes apart, to contiguous device memory.
+int copy_h2d_rows(void* dst, const void* src, size_t rows, size_t row, size_t stride, cudaStream_t s);
+bool pageable_memory(const void* p);            // host memory that is not page-locked
+// Replaces a handle's scratch block by a larger one (waits for the device: kernels may still use the old one).
+int grow_scratch(spx_ell* e, void** p, size_t* bytes, size_t need);
 void pool_trim(int device);                     // waits for the device, then gives all free memory back
 // A non-blocking stream per device for small transfers beside the caller's stream, created once (mem.cu).
 int side_stream(int device, cudaStream_t* out);
+// The calling thread's streams for its host-buffer calls on a device: 0 for all of a call, or copies in (0),
+// multiplies (1) and copies out (2).
+int host_stream(int device, int which, cudaStream_t* out);
 // Pinned host memory from a bounded free list (mem.cu).
-struct PinnedBlock {
-    void* host = nullptr;
-    size_t bytes = 0;
-};
 int pinned_acquire(size_t bytes, PinnedBlock* out);
 void pinned_release(const PinnedBlock& b);
 }  // namespace spx

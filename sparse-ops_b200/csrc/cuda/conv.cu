@@ -654,7 +654,8 @@ static int ensure_taps(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s)
 {
     if (e->taps && e->taps_kH == kH && e->taps_kW == kW) return SPX_OK;
     if (e->r == 0) return SPX_OK;
-    if (!e->taps) SPX_CUDA(cudaMalloc(&e->taps, (size_t)e->m * e->pitch * sizeof(uint32_t)));
+    if (!e->taps)
+        if (int rc = pool_alloc_now(reinterpret_cast<void**>(&e->taps), (size_t)e->m * e->pitch * sizeof(uint32_t), e->device)) return rc;
     build_taps_kernel<<<e->m, 128, 0, s>>>(e->idx, e->nnz, e->m, e->pitch, kH, kW, e->taps);
     SPX_LAUNCH_CHECK("build_taps_kernel");
     e->taps_kH = kH;
@@ -710,11 +711,13 @@ static int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s)
         // per block of 4 rows).  Without room for it the per-row kernel is used instead.
         if (e->rbm_cap == UINT32_MAX) return -1;        // an earlier attempt ran out of memory
         const uint32_t cap = (uint32_t)std::min<uint64_t>((uint64_t)kRbmRows * e->max_nnz, e->n);
-        if (cudaMalloc(&e->rbm_ncols, (size_t)nblocks * sizeof(uint32_t)) != cudaSuccess ||
-            cudaMalloc(&e->rbm_w, (size_t)nblocks * cap * kRbmRows * sizeof(float)) != cudaSuccess ||
-            cudaMalloc(&e->rbm_hdr, (size_t)nblocks * cap * sizeof(uint2)) != cudaSuccess) {
-            (void)cudaGetLastError();
-            cudaFree(e->rbm_ncols); cudaFree(e->rbm_w); cudaFree(e->rbm_hdr);
+        const size_t slots = (size_t)nblocks * cap;
+        if (pool_alloc_now(reinterpret_cast<void**>(&e->rbm_ncols), (size_t)nblocks * sizeof(uint32_t), e->device) != SPX_OK ||
+            pool_alloc_now(reinterpret_cast<void**>(&e->rbm_w), slots * kRbmRows * sizeof(float), e->device) != SPX_OK ||
+            pool_alloc_now(reinterpret_cast<void**>(&e->rbm_hdr), slots * sizeof(uint2), e->device) != SPX_OK) {
+            pool_free(e->rbm_ncols, (size_t)nblocks * sizeof(uint32_t), s);
+            pool_free(e->rbm_w, slots * kRbmRows * sizeof(float), s);
+            pool_free(e->rbm_hdr, slots * sizeof(uint2), s);
             e->rbm_ncols = nullptr; e->rbm_w = nullptr; e->rbm_hdr = nullptr;
             e->rbm_cap = UINT32_MAX;
             return -1;
@@ -1007,11 +1010,7 @@ int launch_conv2d(spx_ell* e, const spx_conv_geom* g, int layout, const float* i
         const uint64_t in_slab = (n_in + 63) / 64 * 64;
         const size_t need = (size_t)(in_slab + n_out) * sizeof(float);
         if (e->fm_scratch_bytes < need) {
-            if (e->fm_scratch) cudaFree(e->fm_scratch);
-            e->fm_scratch = nullptr;
-            e->fm_scratch_bytes = 0;
-            SPX_CUDA(cudaMalloc(&e->fm_scratch, need));
-            e->fm_scratch_bytes = need;
+            if (int rs = grow_scratch(e, &e->fm_scratch, &e->fm_scratch_bytes, need)) return rs;
         }
         float* in_pf = static_cast<float*>(e->fm_scratch);
         float* out_pf = in_pf + in_slab;
@@ -1040,11 +1039,7 @@ int launch_conv2d(spx_ell* e, const spx_conv_geom* g, int layout, const float* i
             const uint64_t n_in = (nchw && pad) ? slab(in_rows * B) : 0, n_out = (nchw && pad) ? slab(out_rows * B) : 0;
             const size_t need = (size_t)(n_in4 + n_out4 + n_in + n_out) * sizeof(float);
             if (e->conv_scratch_bytes < need) {
-                if (e->conv_scratch) cudaFree(e->conv_scratch);
-                e->conv_scratch = nullptr;
-                e->conv_scratch_bytes = 0;
-                SPX_CUDA(cudaMalloc(&e->conv_scratch, need));
-                e->conv_scratch_bytes = need;
+                if (int rs = grow_scratch(e, &e->conv_scratch, &e->conv_scratch_bytes, need)) return rs;
             }
             float* in4 = static_cast<float*>(e->conv_scratch);
             float* out4 = in4 + n_in4;

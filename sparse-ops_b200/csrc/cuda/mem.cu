@@ -20,7 +20,7 @@ namespace spx {
 
 namespace {
 
-constexpr uint64_t kPoolKeep = 1ull << 30;          // of about 180 GB
+constexpr uint64_t kPoolKeep = 2ull << 30;          // of about 180 GB
 // A block that would take a large part of that is mapped and unmapped directly: the pool would not
 // keep it, and growing it by such a block took twice as long as cudaMalloc (slabs of 2 x 0.9 GB).
 constexpr size_t kPoolBlock = kPoolKeep / 4;
@@ -82,6 +82,35 @@ void pool_free(void* p, size_t bytes, cudaStream_t s)
     if (p) (void)(bytes > kPoolBlock ? cudaFree(p) : cudaFreeAsync(p, s));
 }
 
+// Memory that is used on other streams than the one at hand, or while a stream is being captured: it comes
+// through the side stream and is there when the call returns.
+int pool_alloc_now(void** p, size_t bytes, int device)
+{
+    cudaStream_t side = nullptr;
+    if (int rc = side_stream(device, &side)) return rc;
+    if (int rc = pool_alloc(p, bytes, device, side)) return rc;
+    if (bytes && cudaStreamSynchronize(side) != cudaSuccess) {
+        (void)cudaGetLastError();
+        pool_free(*p, bytes, side);
+        *p = nullptr;
+        return fail(SPX_ERR_CUDA, "device allocation of %zu bytes failed", bytes);
+    }
+    return SPX_OK;
+}
+
+int grow_scratch(spx_ell* e, void** p, size_t* bytes, size_t need)
+{
+    if (*p) {
+        (void)cudaDeviceSynchronize();
+        pool_free(*p, *bytes, nullptr);
+    }
+    *p = nullptr;
+    *bytes = 0;
+    if (int rc = pool_alloc_now(p, need, e->device)) return rc;
+    *bytes = need;
+    return SPX_OK;
+}
+
 void pool_trim(int device)
 {
     if (device < 0 || device >= kMaxDevices) return;
@@ -90,14 +119,29 @@ void pool_trim(int device)
     if (g_pools[device]) (void)cudaMemPoolTrimTo(g_pools[device], 0);
 }
 
-int side_stream(int device, cudaStream_t* out)
+static int kept_stream(cudaStream_t (&streams)[kMaxDevices], int device, cudaStream_t* out)
 {
-    static cudaStream_t streams[kMaxDevices] = {};
     if (device < 0 || device >= kMaxDevices) return fail(SPX_ERR_LIMIT, "device ordinal %d not supported", device);
     std::lock_guard<std::mutex> lk(g_pool_mu);
     if (!streams[device]) SPX_CUDA(cudaStreamCreateWithFlags(&streams[device], cudaStreamNonBlocking));
     *out = streams[device];
     return SPX_OK;
+}
+
+int side_stream(int device, cudaStream_t* out)
+{
+    static cudaStream_t streams[kMaxDevices] = {};
+    return kept_stream(streams, device, out);
+}
+
+int host_stream(int device, int which, cudaStream_t* out)
+{
+    struct Streams {                            // threads that make host-buffer calls do not wait for one another
+        cudaStream_t s[3][kMaxDevices] = {};
+        ~Streams() { for (auto& k : s) for (cudaStream_t st : k) if (st) (void)cudaStreamDestroy(st); }
+    };
+    thread_local Streams mine;
+    return kept_stream(mine.s[which], device, out);
 }
 
 int pinned_acquire(size_t bytes, PinnedBlock* out)
@@ -140,16 +184,16 @@ void pinned_release(const PinnedBlock& b)
 
 void ensure_tma_words(spx_ell* e)
 {
-    if (e->tma_failed_host || cudaHostAlloc(reinterpret_cast<void**>(&e->tma_failed_host), sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return;
-    }
+    if (e->tma_failed_host || pinned_acquire(sizeof(int), &e->tma_failed_block) != SPX_OK) return;
+    e->tma_failed_host = static_cast<int*>(e->tma_failed_block.host);
     *e->tma_failed_host = 0;
+    cudaStream_t side = nullptr;
     if (cudaHostGetDevicePointer(reinterpret_cast<void**>(&e->tma_failed_mapped), e->tma_failed_host, 0) != cudaSuccess ||
-        cudaMalloc(reinterpret_cast<void**>(&e->tma_failed_dev), sizeof(int)) != cudaSuccess ||
-        cudaMemset(e->tma_failed_dev, 0, sizeof(int)) != cudaSuccess) {
+        side_stream(e->device, &side) != SPX_OK ||
+        pool_alloc(reinterpret_cast<void**>(&e->tma_failed_dev), sizeof(int), e->device, side) != SPX_OK ||
+        cudaMemsetAsync(e->tma_failed_dev, 0, sizeof(int), side) != cudaSuccess || cudaStreamSynchronize(side) != cudaSuccess) {
         e->tma_failed_mapped = nullptr;
-        if (e->tma_failed_dev) cudaFree(e->tma_failed_dev);
+        pool_free(e->tma_failed_dev, sizeof(int), side);
         e->tma_failed_dev = nullptr;
         (void)cudaGetLastError();
     }

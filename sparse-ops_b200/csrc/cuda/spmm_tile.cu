@@ -463,7 +463,7 @@ double gather_us(const spx_ell* e, uint32_t C, bool aligned)
     const double lanes = (double)q * RW / (32.0 * NV * panels);
     double rate = density < 0.04 ? 26e6 : C <= 64 ? 16e6 : C <= 128 ? 20e6 : 23e6;     // bytes per us, measured
     if (!aligned) rate *= 0.6;
-    return 2.0 + std::max((double)e->nnz_total * C * 4.0 / (rate * lanes), e->max_nnz / (NV == 1 ? 32.0 : 16.0) * 0.85);
+    return 2.0 + std::max((double)e->nnz_total * C * 4.0 / (rate * lanes), e->max_nnz / (NV == 1 ? 32.0 : 16.0) * (NV == 1 ? 1.0 : 0.85));
 }
 
 }  // namespace

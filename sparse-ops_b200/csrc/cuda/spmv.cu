@@ -451,11 +451,11 @@ static int ensure_spmv_windows(spx_ell* e, cudaStream_t s)
     if (enabled != 2 && run > 2500.0) return SPX_OK;
     const uint32_t win = round_up((e->n + windows - 1) / windows, 4u);
     const uint64_t entries = (uint64_t)e->m * (windows - 1);
-    if (cudaMalloc(&e->spmv_split, entries * sizeof(uint32_t)) != cudaSuccess) {
-        (void)cudaGetLastError();
+    if (pool_alloc_now(reinterpret_cast<void**>(&e->spmv_split), entries * sizeof(uint32_t), e->device) != SPX_OK) {
         e->spmv_split = nullptr;
         return SPX_OK;                                              // no room: gather x from global memory
     }
+    e->spmv_split_bytes = entries * sizeof(uint32_t);
     spmv_splits_kernel<<<(unsigned)((entries + 255) / 256), 256, 0, s>>>(e->idx, e->nnz, e->m, e->pitch, win, windows - 1,
                                                                        e->spmv_split);
     SPX_LAUNCH_CHECK("spmv_splits_kernel");

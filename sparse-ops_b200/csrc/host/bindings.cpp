@@ -15,6 +15,7 @@
 
 #include "ellpack.hpp"
 #include "rbm.hpp"
+#include "result_pool.hpp"
 #include "sparse_onnx.hpp"
 
 namespace py = pybind11;
@@ -49,6 +50,23 @@ static py::array_t<T> copy2d(const T* src, uint32_t m, uint32_t r)
     py::array_t<T> a({ py::ssize_t(m), py::ssize_t(r) });
     if (m && r) std::memcpy(a.mutable_data(), src, size_t(m) * r * sizeof(T));
     return a;
+}
+
+// A new float32 array for a result; *pinned tells whether its memory is page-locked (see result_pool.hpp).
+static py::array_t<float> result_array(const std::vector<py::ssize_t>& shape, bool* pinned)
+{
+    size_t bytes = sizeof(float);
+    for (py::ssize_t d : shape) bytes *= size_t(d);
+    const spx::ResultPool::Block b = spx::ResultPool::get().acquire(bytes);
+    *pinned = b.ptr != nullptr;
+    if (!b.ptr) return py::array_t<float>(shape);
+    auto* owned = new spx::ResultPool::Block(b);
+    py::capsule owner(owned, [](void* p) {
+        auto* blk = static_cast<spx::ResultPool::Block*>(p);
+        spx::ResultPool::get().release(*blk);
+        delete blk;
+    });
+    return py::array_t<float>(shape, static_cast<float*>(b.ptr), owner);
 }
 
 static const float* optional_bias(const py::object& bias, farray& keep, uint32_t m, const char* msg)
@@ -136,7 +154,8 @@ PYBIND11_MODULE(sparseops_backend, m)
         farray keep;
         const float* b = optional_bias(bias, keep, E.m, "Bias length must equal E.m");
         const uint32_t C = uint32_t(buf_X.shape[1]);
-        py::array_t<float> Y({ py::ssize_t(E.m), py::ssize_t(C) });
+        bool pinned = false;
+        py::array_t<float> Y = result_array({ py::ssize_t(E.m), py::ssize_t(C) }, &pinned);
         float* yp = Y.mutable_data();
         const float* xp = static_cast<const float*>(buf_X.ptr);
         {
@@ -206,12 +225,13 @@ PYBIND11_MODULE(sparseops_backend, m)
                 throw std::runtime_error("X must hold batch x in_features values");
             std::vector<size_t> dims = model.output_shape();
             if (!dims.empty()) dims[0] = B;
-            py::array_t<float> Y(dims);
+            bool pinned = false;
+            py::array_t<float> Y = result_array(std::vector<py::ssize_t>(dims.begin(), dims.end()), &pinned);
             float* yp = Y.mutable_data();
             const float* xp = static_cast<const float*>(buf.ptr);
             {
                 py::gil_scoped_release nogil;
-                model.run(xp, B, yp);
+                model.run(xp, B, yp, pinned);
             }
             return Y;
         }, "Run inference; memory in and out is feature-major ([features x B], B fastest), as in the reference")

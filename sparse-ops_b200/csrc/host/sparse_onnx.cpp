@@ -570,7 +570,7 @@ void SparseOnnxModel::launch_layers(const float* d_in, float* d_out, uint32_t B,
     }
 }
 
-void SparseOnnxModel::run(const float* input, uint32_t B, float* output) const
+void SparseOnnxModel::run(const float* input, uint32_t B, float* output, bool pinned_output) const
 {
     if (!exec_ || exec_->B != B) build_exec(B);
     Exec& ex = *exec_;
@@ -580,7 +580,7 @@ void SparseOnnxModel::run(const float* input, uint32_t B, float* output) const
     if (ex.graph) check(spx_graph_launch(ex.graph, ex.stream), "graph launch");
     else launch_layers(d_in, d_out, B, ex.stream);
     const size_t out_bytes = size_t(out_features_) * B * sizeof(float);
-    if (ex.h_out && ex.h_out_bytes == out_bytes) {
+    if (!pinned_output && ex.h_out && ex.h_out_bytes == out_bytes) {
         check(spx_memcpy_d2h(ex.h_out, d_out, out_bytes, ex.stream), "output copy");
         check(spx_stream_sync(ex.stream), "run");
         std::memcpy(output, ex.h_out, out_bytes);

@@ -64,7 +64,7 @@ public:
 
     /// Host buffers in, host buffers out (see the memory contract above).  Re-plans the device
     /// buffers when B differs from the current batch.
-    void run(const float* input, uint32_t B, float* output) const;
+    void run(const float* input, uint32_t B, float* output, bool pinned_output = false) const;
     /// Device buffers in and out; launches the layer loop on `stream` without synchronising.
     void run_device(const float* d_input, uint32_t B, float* d_output, void* stream) const;
     /// The model's own device buffers for the current batch (valid after resize_buffers / run):
