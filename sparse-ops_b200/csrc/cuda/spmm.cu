@@ -428,7 +428,7 @@ struct RowsGroup {
 };
 
 template <int V, int NV, int U, int MINB, bool PIPE>
-__global__ void __launch_bounds__(kRowsWarps * 32, MINB)
+__global__ void __launch_bounds__(kRowsWarps * 32, MINB)     // MINB x 4 warps: 64, 128 or 255 registers
 spmm_rows(const __grid_constant__ RowsArgs a)
 {
     constexpr int kBatch = kRowsBatch, kRing = kRowsRing, kRowStride = kRowsStride;
@@ -511,11 +511,15 @@ spmm_rows(const __grid_constant__ RowsArgs a)
             const uint32_t cmax = min((uint32_t)kBatch, nmax - bt * kBatch);
             const uint32_t cmin = nmin > bt * kBatch ? min((uint32_t)kBatch, nmin - bt * kBatch) : 0u;
             constexpr int T = U >= 16 ? 8 : 4;
-            uint32_t t = 0;                         // groups that every row of the warp fills, then smaller ones
-            for (; t + U <= cmin; t += U) {
-                RowsGroup<V, NV, U> g;
-                g.template issue<true>(bw + t, bk + t, U, x);
-                g.template multiply<true>(acc, U);
+            // groups that every row of the warp fills, then smaller ones.  Groups of 4 take the predicated path alone:
+            // a second copy of the loop does not fit 64 registers (262144 power-law rows, C = 1024: 4.21 -> 3.91 ms).
+            uint32_t t = 0;
+            if constexpr (U > T) {
+                for (; t + U <= cmin; t += U) {
+                    RowsGroup<V, NV, U> g;
+                    g.template issue<true>(bw + t, bk + t, U, x);
+                    g.template multiply<true>(acc, U);
+                }
             }
             for (; t < cmax; t += T) {
                 const uint32_t have = cnt > t ? cnt - t : 0u;
@@ -1024,22 +1028,22 @@ static int launch_rows(const spx_ell* e, RowsArgs a, cudaStream_t s)
     // Single columns per lane are cheap enough in registers to keep a second group in flight (1312 x 2080, 27 %,
     // C = 37: 34 -> 23 us); 16-byte vectors are not (4096 x 4096, 10 %, C = 128: 42 -> 46 us).
     if constexpr (V == 1) {
-        if (per_sm < 12 && NV == 1) return launch_rows_one<1, 1, 32, 1, true>(e, a, panels, wpb, s);
-        if (per_sm < 12 && NV == 2) return launch_rows_one<1, 2, 16, 1, true>(e, a, panels, wpb, s);
-        if (per_sm < 12) return launch_rows_one<1, 3, 16, 1, true>(e, a, panels, wpb, s);
+        if (per_sm < 12 && NV == 1) return launch_rows_one<1, 1, 32, 2, true>(e, a, panels, wpb, s);
+        if (per_sm < 12 && NV == 2) return launch_rows_one<1, 2, 16, 2, true>(e, a, panels, wpb, s);
+        if (per_sm < 12) return launch_rows_one<1, 3, 16, 2, true>(e, a, panels, wpb, s);
     }
     if (NV == 1)
-        return U == 32   ? launch_rows_one<V, 1, 32, 1>(e, a, panels, wpb, s)
-               : U == 16 ? launch_rows_one<V, 1, 16, 1>(e, a, panels, wpb, s)
-                         : launch_rows_one<V, 1, 4, 4>(e, a, panels, wpb, s);
+        return U == 32   ? launch_rows_one<V, 1, 32, 2>(e, a, panels, wpb, s)
+               : U == 16 ? launch_rows_one<V, 1, 16, 2>(e, a, panels, wpb, s)
+                         : launch_rows_one<V, 1, 4, 8>(e, a, panels, wpb, s);
     if (NV == 2 || V == 4)
-        return U == 16  ? launch_rows_one<V, 2, 16, 1>(e, a, panels, wpb, s)
-               : U == 8 ? launch_rows_one<V, 2, 8, 2>(e, a, panels, wpb, s)
-                        : launch_rows_one<V, 2, 4, 4>(e, a, panels, wpb, s);
+        return U == 16  ? launch_rows_one<V, 2, 16, 2>(e, a, panels, wpb, s)
+               : U == 8 ? launch_rows_one<V, 2, 8, 4>(e, a, panels, wpb, s)
+                        : launch_rows_one<V, 2, 4, 8>(e, a, panels, wpb, s);
     if constexpr (V != 4)
-        return U == 16  ? launch_rows_one<V, 3, 16, 1>(e, a, panels, wpb, s)
-               : U == 8 ? launch_rows_one<V, 3, 8, 2>(e, a, panels, wpb, s)
-                        : launch_rows_one<V, 3, 4, 4>(e, a, panels, wpb, s);
+        return U == 16  ? launch_rows_one<V, 3, 16, 2>(e, a, panels, wpb, s)
+               : U == 8 ? launch_rows_one<V, 3, 8, 4>(e, a, panels, wpb, s)
+                        : launch_rows_one<V, 3, 4, 8>(e, a, panels, wpb, s);
     return fail(SPX_ERR_LIMIT, "spmm: no kernel");
 }
 
