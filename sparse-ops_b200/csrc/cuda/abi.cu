@@ -419,7 +419,6 @@ int spx_ell_destroy(spx_ell* e)
     pool_free(e->rbm_hdr, slots4 * sizeof(uint2), nullptr);
     pool_free(e->stage_dev, e->stage_dev_bytes, nullptr);
     pool_free(e->conv_scratch, e->conv_scratch_bytes, nullptr);
-    pool_free(e->fm_scratch, e->fm_scratch_bytes, nullptr);
     pool_free(e->tma_failed_dev, sizeof(int), nullptr);
     pinned_release(e->tma_failed_block);
     for (cudaStream_t st : e->pipe_streams) if (st) cudaStreamDestroy(st);

@@ -139,36 +139,32 @@ transpose2d_kernel(const float* __restrict__ src, uint64_t rows, uint64_t cols, 
     }
 }
 
-// dst[r * dst_pitch + c] = c < src_cols ? src[r * src_pitch + c] : 0  for c < dst_cols: widens the
-// batch dimension of a [C,H,W,B] tensor to a multiple of 4 (zeros in the added entries) or narrows
-// it back.
+// Any input tensor to [C,H,W,B4], B4 = B rounded up to a multiple of 4 with zeros in the added entries: the
+// one pass in front of the tiled kernels for inputs whose batch is not the innermost dimension or no
+// multiple of 4.  A thread writes one 16-byte quad of a position; consecutive threads take consecutive
+// positions where the source is contiguous along them (NCHW), else the quads of a position first.
+// I: the type of the quad index (32 bits where they do: 64-bit divisions cost more than the copy).
+template <bool POSITIONS_FIRST, class I>
 __global__ void __launch_bounds__(256)
-repitch_kernel(const float* __restrict__ src, uint32_t src_pitch, uint32_t src_cols,
-               float* __restrict__ dst, uint32_t dst_pitch, uint32_t dst_cols, uint64_t rows)
+to_pf_kernel(const float* __restrict__ src, uint64_t sB, uint64_t sC, uint64_t sH, uint64_t sW, uint32_t H, uint32_t W, uint64_t positions,
+             uint32_t B, uint32_t quads, float* __restrict__ dst)
 {
-    const uint64_t total = rows * dst_cols;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t r = i / dst_cols;
-        const uint32_t c = (uint32_t)(i - r * dst_cols);
-        dst[r * dst_pitch + c] = c < src_cols ? src[r * src_pitch + c] : 0.0f;
-    }
-}
-
-// dst[k][j][i][b] = src[i][j][k][b]: reverses the three outer dimensions (D0, D1, D2) of a tensor whose
-// innermost dimension B stays contiguous -- F-major [W,H,C,B] to [C,H,W,B] and back.
-__global__ void __launch_bounds__(256)
-reverse3_kernel(const float* __restrict__ src, uint32_t D0, uint32_t D1, uint32_t D2, uint32_t B,
-                float* __restrict__ dst)
-{
-    const uint64_t total = (uint64_t)D0 * D1 * D2 * B;
-    for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t b = (uint32_t)(t % B);
-        uint64_t r = t / B;
-        const uint32_t i = (uint32_t)(r % D0);
-        r /= D0;
-        const uint32_t j = (uint32_t)(r % D1);
-        const uint32_t k = (uint32_t)(r / D1);
-        dst[t] = __ldg(src + ((((uint64_t)i * D1 + j) * D2 + k) * B + b));
+    spx::pdl_launch();
+    spx::pdl_wait();
+    const uint64_t total = positions * quads;
+    for (uint64_t t64 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t64 < total; t64 += (uint64_t)gridDim.x * blockDim.x) {
+        const I t = (I)t64, q = POSITIONS_FIRST ? t / (I)positions : t / (I)quads;
+        const I pos = POSITIONS_FIRST ? t - q * (I)positions : q;
+        const uint32_t b = 4 * (uint32_t)(POSITIONS_FIRST ? q : t - q * (I)quads);
+        const I ch = pos / W;
+        const uint32_t w = (uint32_t)(pos - ch * W), h = (uint32_t)(ch % H);
+        const float* __restrict__ p = src + (ch / H) * sC + h * sH + w * sW + b * sB;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (b < B) v.x = __ldg(p);
+        if (b + 1 < B) v.y = __ldg(p + sB);
+        if (b + 2 < B) v.z = __ldg(p + 2 * sB);
+        if (b + 3 < B) v.w = __ldg(p + 3 * sB);
+        *reinterpret_cast<float4*>(dst + (uint64_t)pos * (4ull * quads) + b) = v;
     }
 }
 
@@ -195,8 +191,18 @@ reverse3_kernel(const float* __restrict__ src, uint32_t D0, uint32_t D1, uint32_
 #endif
 constexpr int kTileH = 4, kTileW = 8, kTileWarps = 16;
 
+// Strides in floats.  Input: the batch is contiguous, the other strides are multiples of 4.  Output: any
+// layout; vec_out when the batch is contiguous there too and every position starts on 16 bytes.
+struct ConvViews {
+    uint64_t iC, iH, iW;
+    uint64_t oB, oC, oH, oW;
+    uint32_t b_out;     // batch entries that exist in the output (the input may be widened by up to 3)
+    uint32_t vec_out;
+};
+
 struct TileParams {
     ConvParams c;
+    ConvViews v;
     uint32_t BT;        // batch entries per CTA (multiple of 4, <= 32)
     uint32_t CC;        // input channels per staged chunk
     uint32_t THin, TWin;
@@ -209,6 +215,25 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+// Four finished outputs of one position: batch entries b .. b + 3 of channel mo.
+__device__ __forceinline__ void store_quad(float* __restrict__ out, const ConvViews& v, uint32_t mo, uint32_t oh, uint32_t ow, uint32_t b,
+                                           float4 o, int act)
+{
+    if (act != SPX_ACT_NONE) {
+        o.x = spx::apply_act(o.x, act); o.y = spx::apply_act(o.y, act);
+        o.z = spx::apply_act(o.z, act); o.w = spx::apply_act(o.w, act);
+    }
+    float* __restrict__ p = out + mo * v.oC + oh * v.oH + ow * v.oW + b * v.oB;
+    if (v.vec_out) {
+        *reinterpret_cast<float4*>(p) = o;
+        return;
+    }
+    if (b < v.b_out) p[0] = o.x;
+    if (b + 1 < v.b_out) p[v.oB] = o.y;
+    if (b + 2 < v.b_out) p[2 * v.oB] = o.z;
+    if (b + 3 < v.b_out) p[3 * v.oB] = o.w;
+}
 
 // Stages input channels [c0, c1) of a CTA's receptive field in shared memory as
 // [channel][row][column][BT batch entries]: one warp per (channel, row), 16-byte cp.async copies,
@@ -227,11 +252,11 @@ __device__ __forceinline__ void stage_chunk(float* tile, const TileParams& tp, c
         const int ih = ih0 + (int)y;
         const bool rowok = (unsigned)ih < p.H;
         float* srow = tile + (size_t)r * rowUnits * 4;
-        const float* grow = in + (((size_t)(c0 + c) * p.H + (rowok ? ih : 0)) * p.W) * p.B + b0;
+        const float* grow = in + (size_t)(c0 + c) * tp.v.iC + (size_t)(rowok ? ih : 0) * tp.v.iH + b0;
         for (uint32_t u = lane; u < rowUnits; u += 32) {
             const uint32_t x = u / QB, q = u % QB;
             const int iw = iw0 + (int)x;
-            if (rowok && (unsigned)iw < p.W) cp_async16(srow + u * 4, grow + (size_t)iw * p.B + q * 4);
+            if (rowok && (unsigned)iw < p.W) cp_async16(srow + u * 4, grow + (size_t)iw * tp.v.iW + q * 4);
             else *reinterpret_cast<float4*>(srow + u * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
     }
@@ -324,14 +349,7 @@ conv_pf_tile_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ t
         const uint32_t q = lane + 32u * g;
         const uint32_t pix = q / QB, quad = q % QB;
         const uint32_t oh = oh0 + pix / kTileW, ow = ow0 + pix % kTileW;
-        if (oh < p.Ho && ow < p.Wo) {
-            float4 o = acc[g];
-            if (act != SPX_ACT_NONE) {
-                o.x = spx::apply_act(o.x, act); o.y = spx::apply_act(o.y, act);
-                o.z = spx::apply_act(o.z, act); o.w = spx::apply_act(o.w, act);
-            }
-            *reinterpret_cast<float4*>(out + (((size_t)mo * p.Ho + oh) * p.Wo + ow) * p.B + b0 + quad * 4) = o;
-        }
+        if (oh < p.Ho && ow < p.Wo) store_quad(out, tp.v, mo, oh, ow, b0 + quad * 4, acc[g], act);
     }
 }
 
@@ -448,16 +466,30 @@ __device__ __forceinline__ void rbm_row(float4 (&acc)[kRbmRows][G], uint32_t hm,
     }
 }
 
+// The same with the weight at hand.  (FMAs under one predicate each measured 1.6 times slower than this test.)
+template <int G>
+__device__ __forceinline__ void rbm_row_if(float4 (&acc)[G], uint32_t have, float w, const float4 (&x)[G])
+{
+    if (have) {
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            spx::fma_pair(acc[g].x, acc[g].y, w, x[g].x, x[g].y);
+            spx::fma_pair(acc[g].z, acc[g].w, w, x[g].z, x[g].w);
+        }
+    }
+}
+
 // Work units are (tile of positions, group of NB row blocks, batch tile), numbered tile-fastest.
-// G = kRbmG: the CTA takes unit `unit0 + blockIdx.x`.  G = kRbmG / 2 (half-height tiles): CTAs
-// 2u and 2u + 1 take the upper and lower half of unit `unit0 + u`; used for the last, partly
+// The CTA takes unit `unit0 + blockIdx.x`; with `half`, CTAs 2u and 2u + 1 (of a kernel with half the
+// positions per lane) take the upper and lower half of unit `unit0 + u`; used for the last, partly
 // filled wave of a launch so that its work spreads over twice as many SMs.
 struct RbmUnits {
     uint32_t unit0, tiles, groups;     // first unit of this launch; tiles per image; row-block groups
+    uint32_t half;
 };
 
 template <int QB, int NB, int G>
-__global__ void __launch_bounds__(NB * 32, 1)
+__global__ void __launch_bounds__(NB * 32, 16 / NB)
 conv_rbm_tile_kernel(const uint2* __restrict__ hdr, const float4* __restrict__ w4,
                      const uint32_t* __restrict__ ncols, uint32_t cap, TileParams tp, RbmUnits un,
                      const float* __restrict__ in, const float* __restrict__ bias, int act,
@@ -468,16 +500,19 @@ conv_rbm_tile_kernel(const uint2* __restrict__ hdr, const float4* __restrict__ w
     __shared__ __align__(8) uint64_t tile_bar[2];
     __shared__ uint32_t buf_done[2];      // warps that have finished the chunk held by buffer 0 / 1
     __shared__ uint32_t copies_asked;     // bulk copies this CTA has asked for
+    __shared__ __align__(16) float4 s_wgt[G < kRbmG ? NB : 1][32];
+    __shared__ __align__(16) uint32_t s_hdr[G < kRbmG ? NB : 1][32];
     constexpr int RB = (int)kRbmRows;
     constexpr uint32_t BT = QB * 4;
     constexpr uint32_t TH = 32u * G / QB / kTileW;       // rows of output positions per tile
-    constexpr bool kHalf = G != kRbmG;
     const ConvParams& p = tp.c;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t unit = un.unit0 + (kHalf ? blockIdx.x >> 1 : blockIdx.x);
+    const uint32_t unit = un.unit0 + (un.half ? blockIdx.x >> 1 : blockIdx.x);
     const uint32_t t_id = unit % un.tiles, by = (unit / un.tiles) % un.groups, bz = unit / un.tiles / un.groups;
-    const uint32_t ty = kHalf ? (t_id / tp.tilesX) * 2 + (blockIdx.x & 1) : t_id / tp.tilesX, tx = t_id % tp.tilesX;
+    const uint32_t ty = un.half ? (t_id / tp.tilesX) * 2 + (blockIdx.x & 1) : t_id / tp.tilesX, tx = t_id % tp.tilesX;
     const uint32_t oh0 = ty * TH, ow0 = tx * kTileW;
+    spx::pdl_launch();
+    spx::pdl_wait();
     if (oh0 >= p.Ho) return;                             // lower half of a tile that ends above it
     const uint32_t b0 = bz * BT;
     const uint32_t blk = by * NB + warp;
@@ -540,6 +575,15 @@ conv_rbm_tile_kernel(const uint2* __restrict__ hdr, const float4* __restrict__ w
         if (!active) return;        // warps without rows take no part in the counting below
     }
 
+    // lane l: union column at + l of the block, header and weights
+    auto load_batch = [&](uint32_t at, uint2& hh, float4& ww) {
+        hh = make_uint2(0u, 0u);
+        ww = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (at + lane < nn) {
+            hh = __ldg(hrow + at + lane);
+            ww = __ldg(wrow + at + lane);
+        }
+    };
     uint32_t chunk = 0;
     for (uint32_t c0 = 0; c0 < p.Cin; c0 += tp.CC, ++chunk) {
         const uint32_t c1 = min(p.Cin, c0 + tp.CC);
@@ -555,12 +599,9 @@ conv_rbm_tile_kernel(const uint2* __restrict__ hdr, const float4* __restrict__ w
             // operands of the next batch of 32 columns are asked for before this batch's FMAs, so the
             // round trip to L2 runs behind them.
             bool have = pos + lane < nn;
-            uint2 h = make_uint2(0u, 0u);
-            float4 wl = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (have) {
-                h = __ldg(hrow + pos + lane);
-                wl = __ldg(wrow + pos + lane);
-            }
+            uint2 h;
+            float4 wl;
+            load_batch(pos, h, wl);
             for (;;) {
                 const uint32_t cin = have ? (h.x >> 16) : 0xffffffffu;
                 const uint32_t tl = (((cin - c0) * tp.THin + ((h.x >> 8) & 0xffu) * p.dH) * tp.TWin + (h.x & 0xffu) * p.dW) * BT;
@@ -572,21 +613,48 @@ conv_rbm_tile_kernel(const uint2* __restrict__ hdr, const float4* __restrict__ w
                 float4 nw = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (cnt == 32) {
                     nhave = npos + lane < nn;
-                    if (nhave) {
-                        nh = __ldg(hrow + npos + lane);
-                        nw = __ldg(wrow + npos + lane);
-                    }
+                    load_batch(npos, nh, nw);
                 }
-                for (uint32_t t = 0; t < cnt; ++t) {
-                    const uint32_t hm = __shfl_sync(0xffffffffu, hl, t);
-                    const float* xs = cur + (hm >> 8);
-                    float4 x[G];
+                if constexpr (G < kRbmG) {
+                    // Few warps per SM (small problems, tails): a column costs its latency.  The batch is laid down
+                    // in the warp's strip of shared memory and read back four columns at a time by broadcast, their
+                    // operands asked for together.  (Keeping the batch in registers across chunk boundaries: 10 %
+                    // slower, a chunk then starts and ends with a partial strip.)
+                    constexpr int U = 4;
+                    __syncwarp();               // the strip's earlier contents have been read
+                    s_hdr[warp][lane] = lane < (int)cnt ? hl : 0u;      // no rows beyond the batch's end
+                    s_wgt[warp][lane] = wl;
+                    __syncwarp();
+                    for (uint32_t t = 0; t < cnt; t += U) {
+                        const uint4 h4 = *reinterpret_cast<const uint4*>(&s_hdr[warp][t]);
+                        const uint32_t hm[U] = {h4.x, h4.y, h4.z, h4.w};
+                        float4 w[U], x[U][G];
 #pragma unroll
-                    for (int g = 0; g < G; ++g) x[g] = *reinterpret_cast<const float4*>(xs + off[g]);
-                    rbm_row<0, G>(acc, hm, wl.x, t, x);
-                    rbm_row<1, G>(acc, hm, wl.y, t, x);
-                    rbm_row<2, G>(acc, hm, wl.z, t, x);
-                    rbm_row<3, G>(acc, hm, wl.w, t, x);
+                        for (int u = 0; u < U; ++u) {
+                            w[u] = s_wgt[warp][t + u];
+#pragma unroll
+                            for (int g = 0; g < G; ++g) x[u][g] = *reinterpret_cast<const float4*>(cur + (hm[u] >> 8) + off[g]);
+                        }
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            rbm_row_if<G>(acc[0], hm[u] & 1u, w[u].x, x[u]);
+                            rbm_row_if<G>(acc[1], hm[u] & 2u, w[u].y, x[u]);
+                            rbm_row_if<G>(acc[2], hm[u] & 4u, w[u].z, x[u]);
+                            rbm_row_if<G>(acc[3], hm[u] & 8u, w[u].w, x[u]);
+                        }
+                    }
+                } else {
+                    for (uint32_t t = 0; t < cnt; ++t) {
+                        const uint32_t hm = __shfl_sync(0xffffffffu, hl, t);
+                        const float* xs = cur + (hm >> 8);
+                        float4 x[G];
+#pragma unroll
+                        for (int g = 0; g < G; ++g) x[g] = *reinterpret_cast<const float4*>(xs + off[g]);
+                        rbm_row<0, G>(acc, hm, wl.x, t, x);
+                        rbm_row<1, G>(acc, hm, wl.y, t, x);
+                        rbm_row<2, G>(acc, hm, wl.z, t, x);
+                        rbm_row<3, G>(acc, hm, wl.w, t, x);
+                    }
                 }
                 pos = npos;
                 if (cnt < 32) break;
@@ -634,14 +702,7 @@ conv_rbm_tile_kernel(const uint2* __restrict__ hdr, const float4* __restrict__ w
             const uint32_t q = lane + 32u * g;
             const uint32_t pix = q / QB, quad = q % QB;
             const uint32_t oh = oh0 + pix / kTileW, ow = ow0 + pix % kTileW;
-            if (oh < p.Ho && ow < p.Wo) {
-                float4 o = acc[r][g];
-                if (act != SPX_ACT_NONE) {
-                    o.x = spx::apply_act(o.x, act); o.y = spx::apply_act(o.y, act);
-                    o.z = spx::apply_act(o.z, act); o.w = spx::apply_act(o.w, act);
-                }
-                *reinterpret_cast<float4*>(out + (((size_t)mo * p.Ho + oh) * p.Wo + ow) * p.B + b0 + quad * 4) = o;
-            }
+            if (oh < p.Ho && ow < p.Wo) store_quad(out, tp.v, mo, oh, ow, b0 + quad * 4, acc[r][g], act);
         }
     }
 }
@@ -701,6 +762,19 @@ static int transpose2d(const float* src, uint64_t rows, uint64_t cols, float* ds
     return SPX_OK;
 }
 
+// Shared memory for the staged patch of a CTA with nb warps: 16 warps share an SM.
+static size_t rbm_budget(int nb) { return nb == 16 ? 200 * 1024 : (size_t)nb * 13 * 1024; }
+
+// Whether one channel of the receptive field of a tile (qb batch quads, g groups per lane) fits that.
+static bool rbm_fits(const ConvParams& p, uint32_t qb, int nb, int g)
+{
+    const uint32_t TH = 32u * g / qb / kTileW;
+    if (TH == 0) return false;
+    const size_t THin = (size_t)(TH - 1) * p.sH + (size_t)(p.kH - 1) * p.dH + 1;
+    const size_t TWin = (size_t)(kTileW - 1) * p.sW + (size_t)(p.kW - 1) * p.dW + 1;
+    return THin * TWin * qb * 4 * sizeof(float) <= rbm_budget(nb) / (nb == 16 ? 1 : 2);
+}
+
 // Builds (once per handle and kernel shape) the row-block-merged weights.
 static int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s)
 {
@@ -735,21 +809,21 @@ static int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s)
     return SPX_OK;
 }
 
-template <int QB, int G>
+template <int QB, int NB, int G>
 static int launch_rbm_units(const spx_ell* e, TileParams tp, RbmUnits un, uint32_t ctas, const float* in, const float* bias,
                             int act, float* out, cudaStream_t s, uint32_t b_avail)
 {
-    constexpr int NB = 16;
     const ConvParams& p = tp.c;
     constexpr uint32_t TH = 32u * G / QB / kTileW;
     tp.BT = QB * 4;
     tp.THin = (TH - 1) * p.sH + (p.kH - 1) * p.dH + 1;
     tp.TWin = (kTileW - 1) * p.sW + (p.kW - 1) * p.dW + 1;
     const size_t chanBytes = (size_t)tp.THin * tp.TWin * tp.BT * sizeof(float);
-    const size_t budget = 200 * 1024;
+    const size_t budget = rbm_budget(NB);
     tp.CC = (uint32_t)std::min<size_t>(p.Cin, budget / chanBytes);
     // The chunk's patch as one bulk tensor copy (TMA) where a map of the input tensor can be made:
-    // dimensions, innermost first, [B][W][H][Cin]; box [BT][TWin][THin][CC] (each extent at most
+    // dimensions, innermost first, [B][W][H][Cin] with the strides of the layout at hand; box
+    // [BT][TWin][THin][CC] (each extent at most
     // 256); positions outside the tensor read as zero, which is the halo.  The innermost
     // coordinate of every copy is a multiple of BT floats, i.e. of 16 bytes, as the copy unit
     // requires.  SPX_CONV_TMA=0 keeps the per-thread cp.async staging.
@@ -759,11 +833,11 @@ static int launch_rbm_units(const spx_ell* e, TileParams tp, RbmUnits un, uint32
     uint32_t use_tma = 0;
     const PFN_cuTensorMapEncodeTiled encode = tensor_map_encoder();
     if (tma_env && !e->tma_off && encode && e->tma_failed_dev && e->tma_failed_mapped && tp.TWin <= 256 && tp.THin <= 256 &&
-        p.B % 4 == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0) {
+        (p.Cin == 1 || 2 * chanBytes <= budget)) {
         // two buffers: half the channels of the single-buffer chunk each
         const uint32_t cc = std::min<uint32_t>(std::max<uint32_t>(1u, (uint32_t)(budget / 2 / chanBytes)), std::min<uint32_t>(p.Cin, 256));
         const cuuint64_t gdim[4] = {b_avail, p.W, p.H, p.Cin};    // `in` may point into the batch row (a segment)
-        const cuuint64_t gstr[3] = {(cuuint64_t)p.B * 4, (cuuint64_t)p.W * p.B * 4, (cuuint64_t)p.H * p.W * p.B * 4};
+        const cuuint64_t gstr[3] = {tp.v.iW * 4, tp.v.iH * 4, tp.v.iC * 4};
         const cuuint32_t box[4] = {tp.BT, tp.TWin, tp.THin, cc};
         const cuuint32_t estr[4] = {1, 1, 1, 1};
         if (encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(in), gdim, gstr, box, estr,
@@ -779,34 +853,86 @@ static int launch_rbm_units(const spx_ell* e, TileParams tp, RbmUnits un, uint32
     auto kfn = conv_rbm_tile_kernel<QB, NB, G>;
     cudaError_t err = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return fail(SPX_ERR_CUDA, "conv2d: shared memory opt-in failed: %s", cudaGetErrorString(err));
-    kfn<<<ctas, NB * 32, smem, s>>>(e->rbm_hdr, reinterpret_cast<const float4*>(e->rbm_w), e->rbm_ncols, e->rbm_cap,
-                                    tp, un, in, bias, act, out, map, use_tma, e->tma_failed_dev, e->tma_failed_mapped);
-    SPX_LAUNCH_CHECK("conv_rbm_tile_kernel");
+    err = launch_pdl(kfn, dim3(ctas), dim3(NB * 32), smem, s, e->rbm_hdr, reinterpret_cast<const float4*>(e->rbm_w), e->rbm_ncols,
+                     e->rbm_cap, tp, un, in, bias, act, out, map, use_tma, e->tma_failed_dev, e->tma_failed_mapped);
+    if (err != cudaSuccess) return fail(SPX_ERR_CUDA, "launch of conv_rbm_tile_kernel failed: %s", cudaGetErrorString(err));
+    count_launch();
     return SPX_OK;
+}
+
+// How a launch is cut: NB row blocks (warps) per CTA and G float4 groups per lane.  16 x 4 does the least
+// work per output (one staging per 64 channels, operands shared by most positions), but a small problem
+// then leaves most SMs empty, and with few warps on an SM a column costs its latency, not its instructions.
+// Estimate in cycles per cut: waves of CTAs x (union columns x the larger of a column's latency and what all
+// warps on the SM need for it -- shared-memory wavefronts, doubled by the bank conflicts of an even stride, or
+// instructions -- but at least the staging; plus the ends of the CTA and of each chunk).  The constants are
+// fitted to 16 shapes x 5 cuts (1 x 1 to 5 x 5, 7 x 7 to 74 x 74, batch 1 to 32): within 4 % of the best cut
+// for 14 of them.  256 -> 256 channels, 14 x 14, batch 4, 10 %: 150 us as 16 x 4, 35 us as 4 x 1.
+struct RbmCut {
+    int nb, g;
+};
+static RbmCut rbm_cut(const spx_ell* e, const ConvParams& p, uint32_t qb, uint32_t b_len)
+{
+    struct Option { RbmCut cut; double latency, per_warp; };
+    static const Option options[] = {{{16, 4}, 250, 22}, {{8, 4}, 250, 22}, {{8, 2}, 90, 11.4}, {{4, 2}, 90, 11.4}, {{4, 1}, 70, 7.4}};
+    const double sms = sm_count(e->device), d = (double)e->nnz_total / ((double)e->m * e->n);
+    const double un = 1.0 - std::pow(1.0 - std::min(d, 1.0), (double)kRbmRows);
+    const double share = kRbmRows * d / un, cols = un * e->n;
+    const uint32_t nblocks = (p.Cout + kRbmRows - 1) / kRbmRows;
+    const double conflicts = p.sW % 2 ? 1.0 : 2.0;
+    RbmCut best{0, 0};
+    double best_t = 1e300;
+    for (const Option& o : options) {
+        const int nb = o.cut.nb, g = o.cut.g;
+        if (!rbm_fits(p, qb, nb, g)) continue;
+        const uint32_t TH = 32u * g / qb / kTileW;
+        const double tiles = (double)((p.Wo + kTileW - 1) / kTileW) * ((p.Ho + TH - 1) / TH);
+        const double units = tiles * ((nblocks + nb - 1) / nb) * (b_len / (qb * 4)), per_sm = 16.0 / nb;
+        const double resident = std::min(per_sm, std::ceil(units / sms));       // CTAs on the busiest SM
+        const double warps = resident * std::min<double>(nb, nblocks);
+        // a partly filled last wave of the large cut is split up (see launch_rbm_qb)
+        double waves = units / (sms * per_sm);
+        waves = waves <= 1.0 ? 1.0 : nb == 16 ? waves + 0.1 : std::ceil(waves);
+        const double patch = (double)((TH - 1) * p.sH + (p.kH - 1) * p.dH + 1) * ((kTileW - 1) * p.sW + (p.kW - 1) * p.dW + 1) * qb * 16.0;
+        const double chunks = std::ceil(p.Cin / std::max(1.0, std::floor(rbm_budget(nb) / 2 / patch)));
+        // (tiles of 8 entries: a column of the small cuts measured twice as long, at any number of warps)
+        const double latency = qb == 2 && g < kRbmG ? (g == 2 ? 205.0 : 115.0) : o.latency;
+        const double col = std::max(latency, warps * std::max(4.6 * g * conflicts + 2, o.per_warp * (0.6 + 0.3 * share)));
+        const double t = waves * (std::max(cols * col, resident * p.Cin * patch / 64) + 2500 + 500 * chunks);
+        if (t < best_t) { best_t = t; best = o.cut; }
+    }
+    return best;
 }
 
 template <int QB>
 static int launch_rbm_qb(spx_ell* e, TileParams tp, const float* in, const float* bias, int act, float* out,
                          cudaStream_t s, uint32_t b_base, uint32_t b_len)
 {
-    // a batch segment [b_base, b_base + b_len): the batch is the innermost dimension of both tensors,
-    // so the segment is the same kernel on pointers moved by b_base entries
+    // a batch segment [b_base, b_base + b_len): the batch is the innermost dimension of the input, so the
+    // segment is the same kernel on pointers moved by b_base entries
     in += b_base;
-    out += b_base;
+    out += b_base * tp.v.oB;
+    tp.v.b_out = tp.v.b_out > b_base ? tp.v.b_out - b_base : 0u;
     const uint32_t b_avail = tp.c.B - b_base;       // batch entries from the moved pointer to the end of a row
-    constexpr int NB = 16;
     const ConvParams& p = tp.c;
-    constexpr uint32_t TH = 32u * kRbmG / QB / kTileW;
-    const uint32_t THin = (TH - 1) * p.sH + (p.kH - 1) * p.dH + 1, TWin = (kTileW - 1) * p.sW + (p.kW - 1) * p.dW + 1;
-    if ((size_t)THin * TWin * QB * 4 * sizeof(float) > 200 * 1024) return -1;
+    static const int cut_env = [] { const char* v = getenv("SPX_CONV_CUT"); return v ? atoi(v) : 0; }();      // 10 NB + G, for tests
+    RbmCut cut = rbm_cut(e, p, QB, b_len);
+    if (cut_env && rbm_fits(p, QB, cut_env / 10, cut_env % 10) && 32u * (cut_env % 10) / QB / kTileW) cut = RbmCut{cut_env / 10, cut_env % 10};
+    if (!cut.nb) return -1;
+    const uint32_t TH = 32u * cut.g / QB / kTileW;
     tp.tilesX = (p.Wo + kTileW - 1) / kTileW;
     const uint64_t tiles = (uint64_t)tp.tilesX * ((p.Ho + TH - 1) / TH);
     const uint32_t nblocks = (p.Cout + kRbmRows - 1) / kRbmRows;
-    const uint32_t groups = (nblocks + NB - 1) / NB;
+    const uint32_t groups = (nblocks + cut.nb - 1) / cut.nb;
     const uint64_t units = tiles * groups * (b_len / (QB * 4));
     if (units > 0x3fffffffull) return -1;
     const int rc = ensure_rbm(e, p.kH, p.kW, s);
     if (rc != SPX_OK) return rc;                        // -1: no memory for the merged weights
+    RbmUnits un{0u, (uint32_t)tiles, groups, 0u};
+    if (cut.nb == 8 && cut.g == 4) return launch_rbm_units<QB, 8, 4>(e, tp, un, (uint32_t)units, in, bias, act, out, s, b_avail);
+    if (cut.nb == 8) return launch_rbm_units<QB, 8, 2>(e, tp, un, (uint32_t)units, in, bias, act, out, s, b_avail);
+    if (cut.nb == 4 && cut.g == 2) return launch_rbm_units<QB, 4, 2>(e, tp, un, (uint32_t)units, in, bias, act, out, s, b_avail);
+    if (cut.nb == 4) return launch_rbm_units<QB, 4, 1>(e, tp, un, (uint32_t)units, in, bias, act, out, s, b_avail);
     // One CTA per SM, all units equally long: the launch runs in waves of sm_count units.  A last
     // wave that fills less than half of the SMs is issued as a second launch of half-height tiles
     // (twice the CTAs, each about 0.6 of a full unit's time): 784 units on 148 SMs are 5 full waves
@@ -814,14 +940,14 @@ static int launch_rbm_qb(spx_ell* e, TileParams tp, const float* in, const float
     static const int split_tail = [] { const char* v = getenv("SPX_CONV_RBM_SPLIT_TAIL"); return v ? atoi(v) : 1; }();
     const uint32_t sms = (uint32_t)sm_count(e->device);
     const uint32_t rem = (uint32_t)(units % sms);
-    RbmUnits un{0u, (uint32_t)tiles, groups};
     if (split_tail && units > sms && rem && rem * 2 <= sms) {
-        const int rc1 = launch_rbm_units<QB, kRbmG>(e, tp, un, (uint32_t)(units - rem), in, bias, act, out, s, b_avail);
+        const int rc1 = launch_rbm_units<QB, 16, kRbmG>(e, tp, un, (uint32_t)(units - rem), in, bias, act, out, s, b_avail);
         if (rc1 != SPX_OK) return rc1;
         un.unit0 = (uint32_t)(units - rem);
-        return launch_rbm_units<QB, kRbmG / 2>(e, tp, un, rem * 2, in, bias, act, out, s, b_avail);
+        un.half = 1;
+        return launch_rbm_units<QB, 16, kRbmG / 2>(e, tp, un, rem * 2, in, bias, act, out, s, b_avail);
     }
-    return launch_rbm_units<QB, kRbmG>(e, tp, un, (uint32_t)units, in, bias, act, out, s, b_avail);
+    return launch_rbm_units<QB, 16, kRbmG>(e, tp, un, (uint32_t)units, in, bias, act, out, s, b_avail);
 }
 
 // Row-block-merged path.  Taken whenever K fits the builder's set and the batch is a multiple of 4:
@@ -838,7 +964,7 @@ static int launch_rbm_qb(spx_ell* e, TileParams tp, const float* in, const float
 // output channels per staged chunk instead of 16 or 32.  SPX_CONV_RBM=0 turns the path off;
 // SPX_CONV_RBM_MIN_SHARE=x requires an expected 4 d / (1 - (1 - d)^4) >= x rows per union column
 // (density d).  Returns -1 when not taken.
-static int launch_conv_rbm_tile(spx_ell* e, const ConvParams& p, uint32_t BT, const float* in, const float* bias,
+static int launch_conv_rbm_tile(spx_ell* e, const ConvParams& p, const ConvViews& v, const float* in, const float* bias,
                                 int act, float* out, cudaStream_t s)
 {
     static const int enabled = [] { const char* v = getenv("SPX_CONV_RBM"); return v ? atoi(v) : 1; }();
@@ -846,7 +972,6 @@ static int launch_conv_rbm_tile(spx_ell* e, const ConvParams& p, uint32_t BT, co
     if (int rc = check_tma_words(e, "conv2d")) return rc;     // the handle stages with per-thread copies from then on
     // fewer than 8 row blocks would leave most of the CTA's 16 warps without work
     if (!enabled || e->n > kRbmMaxK || e->m < 8 * kRbmRows - 3 || e->max_nnz == 0) return -1;
-    (void)BT;
     if (p.B % 4) return -1;
     const double d = (double)e->nnz_total / ((double)e->m * e->n);
     const double share = d >= 1.0 ? (double)kRbmRows : kRbmRows * d / (1.0 - std::pow(1.0 - d, (double)kRbmRows));
@@ -860,15 +985,11 @@ static int launch_conv_rbm_tile(spx_ell* e, const ConvParams& p, uint32_t BT, co
     if (!segments && n16 && rest) return -1;
     if (!segments && !n16 && rest == 12) return -1;
     // every segment's staged patch must fit shared memory (checked before any launch)
-    const auto fits = [&](uint32_t qb) {
-        const uint32_t TH = 32u * kRbmG / qb / kTileW;
-        const size_t THin = (size_t)(TH - 1) * p.sH + (size_t)(p.kH - 1) * p.dH + 1;
-        const size_t TWin = (size_t)(kTileW - 1) * p.sW + (size_t)(p.kW - 1) * p.dW + 1;
-        return THin * TWin * qb * 4 * sizeof(float) <= 200 * 1024;
-    };
+    const auto fits = [&](uint32_t qb) { return rbm_fits(p, qb, 16, kRbmG); };
     if ((n16 && !fits(4)) || (rest >= 8 && !fits(2)) || (rest % 8 == 4 && !fits(1))) return -1;
     TileParams tp{};
     tp.c = p;
+    tp.v = v;
     uint32_t at = 0;
     if (n16) {
         const int rc = launch_rbm_qb<4>(e, tp, in, bias, act, out, s, 0, n16);
@@ -888,17 +1009,16 @@ static int launch_conv_rbm_tile(spx_ell* e, const ConvParams& p, uint32_t BT, co
 }
 
 // Returns -1 when the shape is not covered (caller falls back to the direct kernel).
-static int launch_conv_pf_tile(spx_ell* e, const ConvParams& p, const float* in, const float* bias, int act,
+static int launch_conv_pf_tile(spx_ell* e, const ConvParams& p, const ConvViews& v, const float* in, const float* bias, int act,
                                float* out, cudaStream_t s)
 {
     if (!e->cols_ascending || !pf_tile_covers(p)) return -1;
-    if ((reinterpret_cast<uintptr_t>(in) & 15) || (reinterpret_cast<uintptr_t>(out) & 15)) return -1;
     // batch entries per CTA: the largest multiple of 4 that divides B and is <= 32
     uint32_t BT = 0;
     for (uint32_t c = 32; c >= 4; c -= 4) if (p.B % c == 0) { BT = c; break; }
     if (!BT) return -1;
     {
-        const int rc = launch_conv_rbm_tile(e, p, BT, in, bias, act, out, s);
+        const int rc = launch_conv_rbm_tile(e, p, v, in, bias, act, out, s);
         if (rc != -1) return rc;
     }
     static const int ctas = [] { const char* v = getenv("SPX_CONV_CTAS"); return v ? atoi(v) : 0; }();
@@ -920,6 +1040,7 @@ static int launch_conv_pf_tile(spx_ell* e, const ConvParams& p, const float* in,
     const uint32_t warps = small ? 32 : kTileWarps;
     TileParams tp{};
     tp.c = p;
+    tp.v = v;
     tp.BT = BT;
     tp.THin = (TH - 1) * p.sH + (p.kH - 1) * p.dH + 1;
     tp.TWin = (kTileW - 1) * p.sW + (p.kW - 1) * p.dW + 1;
@@ -989,88 +1110,56 @@ int launch_conv2d(spx_ell* e, const spx_conv_geom* g, int layout, const float* i
     if (rc != SPX_OK) return rc;
     ConvParams p{g->Cin, g->Cout, g->kH, g->kW, g->sH, g->sW, g->pH, g->pW, g->dH, g->dW,
                  g->H, g->W, g->Ho, g->Wo, B};
-    // The tiled kernels want [C,H,W,B] with B a multiple of 4.  Other inputs are brought into that
-    // form in per-handle scratch and the result is converted back:
-    //   NCHW (B > 1; one NCHW image already is [C,H,W,1]): transpose in, transpose out - two extra
-    //     streaming passes over input and output (about 5 % of the kernel's time at 256 channels);
-    //   B not a multiple of 4 (or cheaper at the next multiple of 16, see padded_batch): the batch
-    //     dimension is widened with zero entries and narrowed again
-    //     (256 -> 256 channels, 56 x 56: batch 3 takes 0.4 ms this way against 1.2 ms with the general
-    //     kernel, batch 1 0.4 against 0.43 ms).
-    // Arithmetic per output element is unchanged in both cases.
+    // The tiled kernels read the batch as the innermost dimension, in multiples of 4 and of 16 bytes, and
+    // store through any strides.  So [C,H,W,B] and F-major [W,H,C,B] tensors with B a multiple of 4 go in as
+    // they are; others take one pass into [C,H,W,B4] scratch of the handle, zeros in the added batch entries
+    // (B4: padded_batch).  No pass follows the kernel: it stores the entries that exist where they belong.
+    // 256 -> 256 channels, 56 x 56, batch 3: 0.4 ms this way against 1.2 ms with the general kernel.
+    // Arithmetic per output element is the same in all cases.
     const uint32_t B4 = padded_batch(B, merged_kernel_takes(e));
     ConvParams p4 = p;
     p4.B = B4;
-    // F-major tensors, b + B*(c + C*(h + H*w)): [W,H,C,B] is [C,H,W,B] with the three outer
-    // dimensions reversed, so the tiled kernels are reached through two more streaming passes
-    // (reverse in, reverse out) in scratch of their own; shapes the tiled kernels do not cover
-    // gather straight from the F-major tensor in the general kernel below.
-    if (layout == SPX_LAYOUT_FMAJOR && e->r && e->cols_ascending && pf_tile_covers(p4)) {
-        const uint64_t n_in = (uint64_t)g->Cin * g->H * g->W * B, n_out = (uint64_t)g->Cout * g->Ho * g->Wo * B;
-        const uint64_t in_slab = (n_in + 63) / 64 * 64;
-        const size_t need = (size_t)(in_slab + n_out) * sizeof(float);
-        if (e->fm_scratch_bytes < need) {
-            if (int rs = grow_scratch(e, &e->fm_scratch, &e->fm_scratch_bytes, need)) return rs;
-        }
-        float* in_pf = static_cast<float*>(e->fm_scratch);
-        float* out_pf = in_pf + in_slab;
-        auto reverse3 = [&](const float* src, uint32_t D0, uint32_t D1, uint32_t D2, float* dst, uint64_t total) {
-            const unsigned blocks = (unsigned)std::min<uint64_t>((total + 255) / 256, (uint64_t)sm_count(e->device) * 32);
-            reverse3_kernel<<<blocks, 256, 0, s>>>(src, D0, D1, D2, B, dst);
-            SPX_LAUNCH_CHECK("reverse3_kernel");
-            return SPX_OK;
-        };
-        rc = reverse3(in, g->W, g->H, g->Cin, in_pf, n_in);                   // [W,H,C,B] -> [C,H,W,B]
-        if (rc != SPX_OK) return rc;
-        rc = launch_conv2d(e, g, SPX_LAYOUT_PF, in_pf, B, bias, act, out_pf, s);
-        if (rc != SPX_OK) return rc;
-        return reverse3(out_pf, g->Cout, g->Ho, g->Wo, out, n_out);           // [C,Ho,Wo,B] -> [Wo,Ho,C,B]
-    }
-    if (layout != SPX_LAYOUT_FMAJOR && e->r && e->cols_ascending && pf_tile_covers(p4)) {
-        const bool nchw = layout == SPX_LAYOUT_NCHW && B > 1;
-        const bool pad = B4 != B;
-        if (!nchw && !pad) {
-            rc = launch_conv_pf_tile(e, p, in, bias, act, out, s);
-            if (rc != -1) return rc;             // -1: shape not covered by the tiled kernels
+    if (e->r && e->cols_ascending && pf_tile_covers(p4)) {
+        const uint64_t H = g->H, W = g->W, Ho = g->Ho, Wo = g->Wo;
+        ConvViews v{};
+        v.b_out = B;
+        uint64_t iB = 1;
+        if (layout == SPX_LAYOUT_PF) {
+            v.iC = H * W * B; v.iH = W * B; v.iW = B;
+            v.oB = 1; v.oC = Ho * Wo * B; v.oH = Wo * B; v.oW = B;
+        } else if (layout == SPX_LAYOUT_FMAJOR) {
+            v.iC = B; v.iH = (uint64_t)g->Cin * B; v.iW = H * g->Cin * B;
+            v.oB = 1; v.oC = B; v.oH = (uint64_t)g->Cout * B; v.oW = Ho * g->Cout * B;
         } else {
-            const uint64_t in_rows = (uint64_t)g->Cin * g->H * g->W, out_rows = (uint64_t)g->Cout * g->Ho * g->Wo;
-            auto slab = [](uint64_t floats) { return (floats + 63) / 64 * 64; };
-            const uint64_t n_in4 = slab(in_rows * B4), n_out4 = slab(out_rows * B4);
-            const uint64_t n_in = (nchw && pad) ? slab(in_rows * B) : 0, n_out = (nchw && pad) ? slab(out_rows * B) : 0;
-            const size_t need = (size_t)(n_in4 + n_out4 + n_in + n_out) * sizeof(float);
-            if (e->conv_scratch_bytes < need) {
-                if (int rs = grow_scratch(e, &e->conv_scratch, &e->conv_scratch_bytes, need)) return rs;
-            }
-            float* in4 = static_cast<float*>(e->conv_scratch);
-            float* out4 = in4 + n_in4;
-            float* in_t = out4 + n_out4;          // [C,H,W,B] before widening (NCHW and widening only)
-            float* out_t = in_t + n_in;
-            auto repitch = [&](const float* src, uint32_t sp, uint32_t sc, float* dst, uint32_t dp, uint32_t dc, uint64_t rows) {
-                const uint64_t total = rows * dc;
-                const unsigned blocks = (unsigned)std::min<uint64_t>((total + 255) / 256, (uint64_t)sm_count(e->device) * 32);
-                repitch_kernel<<<blocks, 256, 0, s>>>(src, sp, sc, dst, dp, dc, rows);
-                SPX_LAUNCH_CHECK("repitch_kernel");
-                return SPX_OK;
-            };
-            const float* src_pf = in;
-            if (nchw) {
-                rc = transpose2d(in, B, in_rows, pad ? in_t : in4, s);
-                if (rc != SPX_OK) return rc;
-                src_pf = in_t;
-            }
-            if (pad) {
-                rc = repitch(src_pf, B, B, in4, B4, B4, in_rows);
-                if (rc != SPX_OK) return rc;
-            }
-            rc = launch_conv_pf_tile(e, p4, in4, bias, act, out4, s);
-            if (rc == SPX_OK) {
-                if (!pad) return transpose2d(out4, out_rows, B, out, s);
-                rc = repitch(out4, B4, B, nchw ? out_t : out, B, B, out_rows);
-                if (rc != SPX_OK || !nchw) return rc;
-                return transpose2d(out_t, out_rows, B, out, s);
-            }
-            if (rc != -1) return rc;
+            iB = g->Cin * H * W; v.iC = H * W; v.iH = W; v.iW = 1;
+            v.oB = g->Cout * Ho * Wo; v.oC = Ho * Wo; v.oH = Wo; v.oW = 1;
         }
+        v.vec_out = v.oB == 1 && B4 == B && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+        const float* src = in;
+        if (iB != 1 || B4 != B || (reinterpret_cast<uintptr_t>(in) & 15)) {
+            const uint64_t positions = g->Cin * H * W;
+            const size_t need = positions * B4 * sizeof(float);
+            if (e->conv_scratch_bytes < need)
+                if (int rs = grow_scratch(e, &e->conv_scratch, &e->conv_scratch_bytes, need)) return rs;
+            float* dst = static_cast<float*>(e->conv_scratch);
+            if (iB != 1 && B >= 16 && B4 == B) {        // wide transpose through shared memory: both sides in whole lines
+                if (int rt = transpose2d(in, B, positions, dst, s)) return rt;
+            } else {
+                const uint64_t threads = positions * (B4 / 4);
+                const unsigned blocks = (unsigned)std::min<uint64_t>((threads + 255) / 256, (uint64_t)sm_count(e->device) * 32);
+                const bool wide = threads >= (1ull << 32);
+                auto kfn = iB != 1 ? (wide ? to_pf_kernel<true, uint64_t> : to_pf_kernel<true, uint32_t>)
+                                   : (wide ? to_pf_kernel<false, uint64_t> : to_pf_kernel<false, uint32_t>);
+                const cudaError_t err = launch_pdl(kfn, dim3(blocks), dim3(256), 0, s, in, iB, v.iC, v.iH, v.iW, g->H, g->W, positions, B,
+                                                   B4 / 4, dst);
+                if (err != cudaSuccess) return fail(SPX_ERR_CUDA, "launch of to_pf_kernel failed: %s", cudaGetErrorString(err));
+                count_launch();
+            }
+            v.iC = H * W * B4; v.iH = W * B4; v.iW = B4;
+            src = dst;
+        }
+        rc = launch_conv_pf_tile(e, p4, v, src, bias, act, out, s);
+        if (rc != -1) return rc;                 // -1: shape not covered by the tiled kernels
     }
     const uint64_t per_m = (uint64_t)g->Ho * g->Wo * B;
     const uint64_t gx = (per_m + 255) / 256;

@@ -539,6 +539,48 @@ def test_conv_unsorted_columns(lib, orc, cuda, layout):
     assert_bit_equal(dY.cpu().numpy(), want, "conv, unsorted columns")
 
 
+@pytest.mark.parametrize("cut", ["84", "82", "42", "41", "164"])
+def test_conv_each_cut_forced(cut):
+    """Every way of cutting the merged kernel's work, on the convolution cases that run it (a child process:
+    the choice is read once)."""
+    import os
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    cmd = [sys.executable, "-m", "pytest", "-q", "-x", "-m", "gpu", "-p", "no:cacheprovider",
+           os.path.join(here, "test_parity_gpu.py"), "-k", "test_conv_bit_exact_vs_oracle or conv_views"]
+    r = subprocess.run(cmd, env={**os.environ, "SPX_CONV_CUT": cut}, capture_output=True, text=True, timeout=900)
+    assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("layout", [sx.LAYOUT_PF, sx.LAYOUT_NCHW, sx.LAYOUT_FMAJOR])
+@pytest.mark.parametrize("B,Cin,Cout,H,W,k,s,pad", [(1, 3, 40, 9, 13, 3, 1, 1), (7, 5, 33, 8, 17, 3, 2, 1), (16, 9, 64, 7, 7, 1, 1, 0),
+                                                    (21, 4, 32, 5, 31, 5, 1, 2), (32, 3, 36, 6, 9, 3, 4, 1)])
+def test_conv_views_leave_neighbours_alone(lib, orc, cuda, layout, B, Cin, Cout, H, W, k, s, pad):
+    """Tensors that start 4 bytes off a 16-byte boundary, batches of every remainder: results in place, the
+    memory around the output untouched."""
+    rng = np.random.default_rng([B, Cin, Cout, H, W, layout])
+    wt = sparse(rng, Cout, Cin * k * k, 0.3)
+    E = orc.encode(wt)
+    h = gpu_ell(lib, E)
+    g = sx.conv_geom(Cin, Cout, k, k, H, W, sH=s, sW=s, pH=pad, pW=pad)
+    bias = rng.standard_normal(Cout).astype(np.float32)
+    src = as_layout(rng.standard_normal((B, Cin, H, W)).astype(np.float32), layout)
+    n_out = B * Cout * g.Ho * g.Wo
+    dX = torch.empty(src.size + 1, device=cuda, dtype=torch.float32)
+    dX[1:] = dev(src, cuda).reshape(-1)
+    dB = dev(bias, cuda)
+    gd = dict(Cin=Cin, kH=k, kW=k, sH=s, sW=s, pH=pad, pW=pad, dH=1, dW=1, H=H, W=W)
+    want = orc.conv2d(E, gd, layout, src, B, bias, 1).reshape(-1)
+    for shift in (0, 1):
+        out = torch.full((n_out + 6,), 7.0, device=cuda, dtype=torch.float32)
+        h.conv2d(g, layout, dX.data_ptr() + 4, B, dB.data_ptr(), sx.ACT_RELU, out.data_ptr() + 4 * shift)
+        torch.cuda.synchronize()
+        got = out.cpu().numpy()
+        assert_bit_equal(got[shift:shift + n_out], want, f"shift {shift}")
+        assert (got[:shift] == 7.0).all() and (got[shift + n_out:] == 7.0).all()
+
+
 @pytest.mark.parametrize("env", [{"SPX_CONV_RBM": "0"}, {"SPX_CONV_RBM_MIN_SHARE": "0"},
                                  {"SPX_CONV_RBM_MIN_SHARE": "0", "SPX_CONV_TMA": "0"}, {"SPX_CONV_DIRECT": "1"}],
                          ids=["per-row-tiles", "row-block-merged", "row-block-merged-cp-async", "direct"])
