@@ -21,9 +21,9 @@ namespace spx {
 namespace {
 
 constexpr uint64_t kPoolKeep = 2ull << 30;          // of about 180 GB
-// A block that would take a large part of that is mapped and unmapped directly: the pool would not
-// keep it, and growing it by such a block took twice as long as cudaMalloc (slabs of 2 x 0.9 GB).
-constexpr size_t kPoolBlock = kPoolKeep / 4;
+// Larger blocks are mapped and unmapped directly: growing the pool by them takes longer than cudaMalloc
+// (slabs of 2 x 323 MB: 9 ms against 5), and a few of them are all the pool would keep.
+constexpr size_t kPoolBlock = 128u << 20;
 constexpr size_t kPinnedKeep = 64u << 20;
 constexpr int kMaxDevices = 64;
 
