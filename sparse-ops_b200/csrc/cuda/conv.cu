@@ -1106,6 +1106,21 @@ int launch_conv2d(spx_ell* e, const spx_conv_geom* g, int layout, const float* i
     if (e->m == 0 || B == 0 || g->Ho == 0 || g->Wo == 0) return SPX_OK;
     if (g->kH > 255 || g->kW > 255 || g->Cin > 65535)
         return fail(SPX_ERR_LIMIT, "conv2d: kernel extent > 255 or Cin > 65535 not supported");
+    // A 1 x 1 convolution is an SpMM whose columns are the positions (times the batch where that is the innermost
+    // dimension): no halo, no batch to fill up, the same chain per output.  331 -> 128 channels, 74 x 74, batch 30:
+    // 323 -> 199 us; 283 -> 32, 32 x 32, batch 1: 27 -> 6 us.  NCHW images are a product each, which pays up to a few
+    // of them (16 images of 56 x 56: 95 us against 73).
+    static const int pointwise = [] { const char* v = getenv("SPX_CONV_POINTWISE"); return v ? atoi(v) : 1; }();
+    if (pointwise && g->kH == 1 && g->kW == 1 && g->sH == 1 && g->sW == 1 && g->pH == 0 && g->pW == 0) {
+        const uint64_t hw = (uint64_t)g->H * g->W;
+        if ((layout == SPX_LAYOUT_PF || B == 1) && layout != SPX_LAYOUT_FMAJOR && hw * B < (1ull << 30))
+            return launch_spmm(e, in, (uint32_t)(hw * B), hw * B, bias, act, out, hw * B, s);
+        if (layout == SPX_LAYOUT_NCHW && B <= 3 && hw < (1ull << 30)) {
+            for (uint32_t b = 0; b < B; ++b)
+                if (int rs = launch_spmm(e, in + b * g->Cin * hw, (uint32_t)hw, hw, bias, act, out + b * g->Cout * hw, hw, s)) return rs;
+            return SPX_OK;
+        }
+    }
     int rc = ensure_taps(e, g->kH, g->kW, s);
     if (rc != SPX_OK) return rc;
     ConvParams p{g->Cin, g->Cout, g->kH, g->kW, g->sH, g->sW, g->pH, g->pW, g->dH, g->dW,

@@ -475,7 +475,7 @@ int launch_spmm_tile(spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const
     static const int env = [] { const char* v = getenv("SPX_SPMM_TILE"); return v ? atoi(v) : 1; }();
     if (!env || !e->tiles || !e->cols_ascending || e->tma_off || e->max_nnz == 0) return -1;
     const PFN_cuTensorMapEncodeTiled encode = tensor_map_encoder();
-    if (!encode || ldx > 0xffffffffull || e->n > 65536 || C > 65536) return -1;
+    if (!encode || ldx > 0xffffffffull || e->n > 65536 || C > (1u << 30)) return -1;
     const uint32_t NV = C <= 32 ? 1 : 2;
     const Plan p = plan_tiles(e, C, NV, sm_count(e->device));
     if ((uint64_t)p.slices * e->m > 0x7fffffffull) return -1;

@@ -9,8 +9,9 @@
 // summation order differs from the reference's 16-partial-sum order, so results agree within
 // the stated tolerance 1e-5 * sum|w||x|, not bit for bit.  Padding slots are never multiplied.
 //
-// The kernel is HBM-bound: 8 bytes per nonzero streamed once.  The grid is persistent
-// (a multiple of the SM count) so x is staged once per CTA.
+// HBM-bound: 8 bytes per nonzero streamed once.  All kernels are launched as programmatic dependents:
+// what belongs to the handle (schedule, first slab vectors) is asked for while the predecessor in the
+// stream drains, and only x, bias and y wait for it.
 #include "common.cuh"
 
 #include <algorithm>
@@ -27,23 +28,33 @@ __device__ __forceinline__ float group_sum(float v) {
     return v;
 }
 
-template <int LPR, bool SMEM>
-__global__ void __launch_bounds__(1024)
+// Asks for x[0 .. n) in shared memory, by all threads of the CTA, asynchronously: every thread's copies are
+// in flight together.  landed_x(): they have landed for the whole CTA.
+__device__ __forceinline__ void stage_x(float* xs, const float* __restrict__ x, uint32_t n)
+{
+    const uint32_t n4 = ((reinterpret_cast<uintptr_t>(x) & 15) == 0) ? (n >> 2) : 0;
+    const uint32_t to = (uint32_t)__cvta_generic_to_shared(xs);
+    for (uint32_t i = threadIdx.x; i < n4; i += blockDim.x)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 16 * i), "l"(x + 4 * (size_t)i) : "memory");
+    for (uint32_t i = (n4 << 2) + threadIdx.x; i < n; i += blockDim.x)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to + 4 * i), "l"(x + i) : "memory");
+}
+__device__ __forceinline__ void landed_x()
+{
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+}
+
+// x beyond the windowed kernel's reach, or columns that do not ascend: x gathered through L1 / L2.
+template <int LPR>
+__global__ void __launch_bounds__(512, 2)
 spmv_ell_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ idx,
                 const uint32_t* __restrict__ nnz, const uint2* __restrict__ rows,
                 uint32_t m, uint32_t n, uint32_t pitch,
                 const float* __restrict__ x, const float* __restrict__ bias, float* __restrict__ y)
 {
-    extern __shared__ __align__(16) float xs[];
-    if (SMEM) {
-        // n floats, 16-byte vectors where alignment allows
-        const uint32_t n4 = ((reinterpret_cast<uintptr_t>(x) & 15) == 0) ? (n >> 2) : 0;
-        for (uint32_t i = threadIdx.x; i < n4; i += blockDim.x)
-            reinterpret_cast<float4*>(xs)[i] = __ldg(reinterpret_cast<const float4*>(x) + i);
-        for (uint32_t i = (n4 << 2) + threadIdx.x; i < n; i += blockDim.x) xs[i] = __ldg(x + i);
-        __syncthreads();
-    }
-    const float* __restrict__ xsrc = SMEM ? xs : x;
+    spx::pdl_launch();
+    spx::pdl_wait();
 
     const uint32_t lane = threadIdx.x & (LPR - 1);
     const uint32_t groups_per_block = blockDim.x / LPR;
@@ -82,10 +93,10 @@ spmv_ell_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ idx,
 #pragma unroll
             for (int u = 0; u < UNR; ++u) {
                 const uint32_t ju = j + u * LPR * 4;
-                if (ju < nn) a0 = fmaf(wv[u].x, xsrc[kv[u].x], a0);
-                if (ju + 1 < nn) a1 = fmaf(wv[u].y, xsrc[kv[u].y], a1);
-                if (ju + 2 < nn) a2 = fmaf(wv[u].z, xsrc[kv[u].z], a2);
-                if (ju + 3 < nn) a3 = fmaf(wv[u].w, xsrc[kv[u].w], a3);
+                if (ju < nn) a0 = fmaf(wv[u].x, __ldg(x + kv[u].x), a0);
+                if (ju + 1 < nn) a1 = fmaf(wv[u].y, __ldg(x + kv[u].y), a1);
+                if (ju + 2 < nn) a2 = fmaf(wv[u].z, __ldg(x + kv[u].z), a2);
+                if (ju + 3 < nn) a3 = fmaf(wv[u].w, __ldg(x + kv[u].w), a3);
             }
         }
         float acc = (a0 + a1) + (a2 + a3);
@@ -94,16 +105,17 @@ spmv_ell_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ idx,
     }
 }
 
-// spmv_ell_small_kernel: matrices of a few thousand columns (x up to 32 KB).  They are
-// latency-bound: staging x, the row schedule, the row length and the slabs would be four memory
-// round trips in a row.  So this kernel is software-pipelined: a group asks
-// for its first row's id and length and for that row's first slab vectors BEFORE x is staged (none
-// of them depends on x), and while a row is summed the next row's id, length and first vectors
-// are already in flight.  rows may be null (rows of near-equal length): slot == row then, and
-// one dependent load goes away.
+// spmv_staged_kernel: x fits in shared memory (n <= 51200).  One CTA per SM.  Staging x, the row
+// schedule, the row length and the slabs would be four memory round trips in a row, so the kernel is
+// software-pipelined: a group asks for its first row's id and length and for that row's first slab vectors
+// BEFORE x is staged (none of them depends on x), and while a row is summed the next row's id, length and
+// first vectors are already in flight.  rows may be null (rows of near-equal length): slot == row then, and
+// one dependent load goes away.  Against a kernel that starts a row when the one before is done, for all
+// n (it was used up to 8192 columns): 16384 x 16384, 90 / 95 / 99 % sparse 39.0 / 22.7 / 7.5 -> 33.7 / 18.4 /
+// 4.5 us; 5000 x 40000, 95 %: 28 -> 15 us; 60000 x 50000, 97 %: 143 -> 133 us.
 template <int LPR>
 __global__ void __launch_bounds__(1024)
-spmv_ell_small_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ idx,
+spmv_staged_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ idx,
                 const uint32_t* __restrict__ nnz, const uint2* __restrict__ rows,
                 uint32_t m, uint32_t n, uint32_t pitch,
                 const float* __restrict__ x, const float* __restrict__ bias, float* __restrict__ y)
@@ -113,7 +125,8 @@ spmv_ell_small_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__
     constexpr uint32_t STEP = LPR * 4 * UNR;     // entries a group consumes per chunk
     const uint32_t lane = threadIdx.x & (LPR - 1);
     const uint32_t groups_per_block = blockDim.x / LPR;
-    const uint32_t group = blockIdx.x * groups_per_block + threadIdx.x / LPR;
+    // neighbouring slots go to different CTAs, so that a last, partly filled round is spread over all SMs
+    const uint32_t group = threadIdx.x / LPR * gridDim.x + blockIdx.x;
     const uint32_t stride = gridDim.x * groups_per_block;
     // All lanes of a warp run the same number of row iterations so that the shuffles below
     // always see the full warp.
@@ -144,17 +157,12 @@ spmv_ell_small_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__
     auto row_info = [&](uint32_t sl) { return rows ? __ldg(rows + sl) : make_uint2(sl, __ldg(nnz + sl)); };
     uint2 ri = live ? row_info(slot) : make_uint2(0u, 0u);
     uint32_t row = ri.x, nn = ri.y;
+    spx::pdl_launch();
     load_chunk(row, nn, lane * 4);
 
-    {
-        // n floats, 16-byte vectors where alignment allows
-        const uint32_t n4 = ((reinterpret_cast<uintptr_t>(x) & 15) == 0) ? (n >> 2) : 0;
-        for (uint32_t i = threadIdx.x; i < n4; i += blockDim.x)
-            reinterpret_cast<float4*>(xs)[i] = __ldg(reinterpret_cast<const float4*>(x) + i);
-        for (uint32_t i = (n4 << 2) + threadIdx.x; i < n; i += blockDim.x) xs[i] = __ldg(x + i);
-        __syncthreads();
-    }
-    const float* __restrict__ xsrc = xs;
+    spx::pdl_wait();                            // x, bias and y belong to the stream's order, the handle does not
+    stage_x(xs, x, n);
+    landed_x();
 
     for (uint32_t it = 0; it < iters; ++it) {
         // the next row's id and length travel while this row is summed
@@ -170,10 +178,10 @@ spmv_ell_small_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__
 #pragma unroll
             for (int u = 0; u < UNR; ++u) {
                 const uint32_t ju = j + u * LPR * 4;
-                if (ju < nn) a0 = fmaf(wv[u].x, xsrc[kv[u].x], a0);
-                if (ju + 1 < nn) a1 = fmaf(wv[u].y, xsrc[kv[u].y], a1);
-                if (ju + 2 < nn) a2 = fmaf(wv[u].z, xsrc[kv[u].z], a2);
-                if (ju + 3 < nn) a3 = fmaf(wv[u].w, xsrc[kv[u].w], a3);
+                if (ju < nn) a0 = fmaf(wv[u].x, xs[kv[u].x], a0);
+                if (ju + 1 < nn) a1 = fmaf(wv[u].y, xs[kv[u].y], a1);
+                if (ju + 2 < nn) a2 = fmaf(wv[u].z, xs[kv[u].z], a2);
+                if (ju + 3 < nn) a3 = fmaf(wv[u].w, xs[kv[u].w], a3);
             }
         }
         load_chunk(row_n, nn_n, lane * 4);                      // first vectors of the next row
@@ -185,13 +193,15 @@ spmv_ell_small_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__
 }
 
 // ---------------------------------------------------------------------------------------------
-// x larger than shared memory: the columns are cut into equal windows that do fit, and the kernel
-// runs one phase per window: stage x[window], then every row adds the products of its entries
-// whose column lies in the window (a contiguous run, rows ascend; the run's ends come from a
-// per-row split table built once per handle by binary search).  Each matrix entry is still read
-// once; y is written in phase 0 (bias + partial) and updated by the same lane in later phases.
-// Against gathering x through L1 / L2 (32-byte sectors for 4 useful bytes) this keeps every gather
-// in shared memory.
+// x larger than shared memory: the columns are cut into equal windows, two of which fit; the kernel runs
+// one phase per window, with the next window's copy in flight behind it.  In a phase every row adds the
+// products of its entries whose column lies in the window (a contiguous run, columns ascend; the run's ends
+// come from a per-row split table built once per handle by binary search).  Each matrix entry is read once;
+// y is written in phase 0 (bias + partial) and updated by the same lane in later phases.  A row's first slab
+// vectors, the next row's run and the id of the row after it are on their way while a row is summed: that,
+// not the windows, is what gains (65536 x 65536, 95 % sparse: 306 us with two windows and neither, 325 with
+// double-buffered windows alone, 267 with both = the time a copy of the same bytes takes; 20000 x 60000, 90 %:
+// 214 -> 150 us; gathering x through L1 / L2, 32-byte sectors for 4 useful bytes: 320 and 216 us).
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
 spmv_splits_kernel(const uint32_t* __restrict__ idx, const uint32_t* __restrict__ nnz, uint32_t m, uint32_t pitch,
@@ -217,67 +227,65 @@ spmv_ell_windowed_kernel(const float* __restrict__ Wd, const uint32_t* __restric
                          const uint32_t* __restrict__ split, uint32_t m, uint32_t n, uint32_t win, uint32_t pitch,
                          const float* __restrict__ x, const float* __restrict__ bias, float* __restrict__ y)
 {
-    extern __shared__ __align__(16) float xs[];
+    extern __shared__ __align__(16) float xs_all[];        // two windows of x
     const uint32_t lane = threadIdx.x & (LPR - 1);
     const uint32_t groups_per_block = blockDim.x / LPR;
-    const uint32_t group = blockIdx.x * groups_per_block + threadIdx.x / LPR;
+    // neighbouring slots go to different CTAs, so that a last, partly filled round is spread over all SMs
+    const uint32_t group = threadIdx.x / LPR * gridDim.x + blockIdx.x;
     const uint32_t stride = gridDim.x * groups_per_block;
     const uint32_t iters = (m + stride - 1) / stride;
     const uint32_t phases = (n + win - 1) / win;
-    const bool vec_ok = (reinterpret_cast<uintptr_t>(x) & 15) == 0;      // win is a multiple of 4
+    spx::pdl_launch();
+    spx::pdl_wait();
 
+    constexpr int UNR = 4;                      // 16-byte vectors of Wd and of idx in flight per lane
+    float4 wv[UNR];
+    uint4 kv[UNR];
+    // the vectors from entry j on of a run that ends at j1; entries outside the run belong to other phases
+    auto load_chunk = [&](uint32_t row, uint32_t j, uint32_t j1) {
+        const float4* __restrict__ w4 = reinterpret_cast<const float4*>(Wd + (size_t)row * pitch);
+        const uint4* __restrict__ k4 = reinterpret_cast<const uint4*>(idx + (size_t)row * pitch);
+#pragma unroll
+        for (int u = 0; u < UNR; ++u) {
+            const uint32_t ju = j + u * LPR * 4;
+            if (ju < j1) {
+                wv[u] = __ldcs(w4 + (ju >> 2));
+                kv[u] = __ldcs(k4 + (ju >> 2));
+            }
+        }
+    };
+    // ids only: carrying the lengths along costs the registers of a vector in flight (313 -> 332 us at
+    // 65536 x 65536, 95 % sparse)
+    auto id_of = [&](uint64_t slot) { return slot < m ? __ldg(&rows[slot].x) : 0u; };
+
+    stage_x(xs_all, x, min(win, n));
     for (uint32_t p = 0; p < phases; ++p) {
-        const uint32_t lo = p * win, cnt = min(win, n - lo);
-        if (p) __syncthreads();                 // the previous window is no longer read
-        const uint32_t n4 = vec_ok ? (cnt >> 2) : 0;
-        for (uint32_t i = threadIdx.x; i < n4; i += blockDim.x)
-            reinterpret_cast<float4*>(xs)[i] = __ldg(reinterpret_cast<const float4*>(x + lo) + i);
-        for (uint32_t i = (n4 << 2) + threadIdx.x; i < cnt; i += blockDim.x) xs[i] = __ldg(x + lo + i);
-        __syncthreads();
-
+        const uint32_t lo = p * win;
+        const float* xs = xs_all + (p & 1u) * win;
         // this phase's run [j0, j1) of a row: split table entries p-1 and p (0 and nnz at the ends)
-        auto run_of = [&](uint32_t r, uint32_t& b0, uint32_t& b1) {
+        auto run_of = [&](uint64_t slot, uint32_t r, uint32_t& b0, uint32_t& b1) {
+            b0 = b1 = 0;
+            if (slot >= m) return;
             b0 = p ? __ldg(split + (size_t)(p - 1) * m + r) : 0u;
             b1 = (p + 1 < phases) ? __ldg(split + (size_t)p * m + r) : __ldg(nnz + r);
         };
-        // ids only: carrying the lengths along costs the registers of a vector in flight (313 -> 332 us at
-        // 65536 x 65536, 95 % sparse)
-        auto id_of = [&](uint64_t slot) { return __ldg(&rows[slot].x); };
-        // the next row's run and the id of the row after it are fetched while the current row streams
-        uint32_t row = group < m ? id_of(group) : 0u;
-        uint32_t j0_next = 0, j1_next = 0;
-        if (group < m) run_of(row, j0_next, j1_next);
-        uint32_t row_next = (uint64_t)group + stride < m ? id_of((uint64_t)group + stride) : 0u;
+        // A row's first vectors, the next row's run and the id of the row after it are always on their way.
+        uint32_t row = id_of(group), row_next = id_of((uint64_t)group + stride);
+        uint32_t j0, j1;
+        run_of(group, row, j0, j1);
+        load_chunk(row, (j0 & ~3u) + lane * 4, j1);
+        landed_x();                             // and nobody reads the other window any more: the next one goes there
+        if (p + 1 < phases) stage_x(xs_all + ((p + 1) & 1u) * win, x + lo + win, min(win, n - lo - win));
+
         for (uint32_t it = 0; it < iters; ++it) {
-            const uint32_t slot = group + it * stride;
-            const bool live = slot < m;
-            const uint32_t j0 = j0_next, j1 = j1_next;
-            const uint32_t row_after = row_next;
-            {
-                const uint64_t s1 = (uint64_t)slot + stride, s2 = s1 + stride;
-                j0_next = j1_next = 0;
-                if (s1 < m) run_of(row_after, j0_next, j1_next);
-                row_next = s2 < m ? id_of(s2) : 0u;
-            }
-            const float4* __restrict__ w4 = reinterpret_cast<const float4*>(Wd + (size_t)row * pitch);
-            const uint4* __restrict__ k4 = reinterpret_cast<const uint4*>(idx + (size_t)row * pitch);
+            const uint64_t slot = group + (uint64_t)it * stride;
+            uint32_t n0, n1;
+            run_of(slot + stride, row_next, n0, n1);
+            const uint32_t row_after = id_of(slot + 2 * (uint64_t)stride);
             float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-            constexpr int UNR = 4;
-            // vectors from the one holding entry j0; entries outside [j0, j1) belong to other phases
-            for (uint32_t j = (j0 & ~3u) + lane * 4; j < j1; j += LPR * 4 * UNR) {
-                float4 wv[UNR];
-                uint4 kv[UNR];
-#pragma unroll
-                for (int u = 0; u < UNR; ++u) {
-                    const uint32_t ju = j + u * LPR * 4;
-                    if (ju < j1) {
-                        wv[u] = __ldcs(w4 + (ju >> 2));
-                        kv[u] = __ldcs(k4 + (ju >> 2));
-                    } else {
-                        wv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        kv[u] = make_uint4(lo, lo, lo, lo);
-                    }
-                }
+            const uint32_t first = (j0 & ~3u) + lane * 4;
+            for (uint32_t j = first; j < j1; j += LPR * 4 * UNR) {
+                if (j != first) load_chunk(row, j, j1);
 #pragma unroll
                 for (int u = 0; u < UNR; ++u) {
                     const uint32_t ju = j + u * LPR * 4;
@@ -287,13 +295,14 @@ spmv_ell_windowed_kernel(const float* __restrict__ Wd, const uint32_t* __restric
                     if (ju + 3 >= j0 && ju + 3 < j1) a3 = fmaf(wv[u].w, xs[kv[u].w - lo], a3);
                 }
             }
+            load_chunk(row_next, (n0 & ~3u) + lane * 4, n1);
             float acc = (a0 + a1) + (a2 + a3);
             acc = group_sum<LPR>(acc);
-            if (live && lane == 0) {
+            if (slot < m && lane == 0) {
                 if (p == 0) y[row] = (bias ? __ldg(bias + row) : 0.0f) + acc;
                 else if (j1 > j0) y[row] += acc;
             }
-            row = row_after;
+            row = row_next; row_next = row_after; j0 = n0; j1 = n1;
         }
     }
 }
@@ -301,7 +310,7 @@ spmv_ell_windowed_kernel(const float* __restrict__ Wd, const uint32_t* __restric
 // Reference-order variant: reproduces the summation order of the reference's AVX-512 path bit for
 // bit (src/ellpack_matvec.cpp:72-99): sixteen partial sums, partial l takes entries j = l, l+16, ...
 // with one FMA each starting from 0; then lanes l and l+8, l and l+4, the two horizontal adds, and
-// finally bias + sum.  Sixteen lanes per row; slower than spmv_ell_kernel (4-byte loads, chains of
+// finally bias + sum.  Sixteen lanes per row; slower than the others (4-byte loads, chains of
 // nnz/16), meant for checking, not for throughput.
 __global__ void __launch_bounds__(256)
 spmv_reforder_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ idx,
@@ -323,100 +332,70 @@ spmv_reforder_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ 
     if (live && l == 0) y[row] = (bias ? __ldg(bias + row) : 0.0f) + a;
 }
 
-constexpr size_t kSmallX = 32 * 1024;
-
-template <int LPR, bool SMEM>
-int launch_one(const spx_ell* e, const float* x, const float* bias, float* y, cudaStream_t s,
-               int threads, int blocks, size_t smem)
+int finish(cudaError_t err, const char* name)
 {
-    auto kfn = spmv_ell_kernel<LPR, SMEM>;
-    if (smem > 48 * 1024) {
-        cudaError_t err = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (err != cudaSuccess) return spx::fail(SPX_ERR_CUDA, "spmv: shared memory opt-in failed: %s", cudaGetErrorString(err));
-    }
-    kfn<<<blocks, threads, smem, s>>>(e->Wd, e->idx, e->nnz, e->rows, e->m, e->n, e->pitch, x, bias, y);
-    SPX_LAUNCH_CHECK("spmv_ell_kernel");
+    if (err != cudaSuccess) return spx::fail(SPX_ERR_CUDA, "launch of %s failed: %s", name, cudaGetErrorString(err));
+    spx::count_launch();
     return SPX_OK;
 }
 
-// Shrinks a persistent grid so that every group runs the same number of row iterations
-// (a grid of 9324 groups over 16384 rows would give some groups two rows and others one).
-static int balanced_blocks(uint64_t rows, int groups_per_block, int max_blocks)
+template <class K>
+int opt_in(K kfn, size_t smem)
 {
-    const uint64_t cap = (uint64_t)max_blocks * groups_per_block;
-    const uint64_t iters = (rows + cap - 1) / cap;
-    const uint64_t blocks = (rows + iters * groups_per_block - 1) / (iters * groups_per_block);
-    return (int)(blocks ? blocks : 1);
+    const cudaError_t err = smem > 48 * 1024 ? cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) : cudaSuccess;
+    return err == cudaSuccess ? SPX_OK : spx::fail(SPX_ERR_CUDA, "spmv: shared memory opt-in failed: %s", cudaGetErrorString(err));
 }
 
-// Small x (up to 32 KB): the pipelined kernel on a grid with the same number of CTAs on every SM.
-template <int LPR>
-int launch_small(const spx_ell* e, const float* x, const float* bias, float* y, cudaStream_t s)
-{
-    const int sms = spx::sm_count(e->device);
-    const size_t xbytes = (size_t)e->n * sizeof(float);
-    const uint64_t groups_needed = e->m;
-    // Rows of near-equal length need no schedule: slot == row saves one dependent load per row.
-    const uint2* order = (e->max_nnz - e->min_nnz) * 8u <= e->max_nnz ? nullptr : e->rows;
-    // Rows per group (iters) as if every SM held 4 CTAs of 512 threads; then the same number of CTAs
-    // on every SM -- as few as carry the rows in that many iterations (x is staged once per CTA) --
-    // each with equally many groups.  A grid that is not a multiple of the SM count leaves some SMs
-    // with one CTA more than others for the whole kernel.
-    constexpr int kPerSm = 4, kThreadsFull = 512;
-    const uint64_t cap = (uint64_t)sms * kPerSm * (kThreadsFull / LPR);
-    const uint64_t iters = (groups_needed + cap - 1) / cap;
-    const uint64_t per_iter = (groups_needed + iters - 1) / iters;         // groups that must exist
-    int threads = kThreadsFull, blocks = sms * kPerSm;
-    for (int k = 1; k <= kPerSm; ++k) {       // (forcing 2 or 4 CTAs per SM measured the same 8.1 us on 4096 x 4096)
-        const uint64_t g = (per_iter + (uint64_t)sms * k - 1) / ((uint64_t)sms * k);
-        const uint64_t t = (g * LPR + 31) / 32 * 32;
-        if (t <= std::min<uint64_t>(1024, 2048 / k)) {
-            threads = (int)t;
-            blocks = (int)std::min<uint64_t>((uint64_t)sms * k, (per_iter + g - 1) / g);
-            break;
-        }
-    }
-    spmv_ell_small_kernel<LPR><<<blocks, threads, xbytes, s>>>(e->Wd, e->idx, e->nnz, order, e->m, e->n, e->pitch, x, bias, y);
-    SPX_LAUNCH_CHECK("spmv_ell_small_kernel");
-    return SPX_OK;
-}
+constexpr uint32_t kStaged = 200 * 1024 / sizeof(float);        // columns up to which all of x is staged
 
 template <int LPR>
 int launch_lpr(const spx_ell* e, const float* x, const float* bias, float* y, cudaStream_t s)
 {
-    const int sms = spx::sm_count(e->device);
-    const size_t xbytes = (size_t)e->n * sizeof(float);
-    // Measured on B200: the pipelined kernel wins for 4096 columns at every sparsity (8.7 -> 8.1 us
-    // at 90 %, 12 -> 10.4 us at 80 %); at 16384 columns it is mixed and with x gathered from global
-    // memory it is 6 % slower, so larger matrices keep the kernel below.
-    if (xbytes <= kSmallX) return launch_small<LPR>(e, x, bias, y, s);
-    const size_t kSmemMax = 200 * 1024;      // leaves room for a second small CTA's static needs
-    const uint64_t groups_needed = e->m;
-    if (xbytes <= kSmemMax) {
-        // CTAs per SM limited by the staged copy of x; 2048 threads per SM at most.
-        int per_sm = (int)((220 * 1024) / (xbytes + 1024));
-        if (per_sm < 1) per_sm = 1;
-        if (per_sm > 4) per_sm = 4;
-        int threads = 2048 / per_sm;
-        if (threads > 1024) threads = 1024;
-        threads &= ~31;
-        const int blocks = balanced_blocks(groups_needed, threads / LPR, sms * per_sm);
-        return launch_one<LPR, true>(e, x, bias, y, s, threads, blocks, xbytes);
+    const uint64_t sms = spx::sm_count(e->device);
+    if (e->n <= kStaged) {
+        // Rows of near-equal length need no schedule: slot == row saves one dependent load per row.
+        const uint2* order = (e->max_nnz - e->min_nnz) * 8u <= e->max_nnz ? nullptr : e->rows;
+        // One CTA on every SM, with as many groups as give each the same number of rows (64 registers a
+        // thread: 1024 threads are all an SM holds); fewer threads leave room for the next launch's CTAs.
+        const uint64_t per = (e->m + sms - 1) / sms;
+        const uint64_t iters = (per * LPR + 1023) / 1024, groups = (per + iters - 1) / iters;
+        const unsigned threads = (unsigned)((groups * LPR + 31) / 32 * 32);
+        const size_t smem = (size_t)e->n * sizeof(float);
+        auto kfn = spmv_staged_kernel<LPR>;
+        if (int rc = opt_in(kfn, smem)) return rc;
+        return finish(spx::launch_pdl(kfn, dim3((unsigned)std::min<uint64_t>(sms, e->m)), dim3(threads), smem, s, e->Wd, e->idx, e->nnz, order,
+                                      e->m, e->n, e->pitch, x, bias, y), "spmv_staged_kernel");
     }
     if (e->spmv_split) {
-        const int blocks = balanced_blocks(groups_needed, 1024 / LPR, sms);
-        const size_t smem = (size_t)e->spmv_win * sizeof(float);
+        const size_t smem = (size_t)e->spmv_win * 2 * sizeof(float);
         auto kfn = spmv_ell_windowed_kernel<LPR>;
-        cudaError_t err = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (err != cudaSuccess) return spx::fail(SPX_ERR_CUDA, "spmv: shared memory opt-in failed: %s", cudaGetErrorString(err));
-        kfn<<<blocks, 1024, smem, s>>>(e->Wd, e->idx, e->nnz, e->rows, e->spmv_split, e->m, e->n, e->spmv_win,
-                                       e->pitch, x, bias, y);
-        SPX_LAUNCH_CHECK("spmv_ell_windowed_kernel");
-        return SPX_OK;
+        if (int rc = opt_in(kfn, smem)) return rc;
+        return finish(spx::launch_pdl(kfn, dim3((unsigned)std::min<uint64_t>(sms, e->m)), dim3(1024), smem, s, e->Wd, e->idx, e->nnz, e->rows,
+                                      e->spmv_split, e->m, e->n, e->spmv_win, e->pitch, x, bias, y), "spmv_ell_windowed_kernel");
     }
-    int threads = 512;
-    const int blocks = balanced_blocks(groups_needed, threads / LPR, sms * 4);
-    return launch_one<LPR, false>(e, x, bias, y, s, threads, blocks, 0);
+    // as many CTAs as give every group the same number of rows
+    const uint64_t per_block = 512 / LPR, rounds = (e->m + sms * 4 * per_block - 1) / (sms * 4 * per_block);
+    const uint64_t blocks = (e->m + rounds * per_block - 1) / (rounds * per_block);
+    return finish(spx::launch_pdl(spmv_ell_kernel<LPR>, dim3((unsigned)blocks), dim3(512), 0, s, e->Wd, e->idx, e->nnz, e->rows, e->m, e->n,
+                                  e->pitch, x, bias, y), "spmv_ell_kernel");
+}
+
+// Lanes per row.  A lane consumes 16 entries per round trip, so long rows want many lanes and short ones few.
+// Staged x: all rows of an SM at once, if 1024 threads carry them that way, is best -- the fewest rounds and
+// row changes (16384 x 16384, 90 %: 33.7 us with 8 lanes, 36 with 16 or 32; 33088 x 3904, 402 entries: 19.3 us
+// with 4, 20.2 with 32) -- as long as a row takes at most 16 rounds (26877 x 24384, 2377 entries: 81 us with
+// 8 lanes, 79 with 16) and no lane idles for most of a row.
+int lanes_per_row(const spx_ell* e)
+{
+    const double windows = e->spmv_split ? (double)((e->n + e->spmv_win - 1) / e->spmv_win) : 1.0;
+    const double mean = (double)e->nnz_total / e->m / windows;
+    if (e->spmv_split) return mean > 300.0 ? 32 : mean > 100.0 ? 16 : mean > 40.0 ? 8 : 4;
+    const uint64_t per = (e->m + spx::sm_count(e->device) - 1) / spx::sm_count(e->device);
+    if (e->n > kStaged || per * 4 > 1024) return mean > 192.0 ? 32 : mean > 96.0 ? 16 : mean > 40.0 ? 8 : 4;
+    int lpr = 32;
+    while (lpr > 4 && (per * lpr > 1024 || (lpr > 8 && mean / 12.0 < lpr))) lpr /= 2;
+    while (lpr < 32 && mean > 16.0 * 16 * lpr) lpr *= 2;
+    return lpr;
 }
 
 }  // namespace
@@ -432,23 +411,17 @@ int launch_spmv_reforder(const spx_ell* e, const float* x, const float* bias, fl
     return SPX_OK;
 }
 
-// x beyond shared memory: up to kMaxWindows equal column windows of at most 200 KB; the per-row
-// split table ((windows - 1) * m entries) is built on the first call and cached in the handle.
+// x beyond shared memory: up to kMaxWindows equal column windows of at most 104 KB (two at a time are
+// staged); the per-row split table ((windows - 1) * m entries) is built on the first call and kept.
 static int ensure_spmv_windows(spx_ell* e, cudaStream_t s)
 {
-    constexpr uint32_t kWinMax = 200 * 1024 / sizeof(float), kMaxWindows = 8;
+    constexpr uint32_t kWinMax = 104 * 1024 / sizeof(float), kMaxWindows = 16;
     static const int enabled = [] { const char* v = getenv("SPX_SPMV_WINDOWED"); return v ? atoi(v) : 1; }();
     if (e->spmv_split || e->spmv_win == UINT32_MAX) return SPX_OK;
     e->spmv_win = UINT32_MAX;                                       // decided: stays "no" unless built below
-    if (!enabled || !e->cols_ascending || e->n <= kWinMax || e->max_nnz == 0) return SPX_OK;
+    if (!enabled || !e->cols_ascending || e->n <= kStaged || e->max_nnz == 0) return SPX_OK;
     const uint32_t windows = (e->n + kWinMax - 1) / kWinMax;
     if (windows > kMaxWindows) return SPX_OK;
-    // Measured at 65536 x 65536: 307 vs 321 us at 95 % sparsity and 84 vs 97 us at 99 % (the
-    // gathers of x stop crossing L2 -> SM as 32-byte sectors), equal at 90 %, 1117 vs 1086 us at
-    // 80 % (long rows stream at 97 % of the copy bandwidth either way and the second pass over the
-    // rows only costs): taken when a row's run inside a window is short.  SPX_SPMV_WINDOWED=2 forces it.
-    const double run = (double)e->nnz_total / e->m / windows;
-    if (enabled != 2 && run > 2500.0) return SPX_OK;
     const uint32_t win = round_up((e->n + windows - 1) / windows, 4u);
     const uint64_t entries = (uint64_t)e->m * (windows - 1);
     if (pool_alloc_now(reinterpret_cast<void**>(&e->spmv_split), entries * sizeof(uint32_t), e->device) != SPX_OK) {
@@ -470,13 +443,12 @@ int launch_spmv(spx_ell* e, const float* x, const float* bias, float* y, cudaStr
     if (exact) return launch_spmv_reforder(e, x, bias, y, s);
     const int rcw = ensure_spmv_windows(e, s);
     if (rcw != SPX_OK) return rcw;
-    // Lanes per row from the mean row length: a lane consumes 4 entries per vector load.
-    const double windows = e->spmv_split ? (double)((e->n + e->spmv_win - 1) / e->spmv_win) : 1.0;
-    const double mean = e->m ? (double)e->nnz_total / e->m / windows : 0.0;
-    if (mean > 192.0) return launch_lpr<32>(e, x, bias, y, s);
-    if (mean > 96.0)  return launch_lpr<16>(e, x, bias, y, s);
-    if (mean > 40.0)  return launch_lpr<8>(e, x, bias, y, s);
-    return launch_lpr<4>(e, x, bias, y, s);
+    switch (lanes_per_row(e)) {
+    case 32: return launch_lpr<32>(e, x, bias, y, s);
+    case 16: return launch_lpr<16>(e, x, bias, y, s);
+    case 8:  return launch_lpr<8>(e, x, bias, y, s);
+    default: return launch_lpr<4>(e, x, bias, y, s);
+    }
 }
 
 }  // namespace spx
