@@ -682,38 +682,54 @@ static inline uint32_t host_panel_width(uint32_t c0, uint32_t C)
     return std::min<uint32_t>(256, C - c0);
 }
 
-// One host-buffer call: a stream, and where the operands are small a pinned block through which they travel.
-// Small means that latency is all there is to it: inputs are packed and sent as one copy, and the kernel
-// stores its result straight into the pinned block, so the call is one copy, one kernel and one wait
-// (2048 x 2048 SpMV: 26 us with two pageable copies in and one out).
+// One host-buffer call: a stream, and a pinned block through which operands travel that are too small for
+// copy_h2d's pieces: inputs are packed and sent as one copy, a result is fetched into the block and copied
+// on, or, where it is small, stored there by the kernel -- a pageable copy costs the driver's staging and a
+// wait each (2048 x 2048 SpMV: 26 us with two of them in and one out, 22 us; 672 x 2592: 25 -> 20 us).
 struct HostCall {
-    static constexpr size_t kSmall = 64 * 1024;         // bytes of inputs, and of the result
+    static constexpr size_t kSmall = 64 * 1024;         // result bytes that a kernel stores itself
+    static constexpr size_t kInputs = 256 * 1024;       // input bytes that are packed
+    static constexpr size_t kResult = 1024 * 1024;      // result bytes that are fetched through the block
     cudaStream_t stream = nullptr;
-    PinnedBlock block;                                  // [inputs | result], kSmall each
+    PinnedBlock block;                                  // [inputs | result]
     bool open = false;
 
-    int begin(int device) {
+    // result_bytes: of the result, if it may travel through the block (0: it does not)
+    int begin(int device, size_t result_bytes) {
         if (int rc = host_stream(device, 0, &stream)) return rc;
+        if (int rc = pinned_acquire(kInputs + (result_bytes <= kResult ? result_bytes : 0), &block)) return rc;
         open = true;
         return SPX_OK;
     }
-    int stage(size_t bytes) { return block.host ? SPX_OK : pinned_acquire(bytes, &block); }
     char* host() const { return static_cast<char*>(block.host); }
-    // The result half of the block as the device sees it; null when that is not to be had.
+    // The result part of the block as the device sees it; null when that is not to be had.
     float* mapped_result() {
         void* p = nullptr;
-        if (stage(2 * kSmall) != SPX_OK || cudaHostGetDevicePointer(&p, host() + kSmall, 0) != cudaSuccess) {
+        if (cudaHostGetDevicePointer(&p, host() + kInputs, 0) != cudaSuccess) {
             (void)cudaGetLastError();
             return nullptr;
         }
         return static_cast<float*>(p);
     }
-    // Waits for the result and hands it over: from device memory, or (from == null) from the pinned block.
+    // Two inputs that are neighbours on the device, the second `gap` bytes behind the first's start.
+    int send(void* dst, const void* a, size_t a_bytes, const void* b, size_t b_bytes, size_t gap) {
+        if (gap + b_bytes > kInputs) {
+            if (b_bytes) SPX_CUDA(cudaMemcpyAsync(static_cast<char*>(dst) + gap, b, b_bytes, cudaMemcpyHostToDevice, stream));
+            return copy_h2d(dst, a, a_bytes, stream);
+        }
+        if (a_bytes) std::memcpy(host(), a, a_bytes);
+        if (b_bytes) std::memcpy(host() + gap, b, b_bytes);
+        const size_t both = b_bytes ? gap + b_bytes : a_bytes;
+        if (both) SPX_CUDA(cudaMemcpyAsync(dst, host(), both, cudaMemcpyHostToDevice, stream));
+        return SPX_OK;
+    }
+    // Waits for the result and hands it over: from device memory, or (from == null) from the block.
     int finish(float* to, const float* from, size_t bytes) {
-        if (from) SPX_CUDA(cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, stream));
+        const bool through = !from || (bytes <= kResult && pageable_memory(to));
+        if (from) SPX_CUDA(cudaMemcpyAsync(through ? static_cast<void*>(host() + kInputs) : to, from, bytes, cudaMemcpyDeviceToHost, stream));
         open = false;
         SPX_CUDA(cudaStreamSynchronize(stream));
-        if (!from) std::memcpy(to, host() + kSmall, bytes);
+        if (through) std::memcpy(to, host() + kInputs, bytes);
         return SPX_OK;
     }
     ~HostCall() {
@@ -818,23 +834,12 @@ int spx_spmm_host(const spx_ell* ce, const float* X, uint32_t C, const float* bi
         rc = spmm_host_panels(e, X, C, bias, act, Y, dX, dB, dY);
         return rc;
     }
+    const size_t y_bytes = (size_t)e->m * C * 4;
     HostCall call;
-    rc = call.begin(e->device);
+    rc = call.begin(e->device, y_bytes);
+    if (rc == SPX_OK) rc = call.send(dX, X, (size_t)e->n * C * 4, bias, bias ? (size_t)e->m * 4 : 0, xb);
     if (rc != SPX_OK) return rc;
-    const size_t x_bytes = (size_t)e->n * C * 4, bias_bytes = bias ? (size_t)e->m * 4 : 0, y_bytes = (size_t)e->m * C * 4;
-    // X and the bias are neighbours on the device: where both are small they go over in one copy
-    if (xb + bb <= HostCall::kSmall) {
-        rc = call.stage(2 * HostCall::kSmall);
-        if (rc != SPX_OK) return rc;
-        if (x_bytes) std::memcpy(call.host(), X, x_bytes);
-        if (bias) std::memcpy(call.host() + xb, bias, bias_bytes);
-        const size_t both = bias ? xb + bias_bytes : x_bytes;
-        if (both) SPX_CUDA(cudaMemcpyAsync(dX, call.host(), both, cudaMemcpyHostToDevice, call.stream));
-    } else {
-        if (bias) SPX_CUDA(cudaMemcpyAsync(dB, bias, bias_bytes, cudaMemcpyHostToDevice, call.stream));
-        if (int rx = copy_h2d(dX, X, x_bytes, call.stream)) return rx;
-    }
-    float* direct = y_bytes <= HostCall::kSmall ? call.mapped_result() : nullptr;
+    float* direct = y_bytes <= HostCall::kSmall && C >= 8 ? call.mapped_result() : nullptr;
     rc = spx_spmm(e, dX, C, C, bias ? dB : nullptr, act, direct ? direct : dY, C, call.stream);
     if (rc != SPX_OK) return rc;
     return call.finish(Y, direct ? nullptr : dY, y_bytes);
@@ -949,22 +954,13 @@ int spx_spmv_host(const spx_ell* ce, const float* x, const float* bias, float* y
     float* dx = reinterpret_cast<float*>(base);
     float* dB = reinterpret_cast<float*>(base + xb);
     float* dy = reinterpret_cast<float*>(base + xb + bb);
+    const size_t y_bytes = (size_t)e->m * 4;
     HostCall call;
-    rc = call.begin(e->device);
+    rc = call.begin(e->device, y_bytes);
+    if (rc == SPX_OK) rc = call.send(dx, x, (size_t)e->n * 4, bias, bias ? y_bytes : 0, xb);
     if (rc != SPX_OK) return rc;
-    const size_t x_bytes = (size_t)e->n * 4, y_bytes = (size_t)e->m * 4;
-    if (xb + y_bytes <= HostCall::kSmall) {     // x and the bias in one copy
-        rc = call.stage(2 * HostCall::kSmall);
-        if (rc != SPX_OK) return rc;
-        if (x_bytes) std::memcpy(call.host(), x, x_bytes);
-        if (bias) std::memcpy(call.host() + xb, bias, y_bytes);
-        const size_t both = bias ? xb + y_bytes : x_bytes;
-        if (both) SPX_CUDA(cudaMemcpyAsync(dx, call.host(), both, cudaMemcpyHostToDevice, call.stream));
-    } else {
-        if (bias) SPX_CUDA(cudaMemcpyAsync(dB, bias, y_bytes, cudaMemcpyHostToDevice, call.stream));
-        if (int rx = copy_h2d(dx, x, x_bytes, call.stream)) return rx;
-    }
-    float* direct = y_bytes <= HostCall::kSmall ? call.mapped_result() : nullptr;
+    // single floats to the host cost more than a copy beyond a thousand of them (5519 rows: 28 us against 24)
+    float* direct = e->m <= 1024 ? call.mapped_result() : nullptr;
     rc = spx_spmv(e, dx, bias ? dB : nullptr, direct ? direct : dy, call.stream);
     if (rc != SPX_OK) return rc;
     return call.finish(y, direct ? nullptr : dy, y_bytes);

@@ -9,8 +9,8 @@
 // summation order differs from the reference's 16-partial-sum order, so results agree within
 // the stated tolerance 1e-5 * sum|w||x|, not bit for bit.  Padding slots are never multiplied.
 //
-// HBM-bound: 8 bytes per nonzero streamed once.  All kernels are launched as programmatic dependents:
-// what belongs to the handle (schedule, first slab vectors) is asked for while the predecessor in the
+// HBM-bound: 8 bytes per nonzero streamed once.  The kernels that stage x are launched as programmatic
+// dependents: // what belongs to the handle (schedule, first slab vectors) is asked for while the predecessor in the
 // stream drains, and only x, bias and y wait for it.
 #include "common.cuh"
 
@@ -53,9 +53,6 @@ spmv_ell_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ idx,
                 uint32_t m, uint32_t n, uint32_t pitch,
                 const float* __restrict__ x, const float* __restrict__ bias, float* __restrict__ y)
 {
-    spx::pdl_launch();
-    spx::pdl_wait();
-
     const uint32_t lane = threadIdx.x & (LPR - 1);
     const uint32_t groups_per_block = blockDim.x / LPR;
     const uint32_t group = blockIdx.x * groups_per_block + threadIdx.x / LPR;
@@ -376,8 +373,9 @@ int launch_lpr(const spx_ell* e, const float* x, const float* bias, float* y, cu
     // as many CTAs as give every group the same number of rows
     const uint64_t per_block = 512 / LPR, rounds = (e->m + sms * 4 * per_block - 1) / (sms * 4 * per_block);
     const uint64_t blocks = (e->m + rounds * per_block - 1) / (rounds * per_block);
-    return finish(spx::launch_pdl(spmv_ell_kernel<LPR>, dim3((unsigned)blocks), dim3(512), 0, s, e->Wd, e->idx, e->nnz, e->rows, e->m, e->n,
-                                  e->pitch, x, bias, y), "spmv_ell_kernel");
+    spmv_ell_kernel<LPR><<<(unsigned)blocks, 512, 0, s>>>(e->Wd, e->idx, e->nnz, e->rows, e->m, e->n, e->pitch, x, bias, y);
+    SPX_LAUNCH_CHECK("spmv_ell_kernel");
+    return SPX_OK;
 }
 
 // Lanes per row.  A lane consumes 16 entries per round trip, so long rows want many lanes and short ones few.

@@ -17,7 +17,7 @@ namespace spx {
 
 class ResultPool {
 public:
-    static constexpr size_t kMinBytes = 256 * 1024;     // below, a plain array is as fast
+    static constexpr size_t kMinBytes = 64 * 1024;      // below, a plain array is as fast
     static constexpr size_t kMaxBytes = size_t(256) << 20;
     static constexpr int kMaxLive = 8;
 
