@@ -1015,16 +1015,18 @@ static int launch_rows(const spx_ell* e, RowsArgs a, cudaStream_t s)
     const uint32_t nv_max = V == 4 ? 2 : 3;
     const uint32_t NV = std::min(nv_max, (q + 31) / 32);
     const uint32_t panels = (q + 32 * NV - 1) / (32 * NV);
-    const uint32_t per = (q + panels - 1) / panels;
-    a.G = (per + NV - 1) / NV;
+    // One vector per lane: as few lanes as cover the row.  More: whole warps, the rest in the last vector; equal parts
+    // would start off the 128-byte lines (2690 x 3809, 3.4 %, C = 704: 77 -> 52 us; 4096 x 4096, 10 %, C = 320: 157 -> 144).
+    a.G = NV > 1 ? 32u : q;
     a.RW = std::min(32u / a.G, 16u);
     const uint64_t warps = (uint64_t)((e->m + a.RW - 1) / a.RW) * panels;
     uint32_t wpb = 4;                               // small CTAs: a finished one frees its warps at once
     while (wpb > 1 && (warps + wpb - 1) / wpb < sms * 4) wpb >>= 1;
     const double per_sm = (double)warps / sms;
+    const bool brief = e->nnz_total < 100ull * e->m;    // rows too short for a deep group to pay for its registers
     int U;
-    if (NV == 1) U = per_sm < 12 ? 32 : per_sm < 48 ? 16 : 4;
-    else         U = per_sm < (V == 4 ? 12 : 24) ? 16 : per_sm < 48 ? 8 : 4;
+    if (NV == 1) U = per_sm <= 8 ? 32 : per_sm < 48 || !brief ? 16 : 4;
+    else         U = per_sm < (V == 4 ? 12 : 24) ? 16 : per_sm < 48 || !brief ? 8 : 4;
     // Single columns per lane are cheap enough in registers to keep a second group in flight (1312 x 2080, 27 %,
     // C = 37: 34 -> 23 us); 16-byte vectors are not (4096 x 4096, 10 %, C = 128: 42 -> 46 us).
     if constexpr (V == 1) {
@@ -1078,12 +1080,21 @@ int launch_spmm_bcast(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx
     RowsArgs a{};
     a.Wd = e->Wd; a.idx = e->idx; a.rows = e->rows; a.m = e->m; a.pitch = e->pitch; a.n = e->n;
     a.X = X; a.C = C; a.ldx = ldx; a.bias = bias; a.act = act; a.ldy = ldy; a.out = out;
-    // Few columns, X in shared memory: the chain kernel up to 4 columns (or 8 of a small X), the direct
-    // kernel for aligned operands while one CTA per SM carries the rows.
+    // Few columns and X small enough for shared memory: spmm_rows pays a trip to L2 per group of entries, the staged
+    // kernels pay for bringing X in, for their barriers, and in CTAs that share an SM.  They win where rows
+    // are long and few.  Measured, rows against staged: 1024 rows of 300 entries C = 1 / 4 / 8 8.5 / 10.4 / 10.6 us
+    // against 4.0 / 4.8 / 5.1; of 30 entries, C = 3 2.1 against 3.2; 8192 rows of 300, C = 3 13.9 against 18.5; 8192 of
+    // 30, C = 7 4.5 against 20.  Odd widths above 4 serialise most; 4 and 8 columns are whole vectors.
     const uint64_t x_bytes = (uint64_t)e->n * chain_pitch(C) * 4;
     const bool staged = x_bytes <= kChainX && e->max_nnz > 0;      // without entries X is not read and may be null
-    if (staged && (C <= 4 || (C <= 8 && x_bytes <= 32 * 1024))) return launch_chain(e, a, s);
-    if (staged && vec_ok && C <= 64 && e->m <= (uint64_t)sm_count(e->device) * (kChainConsumers / (C / 4)))
+    const uint64_t len = e->max_nnz, m = e->m;
+    const bool chain = C == 1 ? len >= 80 && m <= 6000
+                     : C == 3 ? (len >= 200 || (len >= 80 && x_bytes <= 32 * 1024)) && m <= (len >= 1000 ? 4500u : 2000u)
+                     : C <= 4 ? len >= 60 && m <= 4500
+                     : C < 8  ? len >= 250 && m <= len
+                              : C == 8 && len >= 80 && m <= 2048;
+    if (staged && chain) return launch_chain(e, a, s);
+    if (staged && vec_ok && C >= 8 && C <= 64 && len >= 80 && m <= (uint64_t)sm_count(e->device) * (kChainConsumers / (C / 4)))
         return launch_direct(e, a, true, s);
     {
         const bool vec_x = C % 4 == 0 && ldx % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;

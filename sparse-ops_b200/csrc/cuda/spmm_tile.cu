@@ -457,10 +457,10 @@ struct Plan {
 };
 
 // Launch shape and expected time.  As few waves of CTAs as kMaxWarps warps each allow, and then equally
-// many warps in every CTA.  Time: about half a microsecond per phase (wait, hand-off, a block of steps cut
-// short), and per step of a warp the larger of its latency and the shared-memory wavefronts of all the
-// SM's warps (16 NV gathers + 4 of hand-off, one per cycle).  Fitted to 37 shapes of 512 to 8192 rows and
-// columns, 2 to 38 % dense, C = 16 to 512: rms 6 %, worst 17 %.
+// many warps in every CTA.  Time: the results' way out, about half a microsecond per phase (wait, hand-off, a
+// block of steps cut short; more where X's rows do not begin on lines), and per step of a warp the
+// larger of its latency and the shared-memory wavefronts of all the SM's warps (16 NV gathers + 4 of hand-off,
+// one per cycle).  Fitted to 65 shapes of 256 to 8192 rows and columns, 2 to 50 % dense, C = 9 to 1000: rms 11 %.
 Plan plan_tiles(const spx_ell* e, uint32_t C, uint32_t NV, uint32_t sms)
 {
     Plan p;
@@ -470,23 +470,26 @@ Plan plan_tiles(const spx_ell* e, uint32_t C, uint32_t NV, uint32_t sms)
     p.waves = (units + (uint64_t)sms * kMaxWarps - 1) / ((uint64_t)sms * kMaxWarps);
     p.warps = (uint32_t)std::min<uint64_t>(kMaxWarps, (units + sms * p.waves - 1) / (sms * p.waves));
     while (p.warps < kMaxWarps && (uint64_t)((groups + p.warps - 1) / p.warps) * p.slices > p.waves * sms) ++p.warps;
-    const double len = (double)e->nnz_total / e->m, steps = (len + 0.9 * std::sqrt(len)) / 4.0;
-    p.us = 1.9 + p.waves * (chunks * (NV == 1 ? 0.51 : 0.46) + steps * std::max(NV == 1 ? 0.064 : 0.104, p.warps * (16.0 * NV + 4.0) / 1870.0));
+    const double len = (double)e->nnz_total / e->m, steps = (len + 1.1 * std::sqrt(len)) / 4.0;
+    p.us = 0.9 + (double)e->m * C * 0.62e-6 + (C % 32 ? 0.2 * chunks : 0.0) +
+           p.waves * (1.4 + chunks * (NV == 1 ? 0.50 : 0.37) + steps * std::max(NV == 1 ? 0.053 : 0.098, p.warps * (16.0 * NV + 4.0) / 1950.0));
     return p;
 }
 
-// Expected time of the gather kernel (spmm_rows): bytes of gathered operands over the rate it reaches, which
-// grows with the width and falls with idle lanes (C = 160: 20 of 32 lanes), or the rounds of its longest row.
+// Expected time of the gather kernel (spmm_rows): its warps' load instructions, which L1 passes at 4 (16-byte
+// vectors) or 2 cycles and some, and about 0.1 us of each warp's own; or the rounds of the longest row, for every wave
+// of warps where the deep groups let only 8 to 9 per SM reside.  Fitted to the same shapes: rms 11 %.
 double gather_us(const spx_ell* e, uint32_t C, bool aligned)
 {
-    const double density = (double)e->nnz_total / ((double)e->m * e->n);
-    const uint32_t V = aligned ? 4 : 1, q = (C + V - 1) / V, nv_max = aligned ? 2 : 3;
+    const double sms = sm_count(e->device);
+    const uint32_t q = aligned ? (C + 3) / 4 : C, nv_max = aligned ? 2 : 3;
     const uint32_t NV = std::min(nv_max, (q + 31) / 32), panels = (q + 32 * NV - 1) / (32 * NV);
-    const uint32_t per = (q + panels - 1) / panels, G = (per + NV - 1) / NV, RW = std::min(32 / G, 16u);
-    const double lanes = (double)q * RW / (32.0 * NV * panels);
-    double rate = density < 0.04 ? 26e6 : C <= 64 ? 16e6 : C <= 128 ? 20e6 : 23e6;     // bytes per us, measured
-    if (!aligned) rate *= 0.6;
-    return 2.0 + std::max((double)e->nnz_total * C * 4.0 / (rate * lanes), e->max_nnz / (NV == 1 ? 40.0 : 16.0) * (NV == 1 ? 1.0 : 0.85));
+    const uint32_t RW = NV > 1 ? 1u : std::min(32 / q, 16u);
+    const double per_sm = std::ceil((double)e->m / RW) * panels / sms;
+    const double loads = e->nnz_total / sms * ((aligned ? 3.2e-3 : 1.5e-3) * panels * NV / RW + (C % 32 ? 0.64e-3 : 0.0)) + 0.09 * per_sm;
+    const bool deep = NV == 1 && (per_sm < 48 || e->nnz_total >= 100ull * e->m);
+    const double rounds = e->max_nnz * (NV == 1 ? 0.0275 : 0.0526) * (deep ? std::max(1.0, std::ceil(per_sm / 8.75)) : 1.0);
+    return 1.6 + std::sqrt(std::sqrt(std::pow(loads, 4) + std::pow(rounds, 4)));
 }
 
 }  // namespace
@@ -502,7 +505,7 @@ int launch_spmm_tile(spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const
     const uint32_t NV = C <= 32 ? 1 : 2;
     const Plan p = plan_tiles(e, C, NV, sm_count(e->device));
     if ((uint64_t)p.slices * e->m > 0x7fffffffull) return -1;
-    if (env != 2 && (e->n < kChunk || p.us + (vec_x ? 0.0 : 4.0) > 0.95 * gather_us(e, C, vec_x))) return -1;
+    if (env != 2 && (e->n < kChunk || p.us + (vec_x ? 0.0 : 4.0) > 0.97 * gather_us(e, C, vec_x))) return -1;
     spx_tiles_impl* t = static_cast<spx_tiles_impl*>(e->tiles);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (t->state != 1 || !vec_x) {              // building and the scratch below allocate: not while a graph is captured
