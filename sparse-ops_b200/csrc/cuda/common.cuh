@@ -113,8 +113,9 @@ __device__ __forceinline__ float apply_act(float v, int act) {
 // Programmatic dependent launch: a kernel launched with launch_pdl() may start while its predecessor
 // in the stream is still draining.  Before pdl_wait() it may only touch what no kernel of the stream
 // writes -- the arrays of a finished handle; after it everything the predecessors wrote is visible.
-// pdl_launch() lets the successor in as soon as every CTA of this grid has reached it.  Every thread
-// calls pdl_wait() before it leaves.
+// pdl_launch() lets the successor in as soon as every CTA of this grid has reached it; it comes after
+// pdl_wait(), so that one successor waits and not a row of them (three that pile up: 645 x 5312, C = 32
+// 24.3 us against 15.7).  Every thread calls pdl_wait() before it leaves.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

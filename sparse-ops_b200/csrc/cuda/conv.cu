@@ -149,8 +149,8 @@ __global__ void __launch_bounds__(256)
 to_pf_kernel(const float* __restrict__ src, uint64_t sB, uint64_t sC, uint64_t sH, uint64_t sW, uint32_t H, uint32_t W, uint64_t positions,
              uint32_t B, uint32_t quads, float* __restrict__ dst)
 {
-    spx::pdl_launch();
     spx::pdl_wait();
+    spx::pdl_launch();
     const uint64_t total = positions * quads;
     for (uint64_t t64 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t64 < total; t64 += (uint64_t)gridDim.x * blockDim.x) {
         const I t = (I)t64, q = POSITIONS_FIRST ? t / (I)positions : t / (I)quads;
@@ -511,8 +511,8 @@ conv_rbm_tile_kernel(const uint2* __restrict__ hdr, const float4* __restrict__ w
     const uint32_t t_id = unit % un.tiles, by = (unit / un.tiles) % un.groups, bz = unit / un.tiles / un.groups;
     const uint32_t ty = un.half ? (t_id / tp.tilesX) * 2 + (blockIdx.x & 1) : t_id / tp.tilesX, tx = t_id % tp.tilesX;
     const uint32_t oh0 = ty * TH, ow0 = tx * kTileW;
-    spx::pdl_launch();
     spx::pdl_wait();
+    spx::pdl_launch();
     if (oh0 >= p.Ho) return;                             // lower half of a tile that ends above it
     const uint32_t b0 = bz * BT;
     const uint32_t blk = by * NB + warp;

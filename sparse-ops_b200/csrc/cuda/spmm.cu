@@ -322,6 +322,7 @@ struct RowsArgs {
     uint64_t ldy;
     uint32_t G, RW;
     BlockMap bm;
+    bool early;                         // spmm_rows: let the successor in before the end
     uint32_t n, Cp, batch, vec_out;     // spmm_chain: rows of X, their pitch in shared memory, entries per batch, 16-byte stores
     PeerOut out;
 };
@@ -441,7 +442,6 @@ spmm_rows(const __grid_constant__ RowsArgs a)
     uint32_t rb = blockIdx.x, panel = 0;
     if (a.bm.panels > 1) decode_block(a.bm, blockIdx.x, rb, panel);
     const uint32_t slot0 = (rb * warps + warp) * RW;
-    spx::pdl_launch();
 
     WarpRows wr(a, slot0);
     wr.template start<kBatch, kRing>(a, s_w, s_k);
@@ -460,6 +460,7 @@ spmm_rows(const __grid_constant__ RowsArgs a)
     const uint32_t lrow = mine ? rl : 0u;
 
     spx::pdl_wait();
+    if (a.early) spx::pdl_launch();
     const float b = (mine && a.bias) ? __ldg(a.bias + row) : 0.0f;
     float acc[NV][V];
 #pragma unroll
@@ -529,6 +530,7 @@ spmm_rows(const __grid_constant__ RowsArgs a)
             }
         }
     }
+    spx::pdl_launch();
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
         if (!on[v]) continue;
@@ -605,7 +607,6 @@ spmm_direct(const __grid_constant__ RowsArgs a)
     uint2* s_info = reinterpret_cast<uint2*>(s_k + kChainRing * R * stride);
     const uint32_t slot0 = blockIdx.x * R;
     const uint32_t consumers = blockDim.x - kChainProducers;
-    spx::pdl_launch();
     for (uint32_t i = threadIdx.x; i < R; i += blockDim.x) s_info[i] = slot0 + i < a.m ? __ldg(a.rows + slot0 + i) : make_uint2(0u, 0u);
     __syncthreads();
     const uint32_t nb = (s_info[0].y + E - 1) / E;                  // rows descend in length
@@ -628,6 +629,7 @@ spmm_direct(const __grid_constant__ RowsArgs a)
     if (producer)
         for (uint32_t b = 0; b + 1 < kChainRing; ++b) fill(b);
     spx::pdl_wait();
+    spx::pdl_launch();
     stage_x(s_mem, a, Cp);
 
     if (producer) {
@@ -726,7 +728,6 @@ spmm_chain(const __grid_constant__ RowsArgs a)
     float* s_x = s_w + 2 * kPreRing * R * stride;                 // [2][row][column][entry]
     uint2* s_info = reinterpret_cast<uint2*>(s_x + 2 * R * C * stride);
     const uint32_t slot0 = blockIdx.x * R;
-    spx::pdl_launch();
     for (uint32_t i = threadIdx.x; i < R; i += kPreThreads) s_info[i] = slot0 + i < a.m ? __ldg(a.rows + slot0 + i) : make_uint2(0u, 0u);
     __syncthreads();
     const uint32_t nb = (s_info[0].y + E - 1) / E;                  // rows descend in length
@@ -751,6 +752,7 @@ spmm_chain(const __grid_constant__ RowsArgs a)
     if (producer)
         for (uint32_t b = 0; b < kPreRing - 2; ++b) fill(b);
     spx::pdl_wait();
+    spx::pdl_launch();
     stage_x(s_mem, a, Cp);
 
     if (producer) {
@@ -929,6 +931,10 @@ static int launch_rows_one(const spx_ell* e, RowsArgs a, uint32_t panels, uint32
     a.bm.panels = panels;
     a.bm.head = panels > 1 ? std::min<uint32_t>(a.bm.row_blocks, (uint32_t)((e->long_rows + rows_per_block - 1) / rows_per_block)) : 0u;
     a.bm.blocks = a.bm.row_blocks * panels;
+    // The successor may come in while this grid runs if both fit the GPU whole; otherwise its first CTAs crowd the SMs
+    // that are done early, and it runs out of balance (690 x 4077, 21 %, C = 128 28.4 us against 24.2; 645 x 5312,
+    // 12 %, C = 32, which fits, 15.7 against 17.6).
+    a.early = (uint64_t)a.bm.blocks * wpb * 2 <= (uint64_t)sm_count(e->device) * MINB * kRowsWarps;
     auto kfn = spmm_rows<V, NV, U, MINB, PIPE>;
     if (smem > 48 * 1024) SPX_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     return finish_launch(launch_pdl(kfn, dim3(a.bm.blocks), dim3(wpb * 32), smem, s, a), "spmm_rows");

@@ -201,8 +201,8 @@ __device__ __forceinline__ void tile_steps(float4 (&acc)[NV], uint32_t at, uint3
 __global__ void __launch_bounds__(256)
 align_rows_kernel(const float* __restrict__ X, uint64_t ldx, uint32_t n, uint32_t C, uint32_t Cp, float* __restrict__ dst)
 {
-    spx::pdl_launch();
     spx::pdl_wait();
+    spx::pdl_launch();
     const uint32_t quads = Cp / 4;
     const uint64_t total = (uint64_t)n * quads;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
@@ -231,7 +231,6 @@ spmm_tile_kernel(const __grid_constant__ TileArgs a, const __grid_constant__ CUt
     const uint32_t group = rb * warps + warp;
     const bool active = group < a.groups;
     const uint32_t nactive = min(warps, a.groups - rb * warps);
-    spx::pdl_launch();
 
     // the warp's steps and counts do not depend on the predecessor kernel
     const uint32_t ring = (uint32_t)__cvta_generic_to_shared(s_mem) + kStages * kBox + kPitch + warp * (a.ring_blocks * 512u);
@@ -260,6 +259,7 @@ spmm_tile_kernel(const __grid_constant__ TileArgs a, const __grid_constant__ CUt
     // an earlier CTA's (or call's) wait ran out: leave at once
     const bool bad = __syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile int*>(a.failed) != 0);
     spx::pdl_wait();
+    spx::pdl_launch();
     if (bad) {
         asm volatile("cp.async.wait_all;" ::: "memory");
         return;

@@ -154,10 +154,10 @@ spmv_staged_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ id
     auto row_info = [&](uint32_t sl) { return rows ? __ldg(rows + sl) : make_uint2(sl, __ldg(nnz + sl)); };
     uint2 ri = live ? row_info(slot) : make_uint2(0u, 0u);
     uint32_t row = ri.x, nn = ri.y;
-    spx::pdl_launch();
     load_chunk(row, nn, lane * 4);
 
     spx::pdl_wait();                            // x, bias and y belong to the stream's order, the handle does not
+    spx::pdl_launch();
     stage_x(xs, x, n);
     landed_x();
 
@@ -232,8 +232,8 @@ spmv_ell_windowed_kernel(const float* __restrict__ Wd, const uint32_t* __restric
     const uint32_t stride = gridDim.x * groups_per_block;
     const uint32_t iters = (m + stride - 1) / stride;
     const uint32_t phases = (n + win - 1) / win;
-    spx::pdl_launch();
     spx::pdl_wait();
+    spx::pdl_launch();
 
     constexpr int UNR = 4;                      // 16-byte vectors of Wd and of idx in flight per lane
     float4 wv[UNR];
