@@ -141,7 +141,7 @@ int spx_spmm(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const f
 /* y[i] = bias[i] + sum_j Wd[i,j] * x[idx[i,j]].  Replaces ellpack_matvec
  * (src/ellpack_matvec.cpp:20-147).  bias may be NULL.  For n above 51200 (x larger than shared
  * memory) the first call builds and caches a per-row table of column-window boundaries in the
- * handle (a device allocation of up to 28 bytes per row; make that call outside a stream capture). */
+ * handle (a device allocation of up to 60 bytes per row; make that call outside a stream capture). */
 int spx_spmv(const spx_ell* e, const float* x, const float* bias, float* y, void* stream);
 /* spx_spmv in the reference's own summation order (sixteen partial sums by j mod 16, then the
  * pairwise tree of src/ellpack_matvec.cpp:88-96): bit-identical to the reference's AVX-512 path,
@@ -193,8 +193,8 @@ int spx_maxpool2d(const float* in, uint32_t C, uint32_t H, uint32_t W, uint32_t 
 int spx_global_avgpool(const float* in, uint32_t C, uint32_t H, uint32_t W, uint32_t B, float* out, void* stream);
 
 /* ---- the same calls on HOST buffers (what the reference's Python binding does) ---------- */
-/* X, bias, Y are host arrays; copies in and out go through pinned staging owned by the
- * handle's device context.  Replaces the ellpack_matmul / ellpack_matvec lambdas of
+/* X, bias, Y are host arrays; copies in and out go through pinned staging of the library
+ * (up to 24 KB with the call, 24 to 64 KB as they are, larger pageable inputs in pieces by helper threads).  Replaces the ellpack_matmul / ellpack_matvec lambdas of
  * src/bindings.cpp:91-139.  Synchronous. */
 int spx_spmm_host(const spx_ell* e, const float* X, uint32_t C, const float* bias, int act, float* Y);
 int spx_spmv_host(const spx_ell* e, const float* x, const float* bias, float* y);
