@@ -213,6 +213,10 @@ int copy_h2d_rows(void* dst, const void* src, size_t rows, size_t row, size_t st
 
 int copy_h2d(void* dst, const void* src, size_t bytes, cudaStream_t s)
 {
+    if (bytes < kPiece) {                       // one copy: each costs microseconds whatever its size
+        if (bytes) SPX_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
+        return SPX_OK;
+    }
     // as rows of 4 KB, and the rest
     const size_t whole = bytes / 4096 * 4096;
     if (int rc = copy_h2d_rows(dst, src, whole / 4096, 4096, 4096, s)) return rc;
