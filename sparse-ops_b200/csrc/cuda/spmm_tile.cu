@@ -19,8 +19,8 @@
 // Bound by shared-memory wavefronts (16 NV + 4 per step and warp) with many warps per SM, by the latency
 // of a warp's steps (0.1 us each) with few; chunks of 128 columns, six of them staged, lose 1 to 60 % to
 // the phases' fixed cost, 192 x 4 up to 4 %.  Measured against gathering: 4096 x 4096, 10 %, C = 64 / 128 / 256 / 512
-// 23.8 / 36.2 / 65.5 / 126.7 us against 28.4 / 42.3 / 72.1 / 142.4 (groups in step: 24.7 / 41.3 / 76 / 144);
-// 8192 x 8192, 10 %, C = 64 69 against 105; 3512 x 3227, 19 %, C = 160 61 against 109; 4927 x 3082, 21 %, C = 160 93 against 170.
+// 23.9 / 35.4 / 61.3 / 121.7 us against 28.4 / 42.3 / 72.1 / 142.4 (groups in step: 24.7 / 41.3 / 76 / 144);
+// 8192 x 8192, 10 %, C = 64 68 against 105; 3512 x 3227, 19 %, C = 160 61 against 109; 4927 x 3082, 21 %, C = 160 93 against 170.
 #include "common.cuh"
 #include "tma.cuh"
 #include "peer_out.cuh"
@@ -228,9 +228,11 @@ spmm_tile_kernel(const __grid_constant__ TileArgs a, const __grid_constant__ CUt
     __shared__ uint32_t s_asked;                            // copies asked for
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const uint32_t slice = blockIdx.x / a.row_blocks, rb = blockIdx.x % a.row_blocks;
-    const uint32_t group = rb * warps + warp;
+    // Groups come in descending length: dealt round, every CTA gets its share of the long ones (4096 x 4096, 10 %: the
+    // first CTA in order had 12 % more to read from shared memory than the average: C = 256 65.7 us against 61.3).
+    const uint32_t group = warp * a.row_blocks + rb;
     const bool active = group < a.groups;
-    const uint32_t nactive = min(warps, a.groups - rb * warps);
+    const uint32_t nactive = (a.groups - rb + a.row_blocks - 1) / a.row_blocks;    // at least warp 0: row_blocks <= groups
 
     // the warp's steps and counts do not depend on the predecessor kernel
     const uint32_t ring = (uint32_t)__cvta_generic_to_shared(s_mem) + kStages * kBox + kPitch + warp * (a.ring_blocks * 512u);
