@@ -270,6 +270,8 @@ SPMM_EDGE_CASES = [
     (50, 40000, 1, 0.01), (90, 3000, 37, 0.2), (300, 900, 139, 0.1), (257, 1200, 258, 0.1), (65, 700, 1007, 0.05), (2, 5000, 132, 0.3),
     # X staged block by block from the second call on: aligned, a last group of 1 row, C not a multiple of 4
     (1312, 2080, 160, 0.27), (601, 1537, 100, 0.5), (1201, 1100, 77, 0.5),
+    # its chunks of 256 columns, three of them staged: one, one and a column, all stages and a column; sparse rows
+    (5, 256, 64, 0.5), (130, 257, 32, 0.3), (700, 769, 68, 0.04), (1031, 3000, 96, 0.01),
 ]
 
 
