@@ -308,10 +308,13 @@ spmm_tile_kernel(const __grid_constant__ TileArgs a, const __grid_constant__ CUt
         if (c + 1 < kWindow) continue;
         __syncwarp();
         // No later phase reads chunk c + 1 - kWindow: the last warp to get here asks for the chunk that takes its
-        // place.  The arrival tells whether it is the last (one pending before it); a fence and an atomic instead
+        // place.  The arrival tells whether it is the last (one pending before it) and releases this warp's reads;
+        // the wait for the phase it has just completed (no waiting: it is complete) acquires the other warps'
+        // arrivals, so that all reads of the stage come before the copy unit's writes.  A fence and an atomic instead
         // would wait for the warp's cp.async in flight, 1500 cycles per chunk.
-        const uint32_t out = c + 1 - kWindow;
-        if (lane == 0 && spx::mbar_arrive_pending(&s_free[out % kStages]) == 1u && landed && out + kStages < a.chunks) {
+        const uint32_t out = c + 1 - kWindow, st = out % kStages;
+        if (lane == 0 && spx::mbar_arrive_pending(&s_free[st]) == 1u && landed && out + kStages < a.chunks &&
+            spx::mbar_wait(&s_free[st], (out / kStages) & 1u)) {
             ask(out + kStages);
             atomicAdd(&s_asked, 1u);
         }
