@@ -190,6 +190,15 @@ int set_row_order(spx_ell* e, const uint32_t* host_nnz);
 // The sort behind it: fills order[m], and the handle's long_rows / min_nnz; e->rows is allocated.
 int sort_rows(spx_ell* e, const uint32_t* host_nnz, uint2* order, cudaStream_t s);
 
+// While it lives, this thread may allocate and wait although it is recording a graph on another stream (such a call
+// would otherwise end that capture with an error).  What runs under it does not touch the stream being recorded.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+    RelaxedCapture(const RelaxedCapture&) = delete;
+};
+
 // Device memory from the library's pool of the given device, stream-ordered (mem.cu).
 int pool_alloc(void** p, size_t bytes, int device, cudaStream_t s);
 void pool_free(void* p, size_t bytes, cudaStream_t s);      // bytes as allocated; p may be null

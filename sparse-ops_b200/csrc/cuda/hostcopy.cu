@@ -155,6 +155,16 @@ bool pageable_memory(const void* p) {
     return at.type == cudaMemoryTypeUnregistered;
 }
 
+// A copy that is being recorded into a graph stays one copy node on the caller's memory: what the ring holds and
+// what its events stand for belong to this call, not to the graph's launches.
+static bool being_captured(cudaStream_t s)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) == cudaSuccess) return cap != cudaStreamCaptureStatusNone;
+    (void)cudaGetLastError();
+    return true;
+}
+
 int copy_h2d_rows(void* dst, const void* src, size_t rows, size_t row, size_t stride, cudaStream_t s)
 {
     const size_t bytes = rows * row;
@@ -165,8 +175,10 @@ int copy_h2d_rows(void* dst, const void* src, size_t rows, size_t row, size_t st
         return SPX_OK;
     };
     int device = -1;
-    if (bytes < kPiece || row > kPiece || !pageable_memory(src) || cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxDevices)
+    if (bytes < kPiece || row > kPiece || !pageable_memory(src) || being_captured(s) || cudaGetDevice(&device) != cudaSuccess ||
+        device < 0 || device >= kMaxDevices)
         return plain();
+    RelaxedCapture relaxed;                     // allocations and waits of the ring: no business of a capture on another stream
     Helpers& h = Helpers::get();
     std::unique_lock<std::mutex> lk(h.user, std::try_to_lock);
     if (lk.owns_lock() && !g_ring.half[0]) {
