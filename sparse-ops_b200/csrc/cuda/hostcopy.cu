@@ -217,7 +217,10 @@ int copy_h2d_rows(void* dst, const void* src, size_t rows, size_t row, size_t st
             if (spins < 20000) SPX_PAUSE(); else std::this_thread::yield();
         }
         if (err == cudaSuccess) err = cudaEventRecord(g_ring.free_at[device][half], s);
-        if (err != cudaSuccess) return fail(SPX_ERR_CUDA, "host to device copy failed: %s", cudaGetErrorString(err));
+        if (err != cudaSuccess) {               // no event tells when this half is free: it is when the stream has run dry
+            (void)cudaStreamSynchronize(s);
+            return fail(SPX_ERR_CUDA, "host to device copy failed: %s", cudaGetErrorString(err));
+        }
         g_ring.last_device[half] = device;
     }
     return SPX_OK;

@@ -109,6 +109,21 @@ int main(int argc, char** argv)
         CHECK(!fake::recording_broken);
         CHECK(cudaStreamSynchronize(a.handle()) == cudaSuccess);
         CHECK(dst == src);
+    } else if (what == "failed_copy") {
+        // a copy that fails half way: what it had sent arrives intact although the ring is used again at once
+        for (int nth = 2; nth <= 6; ++nth) {
+            const size_t n = 12 << 20, piece = 256 * 1024;
+            Bytes src = noise(n, 20 + nth), dst(n, 0x11), none(n, 0x11);
+            fake::fail_copy_in = nth;
+            const int rc = spx::copy_h2d(dst.data(), src.data(), n, a.handle());
+            const bool failed = fake::fail_copy_in == 0;
+            fake::fail_copy_in = 0;
+            CHECK(failed ? rc != 0 : rc == 0);
+            contiguous(b, nth);
+            CHECK(cudaStreamSynchronize(a.handle()) == cudaSuccess);
+            for (size_t at = 0; at < n; at += piece)
+                CHECK(!memcmp(&dst[at], &src[at], piece) || !memcmp(&dst[at], &none[at], piece));
+        }
     } else {
         printf("unknown scenario\n");
         return 2;
