@@ -165,6 +165,16 @@ static bool being_captured(cudaStream_t s)
     return true;
 }
 
+// Whether the stream belongs to the device: the ring's events are made on the current one and can be recorded on no other's.
+static bool stream_of(cudaStream_t s, int device)
+{
+    int owner = device;
+    if (!s || s == cudaStreamLegacy || s == cudaStreamPerThread) return true;
+    if (cudaStreamGetDevice(s, &owner) == cudaSuccess) return owner == device;
+    (void)cudaGetLastError();
+    return false;
+}
+
 int copy_h2d_rows(void* dst, const void* src, size_t rows, size_t row, size_t stride, cudaStream_t s)
 {
     const size_t bytes = rows * row;
@@ -176,7 +186,7 @@ int copy_h2d_rows(void* dst, const void* src, size_t rows, size_t row, size_t st
     };
     int device = -1;
     if (bytes < kPiece || row > kPiece || !pageable_memory(src) || being_captured(s) || cudaGetDevice(&device) != cudaSuccess ||
-        device < 0 || device >= kMaxDevices)
+        device < 0 || device >= kMaxDevices || !stream_of(s, device))
         return plain();
     RelaxedCapture relaxed;                     // allocations and waits of the ring: no business of a capture on another stream
     Helpers& h = Helpers::get();

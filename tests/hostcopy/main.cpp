@@ -124,6 +124,14 @@ int main(int argc, char** argv)
             for (size_t at = 0; at < n; at += piece)
                 CHECK(!memcmp(&dst[at], &src[at], piece) || !memcmp(&dst[at], &none[at], piece));
         }
+    } else if (what == "other_device") {
+        // streams of a device that is not current take copies as well
+        b.device = 1;
+        contiguous(a, 1);
+        contiguous(b, 2);
+        fake::current_device = 1;
+        contiguous(a, 3);
+        contiguous(b, 4);
     } else {
         printf("unknown scenario\n");
         return 2;

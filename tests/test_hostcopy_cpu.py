@@ -25,7 +25,7 @@ def driver(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("scenario", ["sizes", "panels", "threads", "capture", "capture_elsewhere", "failed_copy"])
+@pytest.mark.parametrize("scenario", ["sizes", "panels", "threads", "capture", "capture_elsewhere", "failed_copy", "other_device"])
 def test_staged_copies(driver, scenario):
     r = subprocess.run([driver, scenario], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
