@@ -121,6 +121,14 @@ int spx_ell_create_csr(uint32_t m, uint32_t n, const uint64_t* rowptr, const uin
  * convert_to_ellpack (src/ellpack_encoder.cpp:6-44): entries with v != 0.0f, ascending columns. */
 int spx_ell_encode_device(const float* dW, uint32_t m, uint32_t n, void* stream, spx_ell** out);
 int spx_ell_destroy(spx_ell* e);
+/* Kernels that fetch an operand with bulk tensor copies (spx_spmm where it stages X block by block, spx_conv2d's
+ * row-block-merged kernel) wait for them with a limit of about a second.  Should a wait ever run out, the call in
+ * flight has returned SPX_OK but its output is invalid.  The failure is then reported as SPX_ERR_CUDA: by the
+ * *_host call itself, else by the next spx_spmm or spx_conv2d on the handle, before it launches anything, or by this
+ * function, for callers that replay a captured graph (ask after the stream has been waited for).  From then on the
+ * handle does without bulk copies; a graph captured before still holds the kernels that use them, writes nothing and
+ * reports again, until it is captured anew.  Does not synchronise. */
+int spx_ell_status(const spx_ell* e);
 int spx_ell_dims(const spx_ell* e, uint32_t* m, uint32_t* n, uint32_t* r, uint64_t* nnz_total);
 /* Copy back in the reference layout (any pointer may be NULL). */
 int spx_ell_download(const spx_ell* e, float* Wd, uint32_t* idx, uint32_t* nnz);
@@ -135,7 +143,8 @@ int spx_ell_decode_device(const spx_ell* e, float* dW, void* stream);
  * Where staging X block by block is the faster way (columns used several times by a CTA's rows), the
  * second such call on a handle builds and keeps another form of the matrix (about the size of its
  * entries; that call waits for the stream, other threads' calls on the handle wait for it) and later
- * calls use it; a call inside a stream capture never builds it.  Results are the same either way. */
+ * calls use it; a call inside a stream capture never builds it.  Results are the same either way.  That
+ * kernel fetches X with bulk tensor copies: see spx_ell_status. */
 int spx_spmm(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const float* bias,
              int act, float* Y, uint64_t ldy, void* stream);
 /* y[i] = bias[i] + sum_j Wd[i,j] * x[idx[i,j]].  Replaces ellpack_matvec
@@ -155,9 +164,7 @@ int spx_spmv_reference_order(const spx_ell* e, const float* x, const float* bias
  * handle and kernel shape builds and caches a tap table and, where the batch size and weight
  * density favour it, the row-block-merged form of the weights (device allocations; make that
  * call outside a stream capture).  Results do not depend on which kernel is chosen.  The
- * row-block-merged kernel fetches its input with bulk tensor copies and bounded waits; should a
- * wait ever run out, the next spx_conv2d on the handle returns SPX_ERR_CUDA once (the output of
- * the call that was in flight is invalid) and the handle falls back to per-thread copies. */
+ * row-block-merged kernel fetches its input with bulk tensor copies: see spx_ell_status. */
 int spx_conv2d(const spx_ell* e, const spx_conv_geom* g, int layout, const float* in, uint32_t B,
                const float* bias, int act, float* out, void* stream);
 /* spx_conv2d for callers that must not allocate device memory (no counterpart in the

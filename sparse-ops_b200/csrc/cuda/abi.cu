@@ -3,6 +3,7 @@
 // argument validation in front of every kernel launcher, and the host-buffer entry points
 // that copy operands through pinned staging.
 #include "common.cuh"
+#include "tma.cuh"
 
 #include <dlfcn.h>
 
@@ -437,6 +438,12 @@ int spx_ell_dims(const spx_ell* e, uint32_t* m, uint32_t* n, uint32_t* r, uint64
     return SPX_OK;
 }
 
+int spx_ell_status(const spx_ell* e)
+{
+    if (!e) return fail(SPX_ERR_ARG, "handle is null");
+    return check_tma_words(const_cast<spx_ell*>(e), "ell_status");
+}
+
 int spx_ell_download(const spx_ell* e, float* Wd, uint32_t* idx, uint32_t* nnz)
 {
     if (!e) return fail(SPX_ERR_ARG, "handle is null");
@@ -834,14 +841,14 @@ int spx_spmm_host(const spx_ell* ce, const float* X, uint32_t C, const float* bi
         cudaStreamSynchronize(s_mm);
         if (rc != SPX_OK) return rc;
         if (err != cudaSuccess) return fail(SPX_ERR_CUDA, "spmm_host: pipelined copy failed: %s", cudaGetErrorString(err));
-        return SPX_OK;
+        return check_tma_words(e, "spmm_host");
     }
     // Medium operands: two column panels, so that the copy in of one runs beside the multiply and the copy out
     // of the other (4096 x 4096, C = 256: 305 -> 260 us).  A panel of X is packed on its way in.
     // Panel rows of whole 128-byte lines only: the copy unit moved 4096 rows of 272 bytes in 600 us.
     if (C % 64 == 0 && (size_t)e->n * C * 4 >= kPanelBytes && (size_t)e->m * C * 4 >= kPanelBytes) {
         rc = spmm_host_panels(e, X, C, bias, act, Y, dX, dB, dY);
-        return rc;
+        return rc != SPX_OK ? rc : check_tma_words(e, "spmm_host");
     }
     const size_t y_bytes = (size_t)e->m * C * 4;
     HostCall call;
@@ -850,8 +857,8 @@ int spx_spmm_host(const spx_ell* ce, const float* X, uint32_t C, const float* bi
     if (rc != SPX_OK) return rc;
     float* direct = y_bytes <= HostCall::kSmall && C >= 8 ? call.mapped_result() : nullptr;
     rc = spx_spmm(e, dX, C, C, bias ? dB : nullptr, act, direct ? direct : dY, C, call.stream);
-    if (rc != SPX_OK) return rc;
-    return call.finish(Y, direct ? nullptr : dY, y_bytes);
+    if (rc == SPX_OK) rc = call.finish(Y, direct ? nullptr : dY, y_bytes);
+    return rc != SPX_OK ? rc : check_tma_words(e, "spmm_host");
 }
 
 // Row-sharded SpMM on host buffers, one process per GPU.  Every rank holds the same host X but
@@ -945,7 +952,7 @@ int spx_spmm_host_sharded(spx_comm* comm, const spx_ell* ce, const float* X, uin
                 float ms = 0.0f;
                 if (cudaEventElapsedTime(&ms, ev(p, ph, 0), ev(p, ph, 1)) == cudaSuccess) phase_ms[ph] += ms;
             }
-    return SPX_OK;
+    return check_tma_words(e, "spmm_host_sharded");
 }
 
 int spx_spmv_host(const spx_ell* ce, const float* x, const float* bias, float* y)

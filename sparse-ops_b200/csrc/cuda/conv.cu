@@ -563,7 +563,10 @@ conv_rbm_tile_kernel(const uint2* __restrict__ hdr, const float4* __restrict__ w
             buf_done[1] = 0;
             copies_asked = min(2u, nchunks);
         }
-        if (__syncthreads_or(*reinterpret_cast<volatile int*>(tma_failed) != 0)) return;
+        if (__syncthreads_or(*reinterpret_cast<volatile int*>(tma_failed) != 0)) {
+            if (threadIdx.x == 0) *tma_failed_host = 1;     // nothing is written: said again, for a graph's launches
+            return;
+        }
         if (threadIdx.x == 0) {
             mbar_expect_tx(&tile_bar[0], box_bytes);
             tma_load_4d(tile, &tmap, (int)b0, iw0, ih0, 0, &tile_bar[0]);
@@ -969,7 +972,6 @@ static int launch_conv_rbm_tile(spx_ell* e, const ConvParams& p, const ConvViews
 {
     static const int enabled = [] { const char* v = getenv("SPX_CONV_RBM"); return v ? atoi(v) : 1; }();
     static const double share_env = [] { const char* v = getenv("SPX_CONV_RBM_MIN_SHARE"); return v ? atof(v) : -1.0; }();
-    if (int rc = check_tma_words(e, "conv2d")) return rc;     // the handle stages with per-thread copies from then on
     // fewer than 8 row blocks would leave most of the CTA's 16 warps without work
     if (!enabled || e->n > kRbmMaxK || e->m < 8 * kRbmRows - 3 || e->max_nnz == 0) return -1;
     if (p.B % 4) return -1;
@@ -1104,6 +1106,7 @@ int launch_conv2d(spx_ell* e, const spx_conv_geom* g, int layout, const float* i
                   const float* bias, int act, float* out, cudaStream_t s)
 {
     if (e->m == 0 || B == 0 || g->Ho == 0 || g->Wo == 0) return SPX_OK;
+    if (int rc = check_tma_words(e, "conv2d")) return rc;     // the handle stages with per-thread copies from then on
     if (g->kH > 255 || g->kW > 255 || g->Cin > 65535)
         return fail(SPX_ERR_LIMIT, "conv2d: kernel extent > 255 or Cin > 65535 not supported");
     // A 1 x 1 convolution is an SpMM whose columns are the positions (times the batch where that is the innermost

@@ -204,7 +204,7 @@ int check_tma_words(spx_ell* e, const char* what)
     if (!e->tma_failed_host || !*e->tma_failed_host) return SPX_OK;
     *e->tma_failed_host = 0;
     e->tma_off = true;
-    return fail(SPX_ERR_CUDA, "%s: a bulk tensor copy of an earlier call on this handle did not complete; its output is invalid", what);
+    return fail(SPX_ERR_CUDA, "%s: a bulk tensor copy of a call on this handle did not complete; that call's output is invalid", what);
 }
 
 PFN_cuTensorMapEncodeTiled tensor_map_encoder()

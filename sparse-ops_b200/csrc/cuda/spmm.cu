@@ -19,6 +19,7 @@
 // and the CTAs of a wave carry equal work.
 #include "common.cuh"
 #include "peer_out.cuh"
+#include "tma.cuh"
 
 #include <algorithm>
 #include <cstdlib>
@@ -1071,6 +1072,7 @@ int launch_spmm_bcast(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx
     if (e->m == 0 || C == 0) return SPX_OK;
     if (npeers == 0 || npeers > (uint32_t)kMaxPeers) return fail(SPX_ERR_LIMIT, "spmm: 1..%d destination buffers supported", kMaxPeers);
     if (mcast && npeers != 1) return fail(SPX_ERR_ARG, "spmm: a multicast destination is one address");
+    if (int rc = check_tma_words(const_cast<spx_ell*>(e), "spmm")) return rc;
     PeerOut out{};
     out.n = (int)npeers;
     out.mcast = mcast ? 1 : 0;

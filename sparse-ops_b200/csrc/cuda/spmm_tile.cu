@@ -149,6 +149,7 @@ struct TileArgs {
     uint64_t ldy;
     int* failed;
     int* failed_host;
+    uint32_t missing;           // tests: bytes waited for that no copy brings
     PeerOut out;
 };
 
@@ -226,7 +227,7 @@ spmm_tile_kernel(const __grid_constant__ TileArgs a, const __grid_constant__ CUt
     __shared__ __align__(8) uint64_t s_bar[kStages];
     __shared__ __align__(8) uint64_t s_free[kStages];       // arrivals of the warps that no longer read the chunk in stage s
     __shared__ uint32_t s_asked;                            // copies asked for
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t slice = blockIdx.x / a.row_blocks, rb = blockIdx.x % a.row_blocks;
     // Groups come in descending length: dealt round, every CTA gets its share of the long ones (4096 x 4096, 10 %: the
     // first CTA in order had 12 % more to read from shared memory than the average: C = 256 65.7 us against 61.3).
@@ -262,13 +263,14 @@ spmm_tile_kernel(const __grid_constant__ TileArgs a, const __grid_constant__ CUt
     const bool bad = __syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile int*>(a.failed) != 0);
     spx::pdl_wait();
     spx::pdl_launch();
-    if (bad) {
+    if (bad) {                                  // this call's output is not written either: said again, for a graph's launches
+        if (threadIdx.x == 0) *a.failed_host = 1;
         asm volatile("cp.async.wait_all;" ::: "memory");
         return;
     }
     auto ask = [&](uint32_t c) {                // by one thread: chunk c into stage c % kStages
         const uint32_t st = c % kStages;
-        spx::mbar_expect_tx(&s_bar[st], kBox);
+        spx::mbar_expect_tx(&s_bar[st], kBox + a.missing);
         spx::tma_load_2d(s_mem + st * kBox, &tmap, (int)(slice * 32u * NV), (int)(c * kChunk), &s_bar[st]);
     };
     if (threadIdx.x == 0)
@@ -524,7 +526,6 @@ int launch_spmm_tile(spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const
         }
         if (t->state != 1) return -1;
     }
-    if (int rc = check_tma_words(e, "spmm")) return rc;
     void* aligned = nullptr;
     const uint32_t Cp = round_up(C, 4u);
     const size_t aligned_bytes = (size_t)e->n * Cp * 4;
@@ -551,6 +552,10 @@ int launch_spmm_tile(spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const
         a.m = e->m; a.groups = t->groups; a.chunks = t->chunks; a.C = C; a.vec_out = vec_out;
         a.bias = bias; a.act = act; a.ldy = ldy; a.out = out;
         a.failed = e->tma_failed_dev; a.failed_host = e->tma_failed_mapped;
+        // SPX_SPMM_TMA_TEST_TIMEOUT=k: the waits of the process's k-th launch run out
+        static const int timeout_env = [] { const char* v = getenv("SPX_SPMM_TMA_TEST_TIMEOUT"); return v ? atoi(v) : 0; }();
+        static std::atomic<int> launches{0};
+        if (timeout_env && ++launches == timeout_env) a.missing = 16;
         rc = NV == 1 ? launch_tile_nv<1>(e, a, map, p.warps, p.slices, s) : launch_tile_nv<2>(e, a, map, p.warps, p.slices, s);
     }
     pool_free(aligned, aligned_bytes, s);

@@ -480,16 +480,45 @@ void SparseOnnxModel::build_exec(uint32_t B) const
     check(spx_memset(d_in, 0, size_t(in_features_) * B * sizeof(float), exec_->stream), "memset");
     for (int pass = 0; pass < 2; ++pass) launch_layers(d_in, d_out, B, exec_->stream);
     check(spx_stream_sync(exec_->stream), "warm-up pass");
+    (void)copies_failed();                      // its output is nobody's; a weight whose copies fail does without them
+    capture_layers();
+}
+
+void SparseOnnxModel::capture_layers() const
+{
+    Exec& ex = *exec_;
+    if (ex.graph) spx_graph_destroy(ex.graph);
+    ex.graph = nullptr;
     const char* no_graph = std::getenv("SPX_NO_GRAPH");
-    if (!(no_graph && no_graph[0] == '1')) {
-        if (spx_graph_capture_begin(exec_->stream) == SPX_OK) {
-            bool ok = true;
-            try { launch_layers(d_in, d_out, B, exec_->stream); } catch (...) { ok = false; }
-            void* g = nullptr;
-            if (spx_graph_capture_end(exec_->stream, &g) == SPX_OK && ok) exec_->graph = g;
-            else if (g) spx_graph_destroy(g);
-        }
+    if (no_graph && no_graph[0] == '1') return;
+    if (spx_graph_capture_begin(ex.stream) == SPX_OK) {
+        bool ok = true;
+        try { launch_layers(ex.buf.at(input_name_), ex.buf.at(output_name_), ex.B, ex.stream); } catch (...) { ok = false; }
+        void* g = nullptr;
+        if (spx_graph_capture_end(ex.stream, &g) == SPX_OK && ok) ex.graph = g;
+        else if (g) spx_graph_destroy(g);
     }
+}
+
+// Whether a bounded wait ran out in a layer's kernel since the last time this was asked.
+bool SparseOnnxModel::copies_failed() const
+{
+    bool failed = false;
+    for (const auto& L : layers_)
+        for (const Ellpack* E : {L.E.get(), L.shard.get()})
+            if (E && E->dev && spx_ell_status(E->dev) != SPX_OK) failed = true;
+    return failed;
+}
+
+// A graph's launches do not pass the check that each spx_spmm and spx_conv2d makes: it is made here, and the graph,
+// which still holds the kernels that wait for bulk copies, is captured again without them.
+void SparseOnnxModel::report_failed_copies(const char* what) const
+{
+    if (!copies_failed()) return;
+    const std::string why = spx_last_error();
+    check(spx_stream_sync(exec_->stream), what);
+    capture_layers();
+    throw std::runtime_error(std::string(what) + ": " + why);
 }
 
 // The layer loop (reference: src/model_run.cpp:28-127).  Buffers were planned in build_exec;
@@ -583,11 +612,13 @@ void SparseOnnxModel::run(const float* input, uint32_t B, float* output, bool pi
     if (!pinned_output && ex.h_out && ex.h_out_bytes == out_bytes) {
         check(spx_memcpy_d2h(ex.h_out, d_out, out_bytes, ex.stream), "output copy");
         check(spx_stream_sync(ex.stream), "run");
+        report_failed_copies("run");
         std::memcpy(output, ex.h_out, out_bytes);
         return;
     }
     check(spx_memcpy_d2h(output, d_out, out_bytes, ex.stream), "output copy");
     check(spx_stream_sync(ex.stream), "run");
+    report_failed_copies("run");
 }
 
 size_t SparseOnnxModel::activation_buffers() const
@@ -611,6 +642,7 @@ float* SparseOnnxModel::device_output() const
 void SparseOnnxModel::run_resident(void* stream) const
 {
     if (!exec_) throw std::runtime_error("run_resident: call resize_buffers(B) first");
+    report_failed_copies("run_resident");       // of the launches before
     if (exec_->graph) check(spx_graph_launch(exec_->graph, stream), "graph launch");
     else launch_layers(device_input(), device_output(), exec_->B, stream);
 }

@@ -102,6 +102,9 @@ private:
     void build_exec(uint32_t B) const;
     bool exchange_peer_buffers(Exec& ex, const std::vector<std::string>& names) const;
     void launch_layers(const float* d_in, float* d_out, uint32_t B, void* stream) const;
+    void capture_layers() const;
+    bool copies_failed() const;
+    void report_failed_copies(const char* what) const;
 
     std::vector<Layer> layers_;
     uint32_t batch_dim_ = 1;

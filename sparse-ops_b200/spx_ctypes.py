@@ -76,6 +76,7 @@ SIGNATURES = {
     "spx_ell_create_csr": (C.c_int, [C.c_uint32, C.c_uint32, _vp, _vp, _vp, C.POINTER(_vp)]),
     "spx_ell_encode_device": (C.c_int, [_vp, C.c_uint32, C.c_uint32, _vp, C.POINTER(_vp)]),
     "spx_ell_destroy": (C.c_int, [_vp]),
+    "spx_ell_status": (C.c_int, [_vp]),
     "spx_ell_dims": (C.c_int, [_vp, _u32p, _u32p, _u32p, _u64p]),
     "spx_ell_download": (C.c_int, [_vp, _vp, _vp, _vp]),
     "spx_ell_decode_device": (C.c_int, [_vp, _vp, _vp]),

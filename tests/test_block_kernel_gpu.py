@@ -60,3 +60,89 @@ def test_stage_refills(lib, orc, cuda, m, n, C, p):
 
 def test_stage_refills_forced():
     in_child("test_stage_refills and not forced", SPX_SPMM_TILE="2")
+
+
+# ---- a bounded wait that runs out -----------------------------------------------------------------
+def small_case(orc, seed=5):
+    rng = np.random.default_rng(seed)
+    m, n, C = 300, 1500, 64
+    W = sparse(rng, m, n, 0.1)
+    X = rng.uniform(-1, 1, (n, C)).astype(np.float32)
+    b = rng.standard_normal(m).astype(np.float32)
+    E = orc.encode(W)
+    return m, n, C, W, X, b, E, orc.spmm(E, X, b, act=1)
+
+
+def test_timeout_of_a_call(lib, orc, cuda):
+    if os.environ.get("SPX_SPMM_TMA_TEST_TIMEOUT") != "1":
+        pytest.skip("runs in a child process of test_timeouts_are_reported")
+    m, n, C, W, X, b, E, want = small_case(orc)
+    h = lib.ell_create(E.Wd, E.idx, E.nnz, E.n)
+    dX, dB, dY = torch.from_numpy(X).to(cuda), torch.from_numpy(b).to(cuda), torch.zeros((m, C), device=cuda)
+    run = lambda: h.spmm(dX.data_ptr(), C, C, dB.data_ptr(), sx.ACT_RELU, dY.data_ptr(), C)
+    run()                                   # gathered
+    run()                                   # enqueued fine; on the GPU a wait gives up after a second
+    torch.cuda.synchronize()                # the context is still usable
+    y1 = torch.zeros(m, device=cuda)
+    with pytest.raises(sx.SpxError, match="bulk tensor copy") as err:       # any width reports it, whichever kernel it would take
+        h.spmm(dX.data_ptr(), 1, C, dB.data_ptr(), 0, y1.data_ptr(), 1)
+    assert err.value.status == 2
+    for k in range(3):                      # no bulk copies from here on
+        dY.fill_(float("nan"))
+        run()
+        torch.cuda.synchronize()
+        assert_bit_equal(dY.cpu().numpy(), want, "after the report")
+    lib.spx_ell_status(h.h)
+
+
+def test_timeout_of_a_host_call(lib, orc, cuda):
+    if os.environ.get("SPX_SPMM_TMA_TEST_TIMEOUT") != "1":
+        pytest.skip("runs in a child process of test_timeouts_are_reported")
+    m, n, C, W, X, b, E, want = small_case(orc)
+    h = lib.ell_create(E.Wd, E.idx, E.nnz, E.n)
+    assert_bit_equal(h.spmm_host(X, b, sx.ACT_RELU), want, "gathered")
+    with pytest.raises(sx.SpxError, match="bulk tensor copy"):
+        h.spmm_host(X, b, sx.ACT_RELU)
+    assert_bit_equal(h.spmm_host(X, b, sx.ACT_RELU), want, "after the report")
+
+
+@pytest.mark.parametrize("how", ["run", "resident"])
+def test_timeout_of_a_replay(lib, orc, backend, cuda, tmp_path, how):
+    """The graph's kernel waits in vain: run() fails instead of handing over a stale output, run_resident() fails on its
+    next call; both work after that."""
+    if os.environ.get("SPX_SPMM_TMA_TEST_TIMEOUT") != "2":
+        pytest.skip("runs in a child process of test_timeouts_are_reported")
+    import onnx_wire
+    m, n, C, W, X, b, E, want = small_case(orc)
+    path = tmp_path / "one.onnx"
+    path.write_bytes(onnx_wire.mlp_model([W], [b], ["Relu"], C))
+    model = backend.SparseOnnxModel(str(path))
+    model.resize_buffers(C)                 # first launch: the warm-up pass; second: the captured one, which fails
+    out = None
+    if how == "run":
+        with pytest.raises(RuntimeError, match="bulk tensor copy"):
+            model.run(X.reshape(C, n))
+        for k in range(2):
+            out = np.asarray(model.run(X.reshape(C, n)))
+            assert_bit_equal(out.reshape(m, C), want, "after the report")
+        return
+    dX, dY = torch.from_numpy(X).to(cuda), torch.full((m, C), 7.0, device=cuda)
+    lib.spx_memcpy_d2d(model.device_input_ptr(), dX.data_ptr(), dX.numel() * 4, 0)
+    torch.cuda.synchronize()
+    model.run_resident(0)
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="bulk tensor copy"):
+        model.run_resident(0)
+    model.run_resident(0)
+    torch.cuda.synchronize()
+    lib.spx_memcpy_d2d(dY.data_ptr(), model.device_output_ptr(), dY.numel() * 4, 0)
+    torch.cuda.synchronize()
+    assert_bit_equal(dY.cpu().numpy(), want, "after the report")
+
+
+@pytest.mark.parametrize("name,launch", [("test_timeout_of_a_call", "1"), ("test_timeout_of_a_host_call", "1"),
+                                         ("test_timeout_of_a_replay and run]", "2"), ("test_timeout_of_a_replay and resident]", "2")])
+def test_timeouts_are_reported(name, launch):
+    """With the switch a barrier expects more bytes than its copy brings, so the kernel's bounded wait runs out (nothing
+    faults, nothing hangs): an error, never a stale result."""
+    in_child(name, SPX_SPMM_TILE="2", SPX_SPMM_TMA_TEST_TIMEOUT=launch)
