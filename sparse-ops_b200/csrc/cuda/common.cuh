@@ -190,6 +190,18 @@ int set_row_order(spx_ell* e, const uint32_t* host_nnz);
 // The sort behind it: fills order[m], and the handle's long_rows / min_nnz; e->rows is allocated.
 int sort_rows(spx_ell* e, const uint32_t* host_nnz, uint2* order, cudaStream_t s);
 
+// Lets a kernel have all the dynamic shared memory a CTA can get.  The limit belongs to the function and not to a
+// launch: were it set to each launch's own size, another thread's call could lower it between this one's setting and
+// its launch, which would be refused.  So it is set once per kernel and device, to the most.
+int allow_smem(const void* kernel, int device, std::atomic<uint64_t>& done);     // mem.cu
+template <auto Kernel>
+int allow_smem(int device)
+{
+    static std::atomic<uint64_t> done{0};           // a bit per device
+    if (device < 64 && (done.load(std::memory_order_relaxed) >> device & 1)) return SPX_OK;
+    return allow_smem(reinterpret_cast<const void*>(Kernel), device, done);
+}
+
 // While it lives, this thread may allocate and wait although it is recording a graph on another stream (such a call
 // would otherwise end that capture with an error).  What runs under it does not touch the stream being recorded.
 struct RelaxedCapture {

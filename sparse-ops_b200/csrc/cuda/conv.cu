@@ -731,10 +731,8 @@ template <int QB, int G, int WARPS, int MINB>
 static int launch_tile_qb(const spx_ell* e, const TileParams& tp, dim3 grid, size_t smem, const float* in,
                           const float* bias, int act, float* out, cudaStream_t s)
 {
-    auto kfn = conv_pf_tile_kernel<QB, G, WARPS, MINB>;
-    cudaError_t err = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err != cudaSuccess) return fail(SPX_ERR_CUDA, "conv2d: shared memory opt-in failed: %s", cudaGetErrorString(err));
-    kfn<<<grid, WARPS * 32, smem, s>>>(e->Wd, e->taps, e->nnz, e->pitch, tp, in, bias, act, out);
+    if (int rc = allow_smem<conv_pf_tile_kernel<QB, G, WARPS, MINB>>(e->device)) return rc;
+    conv_pf_tile_kernel<QB, G, WARPS, MINB><<<grid, WARPS * 32, smem, s>>>(e->Wd, e->taps, e->nnz, e->pitch, tp, in, bias, act, out);
     SPX_LAUNCH_CHECK("conv_pf_tile_kernel");
     return SPX_OK;
 }
@@ -853,10 +851,8 @@ static int launch_rbm_units(const spx_ell* e, TileParams tp, RbmUnits un, uint32
         }
     }
     const size_t smem = use_tma ? (size_t)tp.stage * (p.Cin > tp.CC ? 2 : 1) * sizeof(float) : chanBytes * tp.CC;
-    auto kfn = conv_rbm_tile_kernel<QB, NB, G>;
-    cudaError_t err = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err != cudaSuccess) return fail(SPX_ERR_CUDA, "conv2d: shared memory opt-in failed: %s", cudaGetErrorString(err));
-    err = launch_pdl(kfn, dim3(ctas), dim3(NB * 32), smem, s, e->rbm_hdr, reinterpret_cast<const float4*>(e->rbm_w), e->rbm_ncols,
+    if (int rc = allow_smem<conv_rbm_tile_kernel<QB, NB, G>>(e->device)) return rc;
+    const cudaError_t err = launch_pdl(conv_rbm_tile_kernel<QB, NB, G>, dim3(ctas), dim3(NB * 32), smem, s, e->rbm_hdr, reinterpret_cast<const float4*>(e->rbm_w), e->rbm_ncols,
                      e->rbm_cap, tp, un, in, bias, act, out, map, use_tma, e->tma_failed_dev, e->tma_failed_mapped);
     if (err != cudaSuccess) return fail(SPX_ERR_CUDA, "launch of conv_rbm_tile_kernel failed: %s", cudaGetErrorString(err));
     count_launch();

@@ -182,6 +182,17 @@ void pinned_release(const PinnedBlock& b)
     (void)cudaFreeHost(b.host);
 }
 
+int allow_smem(const void* kernel, int device, std::atomic<uint64_t>& done)
+{
+    int most = 0;
+    cudaFuncAttributes fa{};
+    SPX_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    SPX_CUDA(cudaFuncGetAttributes(&fa, kernel));
+    SPX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fa.sharedSizeBytes));
+    if (device < 64) done.fetch_or(1ull << device, std::memory_order_relaxed);
+    return SPX_OK;
+}
+
 void ensure_tma_words(spx_ell* e)
 {
     if (e->tma_failed_host || pinned_acquire(sizeof(int), &e->tma_failed_block) != SPX_OK) return;

@@ -936,9 +936,8 @@ static int launch_rows_one(const spx_ell* e, RowsArgs a, uint32_t panels, uint32
     // that are done early, and it runs out of balance (690 x 4077, 21 %, C = 128 28.4 us against 24.2; 645 x 5312,
     // 12 %, C = 32, which fits, 15.7 against 17.6).
     a.early = (uint64_t)a.bm.blocks * wpb * 2 <= (uint64_t)sm_count(e->device) * MINB * kRowsWarps;
-    auto kfn = spmm_rows<V, NV, U, MINB, PIPE>;
-    if (smem > 48 * 1024) SPX_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    return finish_launch(launch_pdl(kfn, dim3(a.bm.blocks), dim3(wpb * 32), smem, s, a), "spmm_rows");
+    if (int rc = allow_smem<spmm_rows<V, NV, U, MINB, PIPE>>(e->device)) return rc;
+    return finish_launch(launch_pdl(spmm_rows<V, NV, U, MINB, PIPE>, dim3(a.bm.blocks), dim3(wpb * 32), smem, s, a), "spmm_rows");
 }
 
 static uint32_t chain_pitch(uint32_t C) { return C <= 2 ? C : round_up(C, 4u); }
@@ -946,9 +945,8 @@ static uint32_t chain_pitch(uint32_t C) { return C <= 2 ? C : round_up(C, 4u); }
 template <int V>
 static int launch_direct_one(const spx_ell* e, const RowsArgs& a, uint32_t threads, size_t smem, cudaStream_t s)
 {
-    auto kfn = spmm_direct<V>;
-    if (smem > 48 * 1024) SPX_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    return finish_launch(launch_pdl(kfn, dim3((e->m + a.RW - 1) / a.RW), dim3(threads), smem, s, a), "spmm_direct");
+    if (int rc = allow_smem<spmm_direct<V>>(e->device)) return rc;
+    return finish_launch(launch_pdl(spmm_direct<V>, dim3((e->m + a.RW - 1) / a.RW), dim3(threads), smem, s, a), "spmm_direct");
 }
 
 // X staged whole.  R rows per CTA: one CTA per SM while kChainConsumers threads carry them; the batch
@@ -972,9 +970,8 @@ static int launch_direct(const spx_ell* e, RowsArgs a, bool vec_out, cudaStream_
 template <int C>
 static int launch_chain_one(const spx_ell* e, const RowsArgs& a, size_t smem, cudaStream_t s)
 {
-    auto kfn = spmm_chain<C>;
-    if (smem > 48 * 1024) SPX_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    return finish_launch(launch_pdl(kfn, dim3((e->m + a.RW - 1) / a.RW), dim3(kPreThreads), smem, s, a), "spmm_chain");
+    if (int rc = allow_smem<spmm_chain<C>>(e->device)) return rc;
+    return finish_launch(launch_pdl(spmm_chain<C>, dim3((e->m + a.RW - 1) / a.RW), dim3(kPreThreads), smem, s, a), "spmm_chain");
 }
 // R rows per CTA and batches of E entries.  The kernel takes as many batches as the longest row needs, each
 // about 0.35 us of barriers and latency plus 5 ns per entry of the serial chains, or the time the SM's

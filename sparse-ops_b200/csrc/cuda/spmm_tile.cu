@@ -448,9 +448,8 @@ static int launch_tile_nv(const spx_ell* e, TileArgs a, const CUtensorMap& map, 
     a.row_blocks = (a.groups + warps - 1) / warps;
     a.ring_blocks = warps > 14 ? 2 : 4;
     const size_t smem = (size_t)(kStages * kChunk + 1) * NV * 128 + (size_t)warps * a.ring_blocks * 512;
-    auto kfn = spmm_tile_kernel<NV>;
-    SPX_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    SPX_CUDA(launch_pdl(kfn, dim3(a.row_blocks * slices), dim3(warps * 32), smem, s, a, map));
+    if (int rc = allow_smem<spmm_tile_kernel<NV>>(e->device)) return rc;
+    SPX_CUDA(launch_pdl(spmm_tile_kernel<NV>, dim3(a.row_blocks * slices), dim3(warps * 32), smem, s, a, map));
     count_launch();
     return SPX_OK;
 }

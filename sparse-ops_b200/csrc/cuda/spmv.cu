@@ -336,13 +336,6 @@ int finish(cudaError_t err, const char* name)
     return SPX_OK;
 }
 
-template <class K>
-int opt_in(K kfn, size_t smem)
-{
-    const cudaError_t err = smem > 48 * 1024 ? cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) : cudaSuccess;
-    return err == cudaSuccess ? SPX_OK : spx::fail(SPX_ERR_CUDA, "spmv: shared memory opt-in failed: %s", cudaGetErrorString(err));
-}
-
 constexpr uint32_t kStaged = 200 * 1024 / sizeof(float);        // columns up to which all of x is staged
 
 template <int LPR>
@@ -358,16 +351,14 @@ int launch_lpr(const spx_ell* e, const float* x, const float* bias, float* y, cu
         const uint64_t iters = (per * LPR + 1023) / 1024, groups = (per + iters - 1) / iters;
         const unsigned threads = (unsigned)((groups * LPR + 31) / 32 * 32);
         const size_t smem = (size_t)e->n * sizeof(float);
-        auto kfn = spmv_staged_kernel<LPR>;
-        if (int rc = opt_in(kfn, smem)) return rc;
-        return finish(spx::launch_pdl(kfn, dim3((unsigned)std::min<uint64_t>(sms, e->m)), dim3(threads), smem, s, e->Wd, e->idx, e->nnz, order,
+        if (int rc = spx::allow_smem<spmv_staged_kernel<LPR>>(e->device)) return rc;
+        return finish(spx::launch_pdl(spmv_staged_kernel<LPR>, dim3((unsigned)std::min<uint64_t>(sms, e->m)), dim3(threads), smem, s, e->Wd, e->idx, e->nnz, order,
                                       e->m, e->n, e->pitch, x, bias, y), "spmv_staged_kernel");
     }
     if (e->spmv_split) {
         const size_t smem = (size_t)e->spmv_win * 2 * sizeof(float);
-        auto kfn = spmv_ell_windowed_kernel<LPR>;
-        if (int rc = opt_in(kfn, smem)) return rc;
-        return finish(spx::launch_pdl(kfn, dim3((unsigned)std::min<uint64_t>(sms, e->m)), dim3(1024), smem, s, e->Wd, e->idx, e->nnz, e->rows,
+        if (int rc = spx::allow_smem<spmv_ell_windowed_kernel<LPR>>(e->device)) return rc;
+        return finish(spx::launch_pdl(spmv_ell_windowed_kernel<LPR>, dim3((unsigned)std::min<uint64_t>(sms, e->m)), dim3(1024), smem, s, e->Wd, e->idx, e->nnz, e->rows,
                                       e->spmv_split, e->m, e->n, e->spmv_win, e->pitch, x, bias, y), "spmv_ell_windowed_kernel");
     }
     // as many CTAs as give every group the same number of rows

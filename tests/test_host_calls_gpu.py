@@ -62,3 +62,50 @@ def test_copies_under_capture(lib, cuda):
             lib.spx_stream_sync(st)
             assert_bit_equal(dst.cpu().numpy(), src, "captured copy")
             lib.spx_graph_destroy(graph)
+
+
+def together(*jobs):
+    """Runs the jobs in threads of their own and raises what any of them raised."""
+    errors = []
+
+    def guard(job):
+        try:
+            torch.cuda.set_device(0)
+            job()
+        except BaseException as e:      # noqa: BLE001 - reported below
+            errors.append(e)
+    threads = [threading.Thread(target=guard, args=(j,)) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    if errors:
+        raise errors[0]
+
+
+def test_launches_of_one_kernel_from_several_threads(lib, orc, cuda):
+    """The same kernels with different amounts of shared memory at the same time: no launch is refused, and results
+    are those of one thread."""
+    rng = np.random.default_rng(3)
+    jobs = []
+    for i, (m, n, Cc) in enumerate([(300, 100, 64), (300, 500, 64), (400, 300, 32), (256, 1000, 32)]):
+        E = orc.encode(sparse(rng, m, n, 0.9))
+        X = rng.uniform(-1, 1, (n, Cc)).astype(np.float32)
+        x = rng.uniform(-1, 1, (n, 1)).astype(np.float32)
+        h = lib.ell_create(E.Wd, E.idx, E.nnz, E.n)
+        dX, dx = torch.from_numpy(X).to(cuda), torch.from_numpy(x).to(cuda)
+        dY, dy, dz = torch.zeros((m, Cc), device=cuda), torch.zeros((m, 1), device=cuda), torch.zeros(m, device=cuda)
+        want, want1 = orc.spmm(E, X, None), orc.spmm(E, x, None)
+
+        def job(h=h, dX=dX, dx=dx, dY=dY, dy=dy, dz=dz, Cc=Cc, want=want, want1=want1):
+            with Stream(lib) as st:
+                for k in range(1500):
+                    h.spmm(dX.data_ptr(), Cc, Cc, 0, 0, dY.data_ptr(), Cc, st)
+                    h.spmm(dx.data_ptr(), 1, 1, 0, 0, dy.data_ptr(), 1, st)
+                    h.spmv(dx.data_ptr(), 0, dz.data_ptr(), st)
+                lib.spx_stream_sync(st)
+            assert_bit_equal(dY.cpu().numpy(), want, "wide")
+            assert_bit_equal(dy.cpu().numpy(), want1, "one column")
+        jobs.append(job)
+    torch.cuda.synchronize()
+    together(*jobs)
