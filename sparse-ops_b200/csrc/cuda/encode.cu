@@ -307,11 +307,11 @@ static int encode_rows(const float* dW, uint32_t m, uint32_t n, cudaStream_t s, 
         SPX_LAUNCH_CHECK("pack_kernel");
     }
     uint2* h_order = reinterpret_cast<uint2*>(h_counts + round_up<size_t>(units, 2));
-    if (int rc = sort_rows(e, h_counts, h_order, s)) return rc;
-    // on a stream of its own, beside the packer (nothing on s uses that block: blocks return to the
-    // pool only after the work on them has been waited for)
+    // on a stream of its own, beside the packer: the block is allocated in that stream's order too (the pool may hand
+    // out memory that work queued on another stream still uses, ordered behind it on the allocating stream only)
     cudaStream_t side = nullptr;
     if (int rc = side_stream(e->device, &side)) return rc;
+    if (int rc = sort_rows(e, h_counts, h_order, side)) return rc;
     SPX_CUDA(cudaMemcpyAsync(e->rows, h_order, (size_t)m * sizeof(uint2), cudaMemcpyHostToDevice, side));
     SPX_CUDA(cudaStreamSynchronize(side));
     SPX_CUDA(cudaStreamSynchronize(s));         // the handle may be used on any stream from here on

@@ -109,3 +109,36 @@ def test_launches_of_one_kernel_from_several_threads(lib, orc, cuda):
         jobs.append(job)
     torch.cuda.synchronize()
     together(*jobs)
+
+
+def test_encoding_beside_products_on_one_stream(lib, orc, cuda):
+    """Handles are made and destroyed on a stream on which another thread queues products that use scratch of the
+    library's pool (X re-pitched for bulk copies): neither disturbs the other."""
+    rng = np.random.default_rng(4)
+    m, n, Cc = 1201, 1100, 77                   # the block kernel, with a copy of X in rows of 16-byte multiples
+    E = orc.encode(sparse(rng, m, n, 0.5))
+    X = rng.uniform(-1, 1, (n, Cc)).astype(np.float32)
+    W = sparse(rng, 3000, 200, 0.3)
+    E2 = orc.encode(W)
+    h = lib.ell_create(E.Wd, E.idx, E.nnz, E.n)
+    dX, dW = torch.from_numpy(X).to(cuda), torch.from_numpy(W).to(cuda)
+    dY = [torch.zeros((m, Cc), device=cuda) for _ in range(300)]
+    dx, dy = torch.ones((200, 1), device=cuda), torch.zeros((3000, 1), device=cuda)
+    want, want2 = orc.spmm(E, X, None), orc.spmm(E2, np.ones((200, 1), np.float32), None)
+    torch.cuda.synchronize()
+    with Stream(lib) as st:
+        def products():
+            for y in dY:
+                h.spmm(dX.data_ptr(), Cc, Cc, 0, 0, y.data_ptr(), Cc, st)
+
+        def handles():
+            for k in range(40):
+                h2 = lib.ell_encode_device(dW.data_ptr(), 3000, 200, st)
+                h2.spmm(dx.data_ptr(), 1, 1, 0, 0, dy.data_ptr(), 1, st)
+                lib.spx_stream_sync(st)
+                assert_bit_equal(dy.cpu().numpy(), want2, f"handle {k}")
+                h2.close()
+        together(products, handles)
+        lib.spx_stream_sync(st)
+        for k, y in enumerate(dY):
+            assert_bit_equal(y.cpu().numpy(), want, f"product {k}")
