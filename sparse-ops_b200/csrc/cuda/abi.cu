@@ -369,7 +369,7 @@ int spx_ell_create_csr(uint32_t m, uint32_t n, const uint64_t* rowptr, const uin
         if (err == cudaSuccess && total) err = cudaMemcpy(d_val, val, total * 4, cudaMemcpyHostToDevice);
         if (err == cudaSuccess) {
             rc = csr_to_ell_device(e, d_rowptr, d_col, d_val, nullptr);
-            if (rc == SPX_OK) err = cudaDeviceSynchronize();
+            if (rc == SPX_OK) err = cudaStreamSynchronize(nullptr);
         }
         cudaFree(d_rowptr); cudaFree(d_col); cudaFree(d_val);
         if (err != cudaSuccess || rc != SPX_OK) {
@@ -406,7 +406,7 @@ int spx_ell_destroy(spx_ell* e)
     for (cudaEvent_t ev : e->xchg_events) if (ev) cudaEventDestroy(ev);
     // Kernels that read the handle may still run, on any stream: one wait for the device, after which
     // its arrays go back to the pool without another one.
-    (void)cudaDeviceSynchronize();
+    wait_for_device();
     free_tiles(e);
     pool_free(e->Wd, (size_t)e->m * e->pitch * 4, nullptr);
     pool_free(e->idx, (size_t)e->m * e->pitch * 4, nullptr);

@@ -222,6 +222,7 @@ int copy_h2d_rows(void* dst, const void* src, size_t rows, size_t row, size_t st
 bool pageable_memory(const void* p);            // host memory that is not page-locked
 // Replaces a handle's scratch block by a larger one (waits for the device: kernels may still use the old one).
 int grow_scratch(spx_ell* e, void** p, size_t* bytes, size_t need);
+void wait_for_device();                         // for all work on the current device
 void pool_trim(int device);                     // waits for the device, then gives all free memory back
 // A non-blocking stream per device for small transfers beside the caller's stream, created once (mem.cu).
 int side_stream(int device, cudaStream_t* out);

@@ -98,10 +98,21 @@ int pool_alloc_now(void** p, size_t bytes, int device)
     return SPX_OK;
 }
 
+// cudaDeviceSynchronize would end every stream capture in the process with an error, other threads' too; the free of
+// mapped memory waits for the device as well and leaves their captures alone (4 us for the pair, as for the other).
+void wait_for_device()
+{
+    void* p = nullptr;
+    if (cudaMalloc(&p, 256) == cudaSuccess && cudaFree(p) == cudaSuccess) return;
+    (void)cudaGetLastError();
+    (void)cudaDeviceSynchronize();
+    (void)cudaGetLastError();
+}
+
 int grow_scratch(spx_ell* e, void** p, size_t* bytes, size_t need)
 {
     if (*p) {
-        (void)cudaDeviceSynchronize();
+        wait_for_device();
         pool_free(*p, *bytes, nullptr);
     }
     *p = nullptr;
@@ -114,7 +125,7 @@ int grow_scratch(spx_ell* e, void** p, size_t* bytes, size_t need)
 void pool_trim(int device)
 {
     if (device < 0 || device >= kMaxDevices) return;
-    (void)cudaDeviceSynchronize();
+    wait_for_device();
     std::lock_guard<std::mutex> lk(g_pool_mu);
     if (g_pools[device]) (void)cudaMemPoolTrimTo(g_pools[device], 0);
 }

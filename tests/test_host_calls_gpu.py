@@ -142,3 +142,47 @@ def test_encoding_beside_products_on_one_stream(lib, orc, cuda):
         lib.spx_stream_sync(st)
         for k, y in enumerate(dY):
             assert_bit_equal(y.cpu().numpy(), want, f"product {k}")
+
+
+def test_handles_come_and_go_beside_another_threads_capture(lib, orc, cuda):
+    """A graph that one thread records survives another thread making, using and destroying handles and growing their
+    scratch (spx_graph_capture_begin keeps other threads' calls apart)."""
+    rng = np.random.default_rng(6)
+    E = orc.encode(sparse(rng, 300, 400, 0.2))
+    X = rng.uniform(-1, 1, (400, 48)).astype(np.float32)
+    want = orc.spmm(E, X, None)
+    h = lib.ell_create(E.Wd, E.idx, E.nnz, E.n)
+    dX, dY = torch.from_numpy(X).to(cuda), torch.zeros((300, 48), device=cuda)
+    begun, done = threading.Event(), threading.Event()
+    torch.cuda.synchronize()
+
+    def records():
+        with Stream(lib) as st:
+            try:
+                h.spmm(dX.data_ptr(), 48, 48, 0, 0, dY.data_ptr(), 48, st)
+                lib.spx_stream_sync(st)
+                lib.spx_graph_capture_begin(st)
+                h.spmm(dX.data_ptr(), 48, 48, 0, 0, dY.data_ptr(), 48, st)
+            finally:
+                begun.set()
+            done.wait(60)
+            h.spmm(dX.data_ptr(), 48, 48, 0, 0, dY.data_ptr(), 48, st)
+            graph = C.c_void_p()
+            lib.spx_graph_capture_end(st, C.byref(graph))
+            lib.spx_memset(dY.data_ptr(), 0, dY.numel() * 4, st)
+            lib.spx_graph_launch(graph, st)
+            lib.spx_stream_sync(st)
+            lib.spx_graph_destroy(graph)
+        assert_bit_equal(dY.cpu().numpy(), want, "replay")
+
+    def others():
+        begun.wait(60)
+        try:
+            for k in range(3):
+                h2 = lib.ell_create(E.Wd, E.idx, E.nnz, E.n)
+                assert_bit_equal(h2.spmm_host(X[:, :8].copy(), None), want[:, :8], "host call")
+                assert_bit_equal(h2.spmm_host(X, None), want, "host call, more scratch")
+                h2.close()
+        finally:
+            done.set()
+    together(records, others)
