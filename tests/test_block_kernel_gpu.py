@@ -21,9 +21,9 @@ def sparse(rng, m, n, p):
 
 
 def in_child(name, **env):
-    """Runs the test called `name` of this file in a process of its own: switches are read once per process."""
-    cmd = [sys.executable, "-m", "pytest", "-q", "-x", "-m", "gpu", "-p", "no:cacheprovider", os.path.abspath(__file__), "-k", name]
-    r = subprocess.run(cmd, env={**os.environ, **env}, capture_output=True, text=True, timeout=900)
+    """Runs the test `name` of this file in a process of its own: switches are read once per process."""
+    cmd = [sys.executable, "-m", "pytest", "-q", "-x", "-m", "gpu", "-p", "no:cacheprovider", os.path.abspath(__file__) + "::" + name]
+    r = subprocess.run(cmd, env={**os.environ, **env}, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and " passed" in r.stdout, r.stdout[-3000:] + r.stderr[-2000:]
 
 
@@ -59,7 +59,7 @@ def test_stage_refills(lib, orc, cuda, m, n, C, p):
 
 
 def test_stage_refills_forced():
-    in_child("test_stage_refills and not forced", SPX_SPMM_TILE="2")
+    in_child("test_stage_refills", SPX_SPMM_TILE="2")
 
 
 # ---- a bounded wait that runs out -----------------------------------------------------------------
@@ -141,7 +141,7 @@ def test_timeout_of_a_replay(lib, orc, backend, cuda, tmp_path, how):
 
 
 @pytest.mark.parametrize("name,launch", [("test_timeout_of_a_call", "1"), ("test_timeout_of_a_host_call", "1"),
-                                         ("test_timeout_of_a_replay and run]", "2"), ("test_timeout_of_a_replay and resident]", "2")])
+                                         ("test_timeout_of_a_replay[run]", "2"), ("test_timeout_of_a_replay[resident]", "2")])
 def test_timeouts_are_reported(name, launch):
     """With the switch a barrier expects more bytes than its copy brings, so the kernel's bounded wait runs out (nothing
     faults, nothing hangs): an error, never a stale result."""
