@@ -130,11 +130,11 @@ void pool_trim(int device)
     if (g_pools[device]) (void)cudaMemPoolTrimTo(g_pools[device], 0);
 }
 
-static int kept_stream(cudaStream_t (&streams)[kMaxDevices], int device, cudaStream_t* out)
+static int kept_stream(cudaStream_t (&streams)[kMaxDevices], int device, cudaStream_t* out, unsigned flags)
 {
     if (device < 0 || device >= kMaxDevices) return fail(SPX_ERR_LIMIT, "device ordinal %d not supported", device);
     std::lock_guard<std::mutex> lk(g_pool_mu);
-    if (!streams[device]) SPX_CUDA(cudaStreamCreateWithFlags(&streams[device], cudaStreamNonBlocking));
+    if (!streams[device]) SPX_CUDA(cudaStreamCreateWithFlags(&streams[device], flags));
     *out = streams[device];
     return SPX_OK;
 }
@@ -142,7 +142,7 @@ static int kept_stream(cudaStream_t (&streams)[kMaxDevices], int device, cudaStr
 int side_stream(int device, cudaStream_t* out)
 {
     static cudaStream_t streams[kMaxDevices] = {};
-    return kept_stream(streams, device, out);
+    return kept_stream(streams, device, out, cudaStreamNonBlocking);
 }
 
 int host_stream(int device, int which, cudaStream_t* out)
@@ -152,7 +152,8 @@ int host_stream(int device, int which, cudaStream_t* out)
         ~Streams() { for (auto& k : s) for (cudaStream_t st : k) if (st) (void)cudaStreamDestroy(st); }
     };
     thread_local Streams mine;
-    return kept_stream(mine.s[which], device, out);
+    // ordered behind what the caller has queued on the default stream (a copy into an operand, for instance)
+    return kept_stream(mine.s[which], device, out, cudaStreamDefault);
 }
 
 int pinned_acquire(size_t bytes, PinnedBlock* out)

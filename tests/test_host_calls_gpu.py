@@ -186,3 +186,33 @@ def test_handles_come_and_go_beside_another_threads_capture(lib, orc, cuda):
         finally:
             done.set()
     together(records, others)
+
+
+@pytest.mark.parametrize("m,n,Cc", [(200, 300, 1), (200, 300, 8), (300, 2000, 17), (700, 3000, 48), (4096, 4100, 64)])
+def test_host_calls_follow_the_default_stream(lib, orc, cuda, m, n, Cc):
+    """Operands in page-locked memory that a copy on the default stream is still to fill: the call comes after it,
+    as it does when it runs on that stream itself.  The result's old contents are still being read, too."""
+    rng = np.random.default_rng([m, n, Cc])
+    E = orc.encode(sparse(rng, m, n, 0.1))
+    X = rng.uniform(-1, 1, (n, Cc)).astype(np.float32)
+    b = rng.standard_normal(m).astype(np.float32)
+    h = lib.ell_create(E.Wd, E.idx, E.nnz, E.n)
+    want = orc.spmm(E, X, b)
+    hX, hB, hY = torch.zeros((n, Cc)).pin_memory(), torch.zeros(m).pin_memory(), torch.full((m, Cc), 5.0).pin_memory()
+    dX, dB, old = torch.from_numpy(X).to(cuda), torch.from_numpy(b).to(cuda), torch.zeros((m, Cc), device=cuda)
+    hog = torch.empty(1 << 30, dtype=torch.uint8, device=cuda)
+    h.spmm_host(X, b)
+    torch.cuda.synchronize()
+    for _ in range(40):                     # some milliseconds on the default stream
+        lib.spx_memset(hog.data_ptr(), 1, hog.numel(), 0)
+    lib.spx_memcpy_d2h(hX.data_ptr(), dX.data_ptr(), X.nbytes, 0)
+    lib.spx_memcpy_d2h(hB.data_ptr(), dB.data_ptr(), b.nbytes, 0)
+    lib.spx_memcpy_h2d(old.data_ptr(), hY.data_ptr(), hY.numel() * 4, 0)
+    if Cc == 1:
+        lib.spx_spmv_host(h.h, hX.data_ptr(), hB.data_ptr(), hY.data_ptr())
+        bound = orc.absbound(E, X[:, 0].copy(), b)
+        assert (np.abs(hY.numpy()[:, 0] - want[:, 0]) <= 1e-5 * bound).all()
+    else:
+        lib.spx_spmm_host(h.h, hX.data_ptr(), Cc, hB.data_ptr(), 0, hY.data_ptr())
+        assert_bit_equal(hY.numpy(), want, "host call")
+    assert bool((old == 5.0).all())
