@@ -55,13 +55,13 @@ size_t g_pinned_bytes = 0;
 
 }  // namespace
 
-int pool_alloc(void** p, size_t bytes, int device, cudaStream_t s)
+static int allocate(void** p, size_t bytes, int device, cudaStream_t s, bool pooled)
 {
     *p = nullptr;
     if (bytes == 0) return SPX_OK;
     cudaMemPool_t pool = nullptr;
     if (int rc = device_pool(device, &pool)) return rc;
-    auto get = [&] { return bytes > kPoolBlock ? cudaMalloc(p, bytes) : cudaMallocFromPoolAsync(p, bytes, pool, s); };
+    auto get = [&] { return pooled ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMalloc(p, bytes); };
     cudaError_t err = get();
     if (err == cudaErrorMemoryAllocation) {
         (void)cudaGetLastError();
@@ -76,6 +76,12 @@ int pool_alloc(void** p, size_t bytes, int device, cudaStream_t s)
     }
     return SPX_OK;
 }
+
+int pool_alloc(void** p, size_t bytes, int device, cudaStream_t s) { return allocate(p, bytes, device, s, bytes <= kPoolBlock); }
+
+// Scratch of one call, whatever its size: mapping and freeing memory directly would make the call wait for the device.
+int scratch_alloc(void** p, size_t bytes, int device, cudaStream_t s) { return allocate(p, bytes, device, s, true); }
+void scratch_free(void* p, cudaStream_t s) { if (p) (void)cudaFreeAsync(p, s); }
 
 void pool_free(void* p, size_t bytes, cudaStream_t s)
 {

@@ -527,13 +527,12 @@ int launch_spmm_tile(spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const
     }
     void* aligned = nullptr;
     const uint32_t Cp = round_up(C, 4u);
-    const size_t aligned_bytes = (size_t)e->n * Cp * 4;
     if (!vec_x) {                               // bulk copies need 16-byte rows: X moves into scratch that has them
-        if (int rc = pool_alloc(&aligned, aligned_bytes, e->device, s)) return rc == SPX_ERR_OOM ? -1 : rc;
+        if (int rc = scratch_alloc(&aligned, (size_t)e->n * Cp * 4, e->device, s)) return rc == SPX_ERR_OOM ? -1 : rc;
         const uint64_t quads = (uint64_t)e->n * (Cp / 4);
         const unsigned blocks = (unsigned)std::min<uint64_t>((quads + 255) / 256, (uint64_t)sm_count(e->device) * 16);
         const cudaError_t err = launch_pdl(align_rows_kernel, dim3(blocks), dim3(256), 0, s, X, ldx, e->n, C, Cp, static_cast<float*>(aligned));
-        if (err != cudaSuccess) { pool_free(aligned, aligned_bytes, s); return fail(SPX_ERR_CUDA, "launch of align_rows_kernel failed: %s", cudaGetErrorString(err)); }
+        if (err != cudaSuccess) { scratch_free(aligned, s); return fail(SPX_ERR_CUDA, "launch of align_rows_kernel failed: %s", cudaGetErrorString(err)); }
         count_launch();
         X = static_cast<const float*>(aligned);
         ldx = Cp;
@@ -557,7 +556,7 @@ int launch_spmm_tile(spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const
         if (timeout_env && ++launches == timeout_env) a.missing = 16;
         rc = NV == 1 ? launch_tile_nv<1>(e, a, map, p.warps, p.slices, s) : launch_tile_nv<2>(e, a, map, p.warps, p.slices, s);
     }
-    pool_free(aligned, aligned_bytes, s);
+    scratch_free(aligned, s);
     return rc;
 }
 

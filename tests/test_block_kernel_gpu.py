@@ -146,3 +146,30 @@ def test_timeouts_are_reported(name, launch):
     """With the switch a barrier expects more bytes than its copy brings, so the kernel's bounded wait runs out (nothing
     faults, nothing hangs): an error, never a stale result."""
     in_child(name, SPX_SPMM_TILE="2", SPX_SPMM_TMA_TEST_TIMEOUT=launch)
+
+
+def test_large_unaligned_operand_is_only_enqueued(lib, cuda):
+    """The copy of an X whose rows are no multiple of 16 bytes is scratch of the call, 165 MB here: the call returns
+    while the product runs."""
+    m, n, C = 8192, 8192, 5033
+    g = torch.Generator(device="cuda").manual_seed(7)
+    W = torch.rand((m, n), device=cuda, generator=g)
+    W[torch.rand((m, n), device=cuda, generator=g) >= 0.1] = 0
+    X, Y = torch.rand((n, C), device=cuda, generator=g), torch.zeros((m, C), device=cuda)
+    h = lib.ell_encode_device(W.data_ptr(), m, n)
+    run = lambda: h.spmm(X.data_ptr(), C, C, 0, 0, Y.data_ptr(), C)
+    for k in range(3):
+        run()
+    torch.cuda.synchronize()
+    before = lib.spx_launch_count()
+    run()
+    ended = torch.cuda.Event()
+    ended.record()
+    still_running = not ended.query()
+    assert lib.spx_launch_count() == before + 2, "not the route with a copy of X"
+    assert still_running
+    torch.cuda.synchronize()
+    cols = [0, 1, 2517, C - 1]
+    want = W.double() @ X[:, cols].double()
+    got = Y[:, cols].double()
+    assert float((got - want).norm() / want.norm()) < 1e-5      # 32-bit sums of about 800 terms
