@@ -517,6 +517,7 @@ int launch_spmm_tile(spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const
     if (t->state != 1 || !vec_x) {              // building and the scratch below allocate: not while a graph is captured
         if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) { (void)cudaGetLastError(); return -1; }
     }
+    RelaxedCapture relaxed;                     // s is not being captured; another stream may be, by this thread
     if (t->state != 1) {
         std::lock_guard<std::mutex> lk(t->mu);
         if (t->state == 0) {

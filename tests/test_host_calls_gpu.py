@@ -216,3 +216,31 @@ def test_host_calls_follow_the_default_stream(lib, orc, cuda, m, n, Cc):
         lib.spx_spmm_host(h.h, hX.data_ptr(), Cc, hB.data_ptr(), 0, hY.data_ptr())
         assert_bit_equal(hY.numpy(), want, "host call")
     assert bool((old == 5.0).all())
+
+
+@pytest.mark.parametrize("Cc", [160, 77])
+def test_products_beside_the_same_threads_capture(lib, orc, cuda, Cc):
+    """While a thread records a graph on one stream, its products on another stream may build the block kernel's form of
+    a matrix and take scratch: the graph survives that."""
+    rng = np.random.default_rng(8)
+    m, n = 1312, 2080                           # takes the block kernel at both widths, from the second call on
+    E = orc.encode(sparse(rng, m, n, 0.5))
+    X = rng.uniform(-1, 1, (n, Cc)).astype(np.float32)
+    want = orc.spmm(E, X, None)
+    h, small = lib.ell_create(E.Wd, E.idx, E.nnz, E.n), lib.ell_create(E.Wd, E.idx, E.nnz, E.n)
+    dX, dY, dZ = torch.from_numpy(X).to(cuda), torch.zeros((m, Cc), device=cuda), torch.zeros((m, Cc), device=cuda)
+    torch.cuda.synchronize()
+    with Stream(lib) as st, Stream(lib) as free:
+        lib.spx_graph_capture_begin(st)
+        small.spmm(dX.data_ptr(), Cc, Cc, 0, 0, dZ.data_ptr(), Cc, st)
+        for k in range(3):
+            h.spmm(dX.data_ptr(), Cc, Cc, 0, 0, dY.data_ptr(), Cc, free)
+        small.spmm(dX.data_ptr(), Cc, Cc, 0, 0, dZ.data_ptr(), Cc, st)
+        graph = C.c_void_p()
+        lib.spx_graph_capture_end(st, C.byref(graph))
+        lib.spx_graph_launch(graph, st)
+        lib.spx_stream_sync(st)
+        lib.spx_stream_sync(free)
+        lib.spx_graph_destroy(graph)
+    assert_bit_equal(dY.cpu().numpy(), want, "beside the capture")
+    assert_bit_equal(dZ.cpu().numpy(), want, "replay")
