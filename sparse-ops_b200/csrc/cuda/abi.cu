@@ -465,8 +465,8 @@ int spx_ell_decode_device(const spx_ell* e, float* dW, void* stream)
 }
 
 // ---- kernels ---------------------------------------------------------------------------------
-int spx_spmm(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const float* bias,
-             int act, float* Y, uint64_t ldy, void* stream)
+static int spmm_part(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const float* bias,
+                     int act, float* Y, uint64_t ldy, cudaStream_t s, bool again)
 {
     if (!e) return fail(SPX_ERR_ARG, "handle is null");
     if (act < SPX_ACT_NONE || act > SPX_ACT_TANH) return fail(SPX_ERR_ARG, "unknown activation %d", act);
@@ -475,7 +475,13 @@ int spx_spmm(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const f
     if (!Y) return fail(SPX_ERR_ARG, "Y is null");
     if (!X && e->nnz_total) return fail(SPX_ERR_ARG, "X is null");
     if (int rc = check_current_device(e, "spmm")) return rc;
-    return launch_spmm(e, X, C, ldx, bias, act, Y, ldy, (cudaStream_t)stream);
+    return launch_spmm(e, X, C, ldx, bias, act, Y, ldy, s, again);
+}
+
+int spx_spmm(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const float* bias,
+             int act, float* Y, uint64_t ldy, void* stream)
+{
+    return spmm_part(e, X, C, ldx, bias, act, Y, ldy, (cudaStream_t)stream, false);
 }
 
 int spx_spmm_bcast(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const float* bias, int act,
@@ -783,7 +789,7 @@ static int spmm_host_panels(spx_ell* e, const float* X, uint32_t C, const float*
         if (int rc = copy_h2d_rows(dXp, X + (size_t)p * w, e->n, (size_t)w * 4, (size_t)C * 4, st.s[0])) return rc;
         SPX_CUDA(cudaEventRecord(done.ev[2 * p], st.s[0]));
         SPX_CUDA(cudaStreamWaitEvent(st.s[1], done.ev[2 * p], 0));
-        if (int rc = spx_spmm(e, dXp, w, w, bias ? dB : nullptr, act, dY + (size_t)p * w, C, st.s[1])) return rc;
+        if (int rc = spmm_part(e, dXp, w, w, bias ? dB : nullptr, act, dY + (size_t)p * w, C, st.s[1], p > 0)) return rc;
         SPX_CUDA(cudaEventRecord(done.ev[2 * p + 1], st.s[1]));
         SPX_CUDA(cudaStreamWaitEvent(st.s[2], done.ev[2 * p + 1], 0));
         if (!pageable)
@@ -836,7 +842,7 @@ int spx_spmm_host(const spx_ell* ce, const float* X, uint32_t C, const float* bi
             if (err == cudaSuccess) err = cudaEventRecord(ev_in, s_in);
             if (err == cudaSuccess) err = cudaStreamWaitEvent(s_mm, ev_in, 0);
             if (err != cudaSuccess) break;
-            rc = spx_spmm(e, dX + c0, w, C, bias ? dB : nullptr, act, dY + c0, C, s_mm);
+            rc = spmm_part(e, dX + c0, w, C, bias ? dB : nullptr, act, dY + c0, C, s_mm, c0 > 0);
             if (rc != SPX_OK) break;
             err = cudaEventRecord(ev_mm, s_mm);
             if (err == cudaSuccess) err = cudaStreamWaitEvent(s_out, ev_mm, 0);
@@ -937,7 +943,7 @@ int spx_spmm_host_sharded(spx_comm* comm, const spx_ell* ce, const float* X, uin
         if (err == cudaSuccess) err = cudaStreamWaitEvent(st[2], ev(p, 1, 1), 0);
         if (err == cudaSuccess) err = cudaEventRecord(ev(p, 2, 0), st[2]);
         if (err != cudaSuccess) break;
-        if (e->m) rc = spx_spmm(e, dXp, w, w, bias ? dB : nullptr, act, dY + c0, C, st[2]);
+        if (e->m) rc = spmm_part(e, dXp, w, w, bias ? dB : nullptr, act, dY + c0, C, st[2], p > 0);
         if (rc != SPX_OK) break;
         err = cudaEventRecord(ev(p, 2, 1), st[2]);
         // 3: this rank's rows of Y, device -> host

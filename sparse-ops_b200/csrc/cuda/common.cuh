@@ -167,10 +167,12 @@ __device__ __forceinline__ void fma_pair(float& a0, float& a1, float w, float x0
 
 // Kernel launchers implemented in the individual .cu files.
 namespace spx {
+// again: a further part of a call that has been counted (a matrix gets its block form on its second call).
 int launch_spmm(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const float* bias,
-                int act, float* Y, uint64_t ldy, cudaStream_t s);
+                int act, float* Y, uint64_t ldy, cudaStream_t s, bool again = false);
 int launch_spmm_bcast(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const float* bias, int act,
-                      float* const* Ys, uint32_t npeers, uint64_t row0, uint64_t ldy, cudaStream_t s, bool mcast = false);
+                      float* const* Ys, uint32_t npeers, uint64_t row0, uint64_t ldy, cudaStream_t s, bool mcast = false,
+                      bool again = false);
 void* new_tiles();
 void free_tiles(spx_ell* e);
 int launch_spmv(spx_ell* e, const float* x, const float* bias, float* y, cudaStream_t s);

@@ -1116,7 +1116,7 @@ int launch_conv2d(spx_ell* e, const spx_conv_geom* g, int layout, const float* i
             return launch_spmm(e, in, (uint32_t)(hw * B), hw * B, bias, act, out, hw * B, s);
         if (layout == SPX_LAYOUT_NCHW && B <= 3 && hw < (1ull << 30)) {
             for (uint32_t b = 0; b < B; ++b)
-                if (int rs = launch_spmm(e, in + b * g->Cin * hw, (uint32_t)hw, hw, bias, act, out + b * g->Cout * hw, hw, s)) return rs;
+                if (int rs = launch_spmm(e, in + b * g->Cin * hw, (uint32_t)hw, hw, bias, act, out + b * g->Cout * hw, hw, s, b > 0)) return rs;
             return SPX_OK;
         }
     }

@@ -1054,17 +1054,17 @@ static int launch_rows(const spx_ell* e, RowsArgs a, cudaStream_t s)
 }
 
 int launch_spmm_tile(spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const float* bias, int act, const PeerOut& out,
-                     uint64_t ldy, bool vec_x, bool vec_out, cudaStream_t s);
+                     uint64_t ldy, bool vec_x, bool vec_out, bool again, cudaStream_t s);
 
 int launch_spmm(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const float* bias,
-                int act, float* Y, uint64_t ldy, cudaStream_t s)
+                int act, float* Y, uint64_t ldy, cudaStream_t s, bool again)
 {
     float* one[1] = { Y };
-    return launch_spmm_bcast(e, X, C, ldx, bias, act, one, 1, 0, ldy, s);
+    return launch_spmm_bcast(e, X, C, ldx, bias, act, one, 1, 0, ldy, s, false, again);
 }
 
 int launch_spmm_bcast(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const float* bias, int act,
-                      float* const* Ys, uint32_t npeers, uint64_t row0, uint64_t ldy, cudaStream_t s, bool mcast)
+                      float* const* Ys, uint32_t npeers, uint64_t row0, uint64_t ldy, cudaStream_t s, bool mcast, bool again)
 {
     if (e->m == 0 || C == 0) return SPX_OK;
     if (npeers == 0 || npeers > (uint32_t)kMaxPeers) return fail(SPX_ERR_LIMIT, "spmm: 1..%d destination buffers supported", kMaxPeers);
@@ -1103,7 +1103,7 @@ int launch_spmm_bcast(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx
         return launch_direct(e, a, true, s);
     {
         const bool vec_x = C % 4 == 0 && ldx % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
-        const int rc = launch_spmm_tile(const_cast<spx_ell*>(e), X, C, ldx, bias, act, out, ldy, vec_x, C % 4 == 0 && ldy % 4 == 0 && aligned, s);
+        const int rc = launch_spmm_tile(const_cast<spx_ell*>(e), X, C, ldx, bias, act, out, ldy, vec_x, C % 4 == 0 && ldy % 4 == 0 && aligned, again, s);
         if (rc != -1) return rc;
     }
     if (ldx >= (1ull << 30)) {

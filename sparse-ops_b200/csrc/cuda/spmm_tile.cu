@@ -502,7 +502,7 @@ double gather_us(const spx_ell* e, uint32_t C, bool aligned)
 
 // Returns -1 when the shape or the handle is not for this kernel.
 int launch_spmm_tile(spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const float* bias, int act, const PeerOut& out,
-                     uint64_t ldy, bool vec_x, bool vec_out, cudaStream_t s)
+                     uint64_t ldy, bool vec_x, bool vec_out, bool again, cudaStream_t s)
 {
     static const int env = [] { const char* v = getenv("SPX_SPMM_TILE"); return v ? atoi(v) : 1; }();
     if (!env || !e->tiles || !e->cols_ascending || e->tma_off || e->max_nnz == 0) return -1;
@@ -521,7 +521,7 @@ int launch_spmm_tile(spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const
     if (t->state != 1) {
         std::lock_guard<std::mutex> lk(t->mu);
         if (t->state == 0) {
-            if (++t->calls < 2) return -1;      // a matrix that is multiplied once is not worth the second form
+            if ((again ? t->calls : ++t->calls) < 2) return -1;     // a matrix that is multiplied once is not worth the second form
             if (int rc = build_tiles(e, t, s)) return rc;
         }
         if (t->state != 1) return -1;

@@ -173,3 +173,29 @@ def test_large_unaligned_operand_is_only_enqueued(lib, cuda):
     want = W.double() @ X[:, cols].double()
     got = Y[:, cols].double()
     assert float((got - want).norm() / want.norm()) < 1e-5      # 32-bit sums of about 800 terms
+
+
+def test_one_call_in_parts_builds_nothing(lib, orc, cuda):
+    """A matrix gets its block form when it is multiplied again.  A host call in column panels and a 1 x 1 convolution
+    of several images are one call: the second one builds (two more kernels), the first and third do not."""
+    rng = np.random.default_rng(11)
+    m, n, C = 2048, 2048, 256
+    E = orc.encode(sparse(rng, m, n, 0.2))
+    X = rng.uniform(-1, 1, (n, C)).astype(np.float32)
+    h = lib.ell_create(E.Wd, E.idx, E.nnz, E.n)
+    counts = []
+    for k in range(3):
+        before = lib.spx_launch_count()
+        h.spmm_host(X, None)
+        counts.append(lib.spx_launch_count() - before)
+    assert counts == [2, 4, 2]
+    g = sx.conv_geom(n, m, 1, 1, 16, 16)
+    h = lib.ell_create(E.Wd, E.idx, E.nnz, E.n)
+    dX, dY = torch.rand((3, n, 256), device=cuda), torch.zeros((3, m, 256), device=cuda)
+    counts = []
+    for k in range(3):
+        before = lib.spx_launch_count()
+        h.conv2d(g, sx.LAYOUT_NCHW, dX.data_ptr(), 3, 0, 0, dY.data_ptr())
+        counts.append(lib.spx_launch_count() - before)
+    torch.cuda.synchronize()
+    assert counts == [3, 5, 3]
