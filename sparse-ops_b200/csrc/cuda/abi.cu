@@ -104,6 +104,8 @@ int set_row_order(spx_ell* e, const uint32_t* host_nnz)
     std::vector<uint2> order(e->m);
     if (int rc = sort_rows(e, host_nnz, order.data(), nullptr)) return rc;
     SPX_CUDA(cudaMemcpy(e->rows, order.data(), (size_t)e->m * sizeof(uint2), cudaMemcpyHostToDevice));
+    // a copy of up to 64 KB of pageable memory may still be on its way; streams of the caller's are not ordered behind it
+    SPX_CUDA(cudaStreamSynchronize(nullptr));
     return SPX_OK;
 }
 
@@ -324,9 +326,7 @@ int spx_ell_create(uint32_t m, uint32_t n, uint32_t r, const float* Wd, const ui
         spx_ell_destroy(e);
         return fail(SPX_ERR_CUDA, "ELLPACK upload failed: %s", cudaGetErrorString(err));
     }
-    rc = set_row_order(e, nnz);
-    // copies from pageable memory may still be on their way: the handle is complete for every stream
-    if (rc == SPX_OK && cudaStreamSynchronize(nullptr) != cudaSuccess) rc = fail(SPX_ERR_CUDA, "ELLPACK upload failed");
+    rc = set_row_order(e, nnz);                 // waits: the handle is complete for every stream
     if (rc != SPX_OK) { spx_ell_destroy(e); return rc; }
     *out = e;
     return SPX_OK;
@@ -380,7 +380,6 @@ int spx_ell_create_csr(uint32_t m, uint32_t n, const uint64_t* rowptr, const uin
         std::vector<uint32_t> counts(m);
         for (uint32_t i = 0; i < m; ++i) counts[i] = (uint32_t)(rowptr[i + 1] - rowptr[i]);
         rc = set_row_order(e, counts.data());
-        if (rc == SPX_OK && cudaStreamSynchronize(nullptr) != cudaSuccess) rc = fail(SPX_ERR_CUDA, "CSR upload failed");
         if (rc != SPX_OK) { spx_ell_destroy(e); return rc; }
     }
     *out = e;

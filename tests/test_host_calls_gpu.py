@@ -309,3 +309,23 @@ def test_two_threads_make_host_calls(lib, orc, cuda):
                     assert_bit_equal(h.spmm_host(X, None), want, f"call {k}")
         jobs.append(job)
     together(*jobs)
+
+
+@pytest.mark.parametrize("slices", [1, 4, 16])
+def test_slices_are_complete_on_a_stream_of_the_callers(lib, orc, cuda, slices):
+    """The first exchange call makes the slices and multiplies them at once, here on a non-blocking stream."""
+    rng = np.random.default_rng(12)
+    m, n, Cc = 900, 700, 64
+    E = orc.encode(sparse(rng, m, n, 0.1))
+    X = rng.uniform(-1, 1, (n, Cc)).astype(np.float32)
+    want = orc.spmm(E, X, None)
+    dX = torch.from_numpy(X).to(cuda)
+    torch.cuda.synchronize()
+    for k in range(20):
+        h = lib.ell_create(E.Wd, E.idx, E.nnz, E.n)
+        dY = torch.zeros((m, Cc), device=cuda)
+        torch.cuda.synchronize()
+        with Stream(lib) as st:
+            one = (C.c_void_p * 1)(dY.data_ptr())
+            lib.spx_spmm_exchange(h.h, dX.data_ptr(), Cc, Cc, 0, 0, one, 1, 0, 0, Cc, slices, st)
+        assert_bit_equal(dY.cpu().numpy(), want, f"handle {k}")
