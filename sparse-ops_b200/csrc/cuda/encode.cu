@@ -27,12 +27,13 @@ constexpr int kQuads = 4;       // 16-byte loads in flight per lane
 // `segs` equal column segments of a row (`seg` columns each, a multiple of 4).  Rows start at any
 // element offset, so a segment is walked in 16-byte quads aligned in memory: quads 0 .. count-1 from
 // the aligned address `at`, of which only the first and the last can reach over an end of the
-// segment.  col0 is the column of quad 0's first element (negative when that lies before the row).
+// segment.  Places in a segment count from its first column (n may be anything below 2^32, a segment's
+// length is below 2^31: rows of 2^23 columns and more come in few enough to be cut): quad 0 starts at -lead.
 struct Segment {
     uint32_t row;
     int64_t at;                 // element offset of quad 0 from W (may be below 0 or the segment's start)
-    int32_t col0;
-    int32_t c_lo, c_hi;         // columns [c_lo, c_hi)
+    uint32_t c_lo;              // first column
+    int32_t lead, len;          // elements of quad 0 before the segment; columns
     uint32_t quads;
 };
 
@@ -41,27 +42,27 @@ __device__ __forceinline__ Segment segment_of(uint64_t unit, uint32_t mis, uint3
     Segment s;
     s.row = segs == 1 ? (uint32_t)unit : (uint32_t)(unit / segs);
     const uint64_t part = segs == 1 ? 0 : unit - (uint64_t)s.row * segs;
-    s.c_lo = (int32_t)min(part * seg, (uint64_t)n);
-    s.c_hi = (int32_t)min((part + 1) * seg, (uint64_t)n);
+    s.c_lo = (uint32_t)min(part * seg, (uint64_t)n);
+    s.len = (int32_t)(min((part + 1) * seg, (uint64_t)n) - s.c_lo);
     const uint64_t base = (uint64_t)s.row * n;
     const uint64_t first = base + s.c_lo + mis;             // counted from the aligned address W - mis
     s.at = (int64_t)(first & ~3ull) - (int64_t)mis;
-    s.col0 = (int32_t)(s.at - (int64_t)base);
-    s.quads = (uint32_t)((s.c_hi - s.col0 + 3) >> 2);
+    s.lead = (int32_t)(first & 3u);
+    s.quads = (uint32_t)(s.lead + s.len + 3) >> 2;
     return s;
 }
 
 // Quad i of a segment; elements outside the segment read as 0.0f, which is "no entry".
 __device__ __forceinline__ float4 load_quad(const float* __restrict__ W, const Segment& s, uint32_t i)
 {
-    const int32_t c = s.col0 + 4 * (int32_t)i;
+    const int32_t c = 4 * (int32_t)i - s.lead;
     const float* __restrict__ p = W + s.at + 4ull * i;
-    if (c >= s.c_lo && c + 4 <= s.c_hi) return __ldg(reinterpret_cast<const float4*>(p));
+    if (c >= 0 && c + 4 <= s.len) return __ldg(reinterpret_cast<const float4*>(p));
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (c >= s.c_lo && c < s.c_hi) v.x = __ldg(p);
-    if (c + 1 >= s.c_lo && c + 1 < s.c_hi) v.y = __ldg(p + 1);
-    if (c + 2 >= s.c_lo && c + 2 < s.c_hi) v.z = __ldg(p + 2);
-    if (c + 3 >= s.c_lo && c + 3 < s.c_hi) v.w = __ldg(p + 3);
+    if (c >= 0 && c < s.len) v.x = __ldg(p);
+    if (c + 1 >= 0 && c + 1 < s.len) v.y = __ldg(p + 1);
+    if (c + 2 >= 0 && c + 2 < s.len) v.z = __ldg(p + 2);
+    if (c + 3 >= 0 && c + 3 < s.len) v.w = __ldg(p + 3);
     return v;
 }
 
@@ -131,7 +132,7 @@ pack_kernel(const float* __restrict__ W, uint32_t mis, uint32_t m, uint32_t n, u
             const uint32_t b2 = __ballot_sync(0xffffffffu, v[u].z != 0.0f), b3 = __ballot_sync(0xffffffffu, v[u].w != 0.0f);
             // entries of the lanes below come first, then this lane's own in column order
             uint32_t at = pos + __popc(b0 & below) + __popc(b1 & below) + __popc(b2 & below) + __popc(b3 & below);
-            const uint32_t col = (uint32_t)(s.col0 + 4 * (int32_t)(qb + 32 * u + lane));
+            const uint32_t col = s.c_lo + 4 * (qb + 32 * u + lane) - (uint32_t)s.lead;
             if (v[u].x != 0.0f) { wd[at] = v[u].x; ix[at++] = col; }
             if (v[u].y != 0.0f) { wd[at] = v[u].y; ix[at++] = col + 1; }
             if (v[u].z != 0.0f) { wd[at] = v[u].z; ix[at++] = col + 2; }
@@ -187,18 +188,18 @@ decode_rows_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ id
         uint32_t end = cnt;
         while (pos < end) {
             const uint32_t mid = (pos + end) >> 1;
-            if (__ldg(ix + mid) < (uint32_t)s.c_lo) pos = mid + 1; else end = mid;
+            if (__ldg(ix + mid) < s.c_lo) pos = mid + 1; else end = mid;
         }
     }
-    for (uint32_t qb = 0; qb < s.quads; qb += kDecode / 4) {        // strip element i <-> column c0 + i
-        const int32_t c0 = s.col0 + 4 * (int32_t)qb, c1 = min(c0 + (int32_t)kDecode, s.c_hi);
-        uint32_t k[kRun];
+    for (uint32_t qb = 0; qb < s.quads; qb += kDecode / 4) {        // strip element i <-> place c0 + i of the segment
+        const int32_t c0 = 4 * (int32_t)qb - s.lead, c1 = min(c0 + (int32_t)kDecode, s.len);
+        uint32_t k[kRun];                                           // places; columns ascend, so all are at or behind the first
         float w[kRun];
         auto fetch = [&] {
 #pragma unroll
             for (int u = 0; u < kRun; ++u) {
                 const uint32_t j = pos + 32 * u + lane;
-                k[u] = j < cnt ? __ldg(ix + j) : 0x7fffffffu;
+                k[u] = j < cnt ? __ldg(ix + j) - s.c_lo : 0xffffffffu;
                 w[u] = j < cnt ? __ldg(wd + j) : 0.0f;
             }
         };
@@ -210,7 +211,7 @@ decode_rows_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ id
             uint32_t took = 0;
 #pragma unroll
             for (int u = 0; u < kRun; ++u) {
-                const bool in = (int32_t)k[u] < c1;
+                const bool in = k[u] < (uint32_t)c1;
                 if (in) strip[(int32_t)k[u] - c0] = w[u];
                 took += __popc(__ballot_sync(0xffffffffu, in));     // a prefix: columns ascend
             }
@@ -225,11 +226,11 @@ decode_rows_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ id
             const int32_t c = c0 + 4 * (int32_t)i;
             const float4 v = reinterpret_cast<const float4*>(strip)[i];
             float* __restrict__ o = out + 4 * i;
-            if (c >= s.c_lo && c + 4 <= s.c_hi) { __stcs(reinterpret_cast<float4*>(o), v); continue; }
-            if (c >= s.c_lo && c < s.c_hi) o[0] = v.x;
-            if (c + 1 >= s.c_lo && c + 1 < s.c_hi) o[1] = v.y;
-            if (c + 2 >= s.c_lo && c + 2 < s.c_hi) o[2] = v.z;
-            if (c + 3 >= s.c_lo && c + 3 < s.c_hi) o[3] = v.w;
+            if (c >= 0 && c + 4 <= s.len) { __stcs(reinterpret_cast<float4*>(o), v); continue; }
+            if (c >= 0 && c < s.len) o[0] = v.x;
+            if (c + 1 >= 0 && c + 1 < s.len) o[1] = v.y;
+            if (c + 2 >= 0 && c + 2 < s.len) o[2] = v.z;
+            if (c + 3 >= 0 && c + 3 < s.len) o[3] = v.w;
         }
         __syncwarp();
     }
@@ -261,8 +262,8 @@ Split split_rows(uint32_t m, uint32_t n, int sms)
     const uint64_t want = (uint64_t)sms * 64;
     const uint64_t most = std::max<uint64_t>(1, n / 1024);
     s.segs = (uint32_t)std::min<uint64_t>(most, std::max<uint64_t>(1, (want + m - 1) / m));
-    s.seg = spx::round_up((n + s.segs - 1) / s.segs, 4u);
-    s.segs = (n + s.seg - 1) / s.seg;
+    s.seg = (uint32_t)spx::round_up<uint64_t>(((uint64_t)n + s.segs - 1) / s.segs, 4u);
+    s.segs = (uint32_t)(((uint64_t)n + s.seg - 1) / s.seg);
     s.blocks = (unsigned)(((uint64_t)m * s.segs + kWarps - 1) / kWarps);
     return s;
 }

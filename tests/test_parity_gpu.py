@@ -930,3 +930,29 @@ def test_l2_gather_probe_runs(cuda):
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     assert n.value == sms * 8 * 8 * 4 * 8 * 512 and float(sink.item()) == 7.0
     assert probe(buf.data_ptr(), 512, 4, sink.data_ptr(), 0, ctypes.byref(n)) == -1
+
+
+def test_device_codec_with_rows_beyond_two_to_the_31(lib, cuda):
+    """Columns are 32-bit unsigned: rows longer than 2^31, entries on both sides of it, the second row off the 16-byte
+    grid (34 GB on the device)."""
+    n = (1 << 31) + 4101
+    W = torch.zeros((2, n), device=cuda)
+    cols = [[0, 5, (1 << 31) - 3, (1 << 31) - 1, 1 << 31, (1 << 31) + 2, n - 1], [1, 77777, 1 << 30, (1 << 31) - 2, (1 << 31) + 4000]]
+    rng = np.random.default_rng(13)
+    near = np.unique(rng.integers((1 << 31) - 300000, n, 5000)).tolist()
+    cols[1] = sorted(set(cols[1] + near))
+    for r in range(2):
+        W[r, torch.tensor(cols[r], device=cuda)] = torch.arange(1, len(cols[r]) + 1, device=cuda, dtype=torch.float32)
+    h = lib.ell_encode_device(W.data_ptr(), 2, n)
+    Wd, idx, nnz = h.download()
+    assert nnz.tolist() == [len(c) for c in cols]
+    for r in range(2):
+        c = len(cols[r])
+        assert idx[r, :c].tolist() == cols[r] and Wd[r, :c].tolist() == list(range(1, c + 1))
+        assert not Wd[r, c:].any() and not idx[r, c:].any()
+    out = torch.full((2, n), 7.0, device=cuda)
+    lib.spx_ell_decode_device(h.h, out.data_ptr(), 0)
+    torch.cuda.synchronize()
+    step = 1 << 28
+    for r in range(2):
+        assert all(torch.equal(out[r, at:at + step], W[r, at:at + step]) for at in range(0, n, step))
