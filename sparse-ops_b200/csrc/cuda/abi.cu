@@ -694,6 +694,14 @@ static inline uint32_t host_panel_width(uint32_t c0, uint32_t C)
     return std::min<uint32_t>(256, C - c0);
 }
 
+// Whether an operand is page-locked: work that the caller has queued on the default stream may then still fill or read
+// it, and the call runs on that stream (`queued`).  (A stream that the runtime orders with the default one will not do: its first
+// copy of up to 24 KB from page-locked memory is read when it is submitted.)
+static bool any_page_locked(const void* a, const void* b, const void* c)
+{
+    return (a && !pageable_memory(a)) || (b && !pageable_memory(b)) || (c && !pageable_memory(c));
+}
+
 // One host-buffer call: a stream, and a pinned block through which operands travel that are too small for
 // copy_h2d's pieces: inputs are packed and sent as one copy, a result is fetched into the block and copied
 // on, or, where it is small, stored there by the kernel -- a pageable copy costs the driver's staging and a
@@ -708,8 +716,9 @@ struct HostCall {
     bool open = false;
 
     // result_bytes: of the result, if it may travel through the block (0: it does not)
-    int begin(int device, size_t result_bytes) {
-        if (int rc = host_stream(device, 0, &stream)) return rc;
+    int begin(int device, size_t result_bytes, bool queued) {
+        if (!queued)
+            if (int rc = host_stream(device, 0, &stream)) return rc;
         if (int rc = pinned_acquire(kInputs + (result_bytes <= kResult ? result_bytes : 0), &block)) return rc;
         open = true;
         return SPX_OK;
@@ -728,7 +737,7 @@ struct HostCall {
     int send(void* dst, const void* a, size_t a_bytes, const void* b, size_t b_bytes, size_t gap) {
         // The device reads page-locked inputs itself, in stream order: queued work may still write them, and a copy of
         // them costs more than a second transfer (6000 x 2500, C = 17, page-locked: 70 us through the block, 60 so).
-        if ((a_bytes && !pageable_memory(a)) || (b_bytes && !pageable_memory(b))) {
+        if (any_page_locked(a_bytes ? a : nullptr, b_bytes ? b : nullptr, nullptr)) {
             if (b_bytes) SPX_CUDA(cudaMemcpyAsync(static_cast<char*>(dst) + gap, b, b_bytes, cudaMemcpyHostToDevice, stream));
             return copy_h2d(dst, a, a_bytes, stream);
         }
@@ -760,7 +769,7 @@ struct HostCall {
         return SPX_OK;
     }
     ~HostCall() {
-        if (open && stream) (void)cudaStreamSynchronize(stream);   // an error on the way: nothing may still use the block
+        if (open) (void)cudaStreamSynchronize(stream);   // an error on the way: nothing may still use the block
         pinned_release(block);
     }
 };
@@ -780,6 +789,10 @@ static int spmm_host_panels(spx_ell* e, const float* X, uint32_t C, const float*
     for (int i = 0; i < 3; ++i)
         if (int rc = host_stream(e->device, i, &st.s[i])) return rc;
     for (cudaEvent_t& v : done.ev) SPX_CUDA(cudaEventCreateWithFlags(&v, cudaEventDisableTiming));
+    if (any_page_locked(X, bias, Y)) {          // behind what is queued on the default stream, see above
+        SPX_CUDA(cudaEventRecord(done.ev[3], nullptr));
+        SPX_CUDA(cudaStreamWaitEvent(st.s[0], done.ev[3], 0));
+    }
     if (bias) SPX_CUDA(cudaMemcpyAsync(dB, bias, (size_t)e->m * 4, cudaMemcpyHostToDevice, st.s[0]));
     const uint32_t w = C / 2;                   // a multiple of 4
     const bool pageable = pageable_memory(Y);
@@ -865,7 +878,7 @@ int spx_spmm_host(const spx_ell* ce, const float* X, uint32_t C, const float* bi
     }
     const size_t y_bytes = (size_t)e->m * C * 4;
     HostCall call;
-    rc = call.begin(e->device, y_bytes);
+    rc = call.begin(e->device, y_bytes, any_page_locked(X, bias, Y));
     if (rc == SPX_OK) rc = call.send(dX, X, (size_t)e->n * C * 4, bias, bias ? (size_t)e->m * 4 : 0, xb);
     if (rc != SPX_OK) return rc;
     float* direct = y_bytes <= HostCall::kSmall && C >= 8 ? call.mapped_result() : nullptr;
@@ -985,7 +998,7 @@ int spx_spmv_host(const spx_ell* ce, const float* x, const float* bias, float* y
     float* dy = reinterpret_cast<float*>(base + xb + bb);
     const size_t y_bytes = (size_t)e->m * 4;
     HostCall call;
-    rc = call.begin(e->device, y_bytes);
+    rc = call.begin(e->device, y_bytes, any_page_locked(x, bias, y));
     if (rc == SPX_OK) rc = call.send(dx, x, (size_t)e->n * 4, bias, bias ? y_bytes : 0, xb);
     if (rc != SPX_OK) return rc;
     // single floats to the host cost more than a copy beyond a thousand of them (5519 rows: 28 us against 24)

@@ -143,11 +143,11 @@ void pool_trim(int device)
     if (g_pools[device]) (void)cudaMemPoolTrimTo(g_pools[device], 0);
 }
 
-static int kept_stream(cudaStream_t (&streams)[kMaxDevices], int device, cudaStream_t* out, unsigned flags)
+static int kept_stream(cudaStream_t (&streams)[kMaxDevices], int device, cudaStream_t* out)
 {
     if (device < 0 || device >= kMaxDevices) return fail(SPX_ERR_LIMIT, "device ordinal %d not supported", device);
     std::lock_guard<std::mutex> lk(g_pool_mu);
-    if (!streams[device]) SPX_CUDA(cudaStreamCreateWithFlags(&streams[device], flags));
+    if (!streams[device]) SPX_CUDA(cudaStreamCreateWithFlags(&streams[device], cudaStreamNonBlocking));
     *out = streams[device];
     return SPX_OK;
 }
@@ -155,7 +155,7 @@ static int kept_stream(cudaStream_t (&streams)[kMaxDevices], int device, cudaStr
 int side_stream(int device, cudaStream_t* out)
 {
     static cudaStream_t streams[kMaxDevices] = {};
-    return kept_stream(streams, device, out, cudaStreamNonBlocking);
+    return kept_stream(streams, device, out);
 }
 
 int host_stream(int device, int which, cudaStream_t* out)
@@ -165,8 +165,7 @@ int host_stream(int device, int which, cudaStream_t* out)
         ~Streams() { for (auto& k : s) for (cudaStream_t st : k) if (st) (void)cudaStreamDestroy(st); }
     };
     thread_local Streams mine;
-    // ordered behind what the caller has queued on the default stream (a copy into an operand, for instance)
-    return kept_stream(mine.s[which], device, out, cudaStreamDefault);
+    return kept_stream(mine.s[which], device, out);
 }
 
 int pinned_acquire(size_t bytes, PinnedBlock* out)
