@@ -29,18 +29,14 @@ int fail(int code, const char* fmt, ...)
 
 int sm_count(int device)
 {
-    static std::mutex mu;
-    static int cache[64];
-    static bool have[64];
+    static std::atomic<int> cache[64] = {};
     if (device < 0 || device >= 64) return 148;
-    std::lock_guard<std::mutex> lk(mu);
-    if (!have[device]) {
-        int v = 0;
+    int v = cache[device].load(std::memory_order_relaxed);
+    if (!v) {
         if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || v <= 0) v = 148;
-        cache[device] = v;
-        have[device] = true;
+        cache[device].store(v, std::memory_order_relaxed);
     }
-    return cache[device];
+    return v;
 }
 
 // The zero fill of the slabs is enqueued on `s`, the stream the caller fills them on afterwards:

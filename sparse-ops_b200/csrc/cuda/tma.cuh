@@ -36,6 +36,11 @@ __device__ __forceinline__ uint32_t mbar_arrive_pending(uint64_t* bar) {
                  : "=r"(pending) : "r"((uint32_t)__cvta_generic_to_shared(bar)) : "memory");
     return pending;
 }
+// Acquires the arrivals of a phase that is known to be complete.
+__device__ __forceinline__ void mbar_acquire(uint64_t* bar, uint32_t parity) {
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%0], %1;\n\t}"
+                 ::"r"((uint32_t)__cvta_generic_to_shared(bar)), "r"(parity) : "memory");
+}
 // Waits for the phase with the given parity; gives up one second (of the GPU's wall clock) after
 // its 256th unsuccessful poll and returns false, so a copy that never completes cannot hang the GPU.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
