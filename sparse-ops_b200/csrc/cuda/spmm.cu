@@ -12,7 +12,7 @@
 //   spmm_tile_kernel          (spmm_tile.cu) columns are used often enough by the rows of a CTA to stage X
 //                             block by block
 //   spmm_rows                 everything else: rows of X gathered through L1 / L2
-//   spmm_gather_half          64 < C <= 128 and very many short rows
+//   spmm_gather_half          44 <= C <= 128 and many short rows
 //   spmm_gather_staged        a few long rows decide the duration (row shard of a skewed matrix)
 // Column panels are the slow grid dimension so that all CTAs in flight work on the same X panel.
 // Rows are taken from the handle's sorted row schedule (longest first), so the warps of a CTA
@@ -217,20 +217,20 @@ spmm_gather_staged(const float* __restrict__ Wd, const uint32_t* __restrict__ id
 }
 
 // ---------------------------------------------------------------------------------------
-// spmm_gather_half: 64 < C <= 128.  With a full warp per row a lane would own one float4 and the
+// spmm_gather_half: short rows, 32 < C <= 128.  With a full warp per row a lane would own at most one float4 and the
 // per-entry work that does not scale with the width (two shuffles, the row address, the loop)
-// would be spread over 4 FMAs; here 16 lanes share a row and own two float4 each, a warp carries
+// would be spread over 4 FMAs; here 16 lanes share a row and own NV float4 each, a warp carries
 // two neighbouring rows of the sorted schedule, and every shuffle / address / load instruction
 // serves both rows.  Same chain per output element.
 // ---------------------------------------------------------------------------------------
-template <int G, int MINB>
-__global__ void __launch_bounds__(kGatherWarps * 32, MINB)
-spmm_gather_half(const float* __restrict__ Wd, const uint32_t* __restrict__ idx,
-                 const uint32_t* __restrict__ nnz, const uint2* __restrict__ rows,
+template <int NV>
+__global__ void __launch_bounds__(kGatherWarps * 32, 4)
+spmm_gather_half(const float* __restrict__ Wd, const uint32_t* __restrict__ idx, const uint2* __restrict__ rows,
                  uint32_t m, uint32_t pitch,
                  const float* __restrict__ X, uint32_t C, uint64_t ldx,
-                 const float* __restrict__ bias, int act, PeerOut out, uint64_t ldy)
+                 const float* __restrict__ bias, int act, PeerOut out, uint64_t ldy, bool early)
 {
+    constexpr int G = 4;                        // gathers in flight per vector
     const int lane = threadIdx.x & 31;
     const int sl = lane & 15;
     const uint32_t slot = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 2 + (lane >> 4);
@@ -238,18 +238,20 @@ spmm_gather_half(const float* __restrict__ Wd, const uint32_t* __restrict__ idx,
     const uint2 ri = live ? __ldg(rows + slot) : make_uint2(0u, 0u);
     const uint32_t row = ri.x;
     const uint32_t c0 = 4u * sl;
-    bool on[2];
+    bool on[NV];
 #pragma unroll
-    for (int v = 0; v < 2; ++v) on[v] = live && (c0 + 64u * v) < C;
+    for (int v = 0; v < NV; ++v) on[v] = live && (c0 + 64u * v) < C;
 
-    const float b = (live && bias) ? __ldg(bias + row) : 0.0f;
-    float4 acc[2];
-#pragma unroll
-    for (int v = 0; v < 2; ++v) acc[v] = make_float4(b, b, b, b);
     const uint32_t nn = ri.y;
     const uint32_t nmax = __reduce_max_sync(0xffffffffu, nn);       // the warp runs to its longer row
     const float* __restrict__ w = Wd + (size_t)row * pitch;
     const uint32_t* __restrict__ k = idx + (size_t)row * pitch;
+    spx::pdl_wait();
+    if (early) spx::pdl_launch();
+    const float b = (live && bias) ? __ldg(bias + row) : 0.0f;
+    float4 acc[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) acc[v] = make_float4(b, b, b, b);
 
     for (uint32_t j0 = 0; j0 < nmax; j0 += 16) {
         float wl = 0.0f;
@@ -262,7 +264,7 @@ spmm_gather_half(const float* __restrict__ Wd, const uint32_t* __restrict__ idx,
         const uint32_t cmax = min(16u, nmax - j0);
         for (uint32_t t0 = 0; t0 < cmax; t0 += G) {
             float wt[G];
-            float4 xv[G][2];
+            float4 xv[G][NV];
 #pragma unroll
             for (int u = 0; u < G; ++u) {
                 wt[u] = __shfl_sync(0xffffffffu, wl, (t0 + u) & 15, 16);
@@ -270,20 +272,21 @@ spmm_gather_half(const float* __restrict__ Wd, const uint32_t* __restrict__ idx,
                 const float* xr = X + (size_t)kt * ldx + c0;
                 const bool have = (t0 + u) < cnt;
 #pragma unroll
-                for (int v = 0; v < 2; ++v)
+                for (int v = 0; v < NV; ++v)
                     xv[u][v] = (have && on[v]) ? ldg4(xr + 64 * v) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
 #pragma unroll
             for (int u = 0; u < G; ++u) {
                 if ((t0 + u) < cnt) {
 #pragma unroll
-                    for (int v = 0; v < 2; ++v) fma4(acc[v], wt[u], xv[u][v]);
+                    for (int v = 0; v < NV; ++v) fma4(acc[v], wt[u], xv[u][v]);
                 }
             }
         }
     }
+    spx::pdl_launch();
 #pragma unroll
-    for (int v = 0; v < 2; ++v) {
+    for (int v = 0; v < NV; ++v) {
         if (on[v]) {
             float4 o = acc[v];
             if (act != SPX_ACT_NONE) {
@@ -1054,7 +1057,29 @@ static int launch_rows(const spx_ell* e, RowsArgs a, cudaStream_t s)
 }
 
 int launch_spmm_tile(spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const float* bias, int act, const PeerOut& out,
-                     uint64_t ldy, bool vec_x, bool vec_out, bool again, cudaStream_t s);
+                     uint64_t ldy, bool vec_x, bool vec_out, uint32_t V, bool half, bool again, cudaStream_t s);
+
+// Short rows: the ring of spmm_rows costs more than it hides, and half warps leave fewer lanes idle than its 11 to 31
+// lanes a row do.  Measured, half against rows, back to back / alone: 20000 rows of 16 to 64 entries, C = 96 0.75 / 0.80,
+// C = 48 0.85 / 0.90, C = 64 0.99 - 1.14 / 0.95 - 1.05, C = 40 0.96 - 1.17; 5000 rows, C = 68 to 128 0.72 - 0.86 / 0.82 - 0.91,
+// C = 48 0.83 - 0.96 / 0.87 - 0.97; 3500 rows, C = 68 to 128 0.84 - 1.02 / 0.87 - 0.94, C = 48 0.94 - 1.4.
+static bool takes_half(const spx_ell* e, uint32_t C)
+{
+    const uint64_t sms = sm_count(e->device);
+    if (e->nnz_total >= 128ull * e->m) return false;
+    return C > 64 && C <= 128 ? e->m >= 16 * sms : C >= 44 && C <= 60 && e->m >= 32 * sms;
+}
+
+static int launch_half(const spx_ell* e, const RowsArgs& a, cudaStream_t s)
+{
+    const uint32_t warps = (e->m + 1) / 2;
+    uint32_t wpb = 8;
+    while (wpb > 1 && (uint64_t)((warps + wpb - 1) / wpb) < (uint64_t)sm_count(e->device) * 8) wpb >>= 1;
+    const dim3 grid((warps + wpb - 1) / wpb), block(wpb * 32);
+    const bool early = (uint64_t)warps * 2 <= (uint64_t)sm_count(e->device) * 32;       // as in launch_rows_one: 64 registers
+    return finish_launch(launch_pdl(a.C > 64 ? spmm_gather_half<2> : spmm_gather_half<1>, grid, block, 0, s, a.Wd, a.idx, a.rows, a.m, a.pitch,
+                                    a.X, a.C, a.ldx, a.bias, a.act, a.out, a.ldy, early), "spmm_gather_half");
+}
 
 int launch_spmm(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const float* bias,
                 int act, float* Y, uint64_t ldy, cudaStream_t s, bool again)
@@ -1101,26 +1126,20 @@ int launch_spmm_bcast(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx
     if (staged && chain) return launch_chain(e, a, s);
     if (staged && vec_ok && C >= 8 && C <= 64 && len >= 80 && m <= (uint64_t)sm_count(e->device) * (kChainConsumers / (C / 4)))
         return launch_direct(e, a, true, s);
+    // what gathers X if X is not staged: vectors of V floats
+    const uint32_t V = vec_ok ? 4 : C % 2 == 0 && ldx % 2 == 0 && (reinterpret_cast<uintptr_t>(X) & 7) == 0 ? 2 : 1;
+    const bool half = vec_ok && takes_half(e, C);
     {
         const bool vec_x = C % 4 == 0 && ldx % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
-        const int rc = launch_spmm_tile(const_cast<spx_ell*>(e), X, C, ldx, bias, act, out, ldy, vec_x, C % 4 == 0 && ldy % 4 == 0 && aligned, again, s);
+        const int rc = launch_spmm_tile(const_cast<spx_ell*>(e), X, C, ldx, bias, act, out, ldy, vec_x, C % 4 == 0 && ldy % 4 == 0 && aligned, V, half, again, s);
         if (rc != -1) return rc;
     }
     if (ldx >= (1ull << 30)) {
         const uint64_t blocks = ((uint64_t)e->m * C + 255) / 256;
         if (blocks > 0x7fffffffull) return fail(SPX_ERR_LIMIT, "spmm: grid too large");
         return finish_launch(launch_pdl(spmm_simple, dim3((unsigned)blocks), dim3(256), 0, s, a), "spmm_simple");
-    } else if (vec_ok && C > 64 && C <= 128 && e->m >= (uint64_t)sm_count(e->device) * 64 && e->nnz_total < 128ull * e->m) {
-        // many short rows: the ring of spmm_rows costs more than it hides (100000 power-law rows, mean 64,
-        // C = 96: 144 us against 156)
-        const uint32_t warps = (e->m + 1) / 2;
-        uint32_t wpb = 8;
-        while (wpb > 1 && (uint64_t)((warps + wpb - 1) / wpb) < (uint64_t)sm_count(e->device) * 8) wpb >>= 1;
-        const uint32_t blocks = (warps + wpb - 1) / wpb;
-        spmm_gather_half<4, 4><<<blocks, wpb * 32, 0, s>>>(e->Wd, e->idx, e->nnz, e->rows, e->m, e->pitch,
-                                                          X, C, ldx, bias, act, out, ldy);
-        SPX_LAUNCH_CHECK("spmm_gather_half");
-        return SPX_OK;
+    } else if (half) {
+        return launch_half(e, a, s);
     } else if (vec_ok && C > 128) {
         // A row is one dependent chain of gathers, G rows of X per round trip to L2 (about a
         // microsecond under load).  When the longest row's chain is a large part of the whole
@@ -1149,8 +1168,7 @@ int launch_spmm_bcast(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx
             return SPX_OK;
         }
     }
-    const bool pairs = C % 2 == 0 && ldx % 2 == 0 && (reinterpret_cast<uintptr_t>(X) & 7) == 0;
-    return vec_ok ? launch_rows<4>(e, a, s) : pairs ? launch_rows<2>(e, a, s) : launch_rows<1>(e, a, s);
+    return V == 4 ? launch_rows<4>(e, a, s) : V == 2 ? launch_rows<2>(e, a, s) : launch_rows<1>(e, a, s);
 }
 
 }  // namespace spx

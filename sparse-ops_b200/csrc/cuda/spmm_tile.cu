@@ -467,9 +467,14 @@ struct Plan {
 // Launch shape and expected time.  As few waves of CTAs as kMaxWarps warps each allow, and then equally
 // many warps in every CTA.  Time: the results' way out, about half a microsecond per phase (wait, hand-off, a
 // block of steps cut short; more where X's rows do not begin on lines), and per step of a warp the
-// larger of its latency and the shared-memory wavefronts of all the SM's warps (16 NV gathers + 4 of hand-off,
-// one per cycle).  Fitted to 65 shapes of 256 to 8192 rows and columns, 2 to 50 % dense, C = 9 to 1000: rms 11 %.
-Plan plan_tiles(const spx_ell* e, uint32_t C, uint32_t NV, uint32_t sms)
+// larger of its latency and the shared-memory wavefronts of all the SM's warps (16 NV gathers + 4 of hand-off).
+// A phase in which any row of a group has an entry due takes a step, however few they are: rows of less than a
+// few entries per chunk are mostly empty slots (60000 x 4000, 8 entries a row, C = 33: 91 us against 30 gathered).
+// The constants of both estimates are fitted to 1564 measured shapes (256 to 150000 rows, 256 to 60000 columns, 3 to 2500
+// entries a row, C = 1 to 1000): the kernel they choose takes 0.2 % longer than the faster one on average, more
+// than 10 % longer for 14 of them (without that term, and with one kind of gather for every unaligned X: 1.6 %, 58, and
+// up to 3.6 times).
+Plan plan_tiles(const spx_ell* e, uint32_t C, uint32_t NV, uint32_t sms, bool aligned)
 {
     Plan p;
     const uint32_t groups = (e->m + kGroupRows - 1) / kGroupRows, chunks = (e->n + kChunk - 1) / kChunk;
@@ -478,42 +483,46 @@ Plan plan_tiles(const spx_ell* e, uint32_t C, uint32_t NV, uint32_t sms)
     p.waves = (units + (uint64_t)sms * kMaxWarps - 1) / ((uint64_t)sms * kMaxWarps);
     p.warps = (uint32_t)std::min<uint64_t>(kMaxWarps, (units + sms * p.waves - 1) / (sms * p.waves));
     while (p.warps < kMaxWarps && (uint64_t)((groups + p.warps - 1) / p.warps) * p.slices > p.waves * sms) ++p.warps;
-    const double len = (double)e->nnz_total / e->m, steps = (len + 1.1 * std::sqrt(len)) / 4.0;
-    p.us = 0.9 + (double)e->m * C * 0.62e-6 + (C % 32 ? 0.2 * chunks : 0.0) +
-           p.waves * (1.4 + chunks * (NV == 1 ? 0.50 : 0.37) + steps * std::max(NV == 1 ? 0.053 : 0.098, p.warps * (16.0 * NV + 4.0) / 1950.0));
+    const double len = (double)e->nnz_total / e->m;
+    const double steps = std::max((len + 1.1 * std::sqrt(len)) / 4.0, chunks * (1.0 - std::exp(-(double)kGroupRows * len / chunks)));
+    p.us = 0.9 + (double)e->m * C * 0.62e-6 + (C % 32 ? 0.17 * chunks : 0.0) + (aligned ? 0.0 : 3.5) +
+           p.waves * (2.65 + chunks * (NV == 1 ? 0.45 : 0.40) + steps * std::max(NV == 1 ? 0.0515 : 0.096, p.warps * (16.0 * NV + 4.0) / 2480.0));
     return p;
 }
 
-// Expected time of the gather kernel (spmm_rows): its warps' load instructions, which L1 passes at 4 (16-byte
-// vectors) or 2 cycles and some, and about 0.1 us of each warp's own; or the rounds of the longest row, for every wave
-// of warps where the deep groups let only 8 to 9 per SM reside.  Fitted to the same shapes: rms 11 %.
-double gather_us(const spx_ell* e, uint32_t C, bool aligned)
+// Expected time of gathering in vectors of V floats (spmm_rows, or spmm_gather_half): the warps' load instructions,
+// which L1 passes at 4, 2 or 1 cycles and some, and up to 0.1 us of each warp's own; or the rounds of the longest row,
+// for every wave of warps where the deep groups let only 8 per SM reside.
+double gather_us(const spx_ell* e, uint32_t C, uint32_t V, bool half)
 {
     const double sms = sm_count(e->device);
-    const uint32_t q = aligned ? (C + 3) / 4 : C, nv_max = aligned ? 2 : 3;
+    const uint32_t q = (C + V - 1) / V, nv_max = V == 4 ? 2 : 3;
     const uint32_t NV = std::min(nv_max, (q + 31) / 32), panels = (q + 32 * NV - 1) / (32 * NV);
     const uint32_t RW = NV > 1 ? 1u : std::min(32 / q, 16u);
     const double per_sm = std::ceil((double)e->m / RW) * panels / sms;
-    const double loads = e->nnz_total / sms * ((aligned ? 3.2e-3 : 1.5e-3) * panels * NV / RW + (C % 32 ? 0.64e-3 : 0.0)) + 0.09 * per_sm;
-    const bool deep = NV == 1 && (per_sm < 48 || e->nnz_total >= 100ull * e->m);
-    const double rounds = e->max_nnz * (NV == 1 ? 0.0275 : 0.0526) * (deep ? std::max(1.0, std::ceil(per_sm / 8.75)) : 1.0);
-    return 1.6 + std::sqrt(std::sqrt(std::pow(loads, 4) + std::pow(rounds, 4)));
+    const bool brief = e->nnz_total < 100ull * e->m;
+    const double load = V == 4 ? 3.15e-3 : V == 2 ? 1.7e-3 : 1.34e-3, off_lines = V == 4 ? 0.47e-3 : V == 2 ? 0.5e-3 : 0.39e-3;
+    const double loads = e->nnz_total / sms * panels * (load * NV / RW + (C % 32 ? off_lines : 0.0)) + (brief ? 0.037 : 0.10) * per_sm;
+    double rounds = e->max_nnz;
+    if (V == 1 && per_sm < 12) rounds *= 0.0115 * NV * (NV == 3 ? std::ceil(per_sm / 8.0) : 1.0);
+    else rounds *= (NV == 1 ? 0.0168 : 0.0282) * (NV == 1 && (per_sm < 48 || !brief) ? std::max(1.0, std::ceil(per_sm / 8.0)) : 1.0);
+    return (3.5 + std::sqrt(std::sqrt(std::pow(loads, 4) + std::pow(rounds, 4)))) * (half ? 0.9 : 1.0);
 }
 
 }  // namespace
 
 // Returns -1 when the shape or the handle is not for this kernel.
 int launch_spmm_tile(spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const float* bias, int act, const PeerOut& out,
-                     uint64_t ldy, bool vec_x, bool vec_out, bool again, cudaStream_t s)
+                     uint64_t ldy, bool vec_x, bool vec_out, uint32_t V, bool half, bool again, cudaStream_t s)
 {
     static const int env = [] { const char* v = getenv("SPX_SPMM_TILE"); return v ? atoi(v) : 1; }();
     if (!env || !e->tiles || !e->cols_ascending || e->tma_off || e->max_nnz == 0) return -1;
     const PFN_cuTensorMapEncodeTiled encode = tensor_map_encoder();
     if (!encode || ldx > 0xffffffffull || e->n > 65536 || C > (1u << 30)) return -1;
     const uint32_t NV = C <= 32 ? 1 : 2;
-    const Plan p = plan_tiles(e, C, NV, sm_count(e->device));
+    const Plan p = plan_tiles(e, C, NV, sm_count(e->device), vec_x);
     if ((uint64_t)p.slices * e->m > 0x7fffffffull) return -1;
-    if (env != 2 && (e->n < kChunk || p.us + (vec_x ? 0.0 : 4.0) > 0.97 * gather_us(e, C, vec_x))) return -1;
+    if (env != 2 && (e->n < kChunk || p.us > 1.02 * gather_us(e, C, V, half))) return -1;
     spx_tiles_impl* t = static_cast<spx_tiles_impl*>(e->tiles);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (t->state != 1 || !vec_x) {              // building and the scratch below allocate: not while a graph is captured
