@@ -956,3 +956,18 @@ def test_device_codec_with_rows_beyond_two_to_the_31(lib, cuda):
     step = 1 << 28
     for r in range(2):
         assert all(torch.equal(out[r, at:at + step], W[r, at:at + step]) for at in range(0, n, step))
+
+
+@pytest.mark.parametrize("n", [1, 3, 127, 128, 129])
+def test_device_decode_of_narrow_matrices(lib, orc, cuda, n):
+    """Below 128 columns the decoder clears and scatters, from there on it rebuilds rows in strips."""
+    rng = np.random.default_rng(n)
+    m = 3000
+    W = sparse(rng, m, n, 0.3)
+    W[5] = 0
+    dW = dev(W, cuda)
+    h = lib.ell_encode_device(dW.data_ptr(), m, n)
+    out = torch.full((m, n), 7.0, device=cuda)
+    lib.spx_ell_decode_device(h.h, out.data_ptr(), 0)
+    torch.cuda.synchronize()
+    assert_bit_equal(out.cpu().numpy(), orc.decode(orc.encode(W)), "decode")
