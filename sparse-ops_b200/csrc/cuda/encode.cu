@@ -354,8 +354,8 @@ int decode_device(const spx_ell* e, float* dW, cudaStream_t s)
         return SPX_OK;
     }
     // A row of a few columns is not worth a warp's strip: 100000 x 64 35 us through strips, 25 cleared and scattered;
-    // 300000 x 100 95 and 93, 200000 x 200 74 and 88.
-    if (e->cols_ascending && e->n >= 128) {
+    // 300000 x 100 95 and 93, 200000 x 200 74 and 88.  (Few rows: one launch is less than two, 64 x 64 14 us against 18.)
+    if (e->cols_ascending && (e->n >= 128 || e->m < 32768)) {
         const Split sp = split_rows(e->m, e->n, sm_count(e->device));
         decode_rows_kernel<<<sp.blocks, kWarps * 32, 0, s>>>(e->Wd, e->idx, e->nnz, misalignment(dW), e->m, e->n, sp.segs, sp.seg,
                                                             e->pitch, dW);

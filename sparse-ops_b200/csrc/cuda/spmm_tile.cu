@@ -522,7 +522,7 @@ int launch_spmm_tile(spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const
     const uint32_t NV = C <= 32 ? 1 : 2;
     const Plan p = plan_tiles(e, C, NV, sm_count(e->device), vec_x);
     if ((uint64_t)p.slices * e->m > 0x7fffffffull) return -1;
-    if (env != 2 && (e->n < kChunk || p.us > 1.02 * gather_us(e, C, V, half))) return -1;
+    if (env != 2 && (e->n < kChunk || p.us > 1.05 * gather_us(e, C, V, half))) return -1;
     spx_tiles_impl* t = static_cast<spx_tiles_impl*>(e->tiles);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (t->state != 1 || !vec_x) {              // building and the scratch below allocate: not while a graph is captured

@@ -958,11 +958,10 @@ def test_device_codec_with_rows_beyond_two_to_the_31(lib, cuda):
         assert all(torch.equal(out[r, at:at + step], W[r, at:at + step]) for at in range(0, n, step))
 
 
-@pytest.mark.parametrize("n", [1, 3, 127, 128, 129])
-def test_device_decode_of_narrow_matrices(lib, orc, cuda, n):
-    """Below 128 columns the decoder clears and scatters, from there on it rebuilds rows in strips."""
+@pytest.mark.parametrize("m,n", [(3000, 3), (32767, 7), (32768, 1), (32768, 127), (32768, 128), (40000, 9)])
+def test_device_decode_of_narrow_matrices(lib, orc, cuda, m, n):
+    """Many rows of less than 128 columns are cleared and scattered, all others rebuilt in strips."""
     rng = np.random.default_rng(n)
-    m = 3000
     W = sparse(rng, m, n, 0.3)
     W[5] = 0
     dW = dev(W, cuda)
