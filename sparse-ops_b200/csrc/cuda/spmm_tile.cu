@@ -502,10 +502,15 @@ double gather_us(const spx_ell* e, uint32_t C, uint32_t V, bool half)
     const double per_sm = std::ceil((double)e->m / RW) * panels / sms;
     const bool brief = e->nnz_total < 100ull * e->m;
     const double load = V == 4 ? 3.15e-3 : V == 2 ? 1.7e-3 : 1.34e-3, off_lines = V == 4 ? 0.47e-3 : V == 2 ? 0.5e-3 : 0.39e-3;
-    const double loads = e->nnz_total / sms * panels * (load * NV / RW + (C % 32 ? off_lines : 0.0)) + (brief ? 0.037 : 0.10) * per_sm;
+    double loads = e->nnz_total / sms * panels * (load * NV / RW + (C % 32 ? off_lines : 0.0)) + (brief ? 0.037 : 0.10) * per_sm;
+    if (V == 4 && RW > 1 && !brief) {           // long rows side by side in a warp: half as if each took a power of two of lanes
+        uint32_t lanes = 1;
+        while (lanes < q) lanes *= 2;
+        loads = e->nnz_total / sms * 2.0e-3 * (lanes / 32.0 + 1.0 / RW) + 0.10 * per_sm;
+    }
     double rounds = e->max_nnz;
     if (V == 1 && per_sm < 12) rounds *= 0.0115 * NV * (NV == 3 ? std::ceil(per_sm / 8.0) : 1.0);
-    else rounds *= (NV == 1 ? 0.0168 : 0.0282) * (NV == 1 && (per_sm < 48 || !brief) ? std::max(1.0, std::ceil(per_sm / 8.0)) : 1.0);
+    else rounds *= (NV == 1 ? 0.0168 * (V == 4 && RW > 1 && !brief ? 1.0 + 0.03 * RW : 1.0) : 0.0282) * (NV == 1 && (per_sm < 48 || !brief) ? std::max(1.0, std::ceil(per_sm / 8.0)) : 1.0);
     return (3.5 + std::sqrt(std::sqrt(std::pow(loads, 4) + std::pow(rounds, 4)))) * (half ? 0.9 : 1.0);
 }
 
