@@ -174,7 +174,7 @@ __device__ __forceinline__ void staged_row(const float* __restrict__ w, const ui
 
 __global__ void __launch_bounds__(kGatherWarps * 32, 4)
 spmm_gather_staged(const float* __restrict__ Wd, const uint32_t* __restrict__ idx,
-                   const uint32_t* __restrict__ nnz, const uint2* __restrict__ rows,
+                   const uint2* __restrict__ rows,
                    uint32_t m, uint32_t pitch,
                    const float* __restrict__ X, uint32_t C, uint32_t ldxb,
                    const float* __restrict__ bias, int act, PeerOut out, uint64_t ldy, StagedMap sm)
@@ -327,7 +327,7 @@ struct RowsArgs {
     uint32_t G, RW;
     BlockMap bm;
     bool early;                         // spmm_rows: let the successor in before the end
-    uint32_t n, Cp, batch, vec_out;     // spmm_chain: rows of X, their pitch in shared memory, entries per batch, 16-byte stores
+    uint32_t n, Cp, batch;              // staged X: its rows, their pitch in shared memory, entries per batch
     PeerOut out;
 };
 
@@ -551,12 +551,11 @@ spmm_rows(const __grid_constant__ RowsArgs a)
 }
 
 // ---------------------------------------------------------------------------------------
-// spmm_direct<V>: X fits in shared memory (few columns or few rows of X), any leading dimension.  Such
+// spmm_direct: X fits in shared memory, C is a multiple of 4 from 8 to 64 and the operands are aligned.  Such
 // products are bound by latency: a row's FMA chain is serial, and there are not enough rows to hide
-// a gather per entry.  So a CTA over R rows stages X whole (rows padded to Cp, a multiple of V, so
-// that a gather is one read of V columns), and splits its warps: the last two are producers that keep
+// a gather per entry.  So a CTA over R rows stages X whole, and splits its warps: the last two are producers that keep
 // the rows' slabs coming (cp.async, batches of E entries, kChainRing - 1 ahead), the others are
-// consumers: Cp / V lanes per row, which read (w, k) four entries at a time, gather one group of 8
+// consumers: C / 4 lanes per row, which read (w, k) four entries at a time, gather one group of 8
 // entries ahead of the group being multiplied and do nothing else.
 // ---------------------------------------------------------------------------------------
 constexpr int kChainRing = 4, kChainProducers = 64, kChainConsumers = 256;
@@ -596,13 +595,12 @@ __device__ __forceinline__ void lds_vec(float (&d)[V], uint32_t at) {
         asm("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(at));
 }
 
-template <int V>
 __global__ void __launch_bounds__(kChainConsumers + kChainProducers)
 spmm_direct(const __grid_constant__ RowsArgs a)
 {
     // named barriers: batch in ring slot s has landed (kFull + s), slot s is free again (kFree + s)
     constexpr int kFull = 1, kFree = 1 + kChainRing;
-    constexpr int U = 8;
+    constexpr int U = 8, V = 4;                 // entries per group, columns per lane
     extern __shared__ __align__(16) float s_mem[];
     const uint32_t R = a.RW, E = a.batch, stride = E + 4;           // E: 32, 64, 128 or 256 entries per row and batch
     const uint32_t Cp = a.Cp, L = Cp / V;
@@ -699,13 +697,7 @@ spmm_direct(const __grid_constant__ RowsArgs a)
 #pragma unroll
     for (int v = 0; v < V; ++v) acc[v] = spx::apply_act(acc[v], a.act);
     const size_t at = (size_t)(a.out.row0 + ri.x) * a.ldy + g * V;
-    if (V == 4 && a.vec_out) {
-        if constexpr (V == 4) store_out(a.out, at, make_float4(acc[0], acc[1], acc[2], acc[3]));
-        return;
-    }
-#pragma unroll
-    for (int v = 0; v < V; ++v)
-        if (g * V + v < a.C) store_out(a.out, at + v, acc[v]);
+    store_out(a.out, at, make_float4(acc[0], acc[1], acc[2], acc[3]));
 }
 
 // ---------------------------------------------------------------------------------------
@@ -945,29 +937,21 @@ static int launch_rows_one(const spx_ell* e, RowsArgs a, uint32_t panels, uint32
 
 static uint32_t chain_pitch(uint32_t C) { return C <= 2 ? C : round_up(C, 4u); }
 
-template <int V>
-static int launch_direct_one(const spx_ell* e, const RowsArgs& a, uint32_t threads, size_t smem, cudaStream_t s)
-{
-    if (int rc = allow_smem<spmm_direct<V>>(e->device)) return rc;
-    return finish_launch(launch_pdl(spmm_direct<V>, dim3((e->m + a.RW - 1) / a.RW), dim3(threads), smem, s, a), "spmm_direct");
-}
-
 // X staged whole.  R rows per CTA: one CTA per SM while kChainConsumers threads carry them; the batch
 // grows as R shrinks so that the barriers of a batch are spread over as many entries.
-static int launch_direct(const spx_ell* e, RowsArgs a, bool vec_out, cudaStream_t s)
+static int launch_direct(const spx_ell* e, RowsArgs a, cudaStream_t s)
 {
     const uint32_t sms = sm_count(e->device);
-    a.Cp = chain_pitch(a.C);
-    a.vec_out = vec_out;
-    const uint32_t V = a.Cp <= 2 ? a.Cp : 4, L = a.Cp / V;
+    a.Cp = a.C;
+    const uint32_t L = a.C / 4;
     a.RW = std::min<uint32_t>(kChainConsumers / L, std::max<uint32_t>(1u, (e->m + sms - 1) / sms));
     a.batch = a.RW > 32 ? 32 : a.RW > 16 ? 64 : a.RW > 8 ? 128 : 256;
     const auto bytes = [&] { return (size_t)a.RW * (a.batch + 4) * 2 * kChainRing * 4 + a.RW * sizeof(uint2) + (size_t)round_up(e->n * a.Cp, 4u) * 4; };
     while (a.RW > 1 && bytes() > 200 * 1024) a.RW = (a.RW + 1) / 2;
     const uint32_t threads = round_up(a.RW * L, 32u) + kChainProducers;
     const size_t smem = bytes();
-    return V == 1 ? launch_direct_one<1>(e, a, threads, smem, s) : V == 2 ? launch_direct_one<2>(e, a, threads, smem, s)
-                                                                     : launch_direct_one<4>(e, a, threads, smem, s);
+    if (int rc = allow_smem<spmm_direct>(e->device)) return rc;
+    return finish_launch(launch_pdl(spmm_direct, dim3((e->m + a.RW - 1) / a.RW), dim3(threads), smem, s, a), "spmm_direct");
 }
 
 template <int C>
@@ -1125,7 +1109,7 @@ int launch_spmm_bcast(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx
                               : C == 8 && len >= 80 && m <= 2048;
     if (staged && chain) return launch_chain(e, a, s);
     if (staged && vec_ok && C >= 8 && C <= 64 && len >= 80 && m <= (uint64_t)sm_count(e->device) * (kChainConsumers / (C / 4)))
-        return launch_direct(e, a, true, s);
+        return launch_direct(e, a, s);
     // what gathers X if X is not staged: vectors of V floats
     const uint32_t V = vec_ok ? 4 : C % 2 == 0 && ldx % 2 == 0 && (reinterpret_cast<uintptr_t>(X) & 7) == 0 ? 2 : 1;
     const bool half = vec_ok && takes_half(e, C);
@@ -1162,7 +1146,7 @@ int launch_spmm_bcast(const spx_ell* e, const float* X, uint32_t C, uint64_t ldx
             sm.head_panels = (C + 127) / 128;
             sm.head = all_narrow ? 0u : std::min<uint32_t>(sm.row_blocks, (e->long_rows + wpb - 1) / wpb);
             sm.blocks = sm.head * sm.head_panels + (sm.row_blocks - sm.head) * sm.panels;
-            spmm_gather_staged<<<sm.blocks, wpb * 32, (size_t)wpb * 512, s>>>(e->Wd, e->idx, e->nnz, e->rows, e->m, e->pitch,
+            spmm_gather_staged<<<sm.blocks, wpb * 32, (size_t)wpb * 512, s>>>(e->Wd, e->idx, e->rows, e->m, e->pitch,
                                                                           X, C, (uint32_t)(ldx * 4), bias, act, out, ldy, sm);
             SPX_LAUNCH_CHECK("spmm_gather_staged");
             return SPX_OK;

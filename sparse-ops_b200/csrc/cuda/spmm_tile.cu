@@ -32,7 +32,6 @@
 #include <cstring>
 #include <mutex>
 #include <optional>
-#include <vector>
 
 namespace {
 
@@ -395,7 +394,6 @@ static int build_tiles(spx_ell* e, spx_tiles_impl* t, cudaStream_t s)
     if (!e->tma_failed_dev || !e->tma_failed_mapped) return SPX_OK;
     void *pos = nullptr, *total = nullptr, *cnt = nullptr, *off = nullptr, *steps = nullptr;
     PinnedBlock stage;
-    std::vector<uint32_t> host(t->groups + 1);
     auto body = [&]() -> int {
         if (int rc = pool_alloc(&pos, cells * sizeof(uint4), e->device, s)) return rc;
         if (int rc = pool_alloc(&cnt, cells * 4, e->device, s)) return rc;

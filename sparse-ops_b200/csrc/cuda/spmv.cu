@@ -10,7 +10,7 @@
 // the stated tolerance 1e-5 * sum|w||x|, not bit for bit.  Padding slots are never multiplied.
 //
 // HBM-bound: 8 bytes per nonzero streamed once.  The kernels that stage x are launched as programmatic
-// dependents: // what belongs to the handle (schedule, first slab vectors) is asked for while the predecessor in the
+// dependents: what belongs to the handle (schedule, first slab vectors) is asked for while the predecessor in the
 // stream drains, and only x, bias and y wait for it.
 #include "common.cuh"
 
