@@ -333,3 +333,33 @@ def test_python_onnx_sparse_model(backend, cuda):
     y1, Y = model.run(x1), model.run(X)
     assert y1.shape == (10,) and Y.shape == (10, 8) and Y.dtype == np.float32
     assert np.abs(y1 - dense(x1)).max() <= 1e-5 and np.abs(Y - dense(X)).max() <= 1e-5
+
+
+def test_results_keep_their_memory(backend, orc):
+    """Results of 64 KB and more lie in page-locked blocks that are reused once a result is dropped, eight at a time at
+    most; what is kept is never written again, whichever memory it got, and outlives the objects it came from."""
+    rng = np.random.default_rng(17)
+    m, n, C = 300, 200, 64                                  # 77 KB
+    W = rng.standard_normal((m, n)).astype(np.float32)
+    W[rng.random(W.shape) >= 0.2] = 0
+    ell = backend.convert_to_ellpack(W)
+    E = orc.encode(W)
+    operands = [rng.uniform(-1, 1, (n, C)).astype(np.float32) for _ in range(14)]
+    wants = [orc.spmm(E, X, None) for X in operands]
+    kept = [backend.ellpack_matmul(ell, X, None) for X in operands]
+    for k, (got, want) in enumerate(zip(kept, wants)):
+        assert_bit_equal(got, want, f"result {k}")
+    view = kept[2][5:9]
+    del kept[4], kept[0]
+    for X, want in zip(operands, wants):                    # dropped at once: the same blocks over and over
+        assert_bit_equal(backend.ellpack_matmul(ell, X, None), want, "a later result")
+    del ell
+    import gc
+    gc.collect()
+    for got, want in zip(kept, wants[1:4] + wants[5:]):
+        assert_bit_equal(got, want, "kept result")
+    del kept, got
+    gc.collect()
+    again = backend.ellpack_matmul(backend.convert_to_ellpack(W), operands[7], None)
+    assert_bit_equal(view, wants[2][5:9], "view of a dropped result")
+    assert_bit_equal(again, wants[7], "after all were dropped")

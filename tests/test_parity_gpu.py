@@ -970,3 +970,37 @@ def test_device_decode_of_narrow_matrices(lib, orc, cuda, m, n):
     lib.spx_ell_decode_device(h.h, out.data_ptr(), 0)
     torch.cuda.synchronize()
     assert_bit_equal(out.cpu().numpy(), orc.decode(orc.encode(W)), "decode")
+
+
+@pytest.mark.parametrize("m,n,p", [
+    # x staged whole: several rows per group of lanes, rows of near-equal length (no schedule) and of very different ones
+    (40000, 4000, 0.02), (30011, 1500, 0.1), (20000, 300, 0.5),
+    # x in column windows (n > 51200): several rows per group in each, empty runs among them
+    (9000, 60000, 0.002), (20011, 53001, 0.0005)])
+@pytest.mark.parametrize("skew", [False, True], ids=["even", "skewed"])
+def test_spmv_several_rows_per_group(lib, cuda, m, n, p, skew):
+    """A group of lanes asks for its next row while it sums one; more rows than groups, so that it has a next one.
+    Against float64, within the tolerance of the summation order."""
+    rng = np.random.default_rng([m, n, skew])
+    mean = max(1, int(p * n))
+    lengths = rng.integers(0, 2 * mean, m) if skew else np.full(m, mean)
+    if skew:
+        lengths[[3, m - 1]] = [0, min(n, 6 * mean)]
+    rowptr = np.concatenate([[0], np.cumsum(lengths)]).astype(np.uint64)
+    row = np.repeat(np.arange(m), lengths)
+    step = n // np.maximum(lengths, 1)                       # ascending columns: one per stretch of n / length
+    k = np.arange(len(row)) - np.repeat(rowptr[:-1].astype(np.int64), lengths)
+    col = (k * step[row] + rng.integers(0, 1 << 30, len(row)) % step[row]).astype(np.uint32)
+    val = rng.standard_normal(len(row)).astype(np.float32)
+    x = rng.uniform(-1, 1, n).astype(np.float32)
+    b = rng.standard_normal(m).astype(np.float32)
+    h = lib.ell_create_csr(m, n, rowptr, col, val)
+    prod = val.astype(np.float64) * x[col]
+    want = b + np.bincount(row, prod, m)
+    bound = np.abs(b) + np.bincount(row, np.abs(prod), m)
+    dx, dB, dy = dev(x, cuda), dev(b, cuda), torch.full((m,), float("nan"), device=cuda)
+    for call in range(2):
+        dy.fill_(float("nan"))
+        h.spmv(ptr(dx), ptr(dB), ptr(dy))
+        torch.cuda.synchronize()
+        assert (np.abs(dy.cpu().numpy() - want) <= SPMV_TOL * bound).all(), f"call {call}"
