@@ -517,7 +517,7 @@ spmm_rows(const __grid_constant__ RowsArgs a)
             const uint32_t cmin = nmin > bt * kBatch ? min((uint32_t)kBatch, nmin - bt * kBatch) : 0u;
             constexpr int T = U >= 16 ? 8 : 4;
             // groups that every row of the warp fills, then smaller ones.  Groups of 4 take the predicated path alone:
-            // a second copy of the loop does not fit 64 registers (262144 power-law rows, C = 1024: 4.21 -> 3.91 ms).
+            // a second copy of the loop does not fit 64 registers (262144 power-law rows, C = 1024: 4.39 -> 4.20 ms).
             uint32_t t = 0;
             if constexpr (U > T) {
                 for (; t + U <= cmin; t += U) {
