@@ -620,6 +620,9 @@ def measure(args, c):
             def step():
                 i = rot[0] = (rot[0] + 1) % ncopies
                 ells[i].spmm(dXs[i].data_ptr(), C, C, 0 if dB is None else dB.data_ptr(), sx.ACT_NONE, dYs[i].data_ptr(), C, stream)
+            if ncopies > 1:             # each copy is a matrix in use: its second product has built what later ones read
+                for _ in range(2 * ncopies):
+                    step()
             hX = torch.from_numpy(wk["X"]).pin_memory()
             hY = torch.empty((wk["rows"], C), dtype=torch.float32).pin_memory()
             hB = None if wk["bias"] is None else torch.from_numpy(wk["bias"]).pin_memory()
