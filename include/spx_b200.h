@@ -201,8 +201,9 @@ int spx_global_avgpool(const float* in, uint32_t C, uint32_t H, uint32_t W, uint
 
 /* ---- the same calls on HOST buffers (what the reference's Python binding does) ---------- */
 /* X, bias, Y are host arrays; copies in and out go through pinned staging of the library
- * (up to 24 KB with the call, 24 to 64 KB as they are, larger pageable inputs in pieces by helper threads).  Replaces the ellpack_matmul / ellpack_matvec lambdas of
- * src/bindings.cpp:91-139.  Synchronous. */
+ * (up to 24 KB with the call, 24 to 64 KB as they are, larger pageable inputs in pieces by helper threads).
+ * Page-locked operands are read and written in place, after what is queued on the default stream.  Replaces the
+ * ellpack_matmul / ellpack_matvec lambdas of src/bindings.cpp:91-139.  Synchronous. */
 int spx_spmm_host(const spx_ell* e, const float* X, uint32_t C, const float* bias, int act, float* Y);
 int spx_spmv_host(const spx_ell* e, const float* x, const float* bias, float* y);
 

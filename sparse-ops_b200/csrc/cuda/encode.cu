@@ -277,7 +277,7 @@ namespace spx {
 // Everything but the two kernels is kept off the critical path: counts come back through pinned
 // memory in one copy (the only point the host must wait for, r fixes the pitch), the row schedule is
 // sorted on the host while the packer runs, and the arrays come from the library's pool.
-static int encode_rows(const float* dW, uint32_t m, uint32_t n, cudaStream_t s, const PinnedBlock& stage, const Split& sp,
+static int encode_rows(const float* dW, uint32_t m, uint32_t n, int device, cudaStream_t s, const PinnedBlock& stage, const Split& sp,
                        uint32_t* d_counts, spx_ell** out)
 {
     const uint32_t mis = misalignment(dW);
@@ -286,21 +286,35 @@ static int encode_rows(const float* dW, uint32_t m, uint32_t n, cudaStream_t s, 
     count_kernel<<<sp.blocks, kWarps * 32, 0, s>>>(dW, mis, m, n, sp.segs, sp.seg, d_counts);
     SPX_LAUNCH_CHECK("count_kernel");
     SPX_CUDA(cudaMemcpyAsync(h_counts, d_counts, units * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    SPX_CUDA(cudaStreamSynchronize(s));
+    // The schedule travels on a stream of its own, beside the packer: its block is allocated in that stream's order too
+    // (the pool may hand out memory that work queued on another stream still uses, ordered behind it on the allocating
+    // stream only), and here, where the host would wait anyway and no packer is queued to wait for.
+    void* schedule = nullptr;
+    cudaStream_t side = nullptr;
+    const size_t schedule_bytes = (size_t)m * sizeof(uint2);
+    if (int rc = side_stream(device, &side)) return rc;
+    if (int rc = pool_alloc(&schedule, schedule_bytes, device, side)) return rc;
+    const cudaError_t counted = cudaStreamSynchronize(s);
     uint32_t r = 0;
     uint64_t total = 0;
-    if (sp.segs > 1)
+    if (sp.segs > 1 && counted == cudaSuccess)
         for (uint32_t i = 0; i < m; ++i) {
             uint32_t c = h_counts[(size_t)i * sp.segs];
             for (uint32_t k = 1; k < sp.segs; ++k) c += h_counts[(size_t)i * sp.segs + k];
             h_counts[i] = c;                                        // in place: i <= i * segs
         }
-    for (uint32_t i = 0; i < m; ++i) {
+    for (uint32_t i = 0; i < m && counted == cudaSuccess; ++i) {
         r = std::max(r, h_counts[i]);
         total += h_counts[i];
     }
-    if (int rc = alloc_ell(m, n, r, out, s, r == 0)) return rc;
+    const int rc_ell = counted == cudaSuccess ? alloc_ell(m, n, r, out, s, r == 0)
+                                              : fail(SPX_ERR_CUDA, "encode: count pass failed: %s", cudaGetErrorString(counted));
+    if (rc_ell != SPX_OK) {
+        pool_free(schedule, schedule_bytes, side);
+        return rc_ell;
+    }
     spx_ell* e = *out;
+    e->rows = static_cast<uint2*>(schedule);
     e->nnz_total = total;
     e->max_nnz = r;
     if (r) {
@@ -308,12 +322,8 @@ static int encode_rows(const float* dW, uint32_t m, uint32_t n, cudaStream_t s, 
         SPX_LAUNCH_CHECK("pack_kernel");
     }
     uint2* h_order = reinterpret_cast<uint2*>(h_counts + round_up<size_t>(units, 2));
-    // on a stream of its own, beside the packer: the block is allocated in that stream's order too (the pool may hand
-    // out memory that work queued on another stream still uses, ordered behind it on the allocating stream only)
-    cudaStream_t side = nullptr;
-    if (int rc = side_stream(e->device, &side)) return rc;
     if (int rc = sort_rows(e, h_counts, h_order, side)) return rc;
-    SPX_CUDA(cudaMemcpyAsync(e->rows, h_order, (size_t)m * sizeof(uint2), cudaMemcpyHostToDevice, side));
+    SPX_CUDA(cudaMemcpyAsync(e->rows, h_order, schedule_bytes, cudaMemcpyHostToDevice, side));
     SPX_CUDA(cudaStreamSynchronize(side));
     SPX_CUDA(cudaStreamSynchronize(s));         // the handle may be used on any stream from here on
     return SPX_OK;
@@ -335,7 +345,7 @@ int encode_device(const float* dW, uint32_t m, uint32_t n, cudaStream_t s, spx_e
     if (int rc = pinned_acquire((units + 1) * sizeof(uint32_t) + m * sizeof(uint2), &stage)) return rc;
     void* d_counts = nullptr;
     int rc = pool_alloc(&d_counts, units * sizeof(uint32_t), device, s);
-    if (rc == SPX_OK) rc = encode_rows(dW, m, n, s, stage, sp, static_cast<uint32_t*>(d_counts), out);
+    if (rc == SPX_OK) rc = encode_rows(dW, m, n, device, s, stage, sp, static_cast<uint32_t*>(d_counts), out);
     if (rc != SPX_OK) {
         (void)cudaStreamSynchronize(s);         // nothing may still write the staging block
         if (*out) spx_ell_destroy(*out);
