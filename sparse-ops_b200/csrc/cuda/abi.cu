@@ -3,6 +3,7 @@
 // argument validation in front of every kernel launcher, and the host-buffer entry points
 // that copy operands through pinned staging.
 #include "common.cuh"
+#include "conv.cuh"
 #include "tma.cuh"
 
 #include <dlfcn.h>
@@ -54,6 +55,7 @@ int alloc_ell(uint32_t m, uint32_t n, uint32_t r, spx_ell** out, cudaStream_t s,
     }
     e->m = m; e->n = n; e->r = r;
     e->tiles = new_tiles();
+    e->conv_tmem = new_conv_tmem();
     e->pitch = r ? round_up<uint32_t>(r, 32u) : 0u;
     const size_t slots = (size_t)m * e->pitch;
     int rc = SPX_OK;
@@ -70,6 +72,7 @@ int alloc_ell(uint32_t m, uint32_t n, uint32_t r, spx_ell** out, cudaStream_t s,
     if (rc != SPX_OK || err != cudaSuccess) {
         pool_free(e->Wd, slots * sizeof(float), s); pool_free(e->idx, slots * sizeof(uint32_t), s); pool_free(e->nnz, (size_t)m * sizeof(uint32_t), s);
         free_tiles(e);
+        free_conv_tmem(e);
         delete e;
         return rc != SPX_OK ? rc : fail(SPX_ERR_CUDA, "ELLPACK zero fill (%zu slots) failed: %s", slots, cudaGetErrorString(err));
     }
@@ -403,6 +406,7 @@ int spx_ell_destroy(spx_ell* e)
     // its arrays go back to the pool without another one.
     wait_for_device();
     free_tiles(e);
+    free_conv_tmem(e);
     pool_free(e->Wd, (size_t)e->m * e->pitch * 4, nullptr);
     pool_free(e->idx, (size_t)e->m * e->pitch * 4, nullptr);
     pool_free(e->nnz, (size_t)e->m * 4, nullptr);

@@ -62,6 +62,8 @@ struct spx_ell {
     bool tma_off = false;
     // Tiled form of the matrix for spmm_tile.cu, built on the second SpMM call that can use it.
     void* tiles = nullptr;
+    // The convolution's entries for conv_tmem.cu, built on the first call that uses them.
+    void* conv_tmem = nullptr;
     // SpMV with x larger than shared memory (spmv.cu): column window width and the per-row split
     // table, built on the first spx_spmv of such a handle.  spmv_win == UINT32_MAX: not applicable.
     uint32_t* spmv_split = nullptr;

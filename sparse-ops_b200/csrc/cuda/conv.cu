@@ -13,6 +13,7 @@
 // reference for stride 1 (the reference mis-indexes stride_w > 1, :305-306 and :438-439; this
 // kernel implements the mathematically correct stride).
 #include "common.cuh"
+#include "conv.cuh"
 #include "tma.cuh"
 
 #include <algorithm>
@@ -24,6 +25,8 @@
 
 namespace {
 
+using spx::ConvParams;
+using spx::ConvViews;
 using spx::mbar_init;
 using spx::mbar_expect_tx;
 using spx::mbar_wait;
@@ -45,10 +48,6 @@ __global__ void build_taps_kernel(const uint32_t* __restrict__ idx, const uint32
         taps[(size_t)row * pitch + j] = (cin << 16) | (kh << 8) | kw;
     }
 }
-
-struct ConvParams {
-    uint32_t Cin, Cout, kH, kW, sH, sW, pH, pW, dH, dW, H, W, Ho, Wo, B;
-};
 
 // General kernel: one thread per output element, any layout, any geometry.  Threads of a warp
 // are adjacent along the fastest output dimension (batch for PF, width for NCHW), so input
@@ -190,15 +189,6 @@ to_pf_kernel(const float* __restrict__ src, uint64_t sB, uint64_t sC, uint64_t s
 #define SPX_CONV_FMA2 1         // packed fma.rn.f32x2 in the tiled kernels (same rounding per element)
 #endif
 constexpr int kTileH = 4, kTileW = 8, kTileWarps = 16;
-
-// Strides in floats.  Input: the batch is contiguous, the other strides are multiples of 4.  Output: any
-// layout; vec_out when the batch is contiguous there too and every position starts on 16 bytes.
-struct ConvViews {
-    uint64_t iC, iH, iW;
-    uint64_t oB, oC, oH, oW;
-    uint32_t b_out;     // batch entries that exist in the output (the input may be widened by up to 3)
-    uint32_t vec_out;
-};
 
 struct TileParams {
     ConvParams c;
@@ -777,7 +767,7 @@ static bool rbm_fits(const ConvParams& p, uint32_t qb, int nb, int g)
 }
 
 // Builds (once per handle and kernel shape) the row-block-merged weights.
-static int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s)
+int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s)
 {
     if (e->rbm_hdr && e->rbm_kH == kH && e->rbm_kW == kW) return SPX_OK;
     const uint32_t nblocks = (e->m + kRbmRows - 1) / kRbmRows;
@@ -869,18 +859,18 @@ static int launch_rbm_units(const spx_ell* e, TileParams tp, RbmUnits un, uint32
 // for 14 of them.  256 -> 256 channels, 14 x 14, batch 4, 10 %: 150 us as 16 x 4, 35 us as 4 x 1.
 struct RbmCut {
     int nb, g;
+    double cycles;
 };
 static RbmCut rbm_cut(const spx_ell* e, const ConvParams& p, uint32_t qb, uint32_t b_len)
 {
     struct Option { RbmCut cut; double latency, per_warp; };
-    static const Option options[] = {{{16, 4}, 250, 22}, {{8, 4}, 250, 22}, {{8, 2}, 90, 11.4}, {{4, 2}, 90, 11.4}, {{4, 1}, 70, 7.4}};
+    static const Option options[] = {{{16, 4, 0}, 250, 22}, {{8, 4, 0}, 250, 22}, {{8, 2, 0}, 90, 11.4}, {{4, 2, 0}, 90, 11.4}, {{4, 1, 0}, 70, 7.4}};
     const double sms = sm_count(e->device), d = (double)e->nnz_total / ((double)e->m * e->n);
     const double un = 1.0 - std::pow(1.0 - std::min(d, 1.0), (double)kRbmRows);
     const double share = kRbmRows * d / un, cols = un * e->n;
     const uint32_t nblocks = (p.Cout + kRbmRows - 1) / kRbmRows;
     const double conflicts = p.sW % 2 ? 1.0 : 2.0;
-    RbmCut best{0, 0};
-    double best_t = 1e300;
+    RbmCut best{0, 0, 1e300};
     for (const Option& o : options) {
         const int nb = o.cut.nb, g = o.cut.g;
         if (!rbm_fits(p, qb, nb, g)) continue;
@@ -898,9 +888,20 @@ static RbmCut rbm_cut(const spx_ell* e, const ConvParams& p, uint32_t qb, uint32
         const double latency = qb == 2 && g < kRbmG ? (g == 2 ? 205.0 : 115.0) : o.latency;
         const double col = std::max(latency, warps * std::max(4.6 * g * conflicts + 2, o.per_warp * (0.6 + 0.3 * share)));
         const double t = waves * (std::max(cols * col, resident * p.Cin * patch / 64) + 2500 + 500 * chunks);
-        if (t < best_t) { best_t = t; best = o.cut; }
+        if (t < best.cycles) best = RbmCut{nb, g, t};
     }
     return best;
+}
+
+// Expected time of all segments of a batch.  The factors bring the cuts' estimates to measured times of 267 shapes.
+static double conv_rbm_us(const spx_ell* e, const ConvParams& p)
+{
+    const uint32_t n16 = p.B / 16 * 16, rest = p.B - n16;
+    double us = 0.0;
+    if (n16) us += 1.118 * rbm_cut(e, p, 4, n16).cycles / 1900.0 + 2.46;
+    if (rest >= 8) us += 0.879 * rbm_cut(e, p, 2, 8).cycles / 1900.0 + 2.46;
+    if (rest % 8 == 4) us += rbm_cut(e, p, 1, 4).cycles / 1900.0 + 2.46;
+    return us;
 }
 
 template <int QB>
@@ -916,7 +917,7 @@ static int launch_rbm_qb(spx_ell* e, TileParams tp, const float* in, const float
     const ConvParams& p = tp.c;
     static const int cut_env = [] { const char* v = getenv("SPX_CONV_CUT"); return v ? atoi(v) : 0; }();      // 10 NB + G, for tests
     RbmCut cut = rbm_cut(e, p, QB, b_len);
-    if (cut_env && rbm_fits(p, QB, cut_env / 10, cut_env % 10) && 32u * (cut_env % 10) / QB / kTileW) cut = RbmCut{cut_env / 10, cut_env % 10};
+    if (cut_env && rbm_fits(p, QB, cut_env / 10, cut_env % 10) && 32u * (cut_env % 10) / QB / kTileW) cut = RbmCut{cut_env / 10, cut_env % 10, 0.0};
     if (!cut.nb) return -1;
     const uint32_t TH = 32u * cut.g / QB / kTileW;
     tp.tilesX = (p.Wo + kTileW - 1) / kTileW;
@@ -985,6 +986,10 @@ static int launch_conv_rbm_tile(spx_ell* e, const ConvParams& p, const ConvViews
     // every segment's staged patch must fit shared memory (checked before any launch)
     const auto fits = [&](uint32_t qb) { return rbm_fits(p, qb, 16, kRbmG); };
     if ((n16 && !fits(4)) || (rest >= 8 && !fits(2)) || (rest % 8 == 4 && !fits(1))) return -1;
+    {
+        const int rc = launch_conv_tmem(e, p, v, in, bias, act, out, conv_rbm_us(e, p), s);
+        if (rc != -1) return rc;
+    }
     TileParams tp{};
     tp.c = p;
     tp.v = v;

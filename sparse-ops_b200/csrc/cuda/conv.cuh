@@ -1,0 +1,29 @@
+// conv.cuh -- what the convolution kernels' files share.
+#pragma once
+
+#include "common.cuh"
+
+namespace spx {
+
+struct ConvParams {
+    uint32_t Cin, Cout, kH, kW, sH, sW, pH, pW, dH, dW, H, W, Ho, Wo, B;
+};
+
+// Strides in floats.  Input: the batch is contiguous, the other strides are multiples of 4.  Output: any
+// layout; vec_out when the batch is contiguous there too and every position starts on 16 bytes.
+struct ConvViews {
+    uint64_t iC, iH, iW;
+    uint64_t oB, oC, oH, oW;
+    uint32_t b_out;     // batch entries that exist in the output (the input may be widened by up to 3)
+    uint32_t vec_out;
+};
+
+// conv_tmem.cu: -1 when the shape or the handle is not for this kernel, or the other one's expected time is not above its own.
+int launch_conv_tmem(spx_ell* e, const ConvParams& p, const ConvViews& v, const float* in, const float* bias, int act, float* out,
+                     double other_us, cudaStream_t s);
+// conv.cu: the merged weights of conv_rbm_tile_kernel; -1 where there is no memory for them.
+int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s);
+void* new_conv_tmem();
+void free_conv_tmem(spx_ell* e);
+
+}  // namespace spx

@@ -29,6 +29,9 @@ __device__ __forceinline__ void tma_load_2d(void* smem, const CUtensorMap* map, 
                  ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(map), "r"(c0), "r"(c1),
                    "r"((uint32_t)__cvta_generic_to_shared(bar)) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"((uint32_t)__cvta_generic_to_shared(bar)) : "memory");
+}
 // Arrives, and returns how many arrivals of the phase were pending before this one.
 __device__ __forceinline__ uint32_t mbar_arrive_pending(uint64_t* bar) {
     uint32_t pending;

@@ -1,0 +1,119 @@
+"""GPU: the convolution with its patch in tensor memory (conv_tmem.cu), forced, against the oracle bit for bit: edges of
+tiles, chunks and batch segments, few and many output channels, full and empty rows, infinities under taps that a row
+does not store.  The switch is read once per process, so the cases run in a child."""
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+import torch
+
+import spx_ctypes as sx
+from conftest import assert_bit_equal
+from test_parity_gpu import as_layout, dev, gpu_ell, ptr, sparse
+
+pytestmark = pytest.mark.gpu
+HERE = os.path.dirname(os.path.abspath(__file__))
+forced = pytest.mark.skipif(os.environ.get("SPX_CONV_TMEM") != "2", reason="runs in a child process")
+
+# B, Cin, Cout, H, W, (kH, kW), (sH, dH, dW), density
+CASES = [(32, 6, 64, 6, 8, (3, 3), (1, 1, 1), 0.3),         # one chunk, one unit
+         (32, 7, 65, 7, 9, (3, 3), (1, 1, 1), 0.3),         # a chunk of one channel; a block and a position over
+         (32, 13, 33, 5, 17, (3, 3), (1, 1, 1), 1.0),       # dense: the most entries a chunk can hold
+         (48, 19, 29, 4, 7, (3, 3), (1, 1, 1), 0.2),        # segments of 32 and 16, two patches per CTA
+         (60, 5, 40, 9, 9, (3, 3), (1, 1, 1), 0.2),         # all segment widths
+         (4, 30, 132, 3, 40, (3, 3), (1, 1, 1), 0.1),       # eight lane groups
+         (16, 9, 70, 11, 8, (5, 5), (1, 1, 1), 0.15),
+         (8, 8, 36, 12, 12, (7, 7), (1, 1, 1), 0.1),
+         (12, 10, 32, 14, 10, (3, 3), (1, 2, 2), 0.3),      # dilated
+         (32, 8, 31, 9, 8, (3, 2), (2, 1, 3), 0.3),         # stride along the rows only
+         (32, 600, 29, 2, 3, (3, 3), (1, 1, 1), 0.02),      # many chunks, most rows' runs empty
+         (64, 12, 256, 56, 56, (3, 3), (1, 1, 1), 0.05)]    # several waves and a tail of half units
+
+
+@forced
+@pytest.mark.parametrize("layout", [sx.LAYOUT_PF, sx.LAYOUT_NCHW, sx.LAYOUT_FMAJOR])
+@pytest.mark.parametrize("B,Cin,Cout,H,W,k,sd,density", CASES)
+def test_forced_cases(lib, orc, cuda, layout, B, Cin, Cout, H, W, k, sd, density):
+    (kH, kW), (sH, dH, dW) = k, sd
+    if layout != sx.LAYOUT_PF and H > 50:
+        pytest.skip("once is enough at this size")
+    rng = np.random.default_rng([B, Cin, Cout, H, W, kH])
+    wt = sparse(rng, Cout, Cin * kH * kW, density) * np.float32(0.3)
+    wt[Cout // 2] = 0                                       # an empty row
+    wt[:, 4 % wt.shape[1]] = 0                              # nobody stores this tap ...
+    x = rng.standard_normal((B, Cin, H, W)).astype(np.float32)
+    if kH * kW > 4 and H <= 20:
+        x[0, 0, 0, 0], x[-1, -1, -1, -1] = np.inf, np.nan   # ... and what others meet comes out as it is
+    bias = rng.standard_normal(Cout).astype(np.float32)
+    src = as_layout(x, layout)
+    E = orc.encode(wt)
+    pH, pW = (kH // 2) * dH, (kW // 2) * dW
+    gd = dict(Cin=Cin, kH=kH, kW=kW, sH=sH, sW=1, pH=pH, pW=pW, dH=dH, dW=dW, H=H, W=W)
+    want = orc.conv2d(E, gd, layout, src, B, bias, 0)
+    h = gpu_ell(lib, E)
+    g = sx.conv_geom(Cin, Cout, kH, kW, H, W, sH, 1, pH, pW, dH, dW)
+    dX, dB = dev(src, cuda), dev(bias, cuda)
+    out = torch.full((want.size + 8,), 7.0, device=cuda, dtype=torch.float32)
+    for _ in range(2):
+        h.conv2d(g, layout, ptr(dX), B, ptr(dB), sx.ACT_NONE, out.data_ptr() + 16)
+    torch.cuda.synchronize()
+    got = out.cpu().numpy()
+    nan = np.isnan(want.reshape(-1))
+    assert (np.isnan(got[4:-4]) == nan).all()
+    assert_bit_equal(np.where(nan, 0, got[4:-4]).astype(np.float32), np.where(nan, 0, want.reshape(-1)).astype(np.float32), "conv")
+    assert (got[:4] == 7.0).all() and (got[-4:] == 7.0).all()
+
+
+@forced
+def test_forced_more_shapes_than_forms_and_capture(lib, orc, cuda):
+    """One handle under six kernel shapes, the first call of each but one on a stream that records a graph: results are
+    the same whether a form could be built or not, also when graphs are replayed after others were built."""
+    rng = np.random.default_rng(3)
+    Cin, Cout, B, H, W = 8, 32, 32, 12, 12
+    wt = sparse(rng, Cout, Cin * 9, 0.3)
+    E = orc.encode(wt)
+    h = gpu_ell(lib, E)
+    x = rng.standard_normal((B, Cin, H, W)).astype(np.float32)
+    src = as_layout(x, sx.LAYOUT_PF)
+    dX = dev(src, cuda)
+    runs = []
+    for dil in range(1, 7):
+        gd = dict(Cin=Cin, kH=3, kW=3, sH=1, sW=1, pH=0, pW=0, dH=1, dW=1, H=H, W=W)
+        gd.update(dH=dil if dil < 6 else 1, dW=1, sH=1 if dil < 6 else 2)
+        want = orc.conv2d(E, gd, sx.LAYOUT_PF, src, B, None, 0)
+        g = sx.conv_geom(Cin, Cout, 3, 3, H, W, gd["sH"], 1, 0, 0, gd["dH"], 1)
+        dY = torch.empty(want.shape, device=cuda)
+        if dil == 1:
+            h.conv2d(g, sx.LAYOUT_PF, ptr(dX), B, None, 0, ptr(dY))      # allocates what any kernel needs
+            torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            h.conv2d(g, sx.LAYOUT_PF, ptr(dX), B, None, 0, ptr(dY), torch.cuda.current_stream().cuda_stream)
+        dZ = torch.empty(want.shape, device=cuda)
+        h.conv2d(g, sx.LAYOUT_PF, ptr(dX), B, None, 0, ptr(dZ))
+        torch.cuda.synchronize()
+        assert_bit_equal(dZ.cpu().numpy(), want, f"eager {dil}")
+        runs.append((graph, dY, want))
+    for graph, dY, want in runs:
+        dY.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert_bit_equal(dY.cpu().numpy(), want, "replayed")
+
+
+def child(files, select, env):
+    cmd = [sys.executable, "-m", "pytest", "-q", "-x", "-m", "gpu", "-p", "no:cacheprovider", *[os.path.join(HERE, f) for f in files], "-k", select]
+    r = subprocess.run(cmd, env={**os.environ, **env}, capture_output=True, text=True, timeout=900)
+    assert r.returncode == 0 and " passed" in r.stdout, r.stdout[-3000:] + r.stderr[-2000:]
+
+
+def test_forced_kernel():
+    child(["test_conv_tmem_gpu.py", "test_parity_gpu.py", "test_fuzz_gpu.py"],
+          "forced_cases or forced_more or conv_bit_exact or conv_views or conv_random or golden_conv", {"SPX_CONV_TMEM": "2"})
+
+
+def test_timeout_is_reported():
+    """The waits for its bulk copies are bounded: they are made to run out, the next call says so, the one after works."""
+    child(["test_parity_gpu.py"], "bulk_copy_timeout_child", {"SPX_CONV_TMEM": "2", "SPX_CONV_TMA_TEST_TIMEOUT": "1"})
