@@ -7,12 +7,11 @@
 // decode_device replaces decode_from_ellpack (:46-60).  csr_to_ell_device fills the padded slabs
 // from CSR arrays for matrices that never exist densely.
 //
-// All three passes are bound by HBM: 4*m*n bytes read by each encoder pass, 4*m*n written by the
-// decoder, so the kernels move 16-byte vectors with several in flight per lane and touch every byte
-// once.  The packer walks the rows backwards: what the counter read last is then still in L2.
-// Measured at 8192 x 8192, 10 % kept: count 54 us (5.0 TB/s), pack 67 us (4.8 TB/s), decode 54 us
-// (6.0 TB/s; 79 us when a warp fetched 32 entries at a time); encode + decode + destroy through the
-// C ABI 2.4 ms and more before the handle's memory came from a pool, 0.24 ms now.
+// The passes are bound by HBM: 4*m*n bytes read by the counter, 4*m*n written by the decoder, so the kernels move
+// 16-byte vectors with several in flight per lane.  A large matrix is read once: the counter keeps the entries it finds,
+// the packer fetches them from L2; a small one is read again, backwards: what the counter read last is then still in L2.
+// Measured at 8192 x 8192, 10 % kept: count and keep 58 us, pack 29, decode 56 (6.0 TB/s); encode + decode + destroy
+// through the C ABI 185 us (244 with two reads and a schedule sorted on the host).
 #include "common.cuh"
 
 #include <algorithm>
@@ -67,12 +66,13 @@ __device__ __forceinline__ float4 load_quad(const float* __restrict__ W, const S
 }
 
 // Quads qb + lane + 32 u of the segment for u = 0 .. kQuads-1; whole blocks inside it without checks.
+template <bool STREAM>              // read once: first to leave the caches
 __device__ __forceinline__ void load_block(float4 (&v)[kQuads], const float* __restrict__ W, const Segment& s, uint32_t qb, int lane)
 {
     if (qb > 0 && qb + 32 * kQuads < s.quads) {
         const float4* __restrict__ p = reinterpret_cast<const float4*>(W + s.at) + qb + lane;
 #pragma unroll
-        for (int u = 0; u < kQuads; ++u) v[u] = __ldg(p + 32 * u);
+        for (int u = 0; u < kQuads; ++u) v[u] = STREAM ? __ldcs(p + 32 * u) : __ldg(p + 32 * u);
         return;
     }
 #pragma unroll
@@ -93,7 +93,7 @@ count_kernel(const float* __restrict__ W, uint32_t mis, uint32_t m, uint32_t n, 
     uint32_t cnt = 0;
     for (uint32_t qb = 0; qb < s.quads; qb += 32 * kQuads) {
         float4 v[kQuads];
-        load_block(v, W, s, qb, lane);
+        load_block<false>(v, W, s, qb, lane);
 #pragma unroll
         for (int u = 0; u < kQuads; ++u)
             cnt += (v[u].x != 0.0f) + (v[u].y != 0.0f) + (v[u].z != 0.0f) + (v[u].w != 0.0f);
@@ -102,15 +102,150 @@ count_kernel(const float* __restrict__ W, uint32_t mis, uint32_t m, uint32_t n, 
     if (lane == 0) counts[unit] = cnt;
 }
 
-// Unit u of the grid is the matrix's unit (last - u): the counter has just read the end of W.
+// The counter that also keeps what it finds: per unit up to `cap` entries as (value, column) pairs in scratch, so that
+// the matrix is read once.  A block of 512 elements is compacted in the warp's strip of shared memory (one scan of four
+// byte-sized counts per lane gives all places) and leaves it in whole 8-byte rows of 32 lanes.  W is read with an
+// evict-first hint, so that the pairs are still in L2 when pack_kernel fetches them.
+// 8192 x 8192, 10 %: 58 us (count_kernel 53), and pack_kernel 29 instead of 67.
+__global__ void __launch_bounds__(kWarps * 32)
+count_keep_kernel(const float* __restrict__ W, uint32_t mis, uint32_t m, uint32_t n, uint32_t segs, uint32_t seg, uint32_t cap,
+                  uint32_t* __restrict__ counts, uint2* __restrict__ kept)
+{
+    __shared__ __align__(16) uint2 strips[kWarps][128 * kQuads];
+    const int lane = threadIdx.x & 31;
+    uint2* strip = strips[threadIdx.x >> 5];
+    const uint64_t unit = (uint64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
+    if (unit >= (uint64_t)m * segs) return;
+    const Segment s = segment_of(unit, mis, n, segs, seg);
+    uint2* __restrict__ dst = kept + unit * cap;
+    uint32_t pos = 0;
+    for (uint32_t qb = 0; qb < s.quads; qb += 32 * kQuads) {
+        float4 v[kQuads];
+        load_block<true>(v, W, s, qb, lane);
+        uint32_t own = 0;                                   // byte u: entries of this lane's quad u
+#pragma unroll
+        for (int u = 0; u < kQuads; ++u)
+            own |= ((v[u].x != 0.0f) + (v[u].y != 0.0f) + (v[u].z != 0.0f) + (v[u].w != 0.0f)) << (8 * u);
+        uint32_t upto = own;                                // at most 128 in a byte
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t b = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += b;
+        }
+        const uint32_t all = __shfl_sync(0xffffffffu, upto, 31), before = upto - own;
+        uint32_t base = 0;
+#pragma unroll
+        for (int u = 0; u < kQuads; ++u) {
+            uint32_t at = base + ((before >> (8 * u)) & 255u);
+            const uint32_t col = s.c_lo + 4 * (qb + 32 * u + lane) - (uint32_t)s.lead;
+            if (v[u].x != 0.0f) strip[at++] = make_uint2(__float_as_uint(v[u].x), col);
+            if (v[u].y != 0.0f) strip[at++] = make_uint2(__float_as_uint(v[u].y), col + 1);
+            if (v[u].z != 0.0f) strip[at++] = make_uint2(__float_as_uint(v[u].z), col + 2);
+            if (v[u].w != 0.0f) strip[at] = make_uint2(__float_as_uint(v[u].w), col + 3);
+            base += (all >> (8 * u)) & 255u;
+        }
+        __syncwarp();
+        if (pos + base <= cap)                              // else the unit will be read again
+            for (uint32_t j = lane; j < base; j += 32) dst[pos + j] = strip[j];
+        pos += base;
+        __syncwarp();
+    }
+    if (lane == 0) counts[unit] = pos;
+}
+
+// What the host has to know before the arrays can be allocated, where the device makes the row schedule (up to kRankRows
+// rows of less than kRankColumns): one CTA adds up the rows' segments and leaves the result in page-locked memory, where
+// the host finds it after one wait (instead of a copy of all counts and three loops over them).
+constexpr uint32_t kRankRows = 16384, kRankColumns = 1u << 18;
+struct RowStats {
+    uint64_t total;
+    uint32_t longest, shortest, long_rows, pad;
+};
+
+__global__ void __launch_bounds__(1024)
+row_stats_kernel(const uint32_t* __restrict__ counts, uint32_t m, uint32_t segs, uint32_t* __restrict__ keys, RowStats* __restrict__ out)
+{
+    __shared__ uint32_t s_hi[32], s_lo[32], s_long[32];
+    __shared__ unsigned long long s_sum[32];
+    uint32_t hi = 0, lo = 0xffffffffu, n_long = 0;
+    unsigned long long sum = 0;
+    constexpr uint32_t U = 8;                               // rows of a thread in flight
+    for (uint32_t i0 = threadIdx.x; i0 < m; i0 += 1024 * U) {
+        uint32_t len[U] = {};
+        for (uint32_t k = 0; k < segs; ++k)
+#pragma unroll
+            for (uint32_t u = 0; u < U; ++u)
+                if (i0 + 1024 * u < m) len[u] += __ldg(counts + (size_t)(i0 + 1024 * u) * segs + k);
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u) {
+            const uint32_t i = i0 + 1024 * u;
+            if (i >= m) break;
+            keys[i] = len[u] * kRankRows + (kRankRows - 1 - i);
+            hi = max(hi, len[u]);
+            lo = min(lo, len[u]);
+            n_long += len[u] >= 512u;
+            sum += len[u];
+        }
+    }
+    auto reduce = [&] {
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        n_long = __reduce_add_sync(0xffffffffu, n_long);
+#pragma unroll
+        for (int o = 16; o; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+    };
+    reduce();
+    const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (lane == 0) { s_hi[w] = hi; s_lo[w] = lo; s_long[w] = n_long; s_sum[w] = sum; }
+    __syncthreads();
+    if (w) return;
+    hi = s_hi[lane]; lo = s_lo[lane]; n_long = s_long[lane]; sum = s_sum[lane];
+    reduce();
+    if (lane == 0) *out = RowStats{sum, hi, lo, n_long, 0u};
+}
+
+// A row's place in the schedule (longest first, equal ones by id) is the number of rows with a larger key, length before
+// reversed id.  4 lanes count for a row, over keys staged in shared memory (from global memory, one load after the
+// other, 8192 rows took 110 us).
+constexpr uint32_t kRankPerCta = kWarps * 32 / 4, kRankTile = 2048;
+__device__ __forceinline__ void rank_rows(uint32_t cta, const uint32_t* __restrict__ keys, uint32_t m, uint2* __restrict__ rows, uint4* tile)
+{
+    const uint32_t i = cta * kRankPerCta + threadIdx.x / 4, part = threadIdx.x & 3;
+    const uint32_t key = i < m ? __ldg(keys + i) : 0u;
+    uint32_t rank = 0;
+    for (uint32_t t0 = 0; t0 < m; t0 += kRankTile) {
+        __syncthreads();
+        for (uint32_t j = threadIdx.x; j < kRankTile; j += kWarps * 32)
+            reinterpret_cast<uint32_t*>(tile)[j] = t0 + j < m ? __ldg(keys + t0 + j) : 0u;     // 0 is larger than nothing
+        __syncthreads();
+#pragma unroll 8
+        for (uint32_t q = part; q < kRankTile / 4; q += 4) {
+            const uint4 o = tile[q];
+            rank += (o.x > key) + (o.y > key) + (o.z > key) + (o.w > key);
+        }
+    }
+    rank += __shfl_xor_sync(0xffffffffu, rank, 1);
+    rank += __shfl_xor_sync(0xffffffffu, rank, 2);
+    if (part == 0 && i < m) rows[rank] = make_uint2(i, key / kRankRows);
+}
+
+// Entries into their rows: from the pairs that the counter kept, or, where a unit had more of them than fit (or none were
+// kept), out of the matrix again.  Unit u of the grid is the matrix's unit (last - u): the counter has just read the end
+// of W.  The first rank_ctas CTAs make the row schedule.
 __global__ void __launch_bounds__(kWarps * 32)
 pack_kernel(const float* __restrict__ W, uint32_t mis, uint32_t m, uint32_t n, uint32_t segs, uint32_t seg,
             const uint32_t* __restrict__ counts, uint32_t pitch, float* __restrict__ Wd, uint32_t* __restrict__ idx,
-            uint32_t* __restrict__ nnz)
+            uint32_t* __restrict__ nnz, const uint2* __restrict__ kept, uint32_t cap, const uint32_t* __restrict__ keys,
+            uint2* __restrict__ rows, uint32_t rank_ctas)
 {
+    __shared__ __align__(16) uint4 tile[kRankTile / 4];
+    if (blockIdx.x < rank_ctas) {
+        rank_rows(blockIdx.x, keys, m, rows, tile);
+        return;
+    }
     const int lane = threadIdx.x & 31;
     const uint64_t units = (uint64_t)m * segs;
-    const uint64_t u_rev = (uint64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
+    const uint64_t u_rev = (uint64_t)(blockIdx.x - rank_ctas) * kWarps + (threadIdx.x >> 5);
     if (u_rev >= units) return;
     const uint64_t unit = units - 1 - u_rev;
     const Segment s = segment_of(unit, mis, n, segs, seg);
@@ -122,22 +257,40 @@ pack_kernel(const float* __restrict__ W, uint32_t mis, uint32_t m, uint32_t n, u
         for (uint64_t k = first + lane; k < unit; k += 32) pos += counts[k];
         pos = __reduce_add_sync(0xffffffffu, pos);
     }
-    const uint32_t below = (1u << lane) - 1u;
-    for (uint32_t qb = 0; qb < s.quads; qb += 32 * kQuads) {
-        float4 v[kQuads];
-        load_block(v, W, s, qb, lane);
+    const uint32_t mine = kept ? __ldg(counts + unit) : 0u;
+    if (kept && mine <= cap) {
+        const uint2* __restrict__ src = kept + unit * cap;
+        constexpr uint32_t kRun = 4;                        // pairs per lane in flight
+        for (uint32_t j0 = lane; j0 < mine; j0 += 32 * kRun) {
+            uint2 p[kRun];
 #pragma unroll
-        for (int u = 0; u < kQuads; ++u) {
-            const uint32_t b0 = __ballot_sync(0xffffffffu, v[u].x != 0.0f), b1 = __ballot_sync(0xffffffffu, v[u].y != 0.0f);
-            const uint32_t b2 = __ballot_sync(0xffffffffu, v[u].z != 0.0f), b3 = __ballot_sync(0xffffffffu, v[u].w != 0.0f);
-            // entries of the lanes below come first, then this lane's own in column order
-            uint32_t at = pos + __popc(b0 & below) + __popc(b1 & below) + __popc(b2 & below) + __popc(b3 & below);
-            const uint32_t col = s.c_lo + 4 * (qb + 32 * u + lane) - (uint32_t)s.lead;
-            if (v[u].x != 0.0f) { wd[at] = v[u].x; ix[at++] = col; }
-            if (v[u].y != 0.0f) { wd[at] = v[u].y; ix[at++] = col + 1; }
-            if (v[u].z != 0.0f) { wd[at] = v[u].z; ix[at++] = col + 2; }
-            if (v[u].w != 0.0f) { wd[at] = v[u].w; ix[at++] = col + 3; }
-            pos += __popc(b0) + __popc(b1) + __popc(b2) + __popc(b3);
+            for (uint32_t u = 0; u < kRun; ++u) if (j0 + 32 * u < mine) p[u] = __ldcs(src + j0 + 32 * u);
+#pragma unroll
+            for (uint32_t u = 0; u < kRun; ++u)
+                if (j0 + 32 * u < mine) {
+                    wd[pos + j0 + 32 * u] = __uint_as_float(p[u].x);
+                    ix[pos + j0 + 32 * u] = p[u].y;
+                }
+        }
+        pos += mine;
+    } else {
+        const uint32_t below = (1u << lane) - 1u;
+        for (uint32_t qb = 0; qb < s.quads; qb += 32 * kQuads) {
+            float4 v[kQuads];
+            load_block<false>(v, W, s, qb, lane);
+#pragma unroll
+            for (int u = 0; u < kQuads; ++u) {
+                const uint32_t b0 = __ballot_sync(0xffffffffu, v[u].x != 0.0f), b1 = __ballot_sync(0xffffffffu, v[u].y != 0.0f);
+                const uint32_t b2 = __ballot_sync(0xffffffffu, v[u].z != 0.0f), b3 = __ballot_sync(0xffffffffu, v[u].w != 0.0f);
+                // entries of the lanes below come first, then this lane's own in column order
+                uint32_t at = pos + __popc(b0 & below) + __popc(b1 & below) + __popc(b2 & below) + __popc(b3 & below);
+                const uint32_t col = s.c_lo + 4 * (qb + 32 * u + lane) - (uint32_t)s.lead;
+                if (v[u].x != 0.0f) { wd[at] = v[u].x; ix[at++] = col; }
+                if (v[u].y != 0.0f) { wd[at] = v[u].y; ix[at++] = col + 1; }
+                if (v[u].z != 0.0f) { wd[at] = v[u].z; ix[at++] = col + 2; }
+                if (v[u].w != 0.0f) { wd[at] = v[u].w; ix[at++] = col + 3; }
+                pos += __popc(b0) + __popc(b1) + __popc(b2) + __popc(b3);
+            }
         }
     }
     if (unit + 1 == first + segs) {                         // the row's last segment also owns its padding and count
@@ -274,38 +427,72 @@ inline uint32_t misalignment(const float* p) { return (uint32_t)((reinterpret_ca
 
 namespace spx {
 
-// Everything but the two kernels is kept off the critical path: counts come back through pinned
-// memory in one copy (the only point the host must wait for, r fixes the pitch), the row schedule is
-// sorted on the host while the packer runs, and the arrays come from the library's pool.
+// Pairs kept by the counter: a quarter of a unit's columns (denser units are read again, which is then no more to move
+// than pairs would be), and no more scratch than the pool keeps for the next call in any case.  A matrix that stays in L2
+// is read again for less than the pairs cost, short units end in blocks of 512 columns that are mostly empty, and beyond
+// kRankRows rows the host's sort shows that the packer hid (10 % dense, with and without the pairs: 5000 x 5000 110 and
+// 124 us, 14000 x 3000 161 and 183, 10000 x 10000 269 and 326; 3000 x 3000 73.5 and 71.5, 30000 x 1500 229 and 223).
+constexpr size_t kKeepBytes = 256u << 20, kKeepFrom = 64u << 20;
+constexpr uint32_t kKeepColumns = 2048, kKeepColumnsHostSort = 4096;
+// Without the pairs the packer takes longer and hides the host's sort of more rows: 8192 x 2000 98 us ranked, 109 sorted;
+// 9472 x 3000 140 and 139; 16384 x 1000 140 and 129.
+constexpr uint32_t kRankRowsReread = 8192;
+
+// Device memory of one call beside the handle's own.
+struct EncodeScratch {
+    uint32_t* counts = nullptr;     // per unit
+    uint32_t* keys = nullptr;       // per row, where the device ranks them: length * kRankRows + reversed id
+    uint2* kept = nullptr;
+    uint32_t cap = 0;
+};
+
+// Everything but the two passes is kept off the critical path: what the host must know (r fixes the pitch) is one wait
+// away, the row schedule is made beside the packer -- on the device for few rows (a row costs m comparisons), else sorted
+// on the host -- and the arrays come from the library's pool.
 static int encode_rows(const float* dW, uint32_t m, uint32_t n, int device, cudaStream_t s, const PinnedBlock& stage, const Split& sp,
-                       uint32_t* d_counts, spx_ell** out)
+                       const EncodeScratch& sc, spx_ell** out)
 {
     const uint32_t mis = misalignment(dW);
-    uint32_t* h_counts = static_cast<uint32_t*>(stage.host);    // m * segs counts, then the schedule
+    const bool ranked = sc.keys != nullptr;
+    uint32_t* h_counts = static_cast<uint32_t*>(stage.host);    // m * segs counts, then the schedule; or the statistics
     const size_t units = (size_t)m * sp.segs;
-    count_kernel<<<sp.blocks, kWarps * 32, 0, s>>>(dW, mis, m, n, sp.segs, sp.seg, d_counts);
+    if (sc.kept) count_keep_kernel<<<sp.blocks, kWarps * 32, 0, s>>>(dW, mis, m, n, sp.segs, sp.seg, sc.cap, sc.counts, sc.kept);
+    else count_kernel<<<sp.blocks, kWarps * 32, 0, s>>>(dW, mis, m, n, sp.segs, sp.seg, sc.counts);
     SPX_LAUNCH_CHECK("count_kernel");
-    SPX_CUDA(cudaMemcpyAsync(h_counts, d_counts, units * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    // The schedule travels on a stream of its own, beside the packer: its block is allocated in that stream's order too
-    // (the pool may hand out memory that work queued on another stream still uses, ordered behind it on the allocating
-    // stream only), and here, where the host would wait anyway and no packer is queued to wait for.
+    if (ranked) {
+        void* stats = nullptr;
+        SPX_CUDA(cudaHostGetDevicePointer(&stats, stage.host, 0));
+        row_stats_kernel<<<1, 1024, 0, s>>>(sc.counts, m, sp.segs, sc.keys, static_cast<RowStats*>(stats));
+        SPX_LAUNCH_CHECK("row_stats_kernel");
+    } else {
+        SPX_CUDA(cudaMemcpyAsync(h_counts, sc.counts, units * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    }
+    // A schedule from the host travels on a stream of its own, beside the packer: its block is allocated in that stream's
+    // order too (the pool may hand out memory that work queued on another stream still uses, ordered behind it on the
+    // allocating stream only), and here, where the host would wait anyway and no packer is queued to wait for.
     void* schedule = nullptr;
-    cudaStream_t side = nullptr;
+    cudaStream_t side = s;
     const size_t schedule_bytes = (size_t)m * sizeof(uint2);
-    if (int rc = side_stream(device, &side)) return rc;
+    if (!ranked)
+        if (int rc = side_stream(device, &side)) return rc;
     if (int rc = pool_alloc(&schedule, schedule_bytes, device, side)) return rc;
     const cudaError_t counted = cudaStreamSynchronize(s);
     uint32_t r = 0;
     uint64_t total = 0;
-    if (sp.segs > 1 && counted == cudaSuccess)
+    if (counted == cudaSuccess && ranked) {
+        r = static_cast<const RowStats*>(stage.host)->longest;
+        total = static_cast<const RowStats*>(stage.host)->total;
+    } else if (counted == cudaSuccess) {
+        if (sp.segs > 1)
+            for (uint32_t i = 0; i < m; ++i) {
+                uint32_t c = h_counts[(size_t)i * sp.segs];
+                for (uint32_t k = 1; k < sp.segs; ++k) c += h_counts[(size_t)i * sp.segs + k];
+                h_counts[i] = c;                                    // in place: i <= i * segs
+            }
         for (uint32_t i = 0; i < m; ++i) {
-            uint32_t c = h_counts[(size_t)i * sp.segs];
-            for (uint32_t k = 1; k < sp.segs; ++k) c += h_counts[(size_t)i * sp.segs + k];
-            h_counts[i] = c;                                        // in place: i <= i * segs
+            r = std::max(r, h_counts[i]);
+            total += h_counts[i];
         }
-    for (uint32_t i = 0; i < m && counted == cudaSuccess; ++i) {
-        r = std::max(r, h_counts[i]);
-        total += h_counts[i];
     }
     const int rc_ell = counted == cudaSuccess ? alloc_ell(m, n, r, out, s, r == 0)
                                               : fail(SPX_ERR_CUDA, "encode: count pass failed: %s", cudaGetErrorString(counted));
@@ -317,14 +504,23 @@ static int encode_rows(const float* dW, uint32_t m, uint32_t n, int device, cuda
     e->rows = static_cast<uint2*>(schedule);
     e->nnz_total = total;
     e->max_nnz = r;
-    if (r) {
-        pack_kernel<<<sp.blocks, kWarps * 32, 0, s>>>(dW, mis, m, n, sp.segs, sp.seg, d_counts, e->pitch, e->Wd, e->idx, e->nnz);
+    const uint32_t rank_ctas = ranked ? (m + kRankPerCta - 1) / kRankPerCta : 0;
+    const uint32_t pack_ctas = r ? sp.blocks : 0;
+    if (rank_ctas + pack_ctas) {
+        pack_kernel<<<rank_ctas + pack_ctas, kWarps * 32, 0, s>>>(dW, mis, m, n, sp.segs, sp.seg, sc.counts, e->pitch, e->Wd, e->idx, e->nnz,
+                                                                  sc.kept, sc.cap, sc.keys, e->rows, rank_ctas);
         SPX_LAUNCH_CHECK("pack_kernel");
     }
-    uint2* h_order = reinterpret_cast<uint2*>(h_counts + round_up<size_t>(units, 2));
-    if (int rc = sort_rows(e, h_counts, h_order, side)) return rc;
-    SPX_CUDA(cudaMemcpyAsync(e->rows, h_order, schedule_bytes, cudaMemcpyHostToDevice, side));
-    SPX_CUDA(cudaStreamSynchronize(side));
+    if (ranked) {
+        const RowStats& st = *static_cast<const RowStats*>(stage.host);
+        e->min_nnz = st.shortest;
+        e->long_rows = st.long_rows;
+    } else {
+        uint2* h_order = reinterpret_cast<uint2*>(h_counts + round_up<size_t>(units, 2));
+        if (int rc = sort_rows(e, h_counts, h_order, side)) return rc;
+        SPX_CUDA(cudaMemcpyAsync(e->rows, h_order, schedule_bytes, cudaMemcpyHostToDevice, side));
+        SPX_CUDA(cudaStreamSynchronize(side));
+    }
     SPX_CUDA(cudaStreamSynchronize(s));         // the handle may be used on any stream from here on
     return SPX_OK;
 }
@@ -341,17 +537,35 @@ int encode_device(const float* dW, uint32_t m, uint32_t n, cudaStream_t s, spx_e
     SPX_CUDA(cudaGetDevice(&device));
     const Split sp = split_rows(m, n, sm_count(device));
     const size_t units = (size_t)m * sp.segs;
+    EncodeScratch sc;
+    sc.cap = sp.seg / 4;
+    const size_t keep = units * sc.cap * sizeof(uint2);
+    bool keeps = sp.seg >= kKeepColumns && (m <= kRankRows || sp.seg >= kKeepColumnsHostSort) &&
+                 (size_t)m * n * sizeof(float) >= kKeepFrom && keep <= kKeepBytes;
+    const bool ranked = m <= (keeps ? kRankRows : kRankRowsReread) && n < kRankColumns;
     PinnedBlock stage;
-    if (int rc = pinned_acquire((units + 1) * sizeof(uint32_t) + m * sizeof(uint2), &stage)) return rc;
-    void* d_counts = nullptr;
-    int rc = pool_alloc(&d_counts, units * sizeof(uint32_t), device, s);
-    if (rc == SPX_OK) rc = encode_rows(dW, m, n, device, s, stage, sp, static_cast<uint32_t*>(d_counts), out);
+    if (int rc = pinned_acquire(ranked ? sizeof(RowStats) : (units + 1) * sizeof(uint32_t) + m * sizeof(uint2), &stage)) return rc;
+    // counts, the rows' keys, the pairs, each on a 16-byte boundary
+    const size_t keys_at = round_up<size_t>(units * sizeof(uint32_t), 16), kept_at = keys_at + (ranked ? round_up<size_t>(m * sizeof(uint32_t), 16) : 0);
+    void* scratch = nullptr;
+    int rc = scratch_alloc(&scratch, kept_at + (keeps ? keep : 0), device, s);
+    if (rc == SPX_ERR_OOM && keeps) {           // it goes without
+        keeps = false;
+        rc = scratch_alloc(&scratch, kept_at, device, s);
+    }
+    if (rc == SPX_OK) {
+        unsigned char* base = static_cast<unsigned char*>(scratch);
+        sc.counts = reinterpret_cast<uint32_t*>(base);
+        if (ranked) sc.keys = reinterpret_cast<uint32_t*>(base + keys_at);
+        if (keeps) sc.kept = reinterpret_cast<uint2*>(base + kept_at);
+        rc = encode_rows(dW, m, n, device, s, stage, sp, sc, out);
+    }
     if (rc != SPX_OK) {
         (void)cudaStreamSynchronize(s);         // nothing may still write the staging block
         if (*out) spx_ell_destroy(*out);
         *out = nullptr;
     }
-    pool_free(d_counts, units * sizeof(uint32_t), s);
+    scratch_free(scratch, s);
     pinned_release(stage);
     return rc;
 }
