@@ -15,12 +15,12 @@
 //
 // What bounds it: issue slots.  A tap costs a warp 8 packed FMAs (16 clocks of the FMA pipe) and about 8 other
 // instructions, 24 clocks with four warps to an SM quarter; filling costs 4 clocks per column, a shared-memory wavefront
-// for each quadrant.  Measured, 256 -> 256 channels, 3 x 3, 56 x 56, batch 32: 80 % sparse 742 us against 1342 with
-// conv_rbm_tile_kernel, 50 % 1430 / 2370, 95 % 436 / 465; batch 8 272 / 375; 64 -> 64, 112 x 112 252 / 378; 5 x 5, 64 -> 96,
-// 28 x 28, batch 16 58 / 100.  Tried: scalar FMAs 1221 against 1021 us at the time, 4 x 8 positions and 2 channels a warp
+// for each quadrant.  Measured, 256 -> 256 channels, 3 x 3, 56 x 56, batch 32: 80 % sparse 697 us against 1342 with
+// conv_rbm_tile_kernel, 50 % 1359 / 2370, 95 % 391 / 465; batch 8 256 / 375; 64 -> 64, 112 x 112 201 / 378; 5 x 5, 64 -> 96,
+// 28 x 28, batch 16 56 / 100.  Tried: scalar FMAs 1221 against 1021 us at the time, 4 x 8 positions and 2 channels a warp
 // 1272 (spills), no warps of their own for the copying 1010 against 819 (its waits add up), entries read through L1
 // instead of shared memory 807 against 732, weights stored twice so that the packed FMA can take them as they are 760
-// against 732.
+// against 732, CTAs that go on to further units by themselves 764 against 743.
 #include "conv.cuh"
 #include "tma.cuh"
 #include "tmem.cuh"
@@ -196,6 +196,10 @@ __device__ __forceinline__ void fill_columns(uint32_t from, uint32_t pitch, uint
         spx::tmem_st8(to, v);
     }
 }
+
+// Sigmoid and tanh: one copy of their code.  Inlined for each of a thread's 64 results they made the instruction cache
+// miss at the end of every CTA: 256 -> 256, 56 x 56 742 against 697 us, 3 -> 416, 80 x 80 242 against 147.
+__device__ __noinline__ float activate(float v, int act) { return spx::apply_act(v, act); }
 
 // RW: output channels per warp (4, or half a block: the last wave of a launch on twice the CTAs); GP: row_cols, where
 // it is known.  Work units are (group of output channels, tiles, batch entries), groups fastest, so that the CTAs that
@@ -380,16 +384,32 @@ conv_tmem_kernel(const __grid_constant__ TmemArgs a, const __grid_constant__ CUt
     const uint32_t tile = first_tile + sub, b = bz * a.BT + lane % a.BT;
     const uint32_t oh0 = tile / a.tilesX * kTH, ow0 = tile % a.tilesX * kTW;
     if (active && tile < a.tiles && b < a.v.b_out) {
+        if (a.act == SPX_ACT_RELU) {
+#pragma unroll
+            for (int r = 0; r < RW; ++r)
+#pragma unroll
+                for (int g = 0; g < (int)kTH; ++g)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) acc[r][g][i] = acc[r][g][i] > 0.0f ? acc[r][g][i] : 0.0f;
+        } else if (a.act != SPX_ACT_NONE) {
+#pragma unroll
+            for (int r = 0; r < RW; ++r)
+#pragma unroll
+                for (int g = 0; g < (int)kTH; ++g)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) acc[r][g][i] = activate(acc[r][g][i], a.act);
+        }
+        const int cols = (int)min(8u, p.Wo - ow0), rows = (int)min(kTH, p.Ho - oh0);
 #pragma unroll
         for (int r = 0; r < RW; ++r) {
             if (mo0 + r >= p.Cout) break;
 #pragma unroll
             for (int g = 0; g < (int)kTH; ++g) {
-                if (oh0 + g >= p.Ho) break;
+                if (g >= rows) break;
                 float* __restrict__ o = a.out + (mo0 + r) * a.v.oC + (oh0 + g) * a.v.oH + ow0 * a.v.oW + b * a.v.oB;
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    if (ow0 + i < p.Wo) o[i * a.v.oW] = spx::apply_act(acc[r][g][i], a.act);
+                for (int i = 0; i < 8; ++i, o += a.v.oW)
+                    if (i < cols) *o = acc[r][g][i];
             }
         }
     }
