@@ -197,10 +197,6 @@ __device__ __forceinline__ void fill_columns(uint32_t from, uint32_t pitch, uint
     }
 }
 
-// Sigmoid and tanh: one copy of their code.  Inlined for each of a thread's 64 results they made the instruction cache
-// miss at the end of every CTA: 256 -> 256, 56 x 56 742 against 697 us, 3 -> 416, 80 x 80 242 against 147.
-__device__ __noinline__ float activate(float v, int act) { return spx::apply_act(v, act); }
-
 // RW: output channels per warp (4, or half a block: the last wave of a launch on twice the CTAs); GP: row_cols, where
 // it is known.  Work units are (group of output channels, tiles, batch entries), groups fastest, so that the CTAs that
 // read the same patch run side by side.
@@ -397,7 +393,7 @@ conv_tmem_kernel(const __grid_constant__ TmemArgs a, const __grid_constant__ CUt
 #pragma unroll
                 for (int g = 0; g < (int)kTH; ++g)
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) acc[r][g][i] = activate(acc[r][g][i], a.act);
+                    for (int i = 0; i < 8; ++i) acc[r][g][i] = spx::apply_smooth_act(acc[r][g][i], a.act);
         }
         const int cols = (int)min(8u, p.Wo - ow0), rows = (int)min(kTH, p.Ho - oh0);
 #pragma unroll
