@@ -893,14 +893,14 @@ static RbmCut rbm_cut(const spx_ell* e, const ConvParams& p, uint32_t qb, uint32
     return best;
 }
 
-// Expected time of all segments of a batch.  The factors bring the cuts' estimates to measured times of 267 shapes.
+// Expected time of all segments of a batch.  The factors bring the cuts' estimates to measured times of 400 shapes.
 static double conv_rbm_us(const spx_ell* e, const ConvParams& p)
 {
     const uint32_t n16 = p.B / 16 * 16, rest = p.B - n16;
     double us = 0.0;
-    if (n16) us += 1.118 * rbm_cut(e, p, 4, n16).cycles / 1900.0 + 2.46;
-    if (rest >= 8) us += 0.879 * rbm_cut(e, p, 2, 8).cycles / 1900.0 + 2.46;
-    if (rest % 8 == 4) us += rbm_cut(e, p, 1, 4).cycles / 1900.0 + 2.46;
+    if (n16) us += 1.118 * rbm_cut(e, p, 4, n16).cycles / 1900.0 + 2.75;
+    if (rest >= 8) us += 0.865 * rbm_cut(e, p, 2, 8).cycles / 1900.0 + 2.75;
+    if (rest % 8 == 4) us += 0.952 * rbm_cut(e, p, 1, 4).cycles / 1900.0 + 2.75;
     return us;
 }
 

@@ -140,6 +140,7 @@ struct TmemArgs {
     const float* bias;
     float* out;
     int act;
+    uint32_t quads_out;                     // positions are contiguous in the output, in whole 16-byte quads
     uint32_t cap, slot;                     // units per block of the form; per slot of a chunk's units in shared memory
     uint32_t BT, S, QT;                     // batch entries per lane group; lane groups per warp; quadrants with patches of their own
     uint32_t TWin, CC, chunks, chunk_cols, row_cols;    // row_cols: columns from one row of positions to the next
@@ -403,6 +404,11 @@ conv_tmem_kernel(const __grid_constant__ TmemArgs a, const __grid_constant__ CUt
             for (int g = 0; g < (int)kTH; ++g) {
                 if (g >= rows) break;
                 float* __restrict__ o = a.out + (mo0 + r) * a.v.oC + (oh0 + g) * a.v.oH + ow0 * a.v.oW + b * a.v.oB;
+                if (a.quads_out) {              // positions side by side: whole sectors per lane
+                    reinterpret_cast<float4*>(o)[0] = make_float4(acc[r][g][0], acc[r][g][1], acc[r][g][2], acc[r][g][3]);
+                    if (cols > 4) reinterpret_cast<float4*>(o)[1] = make_float4(acc[r][g][4], acc[r][g][5], acc[r][g][6], acc[r][g][7]);
+                    continue;
+                }
 #pragma unroll
                 for (int i = 0; i < 8; ++i, o += a.v.oW)
                     if (i < cols) *o = acc[r][g][i];
@@ -555,13 +561,14 @@ Tail tail_of(uint64_t units, uint32_t sms)
 
 }  // namespace
 
-// Expected time.  Per chunk of a CTA the larger of what its busiest quadrant multiplies (24 clocks an entry, and 134 for
-// each row's run) or the latency of a warp's own runs, and what its fillers copy (8.8 clocks a column; the lane groups
-// of a warp read the same banks, 4.5 clocks for each); 15000 clocks per CTA, 32000 for a launch more.  Fitted with
-// conv_rbm_us to 267 shapes of both kernels (3 to 512 channels, 3 x 3 and 5 x 5, 7 x 7 to 112 x 112, batch 1 to 32, 5 to 50 %
-// dense): taken where it is below 0.93 of that, it was the faster one every time, 58 times; picking the faster each time
-// would gain another 0.5 % on average.
-double conv_tmem_us(const spx_ell* e, const ConvParams& p)
+// Expected time.  Per chunk of a CTA the larger of what its busiest quadrant multiplies (23.5 clocks an entry, and 115 for
+// each row's run) or the latency of a warp's own runs, and what its fillers copy (7.7 clocks a column, and 690; the lane
+// groups of a warp read the same banks, 4.4 clocks for each); 9650 clocks per CTA; results that are not contiguous along
+// the batch by the million, in quads or one by one.  Fitted with conv_rbm_us to 400 shapes of both kernels (3 to 512
+// channels, 3 x 3 and 5 x 5, 7 x 7 to 112 x 112, batch 1 to 32, 5 to 50 % dense, all layouts): taken where it is below 0.92 of
+// that (0.85 for batches below 16, not for few output channels with a batch that is no multiple of 16), it was the faster
+// one every time, some 125 times; picking the faster each time would gain another 1.2 % on average.
+static double conv_tmem_us(const spx_ell* e, const ConvParams& p, const ConvViews& v)
 {
     const uint32_t sms = (uint32_t)sm_count(e->device);
     const double density = (double)e->nnz_total / ((double)e->m * e->n);
@@ -572,15 +579,16 @@ double conv_tmem_us(const spx_ell* e, const ConvParams& p)
         const double run = c.CC * p.kH * p.kW * density;
         const auto cta = [&](double rows) {
             const double quad = std::min(16.0, (p.Cout + kRows - 1) / kRows * c.QT * (kRows / rows)) / 4.0;
-            const double mul = std::max(quad * rows * (24.05 * run + 134.0), rows * (60.0 * run + 150.0) + 300.0);
-            return 15080.0 + c.chunks * std::max(mul, c.chunk_cols * std::max(8.8, 4.5 * c.S) + 380.0);
+            const double mul = std::max(quad * rows * (23.5 * run + 115.0), rows * (60.0 * run + 150.0) + 300.0);
+            return 9650.0 + c.chunks * std::max(mul, c.chunk_cols * std::max(7.7, 4.4 * c.S) + 690.0);
         };
         const Tail t = tail_of(c.units, sms);
         const double full = std::floor((double)c.units / sms), rem = (double)(c.units % sms);
-        clocks += t == Tail::all ? cta(2) : t == Tail::split ? full * cta(4) + cta(2) + 31800.0 : (full + (rem > 0)) * cta(4);
+        clocks += t == Tail::all ? cta(2) : t == Tail::split ? full * cta(4) + cta(2) + 1040.0 : (full + (rem > 0)) * cta(4);
         return 0;
     });
-    return rc ? 1e30 : clocks / 1900.0;
+    const double strided = v.oB == 1 ? 0.0 : p.Wo % 4 == 0 ? 1.15e-6 : 7.2e-6;
+    return rc ? 1e30 : clocks / 1900.0 + strided * p.Cout * p.Ho * p.Wo * p.B;
 }
 
 template <int RW, int GP>
@@ -620,8 +628,9 @@ int launch_conv_tmem(spx_ell* e, const ConvParams& p, const ConvViews& v, const 
     }();
     const PFN_cuTensorMapEncodeTiled encode = tensor_map_encoder();
     if (!env || !e->conv_tmem || e->tma_off || e->max_nnz == 0 || p.B % 4 || !encode) return -1;
-    const double us = conv_tmem_us(e, p);
-    if (us >= 1e30 || (env != 2 && us > 0.93 * other_us)) return -1;
+    const double us = conv_tmem_us(e, p, v);
+    if (us >= 1e30) return -1;
+    if (env != 2 && ((p.B % 16 && p.Cout <= 32) || us > (p.B < 16 ? 0.85 : 0.92) * other_us)) return -1;
     static const int short_env = [] { const char* v = getenv("SPX_CONV_TMA_TEST_TIMEOUT"); return v ? atoi(v) : 0; }();
     bool launched = false;
     return each_segment(p.B, [&](uint32_t BT, uint32_t at, uint32_t len) -> int {
@@ -636,6 +645,7 @@ int launch_conv_tmem(spx_ell* e, const ConvParams& p, const ConvViews& v, const 
         a.v.b_out = v.b_out > at ? v.b_out - at : 0u;
         a.units = form->units; a.cap = form->cap; a.slot = c.slot;
         a.bias = bias; a.out = out + at * v.oB; a.act = act;
+        a.quads_out = v.oW == 1 && p.Wo % 4 == 0 && (v.oB | v.oC | v.oH) % 4 == 0 && reinterpret_cast<uintptr_t>(a.out) % 16 == 0;
         a.BT = BT; a.S = c.S; a.QT = c.QT;
         a.TWin = c.TWin; a.CC = c.CC; a.chunks = c.chunks; a.chunk_cols = c.chunk_cols; a.row_cols = p.sH * c.TWin;
         a.tilesX = c.tilesX; a.tiles = c.tiles; a.tile_units = c.tile_units; a.groups = c.groups;
