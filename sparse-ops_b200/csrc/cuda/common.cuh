@@ -111,14 +111,6 @@ __device__ __forceinline__ float apply_act(float v, int act) {
     default:              return v;
     }
 }
-// The same for kernels with many results per thread: one copy of the code of sigmoid and tanh.  Inlined for each of 64
-// results they made the instruction cache miss at the end of every CTA (conv_tmem.cu: 3 -> 416 channels, 80 x 80 242
-// against 147 us; conv.cu: 146 and 140).  With few results the call costs more (325 x 576, 2 %, C = 1007, tanh 6.4 against 6.6 us).
-static __device__ __noinline__ float apply_smooth_act(float v, int act) { return apply_act(v, act); }
-__device__ __forceinline__ float apply_act_called(float v, int act) {
-    return act == SPX_ACT_NONE ? v : act == SPX_ACT_RELU ? (v > 0.0f ? v : 0.0f) : apply_smooth_act(v, act);
-}
-
 // Programmatic dependent launch: a kernel launched with launch_pdl() may start while its predecessor
 // in the stream is still draining.  Before pdl_wait() it may only touch what no kernel of the stream
 // writes -- the arrays of a finished handle; after it everything the predecessors wrote is visible.

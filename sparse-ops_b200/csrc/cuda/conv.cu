@@ -211,8 +211,8 @@ __device__ __forceinline__ void store_quad(float* __restrict__ out, const ConvVi
                                            float4 o, int act)
 {
     if (act != SPX_ACT_NONE) {
-        o.x = spx::apply_act_called(o.x, act); o.y = spx::apply_act_called(o.y, act);
-        o.z = spx::apply_act_called(o.z, act); o.w = spx::apply_act_called(o.w, act);
+        o.x = spx::apply_act(o.x, act); o.y = spx::apply_act(o.y, act);
+        o.z = spx::apply_act(o.z, act); o.w = spx::apply_act(o.w, act);
     }
     float* __restrict__ p = out + mo * v.oC + oh * v.oH + ow * v.oW + b * v.oB;
     if (v.vec_out) {

@@ -198,6 +198,11 @@ __device__ __forceinline__ void fill_columns(uint32_t from, uint32_t pitch, uint
     }
 }
 
+// Sigmoid and tanh: one copy of their code.  Inlined for each of a thread's 64 results they made the instruction cache
+// miss at the end of every CTA: 256 -> 256, 56 x 56 742 against 697 us, 3 -> 416, 80 x 80 242 against 147.  (The merged kernel's
+// small cuts lose by the call, also where it is not made: 3 -> 160, 45 x 45, batch 30 30.4 against 33.1.)
+__device__ __noinline__ float activate(float v, int act) { return spx::apply_act(v, act); }
+
 // RW: output channels per warp (4, or half a block: the last wave of a launch on twice the CTAs); GP: row_cols, where
 // it is known.  Work units are (group of output channels, tiles, batch entries), groups fastest, so that the CTAs that
 // read the same patch run side by side.
@@ -394,7 +399,7 @@ conv_tmem_kernel(const __grid_constant__ TmemArgs a, const __grid_constant__ CUt
 #pragma unroll
                 for (int g = 0; g < (int)kTH; ++g)
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) acc[r][g][i] = spx::apply_smooth_act(acc[r][g][i], a.act);
+                    for (int i = 0; i < 8; ++i) acc[r][g][i] = activate(acc[r][g][i], a.act);
         }
         const int cols = (int)min(8u, p.Wo - ow0), rows = (int)min(kTH, p.Ho - oh0);
 #pragma unroll
@@ -566,8 +571,8 @@ Tail tail_of(uint64_t units, uint32_t sms)
 // groups of a warp read the same banks, 4.4 clocks for each); 9650 clocks per CTA; results that are not contiguous along
 // the batch by the million, in quads or one by one.  Fitted with conv_rbm_us to 400 shapes of both kernels (3 to 512
 // channels, 3 x 3 and 5 x 5, 7 x 7 to 112 x 112, batch 1 to 32, 5 to 50 % dense, all layouts): taken where it is below 0.92 of
-// that (0.85 for batches below 16, not for few output channels with a batch that is no multiple of 16), it was the faster
-// one every time, some 125 times; picking the faster each time would gain another 1.2 % on average.
+// that (0.85 for batches that leave lanes to a second tile, not for few output channels with a batch that is no multiple
+// of 16), it was the faster one every time, some 115 times; picking the faster each time would gain another 1.2 % on average.
 static double conv_tmem_us(const spx_ell* e, const ConvParams& p, const ConvViews& v)
 {
     const uint32_t sms = (uint32_t)sm_count(e->device);
@@ -630,7 +635,7 @@ int launch_conv_tmem(spx_ell* e, const ConvParams& p, const ConvViews& v, const 
     if (!env || !e->conv_tmem || e->tma_off || e->max_nnz == 0 || p.B % 4 || !encode) return -1;
     const double us = conv_tmem_us(e, p, v);
     if (us >= 1e30) return -1;
-    if (env != 2 && ((p.B % 16 && p.Cout <= 32) || us > (p.B < 16 ? 0.85 : 0.92) * other_us)) return -1;
+    if (env != 2 && ((p.B % 16 && p.Cout <= 32) || us > (p.B % 32 ? 0.85 : 0.92) * other_us)) return -1;
     static const int short_env = [] { const char* v = getenv("SPX_CONV_TMA_TEST_TIMEOUT"); return v ? atoi(v) : 0; }();
     bool launched = false;
     return each_segment(p.B, [&](uint32_t BT, uint32_t at, uint32_t len) -> int {
