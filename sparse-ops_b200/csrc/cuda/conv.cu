@@ -987,7 +987,7 @@ static int launch_conv_rbm_tile(spx_ell* e, const ConvParams& p, const ConvViews
     const auto fits = [&](uint32_t qb) { return rbm_fits(p, qb, 16, kRbmG); };
     if ((n16 && !fits(4)) || (rest >= 8 && !fits(2)) || (rest % 8 == 4 && !fits(1))) return -1;
     {
-        const int rc = launch_conv_tmem(e, p, v, in, bias, act, out, conv_rbm_us(e, p), s);
+        const int rc = launch_conv_tmem(e, p, v, in, bias, act, out, conv_rbm_us, s);
         if (rc != -1) return rc;
     }
     TileParams tp{};

@@ -20,7 +20,7 @@ struct ConvViews {
 
 // conv_tmem.cu: -1 when the shape or the handle is not for this kernel, or the other one's expected time is not above its own.
 int launch_conv_tmem(spx_ell* e, const ConvParams& p, const ConvViews& v, const float* in, const float* bias, int act, float* out,
-                     double other_us, cudaStream_t s);
+                     double (*other_us)(const spx_ell*, const ConvParams&), cudaStream_t s);
 // conv.cu: the merged weights of conv_rbm_tile_kernel; -1 where there is no memory for them.
 int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s);
 void* new_conv_tmem();

@@ -571,7 +571,8 @@ Tail tail_of(uint64_t units, uint32_t sms)
 // groups of a warp read the same banks, 4.4 clocks for each); 9650 clocks per CTA; results that are not contiguous along
 // the batch by the million, in quads or one by one.  Fitted with conv_rbm_us to 400 shapes of both kernels (3 to 512
 // channels, 3 x 3 and 5 x 5, 7 x 7 to 112 x 112, batch 1 to 32, 5 to 50 % dense, all layouts): taken where it is below 0.92 of
-// that (0.85 for batches that leave lanes to a second tile, not for few output channels with a batch that is no multiple
+// that (a launch on less than half of the SMs counted 15 % longer: the other kernel cuts finer, and 453 -> 54 channels, 5 x 5,
+// 32 x 32, batch 16 was 7 % slower here; 0.85 for batches that leave lanes to a second tile, not for few output channels with a batch that is no multiple
 // of 16), it was the faster one every time, some 115 times; picking the faster each time would gain another 1.2 % on average.
 static double conv_tmem_us(const spx_ell* e, const ConvParams& p, const ConvViews& v)
 {
@@ -589,7 +590,7 @@ static double conv_tmem_us(const spx_ell* e, const ConvParams& p, const ConvView
         };
         const Tail t = tail_of(c.units, sms);
         const double full = std::floor((double)c.units / sms), rem = (double)(c.units % sms);
-        clocks += t == Tail::all ? cta(2) : t == Tail::split ? full * cta(4) + cta(2) + 1040.0 : (full + (rem > 0)) * cta(4);
+        clocks += t == Tail::all ? 1.15 * cta(2) : t == Tail::split ? full * cta(4) + cta(2) + 1040.0 : (full + (rem > 0)) * cta(4);
         return 0;
     });
     const double strided = v.oB == 1 ? 0.0 : p.Wo % 4 == 0 ? 1.15e-6 : 7.2e-6;
@@ -622,7 +623,7 @@ static int launch_cut(const spx_ell* e, TmemArgs a, const CUtensorMap& map, uint
 }
 
 int launch_conv_tmem(spx_ell* e, const ConvParams& p, const ConvViews& v, const float* in, const float* bias, int act, float* out,
-                     double other_us, cudaStream_t s)
+                     double (*other_us)(const spx_ell*, const ConvParams&), cudaStream_t s)
 {
     // the switches that force the other kernels turn this one off
     static const int env = [] {
@@ -633,9 +634,11 @@ int launch_conv_tmem(spx_ell* e, const ConvParams& p, const ConvViews& v, const 
     }();
     const PFN_cuTensorMapEncodeTiled encode = tensor_map_encoder();
     if (!env || !e->conv_tmem || e->tma_off || e->max_nnz == 0 || p.B % 4 || !encode) return -1;
+    // Below 25 million FMAs a CTA's fixed cost decides (the smallest gains seen were at 16 million), and a call of 4 us
+    // is the host's: it does without the estimates (3 -> 32, 21 x 21, batch 8 4.3 against 4.7 us).
+    if (env != 2 && ((p.B % 16 && p.Cout <= 32) || (double)e->nnz_total * p.Ho * p.Wo * p.B < 25e6)) return -1;
     const double us = conv_tmem_us(e, p, v);
-    if (us >= 1e30) return -1;
-    if (env != 2 && ((p.B % 16 && p.Cout <= 32) || us > (p.B % 32 ? 0.85 : 0.92) * other_us)) return -1;
+    if (us >= 1e30 || (env != 2 && us > (p.B % 32 ? 0.85 : 0.92) * other_us(e, p))) return -1;
     static const int short_env = [] { const char* v = getenv("SPX_CONV_TMA_TEST_TIMEOUT"); return v ? atoi(v) : 0; }();
     bool launched = false;
     return each_segment(p.B, [&](uint32_t BT, uint32_t at, uint32_t len) -> int {
