@@ -162,9 +162,11 @@ int spx_spmv_reference_order(const spx_ell* e, const float* x, const float* bias
  * conv2d_tiled_im2col_fmajor / conv2d_rbm_fmajor_implicit (src/layers/conv_kernels.cpp:66-470)
  * and, on the device, build_rbm_from_ellpack (src/layers/rbm_conv.cpp:7-73): the first call per
  * handle and kernel shape builds and caches a tap table and, where the batch size and weight
- * density favour it, the row-block-merged form of the weights (device allocations; make that
- * call outside a stream capture).  Results do not depend on which kernel is chosen.  The
- * row-block-merged kernel fetches its input with bulk tensor copies: see spx_ell_status. */
+ * density favour it, the row-block-merged form of the weights and, for larger calls, a second
+ * form for the kernel that keeps its input in tensor memory (device allocations, and a wait for
+ * `stream`; make that call outside a stream capture: a captured call uses the forms that are
+ * there).  Results do not depend on which kernel is chosen.  Both of those kernels fetch their
+ * input with bulk tensor copies: see spx_ell_status. */
 int spx_conv2d(const spx_ell* e, const spx_conv_geom* g, int layout, const float* in, uint32_t B,
                const float* bias, int act, float* out, void* stream);
 /* spx_conv2d for callers that must not allocate device memory (no counterpart in the
