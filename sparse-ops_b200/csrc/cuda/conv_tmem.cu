@@ -440,6 +440,7 @@ struct conv_tmem_impl {
     };
     std::mutex mu;
     int count = 0;
+    bool no_memory = false;     // an earlier attempt found none: a further one would wait for the whole device to give memory back
     Form forms[kForms];
 };
 
@@ -462,7 +463,7 @@ static int find_form(spx_ell* e, const FormShape& f, uint32_t chunks, cudaStream
     std::lock_guard<std::mutex> lk(t->mu);
     for (int i = 0; i < t->count; ++i)
         if (t->forms[i].shape == f) { *out = &t->forms[i]; return SPX_OK; }
-    if (t->count == conv_tmem_impl::kForms) return -1;
+    if (t->no_memory || t->count == conv_tmem_impl::kForms) return -1;
     cudaStreamCaptureStatus cap_status = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cap_status) != cudaSuccess || cap_status != cudaStreamCaptureStatusNone) {
         (void)cudaGetLastError();
@@ -472,7 +473,10 @@ static int find_form(spx_ell* e, const FormShape& f, uint32_t chunks, cudaStream
     // A later call that is recorded may take the other kernel (another batch, say), and cannot build what that needs then.
     if (const int rc = ensure_rbm(e, f.kH, f.kW, s); rc > 0) return rc;
     ensure_tma_words(e);
-    if (!e->tma_failed_dev || !e->tma_failed_mapped) return -1;
+    if (!e->tma_failed_dev || !e->tma_failed_mapped) {
+        t->no_memory = true;
+        return -1;
+    }
     const uint32_t blocks = (e->m + kRows - 1) / kRows;
     // per row at most one half-empty unit per chunk
     const uint64_t cap = chunks + kRows * (((uint64_t)e->max_nnz + chunks + 1) / 2);
@@ -483,7 +487,10 @@ static int find_form(spx_ell* e, const FormShape& f, uint32_t chunks, cudaStream
     form.cap = (uint32_t)cap;
     form.bytes = (size_t)blocks * cap * 16;
     void* units = nullptr;
-    if (pool_alloc(&units, form.bytes, e->device, s) != SPX_OK) return -1;
+    if (pool_alloc(&units, form.bytes, e->device, s) != SPX_OK) {
+        t->no_memory = true;
+        return -1;
+    }
     form.units = static_cast<uint4*>(units);
     const size_t smem = (size_t)((chunks + 1) * kRows + chunks) * 4;
     conv_form_kernel<<<blocks, 256, smem, s>>>(e->Wd, e->idx, e->nnz, e->m, e->pitch, f, chunks, form.cap, form.units);

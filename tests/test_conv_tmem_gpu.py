@@ -1,6 +1,7 @@
 """GPU: the convolution with its patch in tensor memory (conv_tmem.cu), forced, against the oracle bit for bit: edges of
 tiles, chunks and batch segments, few and many output channels, full and empty rows, infinities under taps that a row
 does not store.  The switch is read once per process, so the cases run in a child."""
+import ctypes
 import os
 import subprocess
 import sys
@@ -103,6 +104,74 @@ def test_forced_more_shapes_than_forms_and_capture(lib, orc, cuda):
         assert_bit_equal(dY.cpu().numpy(), want, "replayed")
 
 
+def kernels_of(f):
+    """Names of the kernels that f() launches."""
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as p:
+        f()
+        torch.cuda.synchronize()
+    return " ".join(e.key for e in p.key_averages())
+
+
+def fill_device(lib, leave, step):
+    """Takes device memory until at most `leave` + `step` bytes are free."""
+    held = []
+    for s in (4 << 30, 256 << 20, step):
+        while torch.cuda.mem_get_info()[0] > leave + s:
+            p = ctypes.c_void_p()
+            lib.spx_malloc(ctypes.byref(p), s)
+            held.append(p)
+    return held
+
+
+def waits_for_the_device(f):
+    """Whether f() returns only after what is queued on another stream."""
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        torch.cuda._sleep(400_000_000)                      # 0.2 s and more
+        done = torch.cuda.Event()
+        done.record()
+    f()
+    waited = done.query()
+    torch.cuda.synchronize()
+    return waited
+
+
+@forced
+def test_no_room_for_a_form(lib, orc, cuda):
+    """The form does not fit: the merged kernel takes the call, and the next one does not try again (which would wait for
+    the whole device each time)."""
+    rng = np.random.default_rng(8)
+    Cin, Cout, B, H = 512, 2048, 32, 4
+    wt = sparse(rng, Cout, Cin * 9, 0.01)
+    wt[0] = 1                                               # a full row: the form's capacity is for rows like it, 77 MB
+    E = orc.encode(wt)
+    src = as_layout(rng.standard_normal((B, Cin, H, H)).astype(np.float32), sx.LAYOUT_PF)
+    want = orc.conv2d(E, dict(Cin=Cin, kH=3, kW=3, sH=1, sW=1, pH=1, pW=1, dH=1, dW=1, H=H, W=H), sx.LAYOUT_PF, src, B, None, 0)
+    dX, dY = dev(src, cuda), torch.empty(want.shape, device=cuda)
+    g = sx.conv_geom(Cin, Cout, 3, 3, H, H, 1, 1, 1, 1)
+
+    def call(h):
+        dY.fill_(float("nan"))
+        h.conv2d(g, sx.LAYOUT_PF, ptr(dX), B, None, 0, ptr(dY))
+
+    h = gpu_ell(lib, E)
+    h.conv2d(sx.conv_geom(Cin, Cout, 3, 3, H, H, 2, 2, 1, 1), sx.LAYOUT_PF, ptr(dX), B, None, 0, ptr(dY))   # merged weights only
+    dY.fill_(0.0)
+    assert not waits_for_the_device(lambda: None)           # (makes the stream while there is room)
+    held = fill_device(lib, 32 << 20, 16 << 20)
+    try:
+        for again in (False, True):
+            waited = waits_for_the_device(lambda: call(h))
+            assert not (again and waited), "a call after the failed one waited for another stream's work"
+            assert_bit_equal(dY.cpu().numpy(), want, "short of memory")
+    finally:
+        for p in held:
+            lib.spx_free(p)
+    other = gpu_ell(lib, E)
+    assert "conv_tmem_kernel" in kernels_of(lambda: call(other)) and "conv_tmem_kernel" not in kernels_of(lambda: call(h))
+    assert_bit_equal(dY.cpu().numpy(), want, "room again")
+
+
 def child(files, select, env):
     cmd = [sys.executable, "-m", "pytest", "-q", "-x", "-m", "gpu", "-p", "no:cacheprovider", *[os.path.join(HERE, f) for f in files], "-k", select]
     r = subprocess.run(cmd, env={**os.environ, **env}, capture_output=True, text=True, timeout=900)
@@ -117,3 +186,7 @@ def test_forced_kernel():
 def test_timeout_is_reported():
     """The waits for its bulk copies are bounded: they are made to run out, the next call says so, the one after works."""
     child(["test_parity_gpu.py"], "bulk_copy_timeout_child", {"SPX_CONV_TMEM": "2", "SPX_CONV_TMA_TEST_TIMEOUT": "1"})
+
+
+def test_forced_without_memory():
+    child(["test_conv_tmem_gpu.py"], "no_room_for_a_form", {"SPX_CONV_TMEM": "2"})
