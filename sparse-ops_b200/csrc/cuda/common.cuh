@@ -217,7 +217,7 @@ struct RelaxedCapture {
 // Device memory from the library's pool of the given device, stream-ordered (mem.cu).
 int pool_alloc(void** p, size_t bytes, int device, cudaStream_t s);
 void pool_free(void* p, size_t bytes, cudaStream_t s);      // bytes as allocated; p may be null
-int scratch_alloc(void** p, size_t bytes, int device, cudaStream_t s);      // for one call: allocated and freed in stream order
+int scratch_alloc(void** p, size_t bytes, int device, cudaStream_t s, bool optional = false);   // for one call: allocated and freed in stream order
 void scratch_free(void* p, cudaStream_t s);
 int pool_alloc_now(void** p, size_t bytes, int device);     // usable on every stream at once
 // Host -> device copy in stream order; pageable sources are staged by several threads (hostcopy.cu).

@@ -548,7 +548,7 @@ int encode_device(const float* dW, uint32_t m, uint32_t n, cudaStream_t s, spx_e
     // counts, the rows' keys, the pairs, each on a 16-byte boundary
     const size_t keys_at = round_up<size_t>(units * sizeof(uint32_t), 16), kept_at = keys_at + (ranked ? round_up<size_t>(m * sizeof(uint32_t), 16) : 0);
     void* scratch = nullptr;
-    int rc = scratch_alloc(&scratch, kept_at + (keeps ? keep : 0), device, s);
+    int rc = scratch_alloc(&scratch, kept_at + (keeps ? keep : 0), device, s, keeps);
     if (rc == SPX_ERR_OOM && keeps) {           // it goes without
         keeps = false;
         rc = scratch_alloc(&scratch, kept_at, device, s);

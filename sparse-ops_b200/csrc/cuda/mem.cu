@@ -55,7 +55,7 @@ size_t g_pinned_bytes = 0;
 
 }  // namespace
 
-static int allocate(void** p, size_t bytes, int device, cudaStream_t s, bool pooled)
+static int allocate(void** p, size_t bytes, int device, cudaStream_t s, bool pooled, bool trim = true)
 {
     *p = nullptr;
     if (bytes == 0) return SPX_OK;
@@ -63,7 +63,7 @@ static int allocate(void** p, size_t bytes, int device, cudaStream_t s, bool poo
     if (int rc = device_pool(device, &pool)) return rc;
     auto get = [&] { return pooled ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMalloc(p, bytes); };
     cudaError_t err = get();
-    if (err == cudaErrorMemoryAllocation) {
+    if (err == cudaErrorMemoryAllocation && trim) {
         (void)cudaGetLastError();
         pool_trim(device);
         err = get();
@@ -80,7 +80,8 @@ static int allocate(void** p, size_t bytes, int device, cudaStream_t s, bool poo
 int pool_alloc(void** p, size_t bytes, int device, cudaStream_t s) { return allocate(p, bytes, device, s, bytes <= kPoolBlock); }
 
 // Scratch of one call, whatever its size: mapping and freeing memory directly would make the call wait for the device.
-int scratch_alloc(void** p, size_t bytes, int device, cudaStream_t s) { return allocate(p, bytes, device, s, true); }
+// optional: the caller can do without, and is told at once; to give memory back first would wait for the whole device.
+int scratch_alloc(void** p, size_t bytes, int device, cudaStream_t s, bool optional) { return allocate(p, bytes, device, s, true, !optional); }
 void scratch_free(void* p, cudaStream_t s) { if (p) (void)cudaFreeAsync(p, s); }
 
 void pool_free(void* p, size_t bytes, cudaStream_t s)

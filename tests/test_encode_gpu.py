@@ -1,12 +1,17 @@
 """GPU: the device encoder around its limits -- units with as many entries as the counter keeps, one more, full and empty
 ones in one matrix; row counts (and widths) on both sides of what the device ranks; ties -- against the oracle's arrays,
 and a product through the row schedule."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
 
 import spx_ctypes as sx
 from conftest import assert_bit_equal
+from test_conv_tmem_gpu import fill_device, waits_for_the_device
 from test_parity_gpu import dev, gpu_spmm
 
 pytestmark = pytest.mark.gpu
@@ -38,3 +43,32 @@ def test_units_around_what_is_kept(lib, orc, cuda, m, n, offset):
         assert_bit_equal(Wd, E.Wd, "Wd")
     X = rng.uniform(-1, 1, (n, 12)).astype(np.float32)
     assert_bit_equal(gpu_spmm(h, X, None, sx.ACT_NONE, cuda), orc.spmm(E, X, None, act=0), "product")
+
+
+def test_without_room_for_the_pairs(lib, cuda):
+    """Pairs that do not fit (39 MB) are gone without at once: the call waits for its own stream and for no other."""
+    if os.environ.get("SPX_TEST_FULL_DEVICE") != "1":
+        pytest.skip("runs in a child process, whose pool of freed memory is empty")
+    m, n = 9473, 2050
+    W = torch.zeros((m, n), device=cuda)
+    W[:, ::20] = torch.arange(m, device=cuda)[:, None] + 1.0
+    want = [a.copy() for a in lib.ell_encode_device(W[:2].contiguous().data_ptr(), 2, n).download()]
+    assert not waits_for_the_device(lambda: None)           # (makes the stream while there is room)
+    made = []
+    held = fill_device(lib, 24 << 20, 8 << 20)
+    try:
+        for again in (False, True):
+            waited = waits_for_the_device(lambda: made.append(lib.ell_encode_device(W.data_ptr(), m, n)))
+            assert not (again and waited), "an encode waited for another stream's work"
+            Wd, idx, nnz = made[-1].download()
+            assert (nnz == want[2][0]).all() and (idx == want[1][0]).all() and (Wd[1] == want[0][1]).all() and Wd[-1, 0] == m
+            made.pop().close()
+    finally:
+        for p in held:
+            lib.spx_free(p)
+
+
+def test_without_room_for_the_pairs_alone():
+    cmd = [sys.executable, "-m", "pytest", "-q", "-x", "-m", "gpu", "-p", "no:cacheprovider", os.path.abspath(__file__) + "::test_without_room_for_the_pairs"]
+    r = subprocess.run(cmd, env={**os.environ, "SPX_TEST_FULL_DEVICE": "1"}, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and " passed" in r.stdout, r.stdout[-3000:] + r.stderr[-2000:]
