@@ -169,17 +169,26 @@ row_stats_kernel(const uint32_t* __restrict__ counts, uint32_t m, uint32_t segs,
     __shared__ unsigned long long s_sum[32];
     uint32_t hi = 0, lo = 0xffffffffu, n_long = 0;
     unsigned long long sum = 0;
-    constexpr uint32_t U = 8;                               // rows of a thread in flight
-    for (uint32_t i0 = threadIdx.x; i0 < m; i0 += 1024 * U) {
+    // Up to 32 lanes add up a row: a thread each was a chain of loads where rows are few and cut into many segments
+    // (28 rows of 239 segments 61 us more for the call).
+    constexpr uint32_t U = 8;                               // rows of a group of lanes in flight
+    uint32_t lanes = 1;
+    while (lanes < 32 && lanes < segs) lanes *= 2;
+    const uint32_t part = threadIdx.x % lanes, step = 1024 / lanes;
+    for (uint32_t first = 0; first < m; first += step * U) {
+        const uint32_t i0 = first + threadIdx.x / lanes;
         uint32_t len[U] = {};
-        for (uint32_t k = 0; k < segs; ++k)
+        for (uint32_t k = part; k < segs; k += lanes)
 #pragma unroll
             for (uint32_t u = 0; u < U; ++u)
-                if (i0 + 1024 * u < m) len[u] += __ldg(counts + (size_t)(i0 + 1024 * u) * segs + k);
+                if (i0 + step * u < m) len[u] += __ldg(counts + (size_t)(i0 + step * u) * segs + k);
+        for (uint32_t o = lanes / 2; o; o /= 2)
+#pragma unroll
+            for (uint32_t u = 0; u < U; ++u) len[u] += __shfl_xor_sync(0xffffffffu, len[u], o);
 #pragma unroll
         for (uint32_t u = 0; u < U; ++u) {
-            const uint32_t i = i0 + 1024 * u;
-            if (i >= m) break;
+            const uint32_t i = i0 + step * u;
+            if (i >= m || part) break;
             keys[i] = len[u] * kRankRows + (kRankRows - 1 - i);
             hi = max(hi, len[u]);
             lo = min(lo, len[u]);
@@ -437,6 +446,8 @@ constexpr uint32_t kKeepColumns = 2048, kKeepColumnsHostSort = 4096;
 // Without the pairs the packer takes longer and hides the host's sort of more rows: 8192 x 2000 98 us ranked, 109 sorted;
 // 9472 x 3000 140 and 139; 16384 x 1000 140 and 129.
 constexpr uint32_t kRankRowsReread = 8192;
+// A handful of rows is sorted by the host in less time than a kernel for it takes (4 x 4 38 us sorted, 41 ranked; 7 x 13 41 and 41).
+constexpr uint32_t kRankFrom = 8;
 
 // Device memory of one call beside the handle's own.
 struct EncodeScratch {
@@ -542,7 +553,7 @@ int encode_device(const float* dW, uint32_t m, uint32_t n, cudaStream_t s, spx_e
     const size_t keep = units * sc.cap * sizeof(uint2);
     bool keeps = sp.seg >= kKeepColumns && (m <= kRankRows || sp.seg >= kKeepColumnsHostSort) &&
                  (size_t)m * n * sizeof(float) >= kKeepFrom && keep <= kKeepBytes;
-    const bool ranked = m <= (keeps ? kRankRows : kRankRowsReread) && n < kRankColumns;
+    const bool ranked = m >= kRankFrom && m <= (keeps ? kRankRows : kRankRowsReread) && n < kRankColumns;
     PinnedBlock stage;
     if (int rc = pinned_acquire(ranked ? sizeof(RowStats) : (units + 1) * sizeof(uint32_t) + m * sizeof(uint2), &stage)) return rc;
     // counts, the rows' keys, the pairs, each on a 16-byte boundary
