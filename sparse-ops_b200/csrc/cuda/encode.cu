@@ -156,7 +156,7 @@ count_keep_kernel(const float* __restrict__ W, uint32_t mis, uint32_t m, uint32_
 // What the host has to know before the arrays can be allocated, where the device makes the row schedule (up to kRankRows
 // rows of less than kRankColumns): one CTA adds up the rows' segments and leaves the result in page-locked memory, where
 // the host finds it after one wait (instead of a copy of all counts and three loops over them).
-constexpr uint32_t kRankRows = 16384, kRankColumns = 1u << 18;
+constexpr uint32_t kRankRows = 15104, kRankColumns = 1u << 18;
 struct RowStats {
     uint64_t total;
     uint32_t longest, shortest, long_rows, pad;
@@ -438,11 +438,13 @@ namespace spx {
 
 // Pairs kept by the counter: a quarter of a unit's columns (denser units are read again, which is then no more to move
 // than pairs would be), and no more scratch than the pool keeps for the next call in any case.  A matrix that stays in L2
-// is read again for less than the pairs cost, short units end in blocks of 512 columns that are mostly empty, and beyond
-// kRankRows rows the host's sort shows that the packer hid (10 % dense, with and without the pairs: 5000 x 5000 110 and
-// 124 us, 14000 x 3000 161 and 183, 10000 x 10000 269 and 326; 3000 x 3000 73.5 and 71.5, 30000 x 1500 229 and 223).
+// is read again for less than the pairs cost, and short units end in blocks of 512 columns that are mostly empty.  With
+// many rows the schedule costs more (m comparisons a row on the device) or shows, where the host's sort no longer hides
+// behind the packer: rows have to be longer then (5 %, with and without the pairs: 5000 x 5000 110 and 124 us, 3000 x 3000
+// 73.5 and 71.5; 10000 x 2100 97 and 95, 14000 x 4096 133 and 140, x 8000 178 and 223; sorted by the host 16000 x 4096 161
+// and 148, x 6000 183 and 195).
 constexpr size_t kKeepBytes = 256u << 20, kKeepFrom = 64u << 20;
-constexpr uint32_t kKeepColumns = 2048, kKeepColumnsHostSort = 4096;
+constexpr uint32_t kKeepColumns = 2048, kKeepColumnsRanked = 4096, kKeepColumnsHostSort = 4608;
 // Without the pairs the packer takes longer and hides the host's sort of more rows: 8192 x 2000 98 us ranked, 109 sorted;
 // 9472 x 3000 140 and 139; 16384 x 1000 140 and 129.
 constexpr uint32_t kRankRowsReread = 8192;
@@ -551,7 +553,7 @@ int encode_device(const float* dW, uint32_t m, uint32_t n, cudaStream_t s, spx_e
     EncodeScratch sc;
     sc.cap = sp.seg / 4;
     const size_t keep = units * sc.cap * sizeof(uint2);
-    bool keeps = sp.seg >= kKeepColumns && (m <= kRankRows || sp.seg >= kKeepColumnsHostSort) &&
+    bool keeps = sp.seg >= (m <= kRankRowsReread ? kKeepColumns : m <= kRankRows ? kKeepColumnsRanked : kKeepColumnsHostSort) &&
                  (size_t)m * n * sizeof(float) >= kKeepFrom && keep <= kKeepBytes;
     const bool ranked = m >= kRankFrom && m <= (keeps ? kRankRows : kRankRowsReread) && n < kRankColumns;
     PinnedBlock stage;

@@ -17,7 +17,7 @@ from test_parity_gpu import dev, gpu_spmm
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("m,n", [(1, 3), (5, 4096), (300, 2050), (1200, 512), (8192, 40), (8193, 40), (4099, 4100), (9473, 2050), (16385, 2050),
+@pytest.mark.parametrize("m,n", [(1, 3), (5, 4096), (300, 2050), (1200, 512), (8192, 40), (8193, 40), (4099, 4100), (4800, 4100), (9473, 2050), (16385, 2050),
                                  (3, 300000), (7, 5000), (8, 5000), (9, 262143), (28, 131000), (1300, 7000)])
 @pytest.mark.parametrize("offset", [0, 1])
 def test_units_around_what_is_kept(lib, orc, cuda, m, n, offset):
@@ -45,11 +45,39 @@ def test_units_around_what_is_kept(lib, orc, cuda, m, n, offset):
     assert_bit_equal(gpu_spmm(h, X, None, sx.ACT_NONE, cuda), orc.spmm(E, X, None, act=0), "product")
 
 
+@pytest.mark.parametrize("m,n", [(4800, 4100), (4799, 4101), (9000, 2048), (15104, 4096), (15105, 4096), (15105, 4608)])
+def test_large_matrices(lib, cuda, m, n):
+    """Rows in one and two segments, ranked and sorted by the host, with pairs and without, some too dense for them: the
+    arrays against the same ones made with torch, and the schedule by a product of small whole numbers, which is exact."""
+    g = torch.Generator(device=cuda).manual_seed(m + n)
+    share = torch.tensor([0.0, 0.02, 0.1, 0.1, 0.24, 0.3], device=cuda)[torch.randint(0, 6, (m, 1), device=cuda, generator=g)]
+    share = share.repeat(1, n)
+    share[::7, n // 2:] = 0.4                               # rows whose second half is too dense
+    W = torch.randint(1, 9, (m, n), device=cuda, generator=g).float()
+    W[torch.rand((m, n), device=cuda, generator=g) >= share] = 0
+    del share
+    h = lib.ell_encode_device(W.data_ptr(), m, n)
+    Wd, idx, nnz = (torch.from_numpy(a.view(np.int32)).to(cuda) for a in h.download())
+    cnt = (W != 0).sum(1)
+    assert torch.equal(nnz.long(), cnt) and h.r == int(cnt.max()) and h.nnz_total == int(cnt.sum())
+    rows, cols = W.nonzero(as_tuple=True)
+    place = torch.arange(len(rows), device=cuda) - (torch.cumsum(cnt, 0) - cnt)[rows]
+    want = torch.zeros((m, h.r), dtype=torch.int32, device=cuda)
+    want[rows, place] = cols.int()
+    assert torch.equal(idx.view(m, h.r), want)
+    want[rows, place] = W[rows, cols].view(torch.int32)
+    assert torch.equal(Wd.view(m, h.r), want)
+    X = torch.randint(-4, 5, (n, 4), device=cuda, generator=g).float()
+    Y = torch.full((m, 4), float("nan"), device=cuda)
+    h.spmm(X.data_ptr(), 4, 4, 0, sx.ACT_NONE, Y.data_ptr(), 4)
+    assert torch.equal(Y.double(), W.double() @ X.double())
+
+
 def test_without_room_for_the_pairs(lib, cuda):
     """Pairs that do not fit (39 MB) are gone without at once: the call waits for its own stream and for no other."""
     if os.environ.get("SPX_TEST_FULL_DEVICE") != "1":
         pytest.skip("runs in a child process, whose pool of freed memory is empty")
-    m, n = 9473, 2050
+    m, n = 4800, 4100
     W = torch.zeros((m, n), device=cuda)
     W[:, ::20] = torch.arange(m, device=cuda)[:, None] + 1.0
     want = [a.copy() for a in lib.ell_encode_device(W[:2].contiguous().data_ptr(), 2, n).download()]
