@@ -107,6 +107,14 @@ count_kernel(const float* __restrict__ W, uint32_t mis, uint32_t m, uint32_t n, 
 // byte-sized counts per lane gives all places) and leaves it in whole 8-byte rows of 32 lanes.  W is read with an
 // evict-first hint, so that the pairs are still in L2 when pack_kernel fetches them.
 // 8192 x 8192, 10 %: 58 us (count_kernel 53), and pack_kernel 29 instead of 67.
+// A unit is given up where more than 17/64 of the columns seen so far (and 16) are entries: the pairs written until then
+// are in vain.  It is marked in its first pair.  (Writing them up to a capacity of a quarter cost units that are denser 8
+// to 12 %: 151 x 264025, 30 % 165 us, now 146, 143 without pairs.  A unit that is dense at its front only is read twice,
+// as without pairs.)
+constexpr uint32_t kNotKept = 0xffffffffu;                  // no column: n is at most this
+constexpr uint32_t kKeepSlack = 16;
+__host__ __device__ constexpr uint32_t keep_cap(uint32_t columns) { return columns / 64 * 17 + kKeepSlack; }
+
 __global__ void __launch_bounds__(kWarps * 32)
 count_keep_kernel(const float* __restrict__ W, uint32_t mis, uint32_t m, uint32_t n, uint32_t segs, uint32_t seg, uint32_t cap,
                   uint32_t* __restrict__ counts, uint2* __restrict__ kept)
@@ -119,7 +127,9 @@ count_keep_kernel(const float* __restrict__ W, uint32_t mis, uint32_t m, uint32_
     const Segment s = segment_of(unit, mis, n, segs, seg);
     uint2* __restrict__ dst = kept + unit * cap;
     uint32_t pos = 0;
-    for (uint32_t qb = 0; qb < s.quads; qb += 32 * kQuads) {
+    uint32_t qb = 0, most = kKeepSlack;
+    bool keep = true;
+    for (; keep && qb < s.quads; qb += 32 * kQuads) {
         float4 v[kQuads];
         load_block<true>(v, W, s, qb, lane);
         uint32_t own = 0;                                   // byte u: entries of this lane's quad u
@@ -145,10 +155,24 @@ count_keep_kernel(const float* __restrict__ W, uint32_t mis, uint32_t m, uint32_
             base += (all >> (8 * u)) & 255u;
         }
         __syncwarp();
-        if (pos + base <= cap)                              // else the unit will be read again
+        most = min(most + 34 * kQuads, cap);                // the next block's share
+        keep = pos + base <= most;
+        if (keep)
             for (uint32_t j = lane; j < base; j += 32) dst[pos + j] = strip[j];
         pos += base;
         __syncwarp();
+    }
+    if (!keep) {
+        uint32_t cnt = 0;
+        for (; qb < s.quads; qb += 32 * kQuads) {
+            float4 v[kQuads];
+            load_block<false>(v, W, s, qb, lane);           // pack_kernel reads it again
+#pragma unroll
+            for (int u = 0; u < kQuads; ++u)
+                cnt += (v[u].x != 0.0f) + (v[u].y != 0.0f) + (v[u].z != 0.0f) + (v[u].w != 0.0f);
+        }
+        pos += __reduce_add_sync(0xffffffffu, cnt);
+        if (lane == 0) dst[0].y = kNotKept;                 // (a first pair was lane 0's store, too)
     }
     if (lane == 0) counts[unit] = pos;
 }
@@ -238,8 +262,8 @@ __device__ __forceinline__ void rank_rows(uint32_t cta, const uint32_t* __restri
     if (part == 0 && i < m) rows[rank] = make_uint2(i, key / kRankRows);
 }
 
-// Entries into their rows: from the pairs that the counter kept, or, where a unit had more of them than fit (or none were
-// kept), out of the matrix again.  Unit u of the grid is the matrix's unit (last - u): the counter has just read the end
+// Entries into their rows: from the pairs that the counter kept, or, where it gave the unit up (or kept none at all), out
+// of the matrix again.  Unit u of the grid is the matrix's unit (last - u): the counter has just read the end
 // of W.  The first rank_ctas CTAs make the row schedule.
 __global__ void __launch_bounds__(kWarps * 32)
 pack_kernel(const float* __restrict__ W, uint32_t mis, uint32_t m, uint32_t n, uint32_t segs, uint32_t seg,
@@ -267,8 +291,8 @@ pack_kernel(const float* __restrict__ W, uint32_t mis, uint32_t m, uint32_t n, u
         pos = __reduce_add_sync(0xffffffffu, pos);
     }
     const uint32_t mine = kept ? __ldg(counts + unit) : 0u;
-    if (kept && mine <= cap) {
-        const uint2* __restrict__ src = kept + unit * cap;
+    const uint2* __restrict__ src = kept + unit * cap;
+    if (kept && (mine == 0 || __ldg(&src->y) != kNotKept)) {
         constexpr uint32_t kRun = 4;                        // pairs per lane in flight
         for (uint32_t j0 = lane; j0 < mine; j0 += 32 * kRun) {
             uint2 p[kRun];
@@ -436,14 +460,14 @@ inline uint32_t misalignment(const float* p) { return (uint32_t)((reinterpret_ca
 
 namespace spx {
 
-// Pairs kept by the counter: a quarter of a unit's columns (denser units are read again, which is then no more to move
-// than pairs would be), and no more scratch than the pool keeps for the next call in any case.  A matrix that stays in L2
-// is read again for less than the pairs cost, and short units end in blocks of 512 columns that are mostly empty.  With
+// Pairs kept by the counter: some more than a quarter of a unit's columns (denser units are read again, which is then no
+// more to move than pairs would be), and no more scratch than the pool keeps for the next call in any case.  A matrix that
+// stays in L2 is read again for less than the pairs cost, short units end in blocks of 512 columns that are mostly empty.  With
 // many rows the schedule costs more (m comparisons a row on the device) or shows, where the host's sort no longer hides
 // behind the packer: rows have to be longer then (5 %, with and without the pairs: 5000 x 5000 110 and 124 us, 3000 x 3000
 // 73.5 and 71.5; 10000 x 2100 97 and 95, 14000 x 4096 133 and 140, x 8000 178 and 223; sorted by the host 16000 x 4096 161
 // and 148, x 6000 183 and 195).
-constexpr size_t kKeepBytes = 256u << 20, kKeepFrom = 64u << 20;
+constexpr size_t kKeepBytes = 288u << 20, kKeepFrom = 64u << 20;
 constexpr uint32_t kKeepColumns = 2048, kKeepColumnsRanked = 4096, kKeepColumnsHostSort = 4608;
 // Without the pairs the packer takes longer and hides the host's sort of more rows: 8192 x 2000 98 us ranked, 109 sorted;
 // 9472 x 3000 140 and 139; 16384 x 1000 140 and 129.
@@ -551,7 +575,7 @@ int encode_device(const float* dW, uint32_t m, uint32_t n, cudaStream_t s, spx_e
     const Split sp = split_rows(m, n, sm_count(device));
     const size_t units = (size_t)m * sp.segs;
     EncodeScratch sc;
-    sc.cap = sp.seg / 4;
+    sc.cap = keep_cap(sp.seg);
     const size_t keep = units * sc.cap * sizeof(uint2);
     bool keeps = sp.seg >= (m <= kRankRowsReread ? kKeepColumns : m <= kRankRows ? kKeepColumnsRanked : kKeepColumnsHostSort) &&
                  (size_t)m * n * sizeof(float) >= kKeepFrom && keep <= kKeepBytes;

@@ -28,9 +28,11 @@ def test_units_around_what_is_kept(lib, orc, cuda, m, n, offset):
     W = np.zeros((m, n), np.float32)
     for lo in range(0, n, seg):
         w = min(seg, n - lo)
-        cap = seg // 4
+        cap = seg // 64 * 17 + 16
         lens = rng.choice([0, 1, min(w, cap), min(w, cap + 1), w // 10, w], m, p=[.1, .1, .3, .2, .2, .1])
         order = np.argsort(rng.random((m, w), dtype=np.float32), axis=1)
+        order[::3] = np.arange(w)[::-1]                             # at the end: kept up to the last place
+        order[1::6] = np.arange(w)                                  # at the front: given up where they are many
         W[:, lo:lo + w][order < lens[:, None]] = 1
     W *= rng.standard_normal((m, n), dtype=np.float32)
     flat = torch.zeros(m * n + 1, device=cuda)
