@@ -186,6 +186,9 @@ struct RowStats {
     uint32_t longest, shortest, long_rows, pad;
 };
 
+// A thread adds up a row, or a warp does, where rows come in many segments (16 and more, of at most some 600 rows then: as
+// a chain of loads they cost 28 x 247446 48 us more; as warps, 8192 rows of 2 segments 2 us more).
+template <bool WARPS>
 __global__ void __launch_bounds__(1024)
 row_stats_kernel(const uint32_t* __restrict__ counts, uint32_t m, uint32_t segs, uint32_t* __restrict__ keys, RowStats* __restrict__ out)
 {
@@ -193,11 +196,7 @@ row_stats_kernel(const uint32_t* __restrict__ counts, uint32_t m, uint32_t segs,
     __shared__ unsigned long long s_sum[32];
     uint32_t hi = 0, lo = 0xffffffffu, n_long = 0;
     unsigned long long sum = 0;
-    // Up to 32 lanes add up a row: a thread each was a chain of loads where rows are few and cut into many segments
-    // (28 rows of 239 segments 61 us more for the call).
-    constexpr uint32_t U = 8;                               // rows of a group of lanes in flight
-    uint32_t lanes = 1;
-    while (lanes < 32 && lanes < segs) lanes *= 2;
+    constexpr uint32_t U = 8, lanes = WARPS ? 32 : 1;       // rows of a group of lanes in flight
     const uint32_t part = threadIdx.x % lanes, step = 1024 / lanes;
     for (uint32_t first = 0; first < m; first += step * U) {
         const uint32_t i0 = first + threadIdx.x / lanes;
@@ -472,8 +471,9 @@ constexpr uint32_t kKeepColumns = 2048, kKeepColumnsRanked = 4096, kKeepColumnsH
 // Without the pairs the packer takes longer and hides the host's sort of more rows: 8192 x 2000 98 us ranked, 109 sorted;
 // 9472 x 3000 140 and 139; 16384 x 1000 140 and 129.
 constexpr uint32_t kRankRowsReread = 8192;
-// A handful of rows is sorted by the host in less time than a kernel for it takes (4 x 4 38 us sorted, 41 ranked; 7 x 13 41 and 41).
-constexpr uint32_t kRankFrom = 8;
+// A handful of short rows is sorted by the host in less time than a kernel for it takes (4 x 4 38 us sorted, 41 ranked; 7 x 13
+// 41 and 41); of long ones not, whose lengths it counts one by one (2 x 255065, 78 % 113 us sorted, 80 ranked).
+constexpr uint32_t kRankFrom = 8, kRankLong = 8192;
 
 // Device memory of one call beside the handle's own.
 struct EncodeScratch {
@@ -499,7 +499,8 @@ static int encode_rows(const float* dW, uint32_t m, uint32_t n, int device, cuda
     if (ranked) {
         void* stats = nullptr;
         SPX_CUDA(cudaHostGetDevicePointer(&stats, stage.host, 0));
-        row_stats_kernel<<<1, 1024, 0, s>>>(sc.counts, m, sp.segs, sc.keys, static_cast<RowStats*>(stats));
+        const auto kernel = sp.segs >= 16 ? row_stats_kernel<true> : row_stats_kernel<false>;
+        kernel<<<1, 1024, 0, s>>>(sc.counts, m, sp.segs, sc.keys, static_cast<RowStats*>(stats));
         SPX_LAUNCH_CHECK("row_stats_kernel");
     } else {
         SPX_CUDA(cudaMemcpyAsync(h_counts, sc.counts, units * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
@@ -579,7 +580,7 @@ int encode_device(const float* dW, uint32_t m, uint32_t n, cudaStream_t s, spx_e
     const size_t keep = units * sc.cap * sizeof(uint2);
     bool keeps = sp.seg >= (m <= kRankRowsReread ? kKeepColumns : m <= kRankRows ? kKeepColumnsRanked : kKeepColumnsHostSort) &&
                  (size_t)m * n * sizeof(float) >= kKeepFrom && keep <= kKeepBytes;
-    const bool ranked = m >= kRankFrom && m <= (keeps ? kRankRows : kRankRowsReread) && n < kRankColumns;
+    const bool ranked = (m >= kRankFrom || n >= kRankLong) && m <= (keeps ? kRankRows : kRankRowsReread) && n < kRankColumns;
     PinnedBlock stage;
     if (int rc = pinned_acquire(ranked ? sizeof(RowStats) : (units + 1) * sizeof(uint32_t) + m * sizeof(uint2), &stage)) return rc;
     // counts, the rows' keys, the pairs, each on a 16-byte boundary

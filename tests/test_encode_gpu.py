@@ -18,7 +18,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("m,n", [(1, 3), (5, 4096), (300, 2050), (1200, 512), (8192, 40), (8193, 40), (4099, 4100), (4800, 4100), (9473, 2050), (16385, 2050),
-                                 (3, 300000), (7, 5000), (8, 5000), (9, 262143), (28, 131000), (1300, 7000)])
+                                 (3, 300000), (7, 5000), (8, 5000), (2, 8191), (2, 8192), (900, 9000), (9, 262143), (28, 131000), (1300, 7000)])
 @pytest.mark.parametrize("offset", [0, 1])
 def test_units_around_what_is_kept(lib, orc, cuda, m, n, offset):
     rng = np.random.default_rng([m, n])
