@@ -18,9 +18,16 @@ struct ConvViews {
     uint32_t vec_out;
 };
 
-// conv_tmem.cu: -1 when the shape or the handle is not for this kernel, or the other one's expected time is not above its own.
+// How a handle's entries lie in the merged kernel's CTAs (of 16, 8 or 4 row blocks): the union columns of the CTA's longest
+// block and its work, 0.7 a union column and 0.2 an entry; on average and in the worst CTA.
+struct MergedLoad {
+    double longest = 0.0, work = 0.0, longest_worst = 0.0, work_worst = 0.0;
+};
+
+// conv_tmem.cu: -1 when the shape or the handle is not for this kernel, or the other one's expected time is not above its own
+// (load: for 16, 8 and 4 blocks; null: by the density).
 int launch_conv_tmem(spx_ell* e, const ConvParams& p, const ConvViews& v, const float* in, const float* bias, int act, float* out,
-                     double (*other_us)(const spx_ell*, const ConvParams&), cudaStream_t s);
+                     double (*other_us)(const spx_ell*, const ConvParams&, const MergedLoad* load), cudaStream_t s);
 // conv.cu: the merged weights of conv_rbm_tile_kernel; -1 where there is no memory for them.
 int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s);
 void* new_conv_tmem();

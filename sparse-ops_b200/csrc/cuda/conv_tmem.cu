@@ -68,10 +68,10 @@ __device__ __forceinline__ uint32_t lower_bound(const uint32_t* __restrict__ k, 
     return lo;
 }
 
-// One CTA per block.  Shared memory: [chunks + 1][4] run starts, [chunks] first unit of each chunk.
+// One CTA per block; entries: [block][chunk] how many.  Shared memory: [chunks + 1][4] run starts, [chunks] first unit of each chunk.
 __global__ void __launch_bounds__(256)
 conv_form_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ idx, const uint32_t* __restrict__ nnz, uint32_t m, uint32_t pitch,
-                 FormShape f, uint32_t chunks, uint32_t cap, uint4* __restrict__ units)
+                 FormShape f, uint32_t chunks, uint32_t cap, uint4* __restrict__ units, uint32_t* __restrict__ entries)
 {
     extern __shared__ uint32_t s_form[];
     __shared__ uint32_t total;
@@ -114,8 +114,12 @@ conv_form_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ idx,
     uint4* __restrict__ dst = units + (size_t)blockIdx.x * cap;
     auto end = [&](uint32_t i) { return i < chunks ? first[i] : total; };
     for (uint32_t c = threadIdx.x; c < chunks; c += blockDim.x) {
-        uint32_t counts = 0;
-        for (uint32_t r = 0; r < kRows; ++r) counts |= count(c, r) << (8 * r);
+        uint32_t counts = 0, all = 0;
+        for (uint32_t r = 0; r < kRows; ++r) {
+            counts |= count(c, r) << (8 * r);
+            all += count(c, r);
+        }
+        if (entries) entries[(size_t)blockIdx.x * chunks + c] = all;
         dst[first[c]] = make_uint4(counts, end(c + 1) - end(c), end(min(c + 2, chunks)) - end(c + 1), 0u);
     }
     const uint32_t taps = f.kH * f.kW;
@@ -130,6 +134,67 @@ conv_form_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ idx,
             const uint32_t col = c % kBuffers * f.chunk_cols + ((cin - c * f.CC) * f.THin + kh * f.dH) * f.TWin + kw * f.dW;
             reinterpret_cast<uint2*>(dst + at + place / 2)[place & 1u] = make_uint2(__float_as_uint(Wd[base + j]), col);
         }
+    }
+}
+
+// Clocks that a chunk takes a CTA: the larger of what its busiest quadrant multiplies (an entry of a warp, a block's four
+// runs) or the latency of the longest block's own, and what its fillers copy (a column; the lane groups of a warp read
+// the same banks), and their fixed costs.
+constexpr float kEntryClocks = 23.5f, kRunClocks = 115.0f, kEntryLatency = 60.0f, kRunLatency = 150.0f, kChunkLatency = 300.0f;
+constexpr float kCtaClocks = 9650.0f;
+__host__ __device__ inline float fill_clocks(uint32_t chunk_cols, uint32_t S)
+{
+    const float groups = 4.4f * S;
+    return chunk_cols * (groups > 7.7f ? groups : 7.7f) + 690.0f;
+}
+constexpr int kLaneGroups = 4;                  // S = 1, 2, 4, 8
+struct CtaClocks {
+    float c[2][kLaneGroups];                    // whole CTAs and halves; by S
+};
+
+// The clocks of a CTA of each group of `per_group` blocks, summed over its own chunks' entries, and per block the union
+// columns and the entries.
+__global__ void __launch_bounds__(128)
+conv_load_kernel(const uint32_t* __restrict__ entries, const uint32_t* __restrict__ union_cols, const uint32_t* __restrict__ nnz, uint32_t m,
+                 uint32_t chunks, uint32_t per_group, uint32_t chunk_cols, CtaClocks* __restrict__ ctas, uint2* __restrict__ blocks)
+{
+    __shared__ float s_part[4][2 * kLaneGroups];
+    const uint32_t nblocks = (m + kRows - 1) / kRows, b0 = blockIdx.x * per_group, nq = per_group / 4;
+    if (threadIdx.x < per_group && b0 + threadIdx.x < nblocks) {
+        const uint32_t b = b0 + threadIdx.x;
+        uint32_t all = 0;
+        for (uint32_t r = b * kRows; r < min(m, (b + 1) * kRows); ++r) all += nnz[r];
+        blocks[b] = make_uint2(union_cols[b], all);
+    }
+    float sum[2 * kLaneGroups] = {};
+    for (uint32_t c = threadIdx.x; c < chunks; c += 128) {
+        float mul = 0.0f;
+        for (uint32_t q = 0; q < nq; ++q) {     // blocks q, q + nq, ... share a quadrant
+            float quad = 0.0f;
+            for (uint32_t b = b0 + q; b < min(nblocks, b0 + per_group); b += nq) {
+                const float n = (float)entries[(size_t)b * chunks + c];
+                quad += kEntryClocks * n + kRows * kRunClocks;
+                mul = fmaxf(mul, kEntryLatency * n + kRows * kRunLatency + kChunkLatency);
+            }
+            mul = fmaxf(mul, quad);
+        }
+#pragma unroll
+        for (int i = 0; i < kLaneGroups; ++i) {
+            const float fill = fill_clocks(chunk_cols, 1u << i);
+            sum[i] += fmaxf(mul, fill);
+            sum[kLaneGroups + i] += fmaxf(mul / 2, fill);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 2 * kLaneGroups; ++i) {
+#pragma unroll
+        for (int o = 16; o; o >>= 1) sum[i] += __shfl_down_sync(0xffffffffu, sum[i], o);
+        if (threadIdx.x % 32 == 0) s_part[threadIdx.x / 32][i] = sum[i];
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 * kLaneGroups) {
+        const uint32_t i = threadIdx.x;
+        ctas[blockIdx.x].c[i / kLaneGroups][i % kLaneGroups] = kCtaClocks + s_part[0][i] + s_part[1][i] + s_part[2][i] + s_part[3][i];
     }
 }
 
@@ -437,6 +502,10 @@ struct conv_tmem_impl {
         uint4* units = nullptr;
         size_t bytes = 0;
         uint32_t cap = 0;
+        // what the CTAs' own entries are expected to take, here and in the merged kernel; not known without memory to find out
+        bool loads = false;
+        CtaClocks mean{}, worst{};
+        MergedLoad merged[3];                   // CTAs of 16, 8 and 4 blocks
     };
     std::mutex mu;
     int count = 0;
@@ -455,9 +524,42 @@ void free_conv_tmem(spx_ell* e)
     e->conv_tmem = nullptr;
 }
 
+static void read_loads(conv_tmem_impl::Form& form, const CtaClocks* ctas, uint32_t groups, uint32_t nblocks)
+{
+    for (int h = 0; h < 2; ++h)
+        for (int i = 0; i < kLaneGroups; ++i) {
+            double sum = 0.0;
+            for (uint32_t g = 0; g < groups; ++g) {
+                sum += ctas[g].c[h][i];
+                form.worst.c[h][i] = std::max(form.worst.c[h][i], ctas[g].c[h][i]);
+            }
+            form.mean.c[h][i] = (float)(sum / groups);
+        }
+    const uint2* blocks = reinterpret_cast<const uint2*>(ctas + groups);
+    for (int k = 0; k < 3; ++k) {
+        const uint32_t nb = 16u >> k;
+        MergedLoad& l = form.merged[k];
+        for (uint32_t b0 = 0; b0 < nblocks; b0 += nb) {
+            double longest = 0.0, work = 0.0;
+            for (uint32_t b = b0; b < std::min(nblocks, b0 + nb); ++b) {
+                longest = std::max<double>(longest, blocks[b].x);
+                work += 0.7 * blocks[b].x + 0.2 * blocks[b].y;
+            }
+            l.longest += longest;
+            l.work += work;
+            l.longest_worst = std::max(l.longest_worst, longest);
+            l.work_worst = std::max(l.work_worst, work);
+        }
+        const uint32_t n = (nblocks + nb - 1) / nb;
+        l.longest /= n;
+        l.work /= n;
+    }
+    form.loads = true;
+}
+
 // The form for a shape, built where it is not there yet (the call then waits for its stream, so that every stream may
 // use the form).  -1: it cannot be (no memory, too many shapes, or a graph is being captured).
-static int find_form(spx_ell* e, const FormShape& f, uint32_t chunks, cudaStream_t s, const conv_tmem_impl::Form** out)
+static int find_form(spx_ell* e, const FormShape& f, uint32_t chunks, uint32_t per_group, cudaStream_t s, const conv_tmem_impl::Form** out)
 {
     conv_tmem_impl* t = static_cast<conv_tmem_impl*>(e->conv_tmem);
     std::lock_guard<std::mutex> lk(t->mu);
@@ -471,7 +573,8 @@ static int find_form(spx_ell* e, const FormShape& f, uint32_t chunks, cudaStream
     }
     RelaxedCapture relaxed;                     // s is not being captured; another stream may be, by this thread
     // A later call that is recorded may take the other kernel (another batch, say), and cannot build what that needs then.
-    if (const int rc = ensure_rbm(e, f.kH, f.kW, s); rc > 0) return rc;
+    const int merged = ensure_rbm(e, f.kH, f.kW, s);
+    if (merged > 0) return merged;
     ensure_tma_words(e);
     if (!e->tma_failed_dev || !e->tma_failed_mapped) {
         t->no_memory = true;
@@ -492,12 +595,30 @@ static int find_form(spx_ell* e, const FormShape& f, uint32_t chunks, cudaStream
         return -1;
     }
     form.units = static_cast<uint4*>(units);
+    // the loads' intermediate counts, and where the host finds them
+    const uint32_t groups = (blocks + per_group - 1) / per_group;
+    const size_t entries_bytes = (size_t)blocks * chunks * 4;
+    void *entries = nullptr, *found = nullptr;
+    PinnedBlock host;
+    bool loads = merged == SPX_OK && pinned_acquire(groups * sizeof(CtaClocks) + blocks * sizeof(uint2), &host) == SPX_OK &&
+                 cudaHostGetDevicePointer(&found, host.host, 0) == cudaSuccess &&
+                 scratch_alloc(&entries, entries_bytes, e->device, s, true) == SPX_OK;
+    if (!loads) (void)cudaGetLastError();
     const size_t smem = (size_t)((chunks + 1) * kRows + chunks) * 4;
-    conv_form_kernel<<<blocks, 256, smem, s>>>(e->Wd, e->idx, e->nnz, e->m, e->pitch, f, chunks, form.cap, form.units);
+    conv_form_kernel<<<blocks, 256, smem, s>>>(e->Wd, e->idx, e->nnz, e->m, e->pitch, f, chunks, form.cap, form.units, static_cast<uint32_t*>(entries));
     cudaError_t err = cudaGetLastError();
     if (err == cudaSuccess) count_launch();
+    if (err == cudaSuccess && loads) {
+        conv_load_kernel<<<groups, 128, 0, s>>>(static_cast<uint32_t*>(entries), e->rbm_ncols, e->nnz, e->m, chunks, per_group, f.chunk_cols,
+                                                static_cast<CtaClocks*>(found), reinterpret_cast<uint2*>(static_cast<CtaClocks*>(found) + groups));
+        err = cudaGetLastError();
+        if (err == cudaSuccess) count_launch();
+    }
+    scratch_free(entries, s);
     const cudaError_t done = cudaStreamSynchronize(s);
     if (err == cudaSuccess) err = done;
+    if (err == cudaSuccess && loads) read_loads(form, static_cast<const CtaClocks*>(host.host), groups, blocks);
+    pinned_release(host);
     if (err != cudaSuccess) {
         pool_free(form.units, form.bytes, s);
         return fail(SPX_ERR_CUDA, "conv2d: building the entries' form failed: %s", cudaGetErrorString(err));
@@ -573,15 +694,11 @@ Tail tail_of(uint64_t units, uint32_t sms)
 
 }  // namespace
 
-// Expected time.  Per chunk of a CTA the larger of what its busiest quadrant multiplies (23.5 clocks an entry, and 115 for
-// each row's run) or the latency of a warp's own runs, and what its fillers copy (7.7 clocks a column, and 690; the lane
-// groups of a warp read the same banks, 4.4 clocks for each); 9650 clocks per CTA; results that are not contiguous along
-// the batch by the million, in quads or one by one.  Fitted with conv_rbm_us to 400 shapes of both kernels (3 to 512
-// channels, 3 x 3 and 5 x 5, 7 x 7 to 112 x 112, batch 1 to 32, 5 to 50 % dense, all layouts): taken where it is below 0.92 of
-// that (a launch on less than half of the SMs counted 15 % longer: the other kernel cuts finer, and 453 -> 54 channels, 5 x 5,
-// 32 x 32, batch 16 was 7 % slower here; 0.85 for batches that leave lanes to a second tile, not for few output channels with a batch that is no multiple
-// of 16), it was the faster one every time, some 115 times; picking the faster each time would gain another 1.2 % on average.
-static double conv_tmem_us(const spx_ell* e, const ConvParams& p, const ConvViews& v)
+// Expected time, by the density alone (iid entries) or, where a form is there, by its loads: waves of CTAs, and results
+// that are not contiguous along the batch by the million, in quads or one by one.  Launches on less than half of the SMs
+// count 15 % longer: the other kernel cuts finer.  Fitted with conv_rbm_us to 400 shapes of both kernels (3 to 512
+// channels, 3 x 3 and 5 x 5, 7 x 7 to 112 x 112, batch 1 to 32, 5 to 50 % dense, all layouts).
+static double conv_tmem_us(const spx_ell* e, const ConvParams& p, const ConvViews& v, const conv_tmem_impl::Form* form)
 {
     const uint32_t sms = (uint32_t)sm_count(e->device);
     const double density = (double)e->nnz_total / ((double)e->m * e->n);
@@ -590,18 +707,37 @@ static double conv_tmem_us(const spx_ell* e, const ConvParams& p, const ConvView
         Cut c;
         if (!plan(p, BT, len, c)) return -1;
         const double run = c.CC * p.kH * p.kW * density;
-        const auto cta = [&](double rows) {
-            const double quad = std::min(16.0, (p.Cout + kRows - 1) / kRows * c.QT * (kRows / rows)) / 4.0;
-            const double mul = std::max(quad * rows * (23.5 * run + 115.0), rows * (60.0 * run + 150.0) + 300.0);
-            return 9650.0 + c.chunks * std::max(mul, c.chunk_cols * std::max(7.7, 4.4 * c.S) + 690.0);
+        const int si = c.S == 1 ? 0 : c.S == 2 ? 1 : c.S == 4 ? 2 : 3;
+        const auto cta = [&](uint32_t rows) -> double {
+            if (form) return form->mean.c[rows < kRows][si];
+            const double quad = std::min<double>(16.0, (p.Cout + kRows - 1) / kRows * c.QT * (kRows / rows)) / 4.0;
+            const double mul = std::max(quad * rows * (kEntryClocks * run + kRunClocks), rows * (kEntryLatency * run + kRunLatency) + kChunkLatency);
+            return kCtaClocks + c.chunks * std::max<double>(mul, fill_clocks(c.chunk_cols, c.S));
         };
         const Tail t = tail_of(c.units, sms);
         const double full = std::floor((double)c.units / sms), rem = (double)(c.units % sms);
-        clocks += t == Tail::all ? 1.15 * cta(2) : t == Tail::split ? full * cta(4) + cta(2) + 1040.0 : (full + (rem > 0)) * cta(4);
+        double seg = t == Tail::all ? 1.15 * cta(2) : t == Tail::split ? full * cta(4) + cta(2) + 1040.0 : (full + (rem > 0)) * cta(4);
+        if (form) seg = std::max<double>(seg, t == Tail::all ? 1.15 * form->worst.c[1][si] : form->worst.c[0][si]);
+        clocks += seg;
         return 0;
     });
     const double strided = v.oB == 1 ? 0.0 : p.Wo % 4 == 0 ? 1.15e-6 : 7.2e-6;
     return rc ? 1e30 : clocks / 1900.0 + strided * p.Cout * p.Ho * p.Wo * p.B;
+}
+
+// The rule.  By the density: below 0.92 of the other kernel's expected time (0.85 for a batch that leaves lanes to a second
+// tile), and not for few output channels with a batch that is no multiple of 16.  On the 400 shapes it was the faster
+// one every time it was taken, some 115 times; picking the faster each time would gain another 1.2 % on average.  Then,
+// with the form built, by what the entries' places say: below 1.04 of the other kernel's (the estimates are that close).
+// Weights that are not iid need it: of 415 (see rbm_cut) the density alone made 40 more than 10 % slower than the other
+// kernel (512 -> 512, 14 x 14, batch 32, rows that share their columns, 5 % dense 76 us against 140).  With both, of 792
+// others 5 were more than 5 % slower than with the merged kernel (up to 1.33), 3 than by the density (up to 1.37).
+static bool worth_it(const spx_ell* e, const ConvParams& p, const ConvViews& v, const conv_tmem_impl::Form* form,
+                     double (*other_us)(const spx_ell*, const ConvParams&, const MergedLoad*))
+{
+    const double us = conv_tmem_us(e, p, v, form);
+    if (form) return us <= 1.04 * other_us(e, p, form->merged);
+    return us < 1e30 && us <= (p.B % 32 ? 0.85 : 0.92) * other_us(e, p, nullptr);
 }
 
 template <int RW, int GP>
@@ -630,7 +766,7 @@ static int launch_cut(const spx_ell* e, TmemArgs a, const CUtensorMap& map, uint
 }
 
 int launch_conv_tmem(spx_ell* e, const ConvParams& p, const ConvViews& v, const float* in, const float* bias, int act, float* out,
-                     double (*other_us)(const spx_ell*, const ConvParams&), cudaStream_t s)
+                     double (*other_us)(const spx_ell*, const ConvParams&, const MergedLoad*), cudaStream_t s)
 {
     // the switches that force the other kernels turn this one off
     static const int env = [] {
@@ -644,17 +780,17 @@ int launch_conv_tmem(spx_ell* e, const ConvParams& p, const ConvViews& v, const 
     // Below 25 million FMAs a CTA's fixed cost decides (the smallest gains seen were at 16 million), and a call of 4 us
     // is the host's: it does without the estimates (3 -> 32, 21 x 21, batch 8 4.3 against 4.7 us).
     if (env != 2 && ((p.B % 16 && p.Cout <= 32) || (double)e->nnz_total * p.Ho * p.Wo * p.B < 25e6)) return -1;
-    const double us = conv_tmem_us(e, p, v);
-    if (us >= 1e30 || (env != 2 && us > (p.B % 32 ? 0.85 : 0.92) * other_us(e, p))) return -1;
+    Cut first;                                  // what the form depends on is the same for all segments
+    if (!plan(p, 4, p.B, first) || (env != 2 && !worth_it(e, p, v, nullptr, other_us))) return -1;
+    const conv_tmem_impl::Form* form = nullptr;
+    const FormShape f{p.kH, p.kW, p.dH, p.dW, first.TWin, first.THin, first.CC, first.chunk_cols};
+    if (const int rc = find_form(e, f, first.chunks, 16 / first.QT, s, &form); rc != SPX_OK) return rc;
+    if (env != 2 && form->loads && !worth_it(e, p, v, form, other_us)) return -1;
     static const int short_env = [] { const char* v = getenv("SPX_CONV_TMA_TEST_TIMEOUT"); return v ? atoi(v) : 0; }();
     bool launched = false;
     return each_segment(p.B, [&](uint32_t BT, uint32_t at, uint32_t len) -> int {
         Cut c;
         plan(p, BT, len, c);
-        const conv_tmem_impl::Form* form = nullptr;
-        const FormShape f{p.kH, p.kW, p.dH, p.dW, c.TWin, c.THin, c.CC, c.chunk_cols};
-        int rc = find_form(e, f, c.chunks, s, &form);       // the same for every segment: it can only fail for the first
-        if (rc != SPX_OK) return rc;
         TmemArgs a{};
         a.c = p; a.v = v;
         a.v.b_out = v.b_out > at ? v.b_out - at : 0u;
@@ -676,7 +812,7 @@ int launch_conv_tmem(spx_ell* e, const ConvParams& p, const ConvViews& v, const 
         const cuuint64_t gstr[3] = {v.iW * 4, v.iH * 4, v.iC * 4};
         const cuuint32_t box[4] = {BT, c.TWin, c.THin, c.CC};
         const cuuint32_t estr[4] = {1, 1, 1, 1};
-        rc = -1;
+        int rc = -1;
         if (encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(in + at), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS)
             rc = a.row_cols == 10 ? launch_cut<10>(e, a, map, (uint32_t)c.units, s) : launch_cut<0>(e, a, map, (uint32_t)c.units, s);

@@ -136,6 +136,29 @@ def waits_for_the_device(f):
     return waited
 
 
+@pytest.mark.skipif(any(k.startswith("SPX_CONV") for k in os.environ), reason="the choice is forced")
+@pytest.mark.parametrize("shared,density,kernel", [(False, 0.2, "conv_tmem_kernel"), (True, 0.05, "conv_rbm_tile_kernel"), (True, 0.5, "conv_tmem_kernel")])
+def test_choice_follows_the_entries(lib, orc, cuda, shared, density, kernel):
+    """The merged kernel does a column once for four rows: where rows share theirs it is the faster one at low density (128 ->
+    128, 28 x 28, batch 32, 5 %: 29 us against 41), and has to be taken although the density alone speaks for the other
+    (45 and 37)."""
+    rng = np.random.default_rng(12)
+    C, H, B = 128, 28, 32
+    wt = rng.standard_normal((C, C * 9)).astype(np.float32)
+    wt[np.broadcast_to(rng.random((1 if shared else C, C * 9)) >= density, wt.shape)] = 0
+    E = orc.encode(wt)
+    src = as_layout(rng.standard_normal((B, C, H, H)).astype(np.float32), sx.LAYOUT_PF)
+    want = orc.conv2d(E, dict(Cin=C, kH=3, kW=3, sH=1, sW=1, pH=1, pW=1, dH=1, dW=1, H=H, W=H), sx.LAYOUT_PF, src, B, None, 0)
+    dX, dY = dev(src, cuda), torch.empty(want.shape, device=cuda)
+    h = gpu_ell(lib, E)
+    g = sx.conv_geom(C, C, 3, 3, H, H, 1, 1, 1, 1)
+    for _ in range(2):
+        dY.fill_(float("nan"))
+        names = kernels_of(lambda: h.conv2d(g, sx.LAYOUT_PF, ptr(dX), B, None, 0, ptr(dY)))
+        assert [k in names for k in ("conv_tmem_kernel", "conv_rbm_tile_kernel")] == [kernel == "conv_tmem_kernel", kernel != "conv_tmem_kernel"]
+        assert_bit_equal(dY.cpu().numpy(), want, kernel)
+
+
 @forced
 def test_no_room_for_a_form(lib, orc, cuda):
     """The form does not fit: the merged kernel takes the call, and the next one does not try again (which would wait for
