@@ -287,7 +287,6 @@ conv_tmem_kernel(const __grid_constant__ TmemArgs a, const __grid_constant__ CUt
     const uint32_t subs = a.S * a.QT, first_tile = tile_unit * subs;
     const uint32_t sub = quad % a.QT * a.S + lane / a.BT;       // this lane's patch among the CTA's
 
-    if (warp == 0) spx::tmem_alloc_all(&s_tmem);
     if (threadIdx.x == 32) {
         for (uint32_t s = 0; s < a.stages; ++s) {
             spx::mbar_init(&s_full[s], 1);
@@ -300,12 +299,15 @@ conv_tmem_kernel(const __grid_constant__ TmemArgs a, const __grid_constant__ CUt
             }
         s_asked = min(a.stages, a.chunks);
     }
+    // Tensor memory is taken after the predecessor's end: a CTA that held it and waited would stop for good a predecessor
+    // that lets successors in before it takes its own.
+    spx::pdl_wait();
+    if (warp == 0) spx::tmem_alloc_all(&s_tmem);
     spx::tmem_fence_before();
     // an earlier CTA's (or call's) wait ran out: leave at once
     const bool bad = __syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile int*>(a.failed) != 0);
     spx::tmem_fence_after();
     const uint32_t tmem = s_tmem;
-    spx::pdl_wait();
     spx::pdl_launch();
     if (bad) {                                  // this call's output is not written either: said again, for a graph's launches
         if (threadIdx.x == 0) *a.failed_host = 1;

@@ -14,7 +14,7 @@ namespace spx {
 constexpr uint32_t kTmemColumns = 512;
 
 // By one whole warp; the address of the first column is left in shared memory.  Waits in hardware while another
-// kernel's CTA on the SM holds columns.
+// kernel's CTA on the SM holds columns: not to be called before pdl_wait(), or each could wait for the other.
 __device__ __forceinline__ void tmem_alloc_all(uint32_t* at) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;"
                  ::"r"((uint32_t)__cvta_generic_to_shared(at)) : "memory");
