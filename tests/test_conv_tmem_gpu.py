@@ -18,6 +18,21 @@ pytestmark = pytest.mark.gpu
 HERE = os.path.dirname(os.path.abspath(__file__))
 forced = pytest.mark.skipif(os.environ.get("SPX_CONV_TMEM") != "2", reason="runs in a child process")
 
+def kernels_of(f):
+    """Names of the kernels that f() launches; None where the profiler sees none at all."""
+    probe = torch.empty(1000, device="cuda")
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as p:
+        probe.sin_()
+        f()
+        torch.cuda.synchronize()
+    names = " ".join(e.key for e in p.key_averages())
+    return names.replace("sin_kernel", "") if "sin_kernel" in names else None
+
+
+def assert_ran(names, kernel):
+    assert names is None or kernel in names, names
+
+
 # B, Cin, Cout, H, W, (kH, kW), (sH, dH, dW), density
 CASES = [(32, 6, 64, 6, 8, (3, 3), (1, 1, 1), 0.3),         # one chunk, one unit
          (32, 7, 65, 7, 9, (3, 3), (1, 1, 1), 0.3),         # a chunk of one channel; a block and a position over
@@ -57,9 +72,9 @@ def test_forced_cases(lib, orc, cuda, layout, B, Cin, Cout, H, W, k, sd, density
     g = sx.conv_geom(Cin, Cout, kH, kW, H, W, sH, 1, pH, pW, dH, dW)
     dX, dB = dev(src, cuda), dev(bias, cuda)
     out = torch.full((want.size + 8,), 7.0, device=cuda, dtype=torch.float32)
-    for _ in range(2):
-        h.conv2d(g, layout, ptr(dX), B, ptr(dB), sx.ACT_NONE, out.data_ptr() + 16)
-    torch.cuda.synchronize()
+    call = lambda: h.conv2d(g, layout, ptr(dX), B, ptr(dB), sx.ACT_NONE, out.data_ptr() + 16)
+    call()
+    assert_ran(kernels_of(call), "conv_tmem_kernel")
     got = out.cpu().numpy()
     nan = np.isnan(want.reshape(-1))
     assert (np.isnan(got[4:-4]) == nan).all()
@@ -87,14 +102,14 @@ def test_forced_more_shapes_than_forms_and_capture(lib, orc, cuda):
         g = sx.conv_geom(Cin, Cout, 3, 3, H, W, gd["sH"], 1, 0, 0, gd["dH"], 1)
         dY = torch.empty(want.shape, device=cuda)
         if dil == 1:
-            h.conv2d(g, sx.LAYOUT_PF, ptr(dX), B, None, 0, ptr(dY))      # allocates what any kernel needs
-            torch.cuda.synchronize()
+            # allocates what any kernel needs
+            assert_ran(kernels_of(lambda: h.conv2d(g, sx.LAYOUT_PF, ptr(dX), B, None, 0, ptr(dY))), "conv_tmem_kernel")
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
             h.conv2d(g, sx.LAYOUT_PF, ptr(dX), B, None, 0, ptr(dY), torch.cuda.current_stream().cuda_stream)
         dZ = torch.empty(want.shape, device=cuda)
-        h.conv2d(g, sx.LAYOUT_PF, ptr(dX), B, None, 0, ptr(dZ))
-        torch.cuda.synchronize()
+        # four forms, the first shapes'; the rest goes without
+        assert_ran(kernels_of(lambda: h.conv2d(g, sx.LAYOUT_PF, ptr(dX), B, None, 0, ptr(dZ))), "conv_tmem_kernel" if dil < 5 else "conv_rbm_tile_kernel")
         assert_bit_equal(dZ.cpu().numpy(), want, f"eager {dil}")
         runs.append((graph, dY, want))
     for graph, dY, want in runs:
@@ -102,14 +117,6 @@ def test_forced_more_shapes_than_forms_and_capture(lib, orc, cuda):
         graph.replay()
         torch.cuda.synchronize()
         assert_bit_equal(dY.cpu().numpy(), want, "replayed")
-
-
-def kernels_of(f):
-    """Names of the kernels that f() launches."""
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as p:
-        f()
-        torch.cuda.synchronize()
-    return " ".join(e.key for e in p.key_averages())
 
 
 def fill_device(lib, leave, step):
@@ -136,6 +143,80 @@ def waits_for_the_device(f):
     return waited
 
 
+@forced
+@pytest.mark.parametrize("act", [sx.ACT_RELU, sx.ACT_SIGMOID, sx.ACT_TANH])
+@pytest.mark.parametrize("B,Cin,Cout,H,W", [(32, 9, 37, 7, 8), (20, 7, 66, 5, 11), (8, 12, 32, 6, 20)])
+@pytest.mark.parametrize("layout", [sx.LAYOUT_PF, sx.LAYOUT_NCHW, sx.LAYOUT_FMAJOR])
+def test_forced_cases_activations(lib, orc, cuda, layout, B, Cin, Cout, H, W, act):
+    """Activations in the epilogue, whole and partial tiles, single stores and (NCHW, a width of 4 k) quads: ReLU bit for bit,
+    sigmoid and tanh within the library's bound, and all of them the bits of the kernel that computes one result a thread."""
+    rng = np.random.default_rng([B, Cout, act])
+    wt = sparse(rng, Cout, Cin * 9, 0.3) * np.float32(0.7)
+    x = rng.standard_normal((B, Cin, H, W)).astype(np.float32)
+    x[0] *= 40                                              # saturated results among them
+    bias = rng.standard_normal(Cout).astype(np.float32)
+    src = as_layout(x, layout)
+    E = orc.encode(wt)
+    gd = dict(Cin=Cin, kH=3, kW=3, sH=1, sW=1, pH=1, pW=1, dH=1, dW=1, H=H, W=W)
+    want = orc.conv2d(E, gd, layout, src, B, bias, act)
+    h = gpu_ell(lib, E)
+    g = sx.conv_geom(Cin, Cout, 3, 3, H, W, 1, 1, 1, 1)
+    dX, dB = dev(src, cuda), dev(bias, cuda)
+    dY, dZ = torch.full(want.shape, float("nan"), device=cuda), torch.full(want.shape, float("nan"), device=cuda)
+    assert_ran(kernels_of(lambda: h.conv2d(g, layout, ptr(dX), B, ptr(dB), act, ptr(dY))), "conv_tmem_kernel")
+    got = dY.cpu().numpy()
+    if act == sx.ACT_RELU:
+        assert_bit_equal(got, want, "relu")
+    else:
+        assert np.abs(got - want).max() <= 4e-7             # expf and tanhf of CUDA and of the C library: a few ulp below 1
+    if layout != sx.LAYOUT_FMAJOR:
+        lib.spx_conv2d_static(h.h, ctypes.byref(g), layout, ptr(dX), B, ptr(dB), act, ptr(dZ), 0)
+        assert_bit_equal(got, dZ.cpu().numpy(), "against one result a thread")
+
+
+@forced
+def test_forced_cases_two_streams(lib, orc, cuda):
+    """Two handles on two streams at once, whose CTAs take all of an SM's tensor memory each."""
+    rng = np.random.default_rng(4)
+    runs = []
+    for B, Cin, Cout, H, W in ((32, 20, 64, 28, 28), (16, 33, 96, 30, 21)):
+        E = orc.encode(sparse(rng, Cout, Cin * 9, 0.2))
+        src = as_layout(rng.standard_normal((B, Cin, H, W)).astype(np.float32), sx.LAYOUT_PF)
+        want = orc.conv2d(E, dict(Cin=Cin, kH=3, kW=3, sH=1, sW=1, pH=1, pW=1, dH=1, dW=1, H=H, W=W), sx.LAYOUT_PF, src, B, None, 0)
+        runs.append((gpu_ell(lib, E), sx.conv_geom(Cin, Cout, 3, 3, H, W, 1, 1, 1, 1), dev(src, cuda), B, want,
+                     [torch.full(want.shape, float("nan"), device=cuda) for _ in range(8)], torch.cuda.Stream()))
+    torch.cuda.synchronize()
+
+    def all_calls():
+        for i in range(8):
+            for h, g, dX, B, _, out, stream in runs:
+                h.conv2d(g, sx.LAYOUT_PF, ptr(dX), B, None, 0, ptr(out[i]), stream.cuda_stream)
+
+    assert_ran(kernels_of(all_calls), "conv_tmem_kernel")
+    for _, _, _, _, want, out, _ in runs:
+        for y in out:
+            assert_bit_equal(y.cpu().numpy(), want, "two streams")
+
+
+@pytest.mark.skipif(os.environ.get("SPX_CONV_TMA_TEST_TIMEOUT") != "1" or os.environ.get("SPX_CONV_TMEM") != "2", reason="runs in a child process")
+def test_timeout_of_this_kernel(lib, orc, cuda):
+    """The waits for its bulk copies run out: that call returns, the next says so, the one after does without and is right."""
+    rng = np.random.default_rng(6)
+    B, Cin, Cout, H = 16, 40, 48, 12
+    E = orc.encode(sparse(rng, Cout, Cin * 9, 0.25))
+    src = as_layout(rng.standard_normal((B, Cin, H, H)).astype(np.float32), sx.LAYOUT_PF)
+    want = orc.conv2d(E, dict(Cin=Cin, kH=3, kW=3, sH=1, sW=1, pH=1, pW=1, dH=1, dW=1, H=H, W=H), sx.LAYOUT_PF, src, B, None, 0)
+    h, g, dX, dY = gpu_ell(lib, E), sx.conv_geom(Cin, Cout, 3, 3, H, H, 1, 1, 1, 1), dev(src, cuda), torch.full(want.shape, float("nan"), device=cuda)
+    call = lambda: h.conv2d(g, sx.LAYOUT_PF, ptr(dX), B, None, 0, ptr(dY))
+    assert_ran(kernels_of(call), "conv_tmem_kernel")
+    with pytest.raises(sx.SpxError, match="bulk tensor copy"):
+        call()
+    dY.fill_(float("nan"))
+    names = kernels_of(call)
+    assert names is None or "conv_tmem_kernel" not in names
+    assert_bit_equal(dY.cpu().numpy(), want, "after the reported timeout")
+
+
 @pytest.mark.skipif(any(k.startswith("SPX_CONV") for k in os.environ), reason="the choice is forced")
 @pytest.mark.parametrize("shared,density,kernel", [(False, 0.2, "conv_tmem_kernel"), (True, 0.05, "conv_rbm_tile_kernel"), (True, 0.5, "conv_tmem_kernel")])
 def test_choice_follows_the_entries(lib, orc, cuda, shared, density, kernel):
@@ -155,7 +236,7 @@ def test_choice_follows_the_entries(lib, orc, cuda, shared, density, kernel):
     for _ in range(2):
         dY.fill_(float("nan"))
         names = kernels_of(lambda: h.conv2d(g, sx.LAYOUT_PF, ptr(dX), B, None, 0, ptr(dY)))
-        assert [k in names for k in ("conv_tmem_kernel", "conv_rbm_tile_kernel")] == [kernel == "conv_tmem_kernel", kernel != "conv_tmem_kernel"]
+        assert_ran(names, kernel)
         assert_bit_equal(dY.cpu().numpy(), want, kernel)
 
 
@@ -191,7 +272,8 @@ def test_no_room_for_a_form(lib, orc, cuda):
         for p in held:
             lib.spx_free(p)
     other = gpu_ell(lib, E)
-    assert "conv_tmem_kernel" in kernels_of(lambda: call(other)) and "conv_tmem_kernel" not in kernels_of(lambda: call(h))
+    assert_ran(kernels_of(lambda: call(other)), "conv_tmem_kernel")
+    assert_ran(kernels_of(lambda: call(h)), "conv_rbm_tile_kernel")
     assert_bit_equal(dY.cpu().numpy(), want, "room again")
 
 
@@ -208,7 +290,7 @@ def test_forced_kernel():
 
 def test_timeout_is_reported():
     """The waits for its bulk copies are bounded: they are made to run out, the next call says so, the one after works."""
-    child(["test_parity_gpu.py"], "bulk_copy_timeout_child", {"SPX_CONV_TMEM": "2", "SPX_CONV_TMA_TEST_TIMEOUT": "1"})
+    child(["test_conv_tmem_gpu.py", "test_parity_gpu.py"], "timeout_of_this_kernel or bulk_copy_timeout_child", {"SPX_CONV_TMEM": "2", "SPX_CONV_TMA_TEST_TIMEOUT": "1"})
 
 
 def test_forced_without_memory():
