@@ -9,7 +9,7 @@
 // FMA each: bit-identical to the other kernels.
 //
 // A CTA: 16 warps multiply, each 4 output channels x 2 x 8 positions x 32 lanes (64 accumulators a thread); every
-// quadrant holds the same patch (or one of 2 or 4, where there are few output channels), so a CTA covers up to 64
+// quadrant holds the same patch (or one of two, where there are 32 output channels and less), so a CTA covers up to 64
 // channels.  4 more warps, one per quadrant, copy the patch from shared memory, where bulk tensor copies bring it, into
 // one half of the quadrant's columns while the other half is used.
 //
@@ -642,7 +642,7 @@ bool plan(const ConvParams& p, uint32_t BT, uint32_t b_len, Cut& c)
 {
     const uint32_t nblocks = (p.Cout + kRows - 1) / kRows, taps = p.kH * p.kW;
     c.S = 32 / BT;
-    c.QT = nblocks > 8 ? 1 : nblocks > 4 ? 2 : 4;           // few output channels: the quadrants take tiles of their own
+    c.QT = nblocks > 8 ? 1 : 2;             // 29 to 32 output channels (fewer do not come here): two quadrants share a tile
     c.subs = c.S * c.QT;
     c.TWin = (kTW - 1) * p.sW + (p.kW - 1) * p.dW + 1;
     c.THin = (kTH - 1) * p.sH + (p.kH - 1) * p.dH + 1;
