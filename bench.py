@@ -1110,7 +1110,7 @@ def measure(args, c):
             line["roofline"]["operand_path"] = {
                 "what": "X operands consumed, 4 bytes per FMA (gathered L2->SM for SpMM/MLP; for conv read from "
                         "shared memory, once per FMA by the per-row kernel, once per block of 4 rows by the "
-                        "row-block-merged kernel)",
+                        "row-block-merged kernel, or from tensor memory)",
                 "bytes_per_step": op_bytes, "achieved_tbps": op_bytes / sec / 1e12}
             if l2_gather_tbps:
                 line["roofline"]["operand_path"].update({

@@ -118,11 +118,13 @@ int spx_ell_create(uint32_t m, uint32_t n, uint32_t r, const float* Wd, const ui
 int spx_ell_create_csr(uint32_t m, uint32_t n, const uint64_t* rowptr, const uint32_t* col,
                        const float* val, spx_ell** out);
 /* Encode a dense row-major m*n device matrix on the device: same result as
- * convert_to_ellpack (src/ellpack_encoder.cpp:6-44): entries with v != 0.0f, ascending columns. */
+ * convert_to_ellpack (src/ellpack_encoder.cpp:6-44): entries with v != 0.0f, ascending columns.
+ * Matrices of 64 MB and more take scratch for the call, about half of theirs and up to 288 MB, where it is
+ * to be had.  Waits for `stream`. */
 int spx_ell_encode_device(const float* dW, uint32_t m, uint32_t n, void* stream, spx_ell** out);
 int spx_ell_destroy(spx_ell* e);
 /* Kernels that fetch an operand with bulk tensor copies (spx_spmm where it stages X block by block, spx_conv2d's
- * row-block-merged kernel) wait for them with a limit of about a second.  Should a wait ever run out, the call in
+ * row-block-merged kernel and its tensor-memory kernel) wait for them with a limit of about a second.  Should a wait ever run out, the call in
  * flight has returned SPX_OK but its output is invalid.  The failure is then reported as SPX_ERR_CUDA: by the
  * *_host call itself, else by the next spx_spmm or spx_conv2d on the handle, before it launches anything, or by this
  * function, for callers that replay a captured graph (ask after the stream has been waited for).  From then on the
@@ -161,11 +163,13 @@ int spx_spmv_reference_order(const spx_ell* e, const float* x, const float* bias
  * [Cout x Cin*kH*kW].  Replaces conv2d_patchmajor_tiled / conv2d_tiled_im2col_cmajor /
  * conv2d_tiled_im2col_fmajor / conv2d_rbm_fmajor_implicit (src/layers/conv_kernels.cpp:66-470)
  * and, on the device, build_rbm_from_ellpack (src/layers/rbm_conv.cpp:7-73): the first call per
- * handle and kernel shape builds and caches a tap table and, where the batch size and weight
- * density favour it, the row-block-merged form of the weights and, for larger calls, a second
- * form for the kernel that keeps its input in tensor memory (device allocations, and a wait for
- * `stream`; make that call outside a stream capture: a captured call uses the forms that are
- * there).  Results do not depend on which kernel is chosen.  Both of those kernels fetch their
+ * handle and kernel shape builds and caches a tap table (4 bytes a slot of the slab), where the
+ * batch size and weight density favour it, the row-block-merged form of the weights (up to three
+ * slabs) and, for larger calls, a second form for the kernel that keeps its input in tensor memory
+ * (about a slab per kernel shape, dilation and row stride, at most four), beside which it always builds
+ * the first: the two are compared (device allocations, and a wait for `stream`; make that call outside a stream
+ * capture: a captured call uses the forms that are there).  A form that finds no memory is gone
+ * without from then on.  Results do not depend on which kernel is chosen.  Both of those kernels fetch their
  * input with bulk tensor copies: see spx_ell_status. */
 int spx_conv2d(const spx_ell* e, const spx_conv_geom* g, int layout, const float* in, uint32_t B,
                const float* bias, int act, float* out, void* stream);

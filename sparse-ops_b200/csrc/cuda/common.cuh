@@ -111,6 +111,7 @@ __device__ __forceinline__ float apply_act(float v, int act) {
     default:              return v;
     }
 }
+
 // Programmatic dependent launch: a kernel launched with launch_pdl() may start while its predecessor
 // in the stream is still draining.  Before pdl_wait() it may only touch what no kernel of the stream
 // writes -- the arrays of a finished handle; after it everything the predecessors wrote is visible.

@@ -1093,7 +1093,7 @@ static int launch_conv_pf_tile(spx_ell* e, const ConvParams& p, const ConvViews&
 // of 16 when that is cheaper.  Cost per batch entry on 256 -> 256 channels, 3 x 3, 56 x 56, 80 %
 // sparse (ms per entry).  Merged kernel, which takes any multiple of 4 in segments of 16 / 8 / 4:
 // 0.0436 / 0.0516 / 0.0645 - rounding up to 16 never pays (28 as 16 + 8 + 4: 1.37 ms, as 32 with
-// the widening passes: 1.53 ms).  Per-row kernel (matrices the merged one does not take) with its
+// the widening passes: 1.53 ms; not weighed for conv_tmem_kernel, whose segments are 32 / 16 / 8 / 4).  Per-row kernel (matrices the merged one does not take) with its
 // tiles of 4 .. 32: 0.094, 0.064, 0.064, 0.056, 0.069, 0.066, 0.068, 0.056 - there 28 runs as 32
 // and 44 as 48, while 12, 20, 24 and 36 stay as they are.
 static uint32_t padded_batch(uint32_t B, bool merged)

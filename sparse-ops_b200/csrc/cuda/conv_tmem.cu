@@ -13,14 +13,15 @@
 // channels.  4 more warps, one per quadrant, copy the patch from shared memory, where bulk tensor copies bring it, into
 // one half of the quadrant's columns while the other half is used.
 //
-// What bounds it: issue slots.  A tap costs a warp 8 packed FMAs (16 clocks of the FMA pipe) and about 8 other
-// instructions, 24 clocks with four warps to an SM quarter; filling costs 4 clocks per column, a shared-memory wavefront
-// for each quadrant.  Measured, 256 -> 256 channels, 3 x 3, 56 x 56, batch 32: 80 % sparse 697 us against 1342 with
-// conv_rbm_tile_kernel, 50 % 1359 / 2370, 95 % 391 / 465; batch 8 256 / 375; 64 -> 64, 112 x 112 201 / 378; 5 x 5, 64 -> 96,
-// 28 x 28, batch 16 56 / 100.  Tried: scalar FMAs 1221 against 1021 us at the time, 4 x 8 positions and 2 channels a warp
-// 1272 (spills), no warps of their own for the copying 1010 against 819 (its waits add up), entries read through L1
-// instead of shared memory 807 against 732, weights stored twice so that the packed FMA can take them as they are 760
-// against 732, CTAs that go on to further units by themselves 764 against 743.
+// What bounds it: issue slots (71 % used, FMA pipe 50 %; nothing issues when an SM quarter's four warps wait at once).  A
+// tap costs a warp 8 packed FMAs (16 clocks of the FMA pipe) and about 8 other instructions, 24 clocks with four warps to a
+// quarter; filling costs 4 clocks per column, a shared-memory wavefront for each quadrant.  Measured, 256 -> 256 channels,
+// 3 x 3, 56 x 56, batch 32: 80 % sparse 704 us (708 in a process of its own) against 1341 with conv_rbm_tile_kernel, 50 %
+// 1362 / 2369, 95 % 399 / 464; batch 8 258 / 374; 64 -> 64, 112 x 112 203 / 377; 5 x 5, 64 -> 96, 28 x 28, batch 16 56 / 101.
+// The halves of a last wave (RW = 2) spill 16 bytes, the whole units nothing.  Tried: scalar FMAs 1221 against 1021 us at
+// the time, 4 x 8 positions and 2 channels a warp 1272 (spills), no warps of their own for the copying 1010 against 819 (its
+// waits add up), entries read through L1 instead of shared memory 807 against 732, weights stored twice so that the packed
+// FMA can take them as they are 760 against 732, CTAs that go on to further units by themselves 764 against 743.
 #include "conv.cuh"
 #include "tma.cuh"
 #include "tmem.cuh"
@@ -264,7 +265,7 @@ __device__ __forceinline__ void fill_columns(uint32_t from, uint32_t pitch, uint
 }
 
 // Sigmoid and tanh: one copy of their code.  Inlined for each of a thread's 64 results they made the instruction cache
-// miss at the end of every CTA: 256 -> 256, 56 x 56 742 against 697 us, 3 -> 416, 80 x 80 242 against 147.  (The merged kernel's
+// miss at the end of every CTA: 256 -> 256, 56 x 56 742 against 697 us at the time, 3 -> 416, 80 x 80 242 against 147.  (The merged kernel's
 // small cuts lose by the call, also where it is not made: 3 -> 160, 45 x 45, batch 30 30.4 against 33.1.)
 __device__ __noinline__ float activate(float v, int act) { return spx::apply_act(v, act); }
 
