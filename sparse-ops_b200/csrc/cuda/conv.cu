@@ -861,9 +861,9 @@ struct RbmCut {
     int nb, g;
     double cycles;
 };
-// load: the cut is chosen by the density all the same, but its time is what the CTAs' own entries take.  Against 415 measured
+// load: the cut is chosen by the density all the same, but its time is what the CTAs' own entries take.  Of 1484 measured
 // weights (iid, rows of different density, channels or kernels removed whole, rows that share their columns) that is 1.0
-// times the time, deviation 0.2; by the density it is 0.6 (dense rows side by side) to 1.9 (shared columns).
+// times the time, deviation 0.2; by the density it is 0.6 (dense rows side by side) to 1.8 (shared columns).
 static RbmCut rbm_cut(const spx_ell* e, const ConvParams& p, uint32_t qb, uint32_t b_len, const spx::MergedLoad* load = nullptr)
 {
     struct Option { RbmCut cut; double latency, per_warp; };

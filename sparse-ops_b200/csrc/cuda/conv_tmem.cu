@@ -732,9 +732,9 @@ static double conv_tmem_us(const spx_ell* e, const ConvParams& p, const ConvView
 // tile), and not for few output channels with a batch that is no multiple of 16.  On the 400 shapes it was the faster
 // one every time it was taken, some 115 times; picking the faster each time would gain another 1.2 % on average.  Then,
 // with the form built, by what the entries' places say: below 1.04 of the other kernel's (the estimates are that close).
-// Weights that are not iid need it: of 415 (see rbm_cut) the density alone made 40 more than 10 % slower than the other
-// kernel (512 -> 512, 14 x 14, batch 32, rows that share their columns, 5 % dense 76 us against 140).  With both, of 792
-// others 5 were more than 5 % slower than with the merged kernel (up to 1.33), 3 than by the density (up to 1.37).
+// Weights that are not iid need it: of 1484 measured ones (see rbm_cut) the density alone made 184 more than 10 % slower
+// than the other kernel (512 -> 512, 14 x 14, batch 32, rows that share their columns, 5 % dense 76 us against 140), both
+// rules leave 20 (up to 1.9) and give away more than 10 % of what the density had gained in 7 (up to 1.4).
 static bool worth_it(const spx_ell* e, const ConvParams& p, const ConvViews& v, const conv_tmem_impl::Form* form,
                      double (*other_us)(const spx_ell*, const ConvParams&, const MergedLoad*))
 {
