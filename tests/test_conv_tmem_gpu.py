@@ -134,7 +134,7 @@ def waits_for_the_device(f):
     """Whether f() returns only after what is queued on another stream."""
     torch.cuda.synchronize()
     with torch.cuda.stream(torch.cuda.Stream()):
-        torch.cuda._sleep(400_000_000)                      # 0.2 s and more
+        torch.cuda._sleep(1_000_000_000)                    # 0.5 s and more
         done = torch.cuda.Event()
         done.record()
     f()
