@@ -109,7 +109,8 @@ count_kernel(const float* __restrict__ W, uint32_t mis, uint32_t m, uint32_t n, 
 // 8192 x 8192, 10 %: 58 us (count_kernel 53), and pack_kernel 29 instead of 67.
 // A unit is given up where more than 17/64 of the columns seen so far (and 16) are entries: the pairs written until then
 // are in vain.  It is marked in its first pair.  (Writing them up to a capacity of a quarter cost units that are denser 8
-// to 12 %: 151 x 264025, 30 % 165 us, now 146, 143 without pairs.  A unit that is dense at its front only is read twice,
+// to 12 %: 151 x 264025, 30 % 165 us, now 146, 143 without pairs.  The check costs 8192 x 8192, 10 % 1 us of 188.  A unit
+// that is dense at its front only is read twice,
 // as without pairs.)
 constexpr uint32_t kNotKept = 0xffffffffu;                  // no column: n is at most this
 constexpr uint32_t kKeepSlack = 16;
@@ -289,9 +290,9 @@ pack_kernel(const float* __restrict__ W, uint32_t mis, uint32_t m, uint32_t n, u
         for (uint64_t k = first + lane; k < unit; k += 32) pos += counts[k];
         pos = __reduce_add_sync(0xffffffffu, pos);
     }
-    const uint32_t mine = kept ? __ldg(counts + unit) : 0u;
     const uint2* __restrict__ src = kept + unit * cap;
-    if (kept && (mine == 0 || __ldg(&src->y) != kNotKept)) {
+    const uint32_t mine = kept ? __ldg(counts + unit) : 0u, mark = kept ? __ldg(&src->y) : kNotKept;    // (one trip for both)
+    if (kept && (mine == 0 || mark != kNotKept)) {
         constexpr uint32_t kRun = 4;                        // pairs per lane in flight
         for (uint32_t j0 = lane; j0 < mine; j0 += 32 * kRun) {
             uint2 p[kRun];
