@@ -166,10 +166,10 @@ int spx_spmv_reference_order(const spx_ell* e, const float* x, const float* bias
  * handle and kernel shape builds and caches a tap table (4 bytes a slot of the slab), where the
  * batch size and weight density favour it, the row-block-merged form of the weights (up to three
  * slabs) and, for larger calls, a second form for the kernel that keeps its input in tensor memory
- * (about a slab per kernel shape, dilation and row stride, at most four), beside which it always builds
- * the first: the two are compared (device allocations, and a wait for `stream`; make that call outside a stream
- * capture: a captured call uses the forms that are there).  A form that finds no memory is gone
- * without from then on.  Results do not depend on which kernel is chosen.  Both of those kernels fetch their
+ * (about a slab per kernel shape, dilation and row stride, at most four), beside which it builds
+ * the first as well: the two are compared.  (Device allocations, and a wait for `stream`; make
+ * that call outside a stream capture: a captured call uses the forms that are there.)  A form that
+ * finds no memory is gone without from then on.  Results do not depend on which kernel is chosen.  Both of those kernels fetch their
  * input with bulk tensor copies: see spx_ell_status. */
 int spx_conv2d(const spx_ell* e, const spx_conv_geom* g, int layout, const float* in, uint32_t B,
                const float* bias, int act, float* out, void* stream);

@@ -11,7 +11,7 @@
 // 16-byte vectors with several in flight per lane.  A large matrix is read once: the counter keeps the entries it finds,
 // the packer fetches them from L2; a small one is read again, backwards: what the counter read last is then still in L2.
 // Measured at 8192 x 8192, 10 % kept: count and keep 58 us, pack 29, decode 56 (6.0 TB/s); encode + decode + destroy
-// through the C ABI 185 us (244 with two reads and a schedule sorted on the host).
+// through the C ABI 187 us (244 with two reads and a schedule sorted on the host).
 #include "common.cuh"
 
 #include <algorithm>
@@ -109,9 +109,8 @@ count_kernel(const float* __restrict__ W, uint32_t mis, uint32_t m, uint32_t n, 
 // 8192 x 8192, 10 %: 58 us (count_kernel 53), and pack_kernel 29 instead of 67.
 // A unit is given up where more than 17/64 of the columns seen so far (and 16) are entries: the pairs written until then
 // are in vain.  It is marked in its first pair.  (Writing them up to a capacity of a quarter cost units that are denser 8
-// to 12 %: 151 x 264025, 30 % 165 us, now 146, 143 without pairs.  The check costs 8192 x 8192, 10 % 1 us of 188.  A unit
-// that is dense at its front only is read twice,
-// as without pairs.)
+// to 12 %: 151 x 264025, 30 % 165 us, now 146, 143 without pairs.  The check costs 8192 x 8192, 10 % 1 us of 187.  A unit
+// that is dense at its front only is read twice, as without pairs.)
 constexpr uint32_t kNotKept = 0xffffffffu;                  // no column: n is at most this
 constexpr uint32_t kKeepSlack = 16;
 __host__ __device__ constexpr uint32_t keep_cap(uint32_t columns) { return columns / 64 * 17 + kKeepSlack; }
