@@ -479,8 +479,12 @@ Plan plan_tiles(const spx_ell* e, uint32_t C, uint32_t NV, uint32_t sms, bool al
     p.slices = (C + 32 * NV - 1) / (32 * NV);
     const uint64_t units = (uint64_t)groups * p.slices;
     p.waves = (units + (uint64_t)sms * kMaxWarps - 1) / ((uint64_t)sms * kMaxWarps);
-    p.warps = (uint32_t)std::min<uint64_t>(kMaxWarps, (units + sms * p.waves - 1) / (sms * p.waves));
-    while (p.warps < kMaxWarps && (uint64_t)((groups + p.warps - 1) / p.warps) * p.slices > p.waves * sms) ++p.warps;
+    for (;; ++p.waves) {                        // whole CTAs: the slices' last ones are not full
+        p.warps = (uint32_t)std::min<uint64_t>(kMaxWarps, (units + sms * p.waves - 1) / (sms * p.waves));
+        const auto ctas = [&] { return (uint64_t)((groups + p.warps - 1) / p.warps) * p.slices; };
+        while (p.warps < kMaxWarps && ctas() > p.waves * sms) ++p.warps;
+        if (ctas() <= p.waves * sms) break;
+    }
     const double len = (double)e->nnz_total / e->m;
     const double steps = std::max((len + 1.1 * std::sqrt(len)) / 4.0, chunks * (1.0 - std::exp(-(double)kGroupRows * len / chunks)));
     p.us = 0.9 + (double)e->m * C * 0.62e-6 + (C % 32 ? 0.17 * chunks : 0.0) + (aligned ? 0.0 : 3.5) +
@@ -509,7 +513,8 @@ double gather_us(const spx_ell* e, uint32_t C, uint32_t V, bool half)
     double rounds = e->max_nnz;
     if (V == 1 && per_sm < 12) rounds *= 0.0115 * NV * (NV == 3 ? std::ceil(per_sm / 8.0) : 1.0);
     else rounds *= (NV == 1 ? 0.0168 * (V == 4 && RW > 1 && !brief ? 1.0 + 0.03 * RW : 1.0) : 0.0282) * (NV == 1 && (per_sm < 48 || !brief) ? std::max(1.0, std::ceil(per_sm / 8.0)) : 1.0);
-    return (3.5 + std::sqrt(std::sqrt(std::pow(loads, 4) + std::pow(rounds, 4)))) * (half ? 0.9 : 1.0);
+    const double l2 = loads * loads, r2 = rounds * rounds;
+    return (3.5 + std::sqrt(std::sqrt(l2 * l2 + r2 * r2))) * (half ? 0.9 : 1.0);
 }
 
 }  // namespace
@@ -521,11 +526,31 @@ int launch_spmm_tile(spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const
     static const int env = [] { const char* v = getenv("SPX_SPMM_TILE"); return v ? atoi(v) : 1; }();
     if (!env || !e->tiles || !e->cols_ascending || e->tma_off || e->max_nnz == 0) return -1;
     const PFN_cuTensorMapEncodeTiled encode = tensor_map_encoder();
-    if (!encode || ldx > 0xffffffffull || e->n > 65536 || C > (1u << 30)) return -1;
-    const uint32_t NV = C <= 32 ? 1 : 2;
-    const Plan p = plan_tiles(e, C, NV, sm_count(e->device), vec_x);
+    if (!encode || ldx > 0xffffffffull || e->n > 65536 || C > (1u << 30) || (env != 2 && e->n < kChunk)) return -1;
+    // Slices of 64 columns read the entries half as often, slices of 32 leave fewer columns idle and give the SMs more
+    // warps.  Of 500 shapes (256 to 8192 rows and columns, 2 to 50 %, C = 33 to 1024, 33 to 160 more often than not), the
+    // narrow ones are faster for 283 (3001 x 4999, 6 %, C = 77 24.2 us against 28.7; 600 x 3000, 30 %, C = 128 25.0 / 31.1),
+    // the wide ones for 177 (6000 x 6000, 5 %, C = 93 46.4 / 48.3).  The choice takes 0.3 % longer than the better one on
+    // average, 10 % longer for 3, and 0.93 of what wide slices took; without the 1.5 us, by which the narrow kernel's estimate
+    // is high, 1.7 % and 36.
+    const uint32_t sms = sm_count(e->device);
+    Plan p = plan_tiles(e, C, 1, sms, vec_x);
+    uint32_t NV = 1;
+    const double gather = gather_us(e, C, V, half);
+    bool faster = p.us <= 1.05 * gather;
+    if (C > 32) {
+        const Plan wide = plan_tiles(e, C, 2, sms, vec_x);
+        if (p.us >= wide.us + 1.5) {
+            p = wide;
+            NV = 2;
+        }
+        // Against gathering the narrow estimate is trusted less: at 0.92 the same shapes take 0.98 of the time that wide
+        // slices alone did, one of them 5 % more; at 1.05 two of a hundred take 5 % and more longer (1920 x 896, 20 %, C = 50
+        // 12.0 us against 9.4 gathered).
+        faster = wide.us <= 1.05 * gather || (NV == 1 && p.us <= 0.92 * gather);
+    }
     if ((uint64_t)p.slices * e->m > 0x7fffffffull) return -1;
-    if (env != 2 && (e->n < kChunk || p.us > 1.05 * gather_us(e, C, V, half))) return -1;
+    if (env != 2 && !faster) return -1;
     spx_tiles_impl* t = static_cast<spx_tiles_impl*>(e->tiles);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (t->state != 1 || !vec_x) {              // building and the scratch below allocate: not while a graph is captured

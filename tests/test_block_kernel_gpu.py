@@ -62,6 +62,32 @@ def test_stage_refills_forced():
     in_child("test_stage_refills", SPX_SPMM_TILE="2")
 
 
+@pytest.mark.parametrize("C", [32, 33, 63, 64, 65, 95, 96, 97, 128, 130, 352])
+@pytest.mark.parametrize("m", [5, 300, 1300])
+def test_slices(lib, orc, cuda, m, C):
+    """Slices of 32 and of 64 columns, whole, cut short and with a single column, of aligned rows and of a copy."""
+    if os.environ.get("SPX_SPMM_TILE") != "2":
+        pytest.skip("runs in a child process of test_slices_forced")
+    rng = np.random.default_rng([m, C])
+    n = 700
+    W = sparse(rng, m, n, 0.2)
+    E = orc.encode(W)
+    b = rng.standard_normal(m).astype(np.float32)
+    X = rng.uniform(-1, 1, (n, C)).astype(np.float32)
+    want = orc.spmm(E, X, b, act=1)
+    h = lib.ell_create(E.Wd, E.idx, E.nnz, E.n)
+    dX, dB = torch.from_numpy(X).to(cuda), torch.from_numpy(b).to(cuda)
+    for call in range(3):                   # the first one gathers
+        dY = torch.full((m, C), float("nan"), device=cuda)
+        h.spmm(dX.data_ptr(), C, C, dB.data_ptr(), sx.ACT_RELU, dY.data_ptr(), C)
+        torch.cuda.synchronize()
+        assert_bit_equal(dY.cpu().numpy(), want, f"call {call}")
+
+
+def test_slices_forced():
+    in_child("test_slices", SPX_SPMM_TILE="2")
+
+
 # ---- a bounded wait that runs out -----------------------------------------------------------------
 def small_case(orc, seed=5):
     rng = np.random.default_rng(seed)
