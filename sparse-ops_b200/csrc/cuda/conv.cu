@@ -770,6 +770,7 @@ static bool rbm_fits(const ConvParams& p, uint32_t qb, int nb, int g)
 int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s)
 {
     if (e->rbm_hdr && e->rbm_kH == kH && e->rbm_kW == kW) return SPX_OK;
+    RelaxedCapture relaxed;                     // allocations and waits below end no capture
     const uint32_t nblocks = (e->m + kRbmRows - 1) / kRbmRows;
     if (!e->rbm_hdr) {
         // Up to three times the ELLPACK slab (24 bytes per union column, at most 4 * max_nnz columns
@@ -791,10 +792,19 @@ int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s)
         ensure_tma_words(e);
         (void)cudaGetLastError();
     }
+    // A call that is recorded builds them all the same, beside the recording: eager calls before it may all have gathered.
+    cudaStreamCaptureStatus cap_status = cudaStreamCaptureStatusNone;
+    const bool recorded = cudaStreamIsCapturing(s, &cap_status) == cudaSuccess && cap_status != cudaStreamCaptureStatusNone;
+    cudaStream_t on = s;
+    if (recorded) {
+        if (int rc = side_stream(e->device, &on)) return rc;
+        wait_for_device();                      // for the entries, which may still be on their way
+    }
     const size_t smem = (size_t)((e->n + 31) / 32) * 2 * sizeof(uint32_t);
-    build_rbm_kernel<<<nblocks, 256, smem, s>>>(e->Wd, e->idx, e->nnz, e->m, e->n, e->pitch, kH, kW, e->rbm_cap,
-                                                e->rbm_hdr, e->rbm_w, e->rbm_ncols);
+    build_rbm_kernel<<<nblocks, 256, smem, on>>>(e->Wd, e->idx, e->nnz, e->m, e->n, e->pitch, kH, kW, e->rbm_cap,
+                                                 e->rbm_hdr, e->rbm_w, e->rbm_ncols);
     SPX_LAUNCH_CHECK("build_rbm_kernel");
+    if (recorded) SPX_CUDA(cudaStreamSynchronize(on));
     e->rbm_kH = kH;
     e->rbm_kW = kW;
     return SPX_OK;
@@ -1089,6 +1099,110 @@ static int launch_conv_pf_tile(spx_ell* e, const ConvParams& p, const ConvViews&
     return -1;
 }
 
+// Warp per block of 4 rows: its union columns and its entries.
+__global__ void __launch_bounds__(256)
+union_count_kernel(const uint32_t* __restrict__ idx, const uint32_t* __restrict__ nnz, uint32_t m, uint32_t pitch, uint2* __restrict__ blocks)
+{
+    const uint32_t lane = threadIdx.x & 31, b = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (b * kRbmRows >= m) return;
+    uint32_t fresh = 0, all = 0, len[kRbmRows];
+#pragma unroll
+    for (uint32_t r = 0; r < kRbmRows; ++r) {
+        const uint32_t row = b * kRbmRows + r;
+        len[r] = row < m ? __ldg(nnz + row) : 0u;
+        all += len[r];
+        const uint32_t* __restrict__ k = idx + (size_t)min(row, m - 1) * pitch;
+        for (uint32_t j = lane; j < len[r]; j += 32) {
+            const uint32_t col = __ldg(k + j);
+            bool seen = false;
+            for (uint32_t q = 0; q < r && !seen; ++q) {     // columns ascend in the earlier rows
+                const uint32_t* __restrict__ other = idx + (size_t)(b * kRbmRows + q) * pitch;
+                uint32_t lo = 0, hi = len[q];
+                while (lo < hi) {
+                    const uint32_t mid = (lo + hi) >> 1;
+                    if (__ldg(other + mid) < col) lo = mid + 1; else hi = mid;
+                }
+                seen = lo < len[q] && __ldg(other + lo) == col;
+            }
+            fresh += !seen;
+        }
+    }
+    fresh = __reduce_add_sync(0xffffffffu, fresh);
+    if (lane == 0) blocks[b] = make_uint2(fresh, all);
+}
+
+// Counts once per handle; the call then waits for its stream.  Not while a graph is recorded on it.
+static void count_loads(spx_ell* e, cudaStream_t s)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) { (void)cudaGetLastError(); return; }
+    RelaxedCapture relaxed;                     // s is not being captured; another stream may be, by this thread
+    e->conv_loads_state = 2;
+    const uint32_t nblocks = (e->m + kRbmRows - 1) / kRbmRows;
+    const size_t bytes = (size_t)nblocks * sizeof(uint2);
+    PinnedBlock host;
+    void* blocks = nullptr;
+    if (scratch_alloc(&blocks, bytes, e->device, s, true) == SPX_OK && pinned_acquire(bytes, &host) == SPX_OK) {
+        union_count_kernel<<<(nblocks + 7) / 8, 256, 0, s>>>(e->idx, e->nnz, e->m, e->pitch, static_cast<uint2*>(blocks));
+        count_launch();
+        if (cudaGetLastError() == cudaSuccess && cudaMemcpyAsync(host.host, blocks, bytes, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
+            cudaStreamSynchronize(s) == cudaSuccess) {
+            MergedLoad load[3];
+            merged_loads(static_cast<const uint2*>(host.host), nblocks, load);
+            for (int k = 0; k < 3; ++k) {
+                const double v[4] = {load[k].longest, load[k].work, load[k].longest_worst, load[k].work_worst};
+                std::copy(v, v + 4, e->conv_loads[k]);
+            }
+            e->conv_loads_state = 1;
+        }
+    }
+    pinned_release(host);
+    scratch_free(blocks, s);
+}
+
+// What the tiled kernels are expected to take: the merged kernel, the one in tensor memory, and the copy of an input that is
+// not as they read it.  How the merged kernel fares depends on the columns that the rows of a block share: by the
+// density, by the counted loads, or as if every block's rows shared all of them, which is the least it can take.  Rows of
+// fewer than 29 channels are not merged: the estimate is by the density there, and on the low side (0.7 of the
+// time in the middle).  0 where it is not known.
+enum class Loads { least, density, counted };
+static double tiled_us(const spx_ell* e, const ConvParams& p4, const ConvViews& v, bool copies, uint32_t B, Loads by)
+{
+    MergedLoad load[3];
+    if (by == Loads::least) {
+        const double len = (double)e->nnz_total / e->m;
+        for (int k = 0; k < 3; ++k) {
+            const double work = std::min(16u >> k, (p4.Cout + kRbmRows - 1) / kRbmRows) * (0.7 + 0.2 * kRbmRows) * len;
+            load[k] = MergedLoad{len, work, len, work};
+        }
+    } else if (by == Loads::counted) {
+        for (int k = 0; k < 3; ++k) load[k] = MergedLoad{e->conv_loads[k][0], e->conv_loads[k][1], e->conv_loads[k][2], e->conv_loads[k][3]};
+    }
+    double us = conv_rbm_us(e, p4, by == Loads::density ? nullptr : load);
+    if (e->m >= 8 * kRbmRows - 3) us = std::min(us, conv_tmem_expected(e, p4, v, conv_rbm_us));
+    if (copies) us += 2.5 + 4e-6 / 3 * (double)p4.Cin * p4.H * p4.W * (p4.B + B);
+    return us < 1e20 ? us : 0.0;                // (a patch that no cut of the merged kernel stages)
+}
+
+// Whether gathering is expected to be faster than the tiled kernels: below 0.9 of their time, 0.85 where it takes four batch
+// entries a lane (both kinds' estimates are 10 % off for half of the shapes; at 0.95 two of a hundred calls took 5 to 16 %
+// longer).  Sure if it is so for the least that these can take, and not worth a count if it is not so by the density;
+// else the columns that rows share are counted, which the density does not tell.  Measured on 500 drawn shapes (300 of
+// them fitted to) the calls take 0.71 of the time they took before there was this kernel, with the faster one each time
+// 0.67; on 900 shapes with weights of eleven kinds (iid, rows of different density, channels, kernels or patterns removed)
+// 0.73, 3 of them more than 10 % longer.  By the density alone some structured kinds had calls 1.3 to 1.5 times as long.
+static bool gather_pays(spx_ell* e, const ConvParams& p4, const ConvViews& v, bool copies, uint32_t B, const ConvGatherPlan& plan, cudaStream_t s)
+{
+    const double us = plan.us / (plan.form >= 2 ? 0.85 : 0.9);
+    if (e->m < 8 * kRbmRows - 3) return us <= tiled_us(e, p4, v, copies, B, Loads::density);
+    if (e->conv_loads_state == 0) {
+        if (us <= tiled_us(e, p4, v, copies, B, Loads::least)) return true;
+        if (us > 1.05 * tiled_us(e, p4, v, copies, B, Loads::density)) return false;
+        count_loads(e, s);
+    }
+    return e->conv_loads_state == 1 && us <= tiled_us(e, p4, v, copies, B, Loads::counted);
+}
+
 // Batch size the tiled kernels run at: B rounded up to a multiple of 4, or further up to a multiple
 // of 16 when that is cheaper.  Cost per batch entry on 256 -> 256 channels, 3 x 3, 56 x 56, 80 %
 // sparse (ms per entry).  Merged kernel, which takes any multiple of 4 in segments of 16 / 8 / 4:
@@ -1152,7 +1266,11 @@ int launch_conv2d(spx_ell* e, const spx_conv_geom* g, int layout, const float* i
     const uint32_t B4 = padded_batch(B, merged_kernel_takes(e));
     ConvParams p4 = p;
     p4.B = B4;
-    if (e->r && e->cols_ascending && pf_tile_covers(p4)) {
+    const bool tiled = e->r && e->cols_ascending && pf_tile_covers(p4);
+    ConvGatherPlan gather;
+    const bool gathers = e->r && plan_conv_gather(e, p, layout, in, out, gather);
+    if (gathers && !tiled) return launch_conv_gather(e, p, layout, in, bias, act, out, gather, s);
+    if (tiled) {
         const uint64_t H = g->H, W = g->W, Ho = g->Ho, Wo = g->Wo;
         ConvViews v{};
         v.b_out = B;
@@ -1169,7 +1287,9 @@ int launch_conv2d(spx_ell* e, const spx_conv_geom* g, int layout, const float* i
         }
         v.vec_out = v.oB == 1 && B4 == B && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
         const float* src = in;
-        if (iB != 1 || B4 != B || (reinterpret_cast<uintptr_t>(in) & 15)) {
+        const bool copies = iB != 1 || B4 != B || (reinterpret_cast<uintptr_t>(in) & 15);
+        if (gathers && gather_pays(e, p4, v, copies, B, gather, s)) return launch_conv_gather(e, p, layout, in, bias, act, out, gather, s);
+        if (copies) {
             const uint64_t positions = g->Cin * H * W;
             const size_t need = positions * B4 * sizeof(float);
             if (e->conv_scratch_bytes < need)

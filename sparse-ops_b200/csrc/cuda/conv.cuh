@@ -24,10 +24,23 @@ struct MergedLoad {
     double longest = 0.0, work = 0.0, longest_worst = 0.0, work_worst = 0.0;
 };
 
+// From the blocks' (union columns, entries).
+void merged_loads(const uint2* blocks, uint32_t nblocks, MergedLoad (&out)[3]);
+
 // conv_tmem.cu: -1 when the shape or the handle is not for this kernel, or the other one's expected time is not above its own
 // (load: for 16, 8 and 4 blocks; null: by the density).
 int launch_conv_tmem(spx_ell* e, const ConvParams& p, const ConvViews& v, const float* in, const float* bias, int act, float* out,
                      double (*other_us)(const spx_ell*, const ConvParams&, const MergedLoad* load), cudaStream_t s);
+// Its expected time where it might be taken, 1e30 where it is not.
+double conv_tmem_expected(const spx_ell* e, const ConvParams& p, const ConvViews& v, double (*other_us)(const spx_ell*, const ConvParams&, const MergedLoad*));
+// conv_gather.cu: whether the kernel takes the shape, in which form and what time is expected.
+struct ConvGatherPlan {
+    int form = 0;
+    double us = 0.0;
+};
+bool plan_conv_gather(const spx_ell* e, const ConvParams& p, int layout, const float* in, const float* out, ConvGatherPlan& plan);
+int launch_conv_gather(const spx_ell* e, const ConvParams& p, int layout, const float* in, const float* bias, int act, float* out,
+                       const ConvGatherPlan& plan, cudaStream_t s);
 // conv.cu: the merged weights of conv_rbm_tile_kernel; -1 where there is no memory for them.
 int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s);
 void* new_conv_tmem();

@@ -527,21 +527,11 @@ void free_conv_tmem(spx_ell* e)
     e->conv_tmem = nullptr;
 }
 
-static void read_loads(conv_tmem_impl::Form& form, const CtaClocks* ctas, uint32_t groups, uint32_t nblocks)
+void merged_loads(const uint2* blocks, uint32_t nblocks, MergedLoad (&out)[3])
 {
-    for (int h = 0; h < 2; ++h)
-        for (int i = 0; i < kLaneGroups; ++i) {
-            double sum = 0.0;
-            for (uint32_t g = 0; g < groups; ++g) {
-                sum += ctas[g].c[h][i];
-                form.worst.c[h][i] = std::max(form.worst.c[h][i], ctas[g].c[h][i]);
-            }
-            form.mean.c[h][i] = (float)(sum / groups);
-        }
-    const uint2* blocks = reinterpret_cast<const uint2*>(ctas + groups);
     for (int k = 0; k < 3; ++k) {
         const uint32_t nb = 16u >> k;
-        MergedLoad& l = form.merged[k];
+        MergedLoad& l = out[k];
         for (uint32_t b0 = 0; b0 < nblocks; b0 += nb) {
             double longest = 0.0, work = 0.0;
             for (uint32_t b = b0; b < std::min(nblocks, b0 + nb); ++b) {
@@ -557,6 +547,20 @@ static void read_loads(conv_tmem_impl::Form& form, const CtaClocks* ctas, uint32
         l.longest /= n;
         l.work /= n;
     }
+}
+
+static void read_loads(conv_tmem_impl::Form& form, const CtaClocks* ctas, uint32_t groups, uint32_t nblocks)
+{
+    for (int h = 0; h < 2; ++h)
+        for (int i = 0; i < kLaneGroups; ++i) {
+            double sum = 0.0;
+            for (uint32_t g = 0; g < groups; ++g) {
+                sum += ctas[g].c[h][i];
+                form.worst.c[h][i] = std::max(form.worst.c[h][i], ctas[g].c[h][i]);
+            }
+            form.mean.c[h][i] = (float)(sum / groups);
+        }
+    merged_loads(reinterpret_cast<const uint2*>(ctas + groups), nblocks, form.merged);
     form.loads = true;
 }
 
@@ -743,6 +747,32 @@ static bool worth_it(const spx_ell* e, const ConvParams& p, const ConvViews& v, 
     return us < 1e30 && us <= (p.B % 32 ? 0.85 : 0.92) * other_us(e, p, nullptr);
 }
 
+static int tmem_env()
+{
+    // the switches that force the other kernels turn this one off
+    static const int env = [] {
+        if (const char* v = getenv("SPX_CONV_TMEM")) return atoi(v);
+        for (const char* k : {"SPX_CONV_RBM", "SPX_CONV_RBM_MIN_SHARE", "SPX_CONV_RBM_SEGMENTS", "SPX_CONV_CUT", "SPX_CONV_TMA"})
+            if (getenv(k)) return 0;
+        return 1;
+    }();
+    return env;
+}
+
+// Below 25 million FMAs a CTA's fixed cost decides (the smallest gains seen were at 16 million), and a call of 4 us
+// is the host's: it does without the estimates (3 -> 32, 21 x 21, batch 8 4.3 against 4.7 us).
+static bool too_small(const spx_ell* e, const ConvParams& p)
+{
+    return (p.B % 16 && p.Cout <= 32) || (double)e->nnz_total * p.Ho * p.Wo * p.B < 25e6;
+}
+
+double conv_tmem_expected(const spx_ell* e, const ConvParams& p, const ConvViews& v, double (*other_us)(const spx_ell*, const ConvParams&, const MergedLoad*))
+{
+    Cut first;
+    if (!tmem_env() || !e->conv_tmem || e->tma_off || p.B % 4 || too_small(e, p) || !plan(p, 4, p.B, first) || !worth_it(e, p, v, nullptr, other_us)) return 1e30;
+    return conv_tmem_us(e, p, v, nullptr);
+}
+
 template <int RW, int GP>
 static int launch_units(const spx_ell* e, const TmemArgs& a, const CUtensorMap& map, uint32_t ctas, cudaStream_t s)
 {
@@ -771,18 +801,10 @@ static int launch_cut(const spx_ell* e, TmemArgs a, const CUtensorMap& map, uint
 int launch_conv_tmem(spx_ell* e, const ConvParams& p, const ConvViews& v, const float* in, const float* bias, int act, float* out,
                      double (*other_us)(const spx_ell*, const ConvParams&, const MergedLoad*), cudaStream_t s)
 {
-    // the switches that force the other kernels turn this one off
-    static const int env = [] {
-        if (const char* v = getenv("SPX_CONV_TMEM")) return atoi(v);
-        for (const char* k : {"SPX_CONV_RBM", "SPX_CONV_RBM_MIN_SHARE", "SPX_CONV_RBM_SEGMENTS", "SPX_CONV_CUT", "SPX_CONV_TMA"})
-            if (getenv(k)) return 0;
-        return 1;
-    }();
+    const int env = tmem_env();
     const PFN_cuTensorMapEncodeTiled encode = tensor_map_encoder();
     if (!env || !e->conv_tmem || e->tma_off || e->max_nnz == 0 || p.B % 4 || !encode) return -1;
-    // Below 25 million FMAs a CTA's fixed cost decides (the smallest gains seen were at 16 million), and a call of 4 us
-    // is the host's: it does without the estimates (3 -> 32, 21 x 21, batch 8 4.3 against 4.7 us).
-    if (env != 2 && ((p.B % 16 && p.Cout <= 32) || (double)e->nnz_total * p.Ho * p.Wo * p.B < 25e6)) return -1;
+    if (env != 2 && too_small(e, p)) return -1;
     Cut first;                                  // what the form depends on is the same for all segments
     if (!plan(p, 4, p.B, first) || (env != 2 && !worth_it(e, p, v, nullptr, other_us))) return -1;
     const conv_tmem_impl::Form* form = nullptr;

@@ -1,0 +1,135 @@
+"""GPU: the convolution that gathers its operands (conv_gather.cu), forced, against the oracle bit for bit: edges of its tiles of
+positions, of batches of 32 entries and groups of 8 and 4, both widths of operands, all layouts; and when it is chosen.  The
+switch is read once per process, so the forced cases run in a child."""
+import os
+
+import numpy as np
+import pytest
+import torch
+
+import spx_ctypes as sx
+from conftest import assert_bit_equal
+from test_conv_tmem_gpu import assert_ran, child, kernels_of
+from test_parity_gpu import as_layout, dev, gpu_ell, ptr, sparse
+
+pytestmark = pytest.mark.gpu
+forced = pytest.mark.skipif(os.environ.get("SPX_CONV_GATHER") != "2", reason="runs in a child process")
+chosen = pytest.mark.skipif(any(k.startswith("SPX_CONV") for k in os.environ), reason="the choice is forced")
+
+# B, Cin, Cout, H, W, (kH, kW), (sH, sW), (dH, dW), density
+CASES = [(1, 3, 8, 4, 8, (3, 3), (1, 1), (1, 1), 0.5),          # one tile of 32 positions
+         (1, 5, 9, 3, 11, (3, 3), (1, 1), (1, 1), 1.0),         # a channel and a position over; rows of 45 entries
+         (3, 16, 33, 13, 12, (1, 1), (2, 2), (1, 1), 0.4),      # a tap, a stride
+         (5, 33, 7, 7, 6, (1, 1), (1, 1), (1, 1), 1.0),         # rows of 33 entries, fewer channels than warps
+         (4, 32, 24, 9, 9, (1, 1), (2, 1), (1, 1), 1.0),        # of 32, four batch entries a lane
+         (12, 4, 40, 17, 5, (5, 5), (2, 2), (1, 1), 0.2),
+         (32, 3, 65, 21, 20, (3, 3), (2, 1), (1, 1), 0.3),
+         (8, 6, 16, 15, 14, (3, 3), (1, 2), (2, 3), 0.4),       # dilated
+         (2, 3, 17, 9, 10, (4, 8), (1, 1), (1, 1), 0.5),        # 32 taps
+         (2, 3, 17, 9, 14, (3, 11), (1, 1), (1, 1), 0.5),       # 33: not for this kernel
+         (1, 2, 130, 66, 65, (3, 3), (1, 1), (1, 1), 0.6),      # many positions and channels, short rows
+         (32, 3, 200, 30, 31, (1, 1), (2, 2), (1, 1), 0.7)]
+
+
+@forced
+@pytest.mark.parametrize("off", [0, 1])
+@pytest.mark.parametrize("layout", [sx.LAYOUT_PF, sx.LAYOUT_NCHW, sx.LAYOUT_FMAJOR])
+@pytest.mark.parametrize("B,Cin,Cout,H,W,k,s,d,density", CASES)
+def test_forced_gather(lib, orc, cuda, layout, off, B, Cin, Cout, H, W, k, s, d, density):
+    """off: the tensors start a float off 16 bytes.  The first tap of the first output meets padding; weights there are
+    infinite in one row, so that w * 0 shows as it does in the reference."""
+    (kH, kW), (sH, sW), (dH, dW) = k, s, d
+    rng = np.random.default_rng([B, Cin, Cout, H, W, kH])
+    wt = sparse(rng, Cout, Cin * kH * kW, density)
+    wt[Cout // 2] = 0
+    wt[0, 0] = np.inf
+    x = rng.standard_normal((B, Cin, H, W)).astype(np.float32)
+    x[-1, -1, -1, -1] = np.nan
+    bias = rng.standard_normal(Cout).astype(np.float32)
+    pH, pW = (kH // 2) * dH, (kW // 2) * dW
+    src, E = as_layout(x, layout), orc.encode(wt)
+    want = orc.conv2d(E, dict(Cin=Cin, kH=kH, kW=kW, sH=sH, sW=sW, pH=pH, pW=pW, dH=dH, dW=dW, H=H, W=W), layout, src, B, bias, 1).reshape(-1)
+    h, g = gpu_ell(lib, E), sx.conv_geom(Cin, Cout, kH, kW, H, W, sH, sW, pH, pW, dH, dW)
+    dX = torch.empty(src.size + 4, device=cuda)
+    dX[off:off + src.size] = dev(src.reshape(-1), cuda)
+    dB = dev(bias, cuda)
+    out = torch.full((want.size + 8,), 7.0, device=cuda)
+    call = lambda: h.conv2d(g, layout, dX.data_ptr() + 4 * off, B, ptr(dB), sx.ACT_RELU, out.data_ptr() + 16 + 4 * off)
+    call()
+    names = kernels_of(call)
+    if kH * kW > 32:
+        assert names is None or "conv_gather_kernel" not in names
+    elif not (k == (1, 1) and s == (1, 1)):                 # such a one is an SpMM
+        assert_ran(names, "conv_gather_kernel")
+    got = out.cpu().numpy()
+    y, nan = got[4 + off:4 + off + want.size], np.isnan(want)
+    assert (np.isnan(y) == nan).all()
+    assert_bit_equal(np.where(nan, 0, y).astype(np.float32), np.where(nan, 0, want).astype(np.float32), "conv")
+    assert (got[:4 + off] == 7.0).all() and (got[4 + off + want.size:] == 7.0).all()
+
+
+@forced
+@pytest.mark.parametrize("B,layout", [(1, sx.LAYOUT_NCHW), (8, sx.LAYOUT_PF)])
+def test_forced_gather_any_column_order(lib, orc, cuda, B, layout):
+    """Rows whose columns do not ascend (only raw arrays have such): entries are added in storage order."""
+    rng = np.random.default_rng(4)
+    Cin, Cout, H = 6, 20, 9
+    E = orc.encode(sparse(rng, Cout, Cin * 9, 0.4))
+    for i in range(Cout):
+        p = rng.permutation(E.nnz[i])
+        E.idx[i, :E.nnz[i]], E.Wd[i, :E.nnz[i]] = E.idx[i, :E.nnz[i]][p], E.Wd[i, :E.nnz[i]][p]
+    src = as_layout(rng.standard_normal((B, Cin, H, H)).astype(np.float32), layout)
+    want = orc.conv2d(E, dict(Cin=Cin, kH=3, kW=3, sH=1, sW=1, pH=1, pW=1, dH=1, dW=1, H=H, W=H), layout, src, B, None, 0)
+    h, dX, dY = gpu_ell(lib, E), dev(src, cuda), torch.empty(want.shape, device=cuda)
+    h.conv2d(sx.conv_geom(Cin, Cout, 3, 3, H, H, 1, 1, 1, 1), layout, ptr(dX), B, None, 0, ptr(dY))
+    assert_bit_equal(dY.cpu().numpy(), want, "permuted rows")
+
+
+@chosen
+@pytest.mark.parametrize("shared,kernel", [(False, "conv_gather_kernel"), (True, "conv_rbm_tile_kernel")])
+def test_choice_of_gathering(lib, orc, cuda, shared, kernel):
+    """Rows that share all their columns are merged at a quarter of the work: 54 -> 100 channels, 5 x 5, batch 2 23 us against 34
+    gathered; of rows that share nothing the merged kernel takes longer."""
+    rng = np.random.default_rng(13)
+    Cin, Cout, H, W, B = 54, 100, 8, 63, 2
+    wt = rng.standard_normal((Cout, Cin * 25)).astype(np.float32)
+    wt[np.broadcast_to(rng.random((1 if shared else Cout, Cin * 25)) >= 0.436, wt.shape)] = 0
+    E = orc.encode(wt)
+    src = as_layout(rng.standard_normal((B, Cin, H, W)).astype(np.float32), sx.LAYOUT_PF)
+    want = orc.conv2d(E, dict(Cin=Cin, kH=5, kW=5, sH=1, sW=1, pH=2, pW=2, dH=1, dW=1, H=H, W=W), sx.LAYOUT_PF, src, B, None, 0)
+    h, dX, dY = gpu_ell(lib, E), dev(src, cuda), torch.empty(want.shape, device=cuda)
+    g = sx.conv_geom(Cin, Cout, 5, 5, H, W, 1, 1, 2, 2)
+    for _ in range(2):
+        dY.fill_(float("nan"))
+        assert_ran(kernels_of(lambda: h.conv2d(g, sx.LAYOUT_PF, ptr(dX), B, None, 0, ptr(dY))), kernel)
+        assert_bit_equal(dY.cpu().numpy(), want, kernel)
+
+
+@chosen
+def test_tiled_call_recorded_after_gathered_ones(lib, orc, cuda):
+    """Calls that gather need no merged weights; a later one that is recorded does, and has them: in the graph, and in an
+    eager call before the graph is launched."""
+    rng = np.random.default_rng(14)
+    C, H = 40, 12
+    E = orc.encode(sparse(rng, C, C * 9, 0.3))
+    gd = dict(Cin=C, kH=3, kW=3, sH=1, sW=1, pH=1, pW=1, dH=1, dW=1, H=H, W=H)
+    h, g = gpu_ell(lib, E), sx.conv_geom(C, C, 3, 3, H, H, 1, 1, 1, 1)
+    x = rng.standard_normal((32, C, H, H)).astype(np.float32)
+    one, many = as_layout(x[:1], sx.LAYOUT_PF), as_layout(x, sx.LAYOUT_PF)
+    w1, w32 = orc.conv2d(E, gd, sx.LAYOUT_PF, one, 1, None, 0), orc.conv2d(E, gd, sx.LAYOUT_PF, many, 32, None, 0)
+    d1, d32, y1, y32, z32 = dev(one, cuda), dev(many, cuda), torch.empty(w1.shape, device=cuda), torch.empty(w32.shape, device=cuda), torch.empty(w32.shape, device=cuda)
+    assert_ran(kernels_of(lambda: h.conv2d(g, sx.LAYOUT_PF, ptr(d1), 1, None, 0, ptr(y1))), "conv_gather_kernel")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        h.conv2d(g, sx.LAYOUT_PF, ptr(d32), 32, None, 0, ptr(y32), torch.cuda.current_stream().cuda_stream)
+    h.conv2d(g, sx.LAYOUT_PF, ptr(d32), 32, None, 0, ptr(z32))
+    assert_bit_equal(z32.cpu().numpy(), w32, "eager, before the graph")
+    graph.replay()
+    torch.cuda.synchronize()
+    assert_bit_equal(y32.cpu().numpy(), w32, "replayed")
+    assert_bit_equal(y1.cpu().numpy(), w1, "gathered")
+
+
+def test_forced_kernel():
+    child(["test_conv_gather_gpu.py", "test_parity_gpu.py", "test_fuzz_gpu.py"],
+          "forced_gather or conv_bit_exact or conv_views or conv_random or golden_conv", {"SPX_CONV_GATHER": "2"})
