@@ -17,7 +17,7 @@
 // of a group need not finish a chunk together, which would leave 19 (10 % dense) to 56 % (2 %) of the slots empty.
 //
 // Bound by shared-memory wavefronts (16 NV + 4 per step and warp) with many warps per SM, by the latency
-// of a warp's steps (0.1 us each) with few; chunks of 128 columns, six of them staged, lose 1 to 60 % to
+// of a warp's steps (0.04 us each, 0.05 with slices of 64) and the phases with few; chunks of 128 columns, six of them staged, lose 1 to 60 % to
 // the phases' fixed cost, 192 x 4 up to 4 %.  Measured against gathering: 4096 x 4096, 10 %, C = 64 / 128 / 256 / 512
 // 23.9 / 35.4 / 61.3 / 121.7 us against 28.4 / 42.3 / 72.1 / 142.4 (groups in step: 24.7 / 41.3 / 76 / 144);
 // 8192 x 8192, 10 %, C = 64 68 against 105; 3512 x 3227, 19 %, C = 160 61 against 109; 4927 x 3082, 21 %, C = 160 93 against 170.
@@ -198,7 +198,7 @@ __device__ __forceinline__ void tile_steps(float4 (&acc)[NV], uint32_t at, uint3
     }
 }
 
-// X with rows of C floats at any alignment into rows of Cp floats (a multiple of 4), zeros behind.
+// X with rows of C floats at any alignment into rows of Cp floats (a multiple of 8, at least 32), zeros behind.
 __global__ void __launch_bounds__(256)
 align_rows_kernel(const float* __restrict__ X, uint64_t ldx, uint32_t n, uint32_t C, uint32_t Cp, float* __restrict__ dst)
 {
@@ -209,7 +209,8 @@ align_rows_kernel(const float* __restrict__ X, uint64_t ldx, uint32_t n, uint32_
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t k = (uint32_t)(i / quads), c = (uint32_t)(i - (uint64_t)k * quads) * 4;
         const float* __restrict__ p = X + (size_t)k * ldx + c;
-        float4 v = make_float4(__ldg(p), 0.f, 0.f, 0.f);
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (c < C) v.x = __ldg(p);
         if (c + 1 < C) v.y = __ldg(p + 1);
         if (c + 2 < C) v.z = __ldg(p + 2);
         if (c + 3 < C) v.w = __ldg(p + 3);
@@ -217,10 +218,16 @@ align_rows_kernel(const float* __restrict__ X, uint64_t ldx, uint32_t n, uint32_
     }
 }
 
-template <int NV>
-__global__ void __launch_bounds__(kMaxWarps * 32, 1)
+// For CTAs of up to WARPS warps.  kMaxWarps of them pass their gathers at the rate of shared memory with one step's operands
+// in registers; fewer wait for their own latencies, and have registers for two steps (kDeep below).  2048 x 2048, 30 %,
+// C = 32 16.6 -> 11.2 us, 640 x 1955, 35 %, C = 35 18.9 -> 14.0; 4096 x 4096, 10 %, C = 64 24.7 -> 19.3; 3001 x 4999, 6 %,
+// C = 64 19.0 -> 15.5.  The steps' places in their blocks are known to the compiler: with one loop of steps, whose next block
+// and register set are found at run time, these were 16.1, -, 21.6 and 16.6.
+template <int NV, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 1)
 spmm_tile_kernel(const __grid_constant__ TileArgs a, const __grid_constant__ CUtensorMap tmap)
 {
+    constexpr bool kDeep = WARPS < (int)kMaxWarps;
     constexpr uint32_t kPitch = NV * 128u;                  // bytes of a staged row of X
     constexpr uint32_t kBox = kChunk * kPitch;              // bytes of a staged chunk
     extern __shared__ __align__(128) unsigned char s_mem[]; // [kStages] chunks of X, a row of zeros, a ring per warp
@@ -285,27 +292,116 @@ spmm_tile_kernel(const __grid_constant__ TileArgs a, const __grid_constant__ CUt
     const uint32_t xbase = (uint32_t)__cvta_generic_to_shared(s_mem) + l * 16;
     uint32_t step = 0;                          // of the group's stream
     bool landed = true;
+    // kDeep.  Registers for two steps, the even and the odd ones of the stream: a step's operands are asked for before the
+    // step in front of it is multiplied, its ids right after the operands of that step's predecessor, its weights once that
+    // one is multiplied.  Operands only within a phase: the next chunk may not have landed (looking across it, with the wait
+    // in the step, made every case slower, 11.2 to 14.2 us at 2048 x 2048, 30 %, C = 32).
+    float4 w0, w1, k0, k1, x0[4][NV], x1[4][NV];
+    auto place = [&](uint32_t st) { return ring + ((st & 15u) * 128u) + r * 16; };
+    auto next_block = [&](uint32_t blk) {       // entering it: it has landed, and the one before the last is free
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+        fill(blk + 2);
+    };
+    auto ids = [&](float4& k, uint32_t st) {
+        if ((st & 3u) == 0) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncwarp();
+            if (st) fill(st / 4 + 2);
+        }
+        k = lds128(place(st) + 64);
+    };
+    auto operands = [&](float4 (&x)[4][NV], const float4& k) {
+        const uint32_t id[4] = {__float_as_uint(k.x), __float_as_uint(k.y), __float_as_uint(k.z), __float_as_uint(k.w)};
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int v = 0; v < NV; ++v) x[u][v] = lds128(xbase + id[u] * (NV * 128u) + v * 128u);
+    };
+    auto multiply = [&](const float4& w, const float4 (&x)[4][NV]) {
+        const float wv[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                acc[v].x = fmaf(wv[u], x[u][v].x, acc[v].x);
+                acc[v].y = fmaf(wv[u], x[u][v].y, acc[v].y);
+                acc[v].z = fmaf(wv[u], x[u][v].z, acc[v].z);
+                acc[v].w = fmaf(wv[u], x[u][v].w, acc[v].w);
+            }
+    };
+    // The stream's next step, POS % 4 of its block (kOdd: 1 or 3); whether another of the phase follows.
+    constexpr int kOdd = 5;
+    auto one = [&](auto pos, bool more) {
+        constexpr int POS = decltype(pos)::value;
+        float4 (&x)[4][NV] = POS & 1 ? x1 : x0;
+        float4 (&xn)[4][NV] = POS & 1 ? x0 : x1;
+        float4 &w = POS & 1 ? w1 : w0, &kn = POS & 1 ? k0 : k1;
+        if (more) {
+            operands(xn, kn);
+            if (POS == 1 || (POS == kOdd && (step & 2u) == 0)) next_block((step + 3) / 4);
+            kn = lds128(place(step + 3) + 64);
+        }
+        multiply(w, x);
+        w = lds128(place(step + 2));
+        ++step;
+    };
+    if constexpr (kDeep) {
+        ids(k0, 0);
+        ids(k1, 1);
+        w0 = lds128(place(0));
+        w1 = lds128(place(1));
+    }
     for (uint32_t c = 0; c < a.chunks; ++c) {
         if (c && (c & 31u) == 0) my_cnt = c + lane < a.chunks ? __ldg(a.cnt + (size_t)group * a.chunks + c + lane) : 0u;
         const uint32_t all = __shfl_sync(0xffffffffu, my_cnt, c & 31u);
         if (landed) landed = spx::mbar_wait(&s_bar[c % kStages], (c / kStages) & 1u);
-        for (uint32_t s = 0; s < all;) {
-            const uint32_t in_block = step & 3u, n = min(4u - in_block, all - s);
-            if (in_block == 0) {                // entering a block of the ring: it has landed, and the one before is free
-                if (ring_mask == 1) asm volatile("cp.async.wait_group 0;" ::: "memory");
-                else asm volatile("cp.async.wait_group 2;" ::: "memory");
-                __syncwarp();
-                fill(step / 4 + ring_mask);
+        if constexpr (kDeep) {
+            using std::integral_constant;
+            constexpr integral_constant<int, 0> p0{};
+            constexpr integral_constant<int, 1> p1{};
+            constexpr integral_constant<int, 2> p2{};
+            constexpr integral_constant<int, 3> p3{};
+            constexpr integral_constant<int, kOdd> p_odd{};
+            uint32_t left = all;                // up to the end of a block, whole blocks, the rest
+            if (left) {
+                if (step & 1u) { operands(x1, k1); ids(k1, step + 2); one(p_odd, --left != 0); }
+                else { operands(x0, k0); ids(k0, step + 2); }
+                if (left && (step & 2u)) {
+                    one(p2, --left != 0);
+                    if (left) one(p3, --left != 0);
+                }
+                for (; left >= 4; left -= 4) {
+                    one(p0, true);
+                    one(p1, true);
+                    one(p2, true);
+                    one(p3, left > 4);
+                }
+                if (left) {
+                    one(p0, --left != 0);
+                    if (left) one(p1, --left != 0);
+                    if (left) one(p2, false);
+                }
             }
-            const uint32_t at = ring + ((step & (4 * ring_mask + 3)) * 128u) + r * 16;
-            switch (n) {                        // unrolled: the hand-off and the gathers of a step run ahead of its FMAs
-            case 1: tile_steps<NV, 1>(acc, at, xbase); break;
-            case 2: tile_steps<NV, 2>(acc, at, xbase); break;
-            case 3: tile_steps<NV, 3>(acc, at, xbase); break;
-            default: tile_steps<NV, 4>(acc, at, xbase);
+        } else {
+            for (uint32_t s = 0; s < all;) {
+                const uint32_t in_block = step & 3u, n = min(4u - in_block, all - s);
+                if (in_block == 0) {                // entering a block of the ring: it has landed, and the one before is free
+                    if (ring_mask == 1) asm volatile("cp.async.wait_group 0;" ::: "memory");
+                    else asm volatile("cp.async.wait_group 2;" ::: "memory");
+                    __syncwarp();
+                    fill(step / 4 + ring_mask);
+                }
+                const uint32_t at = ring + ((step & (4 * ring_mask + 3)) * 128u) + r * 16;
+                switch (n) {                        // unrolled: the hand-off and the gathers of a step run ahead of its FMAs
+                case 1: tile_steps<NV, 1>(acc, at, xbase); break;
+                case 2: tile_steps<NV, 2>(acc, at, xbase); break;
+                case 3: tile_steps<NV, 3>(acc, at, xbase); break;
+                default: tile_steps<NV, 4>(acc, at, xbase);
+                }
+                s += n;
+                step += n;
             }
-            s += n;
-            step += n;
         }
         if (c + 1 < kWindow) continue;
         __syncwarp();
@@ -442,37 +538,44 @@ static int build_tiles(spx_ell* e, spx_tiles_impl* t, cudaStream_t s)
     return SPX_OK;
 }
 
-template <int NV>
+template <int NV, int WARPS>
 static int launch_tile_nv(const spx_ell* e, TileArgs a, const CUtensorMap& map, uint32_t warps, uint32_t slices, cudaStream_t s)
 {
     a.row_blocks = (a.groups + warps - 1) / warps;
-    a.ring_blocks = warps > 14 ? 2 : 4;
-    const size_t smem = (size_t)(kStages * kChunk + 1) * NV * 128 + (size_t)warps * a.ring_blocks * 512;
-    if (int rc = allow_smem<spmm_tile_kernel<NV>>(e->device)) return rc;
-    SPX_CUDA(launch_pdl(spmm_tile_kernel<NV>, dim3(a.row_blocks * slices), dim3(warps * 32), smem, s, a, map));
+    a.ring_blocks = WARPS < (int)kMaxWarps ? 4 : 2;
+    size_t smem = (size_t)(kStages * kChunk + 1) * NV * 128 + (size_t)warps * a.ring_blocks * 512;
+    // One CTA to an SM where the grid is one wave: started while the kernel before still fills some of the SMs, two small ones
+    // share one and take twice as long (435 x 3968, 35 %, C = 274, behind the copy of X: 61 us against 34).
+    if (a.row_blocks * slices <= sm_count(e->device)) smem = std::max<size_t>(smem, 116 * 1024);
+    if (int rc = allow_smem<spmm_tile_kernel<NV, WARPS>>(e->device)) return rc;
+    SPX_CUDA(launch_pdl(spmm_tile_kernel<NV, WARPS>, dim3(a.row_blocks * slices), dim3(warps * 32), smem, s, a, map));
     count_launch();
     return SPX_OK;
 }
 
 namespace {
 
+// The kernel for CTAs of `warps`: the one that keeps two steps' operands in registers, compiled for at most so many warps; 0: none.
+constexpr uint32_t deep_limit(uint32_t NV, uint32_t warps) {
+    return NV == 1 ? (warps <= 20 ? 20u : warps <= 24 ? 24u : 0u) : warps <= 16 ? 16u : 0u;
+}
+
 struct Plan {
-    uint32_t slices, warps;
+    uint32_t slices, warps, deep;
     uint64_t waves;
     double us;
 };
 
 // Launch shape and expected time.  As few waves of CTAs as kMaxWarps warps each allow, and then equally
-// many warps in every CTA.  Time: the results' way out, about half a microsecond per phase (wait, hand-off, a
-// block of steps cut short; more where X's rows do not begin on lines), and per step of a warp the
+// many warps in every CTA.  Time: a third of a microsecond per phase (wait, hand-off, a block of steps cut short; more where
+// X's rows do not begin on sectors, or end inside a line), and per step of a warp the
 // larger of its latency and the shared-memory wavefronts of all the SM's warps (16 NV gathers + 4 of hand-off).
 // A phase in which any row of a group has an entry due takes a step, however few they are: rows of less than a
 // few entries per chunk are mostly empty slots (60000 x 4000, 8 entries a row, C = 33: 91 us against 30 gathered).
-// The constants of both estimates are fitted to 1564 measured shapes (256 to 150000 rows, 256 to 60000 columns, 3 to 2500
-// entries a row, C = 1 to 1000): the kernel they choose takes 0.2 % longer than the faster one on average, more
-// than 10 % longer for 14 of them (without that term, and with one kind of gather for every unaligned X: 1.6 %, 58, and
-// up to 3.6 times).
-Plan plan_tiles(const spx_ell* e, uint32_t C, uint32_t NV, uint32_t sms, bool aligned)
+// The constants of both estimates are fitted to 593 measured shapes (256 to 150000 rows, 256 to 60000 columns, 4 to 3200
+// entries a row, C = 1 to 1000): the kernel they choose takes 0.8 % longer than the fastest of the three (gathered, slices of
+// 32 and of 64) on average, more than 10 % longer for 16 of them.
+Plan plan_tiles(const spx_ell* e, uint32_t C, uint32_t NV, uint32_t sms, bool aligned, bool sectors)
 {
     Plan p;
     const uint32_t groups = (e->m + kGroupRows - 1) / kGroupRows, chunks = (e->n + kChunk - 1) / kChunk;
@@ -485,10 +588,13 @@ Plan plan_tiles(const spx_ell* e, uint32_t C, uint32_t NV, uint32_t sms, bool al
         while (p.warps < kMaxWarps && ctas() > p.waves * sms) ++p.warps;
         if (ctas() <= p.waves * sms) break;
     }
+    p.deep = deep_limit(NV, p.warps);
     const double len = (double)e->nnz_total / e->m;
     const double steps = std::max((len + 1.1 * std::sqrt(len)) / 4.0, chunks * (1.0 - std::exp(-(double)kGroupRows * len / chunks)));
-    p.us = 0.9 + (double)e->m * C * 0.62e-6 + (C % 32 ? 0.17 * chunks : 0.0) + (aligned ? 0.0 : 3.5) +
-           p.waves * (2.65 + chunks * (NV == 1 ? 0.45 : 0.40) + steps * std::max(NV == 1 ? 0.0515 : 0.096, p.warps * (16.0 * NV + 4.0) / 2480.0));
+    const double chunk = !p.deep ? 0.365 : p.deep == 24 ? 0.333 : 0.313;
+    const double step = std::max(!p.deep ? 0.0 : NV == 1 ? 0.036 : 0.051, p.warps * (16.0 * NV + 4.0) / 2060.0);
+    p.us = 0.6 + (C % 32 && !(C < 32 && !aligned) ? 0.04 * chunks : 0.0) + (sectors ? 0.0 : 0.12 * chunks) + (aligned ? 0.0 : 3.2) +
+           p.waves * ((NV == 1 ? 1.9 : 2.6) + chunks * chunk + steps * step);
     return p;
 }
 
@@ -505,16 +611,18 @@ double gather_us(const spx_ell* e, uint32_t C, uint32_t V, bool half)
     const bool brief = e->nnz_total < 100ull * e->m;
     const double load = V == 4 ? 3.15e-3 : V == 2 ? 1.7e-3 : 1.34e-3, off_lines = V == 4 ? 0.47e-3 : V == 2 ? 0.5e-3 : 0.39e-3;
     double loads = e->nnz_total / sms * panels * (load * NV / RW + (C % 32 ? off_lines : 0.0)) + (brief ? 0.037 : 0.10) * per_sm;
+    if (V == 4 && NV == 2 && per_sm >= 12 && !brief)        // 16 warps reside: a last round of a few takes as long as a full one
+        loads = e->nnz_total / sms * panels * (5.5e-3 + (C % 32 ? off_lines : 0.0)) * std::ceil(per_sm / 16.0) * 16.0 / per_sm;
     if (V == 4 && RW > 1 && !brief) {           // long rows side by side in a warp: half as if each took a power of two of lanes
         uint32_t lanes = 1;
         while (lanes < q) lanes *= 2;
         loads = e->nnz_total / sms * 2.0e-3 * (lanes / 32.0 + 1.0 / RW) + 0.10 * per_sm;
     }
     double rounds = e->max_nnz;
-    if (V == 1 && per_sm < 12) rounds *= 0.0115 * NV * (NV == 3 ? std::ceil(per_sm / 8.0) : 1.0);
-    else rounds *= (NV == 1 ? 0.0168 * (V == 4 && RW > 1 && !brief ? 1.0 + 0.03 * RW : 1.0) : 0.0282) * (NV == 1 && (per_sm < 48 || !brief) ? std::max(1.0, std::ceil(per_sm / 8.0)) : 1.0);
+    if (V == 1 && per_sm < 12) rounds *= NV == 1 ? 0.0147 : 0.0115 * NV * (NV == 3 ? std::ceil(per_sm / 8.0) : 1.0);
+    else rounds *= (NV == 1 ? 0.0168 * (V == 4 && RW > 1 && !brief ? 1.0 + 0.03 * RW : 1.0) : 0.0282) * (V > 1 && NV == 1 && (per_sm < 48 || !brief) ? std::max(1.0, std::ceil(per_sm / 8.0)) : 1.0);
     const double l2 = loads * loads, r2 = rounds * rounds;
-    return (3.5 + std::sqrt(std::sqrt(l2 * l2 + r2 * r2))) * (half ? 0.9 : 1.0);
+    return (3.5 + std::sqrt(std::sqrt(l2 * l2 + r2 * r2))) * (half ? 0.98 : 1.0);
 }
 
 }  // namespace
@@ -528,27 +636,21 @@ int launch_spmm_tile(spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const
     const PFN_cuTensorMapEncodeTiled encode = tensor_map_encoder();
     if (!encode || ldx > 0xffffffffull || e->n > 65536 || C > (1u << 30) || (env != 2 && e->n < kChunk)) return -1;
     // Slices of 64 columns read the entries half as often, slices of 32 leave fewer columns idle and give the SMs more
-    // warps.  Of 500 shapes (256 to 8192 rows and columns, 2 to 50 %, C = 33 to 1024, 33 to 160 more often than not), the
-    // narrow ones are faster for 283 (3001 x 4999, 6 %, C = 77 24.2 us against 28.7; 600 x 3000, 30 %, C = 128 25.0 / 31.1),
-    // the wide ones for 177 (6000 x 6000, 5 %, C = 93 46.4 / 48.3).  The choice takes 0.3 % longer than the better one on
-    // average, 10 % longer for 3, and 0.93 of what wide slices took; without the 1.5 us, by which the narrow kernel's estimate
-    // is high, 1.7 % and 36.
+    // warps.  Of 411 shapes with C > 32 (256 to 8192 rows and columns, 2 to 50 %), the narrow ones are faster by more than 2 %
+    // for 191 (3001 x 4999, 6 %, C = 77 21.5 us against 25.6; 600 x 3000, 30 %, C = 128 18.6 / 25.1), the wide ones for 220
+    // (4096 x 4096, 10 %, C = 100 33.4 / 37.7).  The choice takes 0.3 % longer than the better one on average.
     const uint32_t sms = sm_count(e->device);
-    Plan p = plan_tiles(e, C, 1, sms, vec_x);
+    const bool sectors = !vec_x || (ldx % 8 == 0 && reinterpret_cast<uintptr_t>(X) % 32 == 0);
+    Plan p = plan_tiles(e, C, 1, sms, vec_x, sectors);
     uint32_t NV = 1;
-    const double gather = gather_us(e, C, V, half);
-    bool faster = p.us <= 1.05 * gather;
     if (C > 32) {
-        const Plan wide = plan_tiles(e, C, 2, sms, vec_x);
-        if (p.us >= wide.us + 1.5) {
+        const Plan wide = plan_tiles(e, C, 2, sms, vec_x, sectors);
+        if (p.us > wide.us) {
             p = wide;
             NV = 2;
         }
-        // Against gathering the narrow estimate is trusted less: at 0.92 the same shapes take 0.98 of the time that wide
-        // slices alone did, one of them 5 % more; at 1.05 two of a hundred take 5 % and more longer (1920 x 896, 20 %, C = 50
-        // 12.0 us against 9.4 gathered).
-        faster = wide.us <= 1.05 * gather || (NV == 1 && p.us <= 0.92 * gather);
     }
+    const bool faster = p.us <= gather_us(e, C, V, half);
     if ((uint64_t)p.slices * e->m > 0x7fffffffull) return -1;
     if (env != 2 && !faster) return -1;
     spx_tiles_impl* t = static_cast<spx_tiles_impl*>(e->tiles);
@@ -567,8 +669,8 @@ int launch_spmm_tile(spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const
         if (t->state != 1) return -1;
     }
     void* aligned = nullptr;
-    const uint32_t Cp = round_up(C, 4u);
-    if (!vec_x) {                               // bulk copies need 16-byte rows: X moves into scratch that has them
+    const uint32_t Cp = C < 32 ? 32u : round_up(C, 8u);
+    if (!vec_x) {                               // bulk copies need 16-byte rows, and are faster with whole sectors: X moves into scratch that has them
         if (int rc = scratch_alloc(&aligned, (size_t)e->n * Cp * 4, e->device, s)) return rc == SPX_ERR_OOM ? -1 : rc;
         const uint64_t quads = (uint64_t)e->n * (Cp / 4);
         const unsigned blocks = (unsigned)std::min<uint64_t>((quads + 255) / 256, (uint64_t)sm_count(e->device) * 16);
@@ -595,7 +697,9 @@ int launch_spmm_tile(spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const
         static const int timeout_env = [] { const char* v = getenv("SPX_SPMM_TMA_TEST_TIMEOUT"); return v ? atoi(v) : 0; }();
         static std::atomic<int> launches{0};
         if (timeout_env && ++launches == timeout_env) a.missing = 16;
-        rc = NV == 1 ? launch_tile_nv<1>(e, a, map, p.warps, p.slices, s) : launch_tile_nv<2>(e, a, map, p.warps, p.slices, s);
+        const auto launch = NV == 1 ? (p.deep == 20 ? launch_tile_nv<1, 20> : p.deep == 24 ? launch_tile_nv<1, 24> : launch_tile_nv<1, kMaxWarps>)
+                                    : (p.deep == 16 ? launch_tile_nv<2, 16> : launch_tile_nv<2, kMaxWarps>);
+        rc = launch(e, a, map, p.warps, p.slices, s);
     }
     scratch_free(aligned, s);
     return rc;

@@ -225,3 +225,42 @@ def test_one_call_in_parts_builds_nothing(lib, orc, cuda):
         counts.append(lib.spx_launch_count() - before)
     torch.cuda.synchronize()
     assert counts == [3, 5, 3]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,C", [
+    # CTAs of 1, 20, 21, 24 and 25 warps for slices of 32 columns (9, 23: X moves into rows of 32 floats), and of 16 and 17
+    # for slices of 64: where the kernels with two steps' operands in registers begin and end
+    (4, 32), (7, 9), (11840, 32), (12000, 23), (14208, 32), (14400, 32), (9472, 64), (9600, 61), (592, 256), (600, 274)])
+def test_phases(lib, orc, cuda, m, C):
+    """Blocks of 256 columns that some rows do not use and others are full of: phases of no step, of one, of a few that
+    begin or end inside a block of four, and of many."""
+    if os.environ.get("SPX_SPMM_TILE") != "2":
+        pytest.skip("runs in a child process of test_phases_forced")
+    rng = np.random.default_rng([m, C])
+    n = 1800
+    share = rng.choice([0.0, 0.004, 0.02, 0.06, 0.3], (m, 8), p=[0.3, 0.2, 0.2, 0.2, 0.1]).astype(np.float32)
+    W = rng.standard_normal((m, n), dtype=np.float32)
+    W[rng.random((m, n), dtype=np.float32) >= np.repeat(share, 256, axis=1)[:, :n]] = 0
+    W[m // 2] = 0
+    E = orc.encode(W)
+    X = (np.arange(n, dtype=np.float32)[:, None] + rng.uniform(-1, 1, (n, C))).astype(np.float32)
+    rows = np.unique(np.concatenate([np.arange(0, m, max(1, m // 200)), [m // 2, m - 1], np.argsort(E.nnz)[-8:]]))
+    from oracle import EllArrays
+    want = orc.spmm(EllArrays(len(rows), n, E.r, E.Wd[rows], E.idx[rows], E.nnz[rows]), X, None)
+    h = lib.ell_create(E.Wd, E.idx, E.nnz, E.n)
+    dX = torch.from_numpy(X).to(cuda)
+    first = None
+    for call in range(6):
+        dY = torch.full((m, C), float("nan"), device=cuda)
+        h.spmm(dX.data_ptr(), C, C, 0, sx.ACT_NONE, dY.data_ptr(), C)
+        torch.cuda.synchronize()
+        if first is None:
+            first = dY
+            assert_bit_equal(dY[torch.from_numpy(rows).to(cuda)].cpu().numpy(), want, "sampled rows")
+        assert torch.equal(dY.view(torch.int32), first.view(torch.int32)), f"call {call} differs from the first (gathered) one"
+
+
+@pytest.mark.gpu
+def test_phases_forced():
+    in_child("test_phases", SPX_SPMM_TILE="2")
