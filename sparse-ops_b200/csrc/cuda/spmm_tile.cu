@@ -19,8 +19,8 @@
 // Bound by shared-memory wavefronts (16 NV + 4 per step and warp) with many warps per SM, by the latency
 // of a warp's steps (0.04 us each, 0.05 with slices of 64) and the phases with few; chunks of 128 columns, six of them staged, lose 1 to 60 % to
 // the phases' fixed cost, 192 x 4 up to 4 %.  Measured against gathering: 4096 x 4096, 10 %, C = 64 / 128 / 256 / 512
-// 23.9 / 35.4 / 61.3 / 121.7 us against 28.4 / 42.3 / 72.1 / 142.4 (groups in step: 24.7 / 41.3 / 76 / 144);
-// 8192 x 8192, 10 %, C = 64 68 against 105; 3512 x 3227, 19 %, C = 160 61 against 109; 4927 x 3082, 21 %, C = 160 93 against 170.
+// 19.5 / 32.7 / 61.5 / 121.7 us against 26.1 / 43.5 / 72.5 / 141.6; 8192 x 8192, 10 %, C = 64 62.9 against 103;
+// 3512 x 3227, 19 %, C = 160 59.5 against 106; 4927 x 3082, 21 %, C = 160 86.8 against 159.
 #include "common.cuh"
 #include "tma.cuh"
 #include "peer_out.cuh"
@@ -593,7 +593,10 @@ Plan plan_tiles(const spx_ell* e, uint32_t C, uint32_t NV, uint32_t sms, bool al
     const double steps = std::max((len + 1.1 * std::sqrt(len)) / 4.0, chunks * (1.0 - std::exp(-(double)kGroupRows * len / chunks)));
     const double chunk = !p.deep ? 0.365 : p.deep == 24 ? 0.333 : 0.313;
     const double step = std::max(!p.deep ? 0.0 : NV == 1 ? 0.036 : 0.051, p.warps * (16.0 * NV + 4.0) / 2060.0);
-    p.us = 0.6 + (C % 32 && !(C < 32 && !aligned) ? 0.04 * chunks : 0.0) + (sectors ? 0.0 : 0.12 * chunks) + (aligned ? 0.0 : 3.2) +
+    double rows = sectors ? 0.0 : 0.12;                     // us per chunk, for the copies of X's rows
+    if (C < 32 && aligned) rows = (C % 8 ? 14.0 : 5.0) / C;     // shorter than a box is wide (2080 x 613, C = 4: 3 us a chunk)
+    else if (C % 32 && C > 32) rows += 0.04;
+    p.us = 0.6 + rows * chunks + (aligned ? 0.0 : 3.2) +
            p.waves * ((NV == 1 ? 1.9 : 2.6) + chunks * chunk + steps * step);
     return p;
 }
@@ -650,7 +653,12 @@ int launch_spmm_tile(spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const
             NV = 2;
         }
     }
-    const bool faster = p.us <= gather_us(e, C, V, half);
+    // By 1.2 us where gathering takes less than 4.5, 0.8 from 6 to 8, by none from 14 on: the estimates are fitted to calls of
+    // 10 us and more, and one of 2 us takes 1 longer staged (245 shapes of up to 2500 rows and columns: 60 of the 130 that
+    // gather in less than 4 us took 5 % longer without it, none with it), nor is it worth the form.
+    const double gather = gather_us(e, C, V, half);
+    const double by = 0.8 * std::clamp((14.0 - gather) / 6.0, 0.0, 1.0) + 0.4 * std::clamp((6.0 - gather) / 1.5, 0.0, 1.0);
+    const bool faster = p.us + by <= gather;
     if ((uint64_t)p.slices * e->m > 0x7fffffffull) return -1;
     if (env != 2 && !faster) return -1;
     spx_tiles_impl* t = static_cast<spx_tiles_impl*>(e->tiles);
