@@ -6,7 +6,7 @@
 // stride, the last three of four batch entries are padding, and NCHW images are copied first.  Here a warp takes one output
 // channel at 32 V positions and loads each operand when it needs it: no staging, no copy, no padding, any batch and layout.
 //
-// Bound by issue slots (65 to 70 % used; some 8 an operand, 200 to 300 a warp for its ends), L1 wavefronts (50 %; a stride
+// Bound by issue slots (65 to 70 % used; 6 to 9 an operand, 200 to 400 a warp for its ends), L1 wavefronts (50 %; a stride
 // of two or positions that are not neighbours in memory take two to 32 a load) and, with few warps, by the round trips of a
 // row's entries, 8 at a time.  Measured against the tiled kernels: 64 -> 128 channels, 3 x 3, stride 2, 57 x 57, batch 3,
 // NCHW 28 -> 15 us; 219 -> 32, 3 x 3, stride 2, 104 x 104, batch 1 100 -> 17; 384 -> 25, 3 x 3, 9 x 9, batch 27 300 -> 44; 96 -> 214,
@@ -45,31 +45,42 @@ struct GatherArgs {
     uint32_t tiles;
 };
 
-// Predicated, not branched: the loads of a group are on their way together.  The tap's bit of the mask is moved to the sign.
-template <bool CHECK, int VEC>
-__device__ __forceinline__ void load_vec(float (&d)[VEC], const float* __restrict__ p, uint32_t mask, uint32_t entry) {
-    if constexpr (VEC == 4 && CHECK)
-        asm("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\tshf.l.wrap.b32 t, 0, %5, %6;\n\tsetp.lt.s32 p, t, 0;\n\tmov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\t"
-            "mov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t@p ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
-            : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "l"(p), "r"(mask), "r"(entry));
-    else if constexpr (VEC == 4)
-        asm("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "l"(p));
-    else if constexpr (CHECK)
-        asm("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\tshf.l.wrap.b32 t, 0, %2, %3;\n\tsetp.lt.s32 p, t, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
-            "@p ld.global.nc.f32 %0, [%1];\n\t}" : "=f"(d[0]) : "l"(p), "r"(mask), "r"(entry));
-    else
-        asm("ld.global.nc.f32 %0, [%1];" : "=f"(d[0]) : "l"(p));
+// Predicated, not branched: the loads of a group are on their way together.  The tap's bit of the mask, which is moved to the
+// sign by a tap's number (PACK), or met by its bit.
+template <bool PACK, bool CHECK, int VEC>
+__device__ __forceinline__ void load_vec(float (&d)[VEC], const void* __restrict__ p, uint32_t mask, uint32_t tap) {
+#define SPX_LOAD4(TEST)                                                                                                          \
+    asm("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\t" TEST "mov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\t"                   \
+        "mov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t@p ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"             \
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "l"(p), "r"(mask), "r"(tap))
+#define SPX_LOAD1(TEST)                                                                                                          \
+    asm("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\t" TEST "mov.f32 %0, 0f00000000;\n\t@p ld.global.nc.f32 %0, [%1];\n\t}"           \
+        : "=f"(d[0]) : "l"(p), "r"(mask), "r"(tap))
+    if constexpr (VEC == 4 && CHECK && PACK) SPX_LOAD4("shf.l.wrap.b32 t, 0, %5, %6;\n\tsetp.lt.s32 p, t, 0;\n\t");
+    else if constexpr (VEC == 4 && CHECK) SPX_LOAD4("and.b32 t, %5, %6;\n\tsetp.ne.u32 p, t, 0;\n\t");
+    else if constexpr (VEC == 4) asm("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "l"(p));
+    else if constexpr (CHECK && PACK) SPX_LOAD1("shf.l.wrap.b32 t, 0, %2, %3;\n\tsetp.lt.s32 p, t, 0;\n\t");
+    else if constexpr (CHECK) SPX_LOAD1("and.b32 t, %2, %3;\n\tsetp.ne.u32 p, t, 0;\n\t");
+    else asm("ld.global.nc.f32 %0, [%1];" : "=f"(d[0]) : "l"(p));
+#undef SPX_LOAD4
+#undef SPX_LOAD1
 }
 
 // A CTA computes 8 output channels, one a warp, at 32 V positions (of VEC batch entries each, where these are contiguous).
 // The positions' places and the taps of each that lie inside the image are worked out once per CTA.  A row's entries are
-// decoded 32 at a time, one a lane, to (weight, offset of the operand from that of the position's first tap and the tap's
-// number), and read back as 16-byte broadcasts of two entries.  Taps outside the image contribute w * 0 like everywhere.
+// decoded 32 at a time, one a lane, to (weight, offset of the operand from that of the position's first tap) and the tap's bit,
+// and read back as 16-byte broadcasts of two entries, or four bits where positions have taps outside.  Taps outside the image contribute w * 0 like everywhere.
 template <int VEC, int V, int U, int MINB>
 __global__ void __launch_bounds__(kWarps * 32, MINB)
 conv_gather_kernel(const __grid_constant__ GatherArgs a)
 {
     __shared__ __align__(16) uint2 s_entry[kWarps][2][kBatch];
+    // Four positions a lane add a 32-bit offset an operand and meet the mask with the tap's bit, 5 instructions, at 16 bytes more
+    // of shared memory for four entries: 721 -> 476 us (290 -> 501 channels, 5 x 5, 84 x 84, batch 1), 376 -> 248 (192 -> 64,
+    // 3 x 3, 32 x 32, batch 20, NCHW).  The others keep offset and tap in one word, 7 instructions and fewer registers: with
+    // the bits one position a lane took 15.4 -> 16.1 us, four batch entries up to 11 % longer.
+    constexpr bool PACK = VEC == 4 || V == 1;
+    __shared__ __align__(16) uint32_t s_tap[PACK ? 1 : kWarps][2][kBatch];
     __shared__ int s_in[32 * V];
     __shared__ uint32_t s_mask[32 * V], s_out[32 * V];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -100,21 +111,34 @@ conv_gather_kernel(const __grid_constant__ GatherArgs a)
     }
     __syncthreads();
     if (slot >= a.m) return;
-    const float* base[V];
+    std::conditional_t<PACK, const float*, uint32_t> base[V];       // or bytes from the input's start, modulo 2^32: a first tap may lie before it
     uint32_t mask[V];
     const uint32_t all = 0xffffffffu >> (32 - a.kH * a.kW);
     bool inside = true;
     float acc[V][VEC];
 #pragma unroll
     for (int v = 0; v < V; ++v) {
-        base[v] = a.in + s_in[v * 32 + lane];
+        if constexpr (PACK) base[v] = a.in + s_in[v * 32 + lane];
+        else base[v] = 4u * (uint32_t)s_in[v * 32 + lane];
         mask[v] = s_mask[v * 32 + lane];
         inside = inside && mask[v] == all;
 #pragma unroll
         for (int i = 0; i < VEC; ++i) acc[v][i] = bias;
     }
-    auto group = [&](const uint2* __restrict__ e, auto check) {         // U entries
+    auto load = [&](float (&x)[VEC], int v, uint32_t entry, uint32_t tap, auto check) {
+        if constexpr (PACK) load_vec<PACK, decltype(check)::value, VEC>(x, base[v] + (entry >> 5), mask[v], entry);
+        else load_vec<PACK, decltype(check)::value, VEC>(x, reinterpret_cast<const char*>(a.in) + (base[v] + entry), mask[v], tap);
+    };
+    auto group = [&](const uint2* __restrict__ e, const uint32_t* __restrict__ taps, auto check) {         // U entries
         uint2 en[U];
+        uint32_t tap[U] = {};
+        if constexpr (decltype(check)::value && !PACK) {
+#pragma unroll
+            for (int u = 0; u < U; u += 4) {
+                const uint4 four = *reinterpret_cast<const uint4*>(taps + u);
+                tap[u] = four.x; tap[u + 1] = four.y; tap[u + 2] = four.z; tap[u + 3] = four.w;
+            }
+        }
 #pragma unroll
         for (int u = 0; u < U; u += 2) {
             const uint4 two = *reinterpret_cast<const uint4*>(e + u);
@@ -126,7 +150,7 @@ conv_gather_kernel(const __grid_constant__ GatherArgs a)
         for (int u = 0; u < U; ++u)
 #pragma unroll
             for (int v = 0; v < V; ++v)
-                load_vec<decltype(check)::value, VEC>(x[u][v], base[v] + (en[u].y >> 5), mask[v], en[u].y);
+                load(x[u][v], v, en[u].y, tap[u], check);
 #pragma unroll
         for (int u = 0; u < U; ++u)
 #pragma unroll
@@ -137,19 +161,23 @@ conv_gather_kernel(const __grid_constant__ GatherArgs a)
     auto run = [&](auto check) {
         for (uint32_t j = 0, buf = 0; j < nn; j += kBatch, buf ^= 1u) {
             uint2* __restrict__ e = s_entry[warp][buf];
+            uint32_t* __restrict__ taps = s_tap[PACK ? 0 : warp][buf];
             const uint32_t kh = t >> 8 & 0xffu, kw = t & 0xffu;
-            e[lane] = make_uint2(__float_as_uint(w), ((t >> 16) * a.iC + kh * a.dH * a.iH + kw * a.dW * a.iW) << 5 | (31 - (kh * a.kW + kw)));
+            const uint32_t at = (t >> 16) * a.iC + kh * a.dH * a.iH + kw * a.dW * a.iW, tap = kh * a.kW + kw;
+            e[lane] = make_uint2(__float_as_uint(w), PACK ? at << 5 | (31 - tap) : 4u * at);
+            if constexpr (decltype(check)::value && !PACK) taps[lane] = 1u << tap;
             __syncwarp();
             if (j + kBatch + lane < nn) { t = __ldg(tp + j + kBatch + lane); w = __ldg(wd + j + kBatch + lane); }
             const uint32_t n = min(kBatch, nn - j);
             uint32_t u = 0;
-            for (; u + U <= n; u += U) group(e + u, check);
+            for (; u + U <= n; u += U) group(e + u, taps + u, check);
             for (; u < n; ++u) {
                 const uint2 en = e[u];
+                const uint32_t tap = decltype(check)::value && !PACK ? taps[u] : 0u;
 #pragma unroll
                 for (int v = 0; v < V; ++v) {
                     float x[VEC];
-                    load_vec<decltype(check)::value, VEC>(x, base[v] + (en.y >> 5), mask[v], en.y);
+                    load(x, v, en.y, tap, check);
 #pragma unroll
                     for (int i = 0; i < VEC; ++i) acc[v][i] = fmaf(__uint_as_float(en.x), x[i], acc[v][i]);
                 }
@@ -186,6 +214,10 @@ struct Form {
 constexpr Form kForms[4] = {{1, 1, 8, 3.5, 208, 3.2, 5.9, 0.42, 366}, {1, 4, 4, 2.8, 297, 3.5, 7.7, 0.42, 729},
                             {4, 2, 4, 2.0, 382, 6.3, 11.2, 0.40, 927}, {4, 1, 4, 2.5, 268, 5.5, 10.1, 0.43, 532}};
 
+// The second one where neighbouring positions are neighbours in memory (elsewhere L1 wavefronts bound it, and the estimate
+// above holds), fitted to 112 shapes with an SM's CTAs counted whole.
+constexpr Form kNear = {1, 4, 4, 2.9, 364, 4.2, 4.9, 0.19, 325};
+
 double form_us(const spx_ell* e, const ConvParams& p, int layout, const Form& f)
 {
     const double sms = sm_count(e->device), len = (double)e->nnz_total / e->m;
@@ -199,7 +231,12 @@ double form_us(const spx_ell* e, const ConvParams& p, int layout, const Form& f)
     } else {
         lines = std::min(32.0, f.VEC * p.sW + 1.0 + 32.0 * f.VEC / ((double)p.Wo * (layout == SPX_LAYOUT_PF ? p.B : 1)));
     }
-    const double busy = warps * (f.warp + len * (f.entry + f.operand * f.V)) / (4 * sms) + warps * len * f.V * lines * f.wavefront / sms;
+    double whole = 1.0;                         // the fullest SM's CTAs to the average
+    if (&f == &kNear) {
+        const double ctas = warps / kWarps / sms;
+        whole = ctas <= 4.0 ? std::ceil(ctas) / ctas : (ctas + 0.5) / ctas;
+    }
+    const double busy = whole * (warps * (f.warp + len * (f.entry + f.operand * f.V)) / (4 * sms) + warps * len * f.V * lines * f.wavefront / sms);
     const double chain = 1000.0 + (e->max_nnz / f.U + 2.0) * f.trip;
     return f.us + std::sqrt(busy * busy + chain * chain) / 1900.0;
 }
@@ -229,18 +266,27 @@ bool plan_conv_gather(const spx_ell* e, const ConvParams& p, int layout, const f
     }();
     const uint64_t H = p.H, W = p.W, B = p.B, Cin = p.Cin, Ho = p.Ho, Wo = p.Wo;
     if (!env || p.kH * p.kW > 32) return false;             // a bit per tap
-    // 27 bits of an entry's offset, 32 of a position's in the input (signed) and in the output
+    // 27 bits of an entry's offset, 32 of an operand's in bytes and of a position's in the output
     const uint64_t iC = layout == SPX_LAYOUT_FMAJOR ? B : layout == SPX_LAYOUT_PF ? H * W * B : H * W;
     const uint64_t iH = layout == SPX_LAYOUT_FMAJOR ? Cin * B : layout == SPX_LAYOUT_PF ? W * B : W;
     const uint64_t iW = layout == SPX_LAYOUT_FMAJOR ? H * Cin * B : layout == SPX_LAYOUT_PF ? B : 1;
     if ((Cin - 1) * iC + (uint64_t)(p.kH - 1) * p.dH * iH + (uint64_t)(p.kW - 1) * p.dW * iW >= 1ull << 27) return false;
-    if ((H + p.pH) * iH + (W + p.pW) * iW + Cin * H * W * B >= 1ull << 31 || p.Cout * Ho * Wo * B >= 1ull << 32) return false;
+    if ((H + p.pH) * iH + (W + p.pW) * iW + Cin * H * W * B >= 1ull << 30 || p.Cout * Ho * Wo * B >= 1ull << 32) return false;
     if ((Ho * Wo * B + 31) / 32 * ((e->m + kWarps - 1) / kWarps) > 0x7fffffffull) return false;
     const bool vec = layout != SPX_LAYOUT_NCHW && B % 4 == 0 && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
     const int f0 = vec ? 2 : 0;
-    const double us0 = form_us(e, p, layout, kForms[f0]), us1 = form_us(e, p, layout, kForms[f0 + 1]);
+    const bool neighbours = layout != SPX_LAYOUT_FMAJOR && p.sW == 1;
+    const Form& other = vec ? kForms[3] : neighbours ? kNear : kForms[1];
+    const double us0 = form_us(e, p, layout, kForms[f0]), us1 = form_us(e, p, layout, other);
     plan.form = us1 < us0 ? f0 + 1 : f0;
-    plan.us = env == 2 ? 0.0 : std::min(us0, us1);
+    double us = std::min(us0, us1);
+    // One batch entry a lane although four are contiguous: more warps, shorter round trips, fewer lanes idle.  Where it is expected
+    // to be faster by a ninth: the estimates are a tenth off for half of the shapes.
+    if (vec && layout == SPX_LAYOUT_PF) {
+        const double one = form_us(e, p, layout, kForms[0]), four = neighbours ? form_us(e, p, layout, kNear) : 1e30;
+        if (std::min(one, four) < 0.9 * us) { us = std::min(one, four); plan.form = four < one ? 1 : 0; }
+    }
+    plan.us = env == 2 ? 0.0 : us;
     return true;
 }
 

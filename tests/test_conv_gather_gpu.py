@@ -28,7 +28,9 @@ CASES = [(1, 3, 8, 4, 8, (3, 3), (1, 1), (1, 1), 0.5),          # one tile of 32
          (2, 3, 17, 9, 10, (4, 8), (1, 1), (1, 1), 0.5),        # 32 taps
          (2, 3, 17, 9, 14, (3, 11), (1, 1), (1, 1), 0.5),       # 33: not for this kernel
          (1, 2, 130, 66, 65, (3, 3), (1, 1), (1, 1), 0.6),      # many positions and channels, short rows
-         (32, 3, 200, 30, 31, (1, 1), (2, 2), (1, 1), 0.7)]
+         (32, 3, 200, 30, 31, (1, 1), (2, 2), (1, 1), 0.7),
+         (4, 64, 24, 17, 13, (3, 3), (1, 1), (1, 1), 0.3),      # one batch entry a lane although four are contiguous
+         (28, 24, 104, 14, 14, (3, 3), (1, 1), (1, 1), 0.3)]    # and of four positions
 
 
 @forced
