@@ -168,7 +168,9 @@ int spx_spmv_reference_order(const spx_ell* e, const float* x, const float* bias
  * slabs) and, for larger calls, a second form for the kernel that keeps its input in tensor memory
  * (about a slab per kernel shape, dilation and row stride, at most four), beside which it builds
  * the first as well: the two are compared.  (Device allocations, and a wait for `stream`; make
- * that call outside a stream capture: a captured call uses the forms that are there.)  A form that
+ * that call outside a stream capture: a captured call uses the forms that are there.)  Small calls gather
+ * their input and use the tap table alone; a handle's first one may wait for `stream` to count the columns that
+ * its rows share.  A form that
  * finds no memory is gone without from then on.  Results do not depend on which kernel is chosen.  Both of those kernels fetch their
  * input with bulk tensor copies: see spx_ell_status. */
 int spx_conv2d(const spx_ell* e, const spx_conv_geom* g, int layout, const float* in, uint32_t B,

@@ -1187,10 +1187,10 @@ static double tiled_us(const spx_ell* e, const ConvParams& p4, const ConvViews& 
 // Whether gathering is expected to be faster than the tiled kernels: below 0.9 of their time, 0.85 where it takes four batch
 // entries a lane (both kinds' estimates are 10 % off for half of the shapes; at 0.95 two of a hundred calls took 5 to 16 %
 // longer).  Sure if it is so for the least that these can take, and not worth a count if it is not so by the density;
-// else the columns that rows share are counted, which the density does not tell.  Measured on 500 drawn shapes (300 of
-// them fitted to) the calls take 0.71 of the time they took before there was this kernel, with the faster one each time
-// 0.67; on 900 shapes with weights of eleven kinds (iid, rows of different density, channels, kernels or patterns removed)
-// 0.73, 3 of them more than 10 % longer.  By the density alone some structured kinds had calls 1.3 to 1.5 times as long.
+// else the columns that rows share are counted, which the density does not tell.  Measured on 173 drawn shapes of 8 us and
+// more that were not fitted to, the calls take 0.65 of the time they took before there was this kernel, none of them 5 % longer;
+// on 500 shapes with weights of eleven kinds (iid, rows of different density, channels, kernels or patterns removed) 0.73, 4 of
+// them more than 10 % longer.  By the density alone some structured kinds had calls 1.3 to 1.5 times as long.
 static bool gather_pays(spx_ell* e, const ConvParams& p4, const ConvViews& v, bool copies, uint32_t B, const ConvGatherPlan& plan, cudaStream_t s)
 {
     const double us = plan.us / (plan.form >= 2 ? 0.85 : 0.9);

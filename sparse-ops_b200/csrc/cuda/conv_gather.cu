@@ -49,27 +49,28 @@ struct GatherArgs {
 // sign by a tap's number (PACK), or met by its bit.
 template <bool PACK, bool CHECK, int VEC>
 __device__ __forceinline__ void load_vec(float (&d)[VEC], const void* __restrict__ p, uint32_t mask, uint32_t tap) {
-#define SPX_LOAD4(TEST)                                                                                                          \
-    asm("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\t" TEST "mov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\t"                   \
-        "mov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t@p ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"             \
-        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "l"(p), "r"(mask), "r"(tap))
-#define SPX_LOAD1(TEST)                                                                                                          \
-    asm("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\t" TEST "mov.f32 %0, 0f00000000;\n\t@p ld.global.nc.f32 %0, [%1];\n\t}"           \
-        : "=f"(d[0]) : "l"(p), "r"(mask), "r"(tap))
-    if constexpr (VEC == 4 && CHECK && PACK) SPX_LOAD4("shf.l.wrap.b32 t, 0, %5, %6;\n\tsetp.lt.s32 p, t, 0;\n\t");
-    else if constexpr (VEC == 4 && CHECK) SPX_LOAD4("and.b32 t, %5, %6;\n\tsetp.ne.u32 p, t, 0;\n\t");
-    else if constexpr (VEC == 4) asm("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "l"(p));
-    else if constexpr (CHECK && PACK) SPX_LOAD1("shf.l.wrap.b32 t, 0, %2, %3;\n\tsetp.lt.s32 p, t, 0;\n\t");
-    else if constexpr (CHECK) SPX_LOAD1("and.b32 t, %2, %3;\n\tsetp.ne.u32 p, t, 0;\n\t");
-    else asm("ld.global.nc.f32 %0, [%1];" : "=f"(d[0]) : "l"(p));
-#undef SPX_LOAD4
-#undef SPX_LOAD1
+    static_assert(PACK || VEC == 1);
+    if constexpr (VEC == 4 && CHECK)
+        asm("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\tshf.l.wrap.b32 t, 0, %5, %6;\n\tsetp.lt.s32 p, t, 0;\n\tmov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\t"
+            "mov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t@p ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+            : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "l"(p), "r"(mask), "r"(tap));
+    else if constexpr (VEC == 4)
+        asm("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "l"(p));
+    else if constexpr (CHECK && PACK)
+        asm("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\tshf.l.wrap.b32 t, 0, %2, %3;\n\tsetp.lt.s32 p, t, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
+            "@p ld.global.nc.f32 %0, [%1];\n\t}" : "=f"(d[0]) : "l"(p), "r"(mask), "r"(tap));
+    else if constexpr (CHECK)
+        asm("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\tand.b32 t, %2, %3;\n\tsetp.ne.u32 p, t, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
+            "@p ld.global.nc.f32 %0, [%1];\n\t}" : "=f"(d[0]) : "l"(p), "r"(mask), "r"(tap));
+    else
+        asm("ld.global.nc.f32 %0, [%1];" : "=f"(d[0]) : "l"(p));
 }
 
 // A CTA computes 8 output channels, one a warp, at 32 V positions (of VEC batch entries each, where these are contiguous).
 // The positions' places and the taps of each that lie inside the image are worked out once per CTA.  A row's entries are
 // decoded 32 at a time, one a lane, to (weight, offset of the operand from that of the position's first tap) and the tap's bit,
-// and read back as 16-byte broadcasts of two entries, or four bits where positions have taps outside.  Taps outside the image contribute w * 0 like everywhere.
+// and read back as 16-byte broadcasts of two entries, or four bits where positions have taps outside.  Taps outside the image
+// contribute w * 0 like everywhere.
 template <int VEC, int V, int U, int MINB>
 __global__ void __launch_bounds__(kWarps * 32, MINB)
 conv_gather_kernel(const __grid_constant__ GatherArgs a)
@@ -111,7 +112,8 @@ conv_gather_kernel(const __grid_constant__ GatherArgs a)
     }
     __syncthreads();
     if (slot >= a.m) return;
-    std::conditional_t<PACK, const float*, uint32_t> base[V];       // or bytes from the input's start, modulo 2^32: a first tap may lie before it
+    // the position's first tap, or its bytes from the input's start modulo 2^32 (it may lie before)
+    std::conditional_t<PACK, const float*, uint32_t> base[V];
     uint32_t mask[V];
     const uint32_t all = 0xffffffffu >> (32 - a.kH * a.kW);
     bool inside = true;

@@ -303,7 +303,7 @@ spmm_tile_kernel(const __grid_constant__ TileArgs a, const __grid_constant__ CUt
         __syncwarp();
         fill(blk + 2);
     };
-    auto ids = [&](float4& k, uint32_t st) {
+    auto ids = [&](float4& k, uint32_t st) {    // where the step's place in its block is not known
         if ((st & 3u) == 0) {
             asm volatile("cp.async.wait_group 1;" ::: "memory");
             __syncwarp();
