@@ -591,7 +591,7 @@ Plan plan_tiles(const spx_ell* e, uint32_t C, uint32_t NV, uint32_t sms, bool al
     p.deep = deep_limit(NV, p.warps);
     const double len = (double)e->nnz_total / e->m;
     const double steps = std::max((len + 1.1 * std::sqrt(len)) / 4.0, chunks * (1.0 - std::exp(-(double)kGroupRows * len / chunks)));
-    const double chunk = !p.deep ? 0.365 : p.deep == 24 ? 0.333 : 0.313;
+    const double chunk = !p.deep || p.warps <= 3 ? 0.365 : p.deep == 24 ? 0.333 : 0.313;     // few warps wait for the copies
     const double step = std::max(!p.deep ? 0.0 : NV == 1 ? 0.036 : 0.051, p.warps * (16.0 * NV + 4.0) / 2060.0);
     double rows = sectors ? 0.0 : 0.12;                     // us per chunk, for the copies of X's rows
     if (C < 32 && aligned) rows = (C % 8 ? 14.0 : 5.0) / C;     // shorter than a box is wide (2080 x 613, C = 4: 3 us a chunk)
