@@ -18,6 +18,13 @@ namespace spx {
 
 static thread_local char g_err[512] = "";
 std::atomic<uint64_t> g_launches{0};
+static thread_local uint64_t t_capture_start = 0;       // g_launches when this thread's capture began
+
+void count_launch_beside()
+{
+    count_launch();
+    ++t_capture_start;
+}
 
 int fail(int code, const char* fmt, ...)
 {
@@ -56,6 +63,13 @@ int alloc_ell(uint32_t m, uint32_t n, uint32_t r, spx_ell** out, cudaStream_t s,
     e->m = m; e->n = n; e->r = r;
     e->tiles = new_tiles();
     e->conv_tmem = new_conv_tmem();
+    e->conv = new_conv_tables();
+    if (!e->conv) {
+        free_tiles(e);
+        free_conv_tmem(e);
+        delete e;
+        return fail(SPX_ERR_OOM, "out of host memory");
+    }
     e->pitch = r ? round_up<uint32_t>(r, 32u) : 0u;
     const size_t slots = (size_t)m * e->pitch;
     int rc = SPX_OK;
@@ -73,6 +87,7 @@ int alloc_ell(uint32_t m, uint32_t n, uint32_t r, spx_ell** out, cudaStream_t s,
         pool_free(e->Wd, slots * sizeof(float), s); pool_free(e->idx, slots * sizeof(uint32_t), s); pool_free(e->nnz, (size_t)m * sizeof(uint32_t), s);
         free_tiles(e);
         free_conv_tmem(e);
+        free_conv_tables(e);
         delete e;
         return rc != SPX_OK ? rc : fail(SPX_ERR_CUDA, "ELLPACK zero fill (%zu slots) failed: %s", slots, cudaGetErrorString(err));
     }
@@ -237,7 +252,6 @@ struct GraphExec {
     cudaGraphExec_t exec = nullptr;
     uint64_t kernels = 0;
 };
-thread_local uint64_t t_capture_start = 0;
 }  // namespace
 
 int spx_graph_capture_begin(void* stream)
@@ -407,6 +421,7 @@ int spx_ell_destroy(spx_ell* e)
     wait_for_device();
     free_tiles(e);
     free_conv_tmem(e);
+    free_conv_tables(e);
     pool_free(e->Wd, (size_t)e->m * e->pitch * 4, nullptr);
     pool_free(e->idx, (size_t)e->m * e->pitch * 4, nullptr);
     pool_free(e->nnz, (size_t)e->m * 4, nullptr);

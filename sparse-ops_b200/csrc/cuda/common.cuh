@@ -15,6 +15,7 @@ struct PinnedBlock {
     void* host = nullptr;
     size_t bytes = 0;
 };
+struct ConvTables;
 }  // namespace spx
 
 // Device-resident ELLPACK (see include/spx_b200.h).  Row i occupies entries
@@ -66,6 +67,8 @@ struct spx_ell {
     // counted, 2 not to be counted (no memory).
     int conv_loads_state = 0;
     double conv_loads[3][4] = {};
+    // Lock of what the convolution builds (conv.cuh).
+    spx::ConvTables* conv = nullptr;
     // The convolution's entries for conv_tmem.cu, built on the first call that uses them.
     void* conv_tmem = nullptr;
     // SpMV with x larger than shared memory (spmv.cu): column window width and the per-row split
@@ -100,6 +103,7 @@ namespace spx {
 int fail(int code, const char* fmt, ...);
 extern std::atomic<uint64_t> g_launches;
 inline void count_launch(uint64_t n = 1) { g_launches.fetch_add(n, std::memory_order_relaxed); }
+void count_launch_beside();     // of a kernel that runs at once although the call is being recorded: not one of the graph's
 int sm_count(int device);
 
 // Rounds up to a multiple of `to`.

@@ -766,12 +766,21 @@ static bool rbm_fits(const ConvParams& p, uint32_t qb, int nb, int g)
     return THin * TWin * qb * 4 * sizeof(float) <= rbm_budget(nb) / (nb == 16 ? 1 : 2);
 }
 
-// Builds (once per handle and kernel shape) the row-block-merged weights.
-int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s)
+ConvTables* new_conv_tables() { return new (std::nothrow) ConvTables(); }
+void free_conv_tables(spx_ell* e) { delete e->conv; e->conv = nullptr; }
+
+// Builds (once per handle and kernel shape) the row-block-merged weights.  On a stream beside the call's, which is waited for:
+// the calls of other threads and streams find them complete, and where the call's stream is being recorded they are there
+// before the graph runs.  (A handle's arrays are complete when it is handed out, so there is nothing to wait for before.)
+int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW)
 {
+    std::lock_guard<std::mutex> lk(e->conv->mu);
     if (e->rbm_hdr && e->rbm_kH == kH && e->rbm_kW == kW) return SPX_OK;
     RelaxedCapture relaxed;                     // allocations and waits below end no capture
+    cudaStream_t side = nullptr;
+    if (int rc = side_stream(e->device, &side)) return rc;
     const uint32_t nblocks = (e->m + kRbmRows - 1) / kRbmRows;
+    if (e->rbm_hdr) wait_for_device();          // another kernel shape's, which calls may still be using
     if (!e->rbm_hdr) {
         // Up to three times the ELLPACK slab (24 bytes per union column, at most 4 * max_nnz columns
         // per block of 4 rows).  Without room for it the per-row kernel is used instead.
@@ -781,9 +790,9 @@ int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s)
         if (pool_alloc_now(reinterpret_cast<void**>(&e->rbm_ncols), (size_t)nblocks * sizeof(uint32_t), e->device) != SPX_OK ||
             pool_alloc_now(reinterpret_cast<void**>(&e->rbm_w), slots * kRbmRows * sizeof(float), e->device) != SPX_OK ||
             pool_alloc_now(reinterpret_cast<void**>(&e->rbm_hdr), slots * sizeof(uint2), e->device) != SPX_OK) {
-            pool_free(e->rbm_ncols, (size_t)nblocks * sizeof(uint32_t), s);
-            pool_free(e->rbm_w, slots * kRbmRows * sizeof(float), s);
-            pool_free(e->rbm_hdr, slots * sizeof(uint2), s);
+            pool_free(e->rbm_ncols, (size_t)nblocks * sizeof(uint32_t), side);
+            pool_free(e->rbm_w, slots * kRbmRows * sizeof(float), side);
+            pool_free(e->rbm_hdr, slots * sizeof(uint2), side);
             e->rbm_ncols = nullptr; e->rbm_w = nullptr; e->rbm_hdr = nullptr;
             e->rbm_cap = UINT32_MAX;
             return -1;
@@ -792,19 +801,12 @@ int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s)
         ensure_tma_words(e);
         (void)cudaGetLastError();
     }
-    // A call that is recorded builds them all the same, beside the recording: eager calls before it may all have gathered.
-    cudaStreamCaptureStatus cap_status = cudaStreamCaptureStatusNone;
-    const bool recorded = cudaStreamIsCapturing(s, &cap_status) == cudaSuccess && cap_status != cudaStreamCaptureStatusNone;
-    cudaStream_t on = s;
-    if (recorded) {
-        if (int rc = side_stream(e->device, &on)) return rc;
-        wait_for_device();                      // for the entries, which may still be on their way
-    }
     const size_t smem = (size_t)((e->n + 31) / 32) * 2 * sizeof(uint32_t);
-    build_rbm_kernel<<<nblocks, 256, smem, on>>>(e->Wd, e->idx, e->nnz, e->m, e->n, e->pitch, kH, kW, e->rbm_cap,
-                                                 e->rbm_hdr, e->rbm_w, e->rbm_ncols);
-    SPX_LAUNCH_CHECK("build_rbm_kernel");
-    if (recorded) SPX_CUDA(cudaStreamSynchronize(on));
+    build_rbm_kernel<<<nblocks, 256, smem, side>>>(e->Wd, e->idx, e->nnz, e->m, e->n, e->pitch, kH, kW, e->rbm_cap,
+                                                   e->rbm_hdr, e->rbm_w, e->rbm_ncols);
+    SPX_CUDA(cudaGetLastError());
+    count_launch_beside();
+    SPX_CUDA(cudaStreamSynchronize(side));
     e->rbm_kH = kH;
     e->rbm_kW = kW;
     return SPX_OK;
@@ -950,7 +952,7 @@ static int launch_rbm_qb(spx_ell* e, TileParams tp, const float* in, const float
     const uint32_t groups = (nblocks + cut.nb - 1) / cut.nb;
     const uint64_t units = tiles * groups * (b_len / (QB * 4));
     if (units > 0x3fffffffull) return -1;
-    const int rc = ensure_rbm(e, p.kH, p.kW, s);
+    const int rc = ensure_rbm(e, p.kH, p.kW);
     if (rc != SPX_OK) return rc;                        // -1: no memory for the merged weights
     RbmUnits un{0u, (uint32_t)tiles, groups, 0u};
     if (cut.nb == 8 && cut.g == 4) return launch_rbm_units<QB, 8, 4>(e, tp, un, (uint32_t)units, in, bias, act, out, s, b_avail);

@@ -3,6 +3,8 @@
 
 #include "common.cuh"
 
+#include <mutex>
+
 namespace spx {
 
 struct ConvParams {
@@ -41,8 +43,15 @@ struct ConvGatherPlan {
 bool plan_conv_gather(const spx_ell* e, const ConvParams& p, int layout, const float* in, const float* out, ConvGatherPlan& plan);
 int launch_conv_gather(const spx_ell* e, const ConvParams& p, int layout, const float* in, const float* bias, int act, float* out,
                        const ConvGatherPlan& plan, cudaStream_t s);
+// What a handle's convolutions share is built by whichever call first needs it, on any thread and stream: under this lock, and
+// complete for every stream when it is let go.
+struct ConvTables {
+    std::mutex mu;
+};
+ConvTables* new_conv_tables();
+void free_conv_tables(spx_ell* e);
 // conv.cu: the merged weights of conv_rbm_tile_kernel; -1 where there is no memory for them.
-int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s);
+int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW);
 void* new_conv_tmem();
 void free_conv_tmem(spx_ell* e);
 

@@ -579,8 +579,8 @@ static int find_form(spx_ell* e, const FormShape& f, uint32_t chunks, uint32_t p
         return -1;
     }
     RelaxedCapture relaxed;                     // s is not being captured; another stream may be, by this thread
-    // A later call that is recorded may take the other kernel (another batch, say), and cannot build what that needs then.
-    const int merged = ensure_rbm(e, f.kH, f.kW, s);
+    // The other kernel's weights, which a later call may take (another batch, say); how many columns they have is counted below.
+    const int merged = ensure_rbm(e, f.kH, f.kW);
     if (merged > 0) return merged;
     ensure_tma_words(e);
     if (!e->tma_failed_dev || !e->tma_failed_mapped) {

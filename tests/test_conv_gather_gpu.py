@@ -1,7 +1,9 @@
 """GPU: the convolution that gathers its operands (conv_gather.cu), forced, against the oracle bit for bit: edges of its tiles of
 positions, of batches of 32 entries and groups of 8 and 4, both widths of operands, all layouts; and when it is chosen.  The
 switch is read once per process, so the forced cases run in a child."""
+import ctypes
 import os
+import threading
 
 import numpy as np
 import pytest
@@ -9,7 +11,7 @@ import torch
 
 import spx_ctypes as sx
 from conftest import assert_bit_equal
-from test_conv_tmem_gpu import assert_ran, child, kernels_of
+from test_conv_tmem_gpu import assert_ran, child, kernels_of, waits_for_the_device
 from test_parity_gpu import as_layout, dev, gpu_ell, ptr, sparse
 
 pytestmark = pytest.mark.gpu
@@ -130,6 +132,91 @@ def test_tiled_call_recorded_after_gathered_ones(lib, orc, cuda):
     torch.cuda.synchronize()
     assert_bit_equal(y32.cpu().numpy(), w32, "replayed")
     assert_bit_equal(y1.cpu().numpy(), w1, "gathered")
+
+
+def merged_after_gathered(lib, orc, cuda, batches):
+    """A handle whose first call gathers (so that nothing is merged yet), and a call per batch size; 32 is merged."""
+    rng, C, H = np.random.default_rng(15), 64, 28
+    E = orc.encode(sparse(rng, C, C * 9, 0.3))
+    gd = dict(Cin=C, kH=3, kW=3, sH=2, sW=2, pH=1, pW=1, dH=1, dW=1, H=H, W=H)
+    h, g = gpu_ell(lib, E), sx.conv_geom(C, C, 3, 3, H, H, 2, 2, 1, 1)
+    x = rng.standard_normal((max(batches), C, H, H)).astype(np.float32)
+    runs = []
+    for B in batches:
+        src = as_layout(x[:B], sx.LAYOUT_PF)
+        want = orc.conv2d(E, gd, sx.LAYOUT_PF, src, B, None, 0)
+        dX, dY = dev(src, cuda), torch.full(want.shape, float("nan"), device=cuda)
+        runs.append((B, dX, dY, want, torch.cuda.Stream()))
+    one, y1 = dev(as_layout(x[:1], sx.LAYOUT_PF), cuda), torch.empty((C, H // 2, H // 2, 1), device=cuda)
+    assert_ran(kernels_of(lambda: h.conv2d(g, sx.LAYOUT_PF, ptr(one), 1, None, 0, ptr(y1))), "conv_gather_kernel")
+    torch.cuda.synchronize()
+    return h, g, runs, lambda run: h.conv2d(g, sx.LAYOUT_PF, ptr(run[1]), run[0], None, 0, ptr(run[2]), run[4].cuda_stream)
+
+
+@chosen
+def test_merged_weights_for_two_streams(lib, orc, cuda):
+    """The first merged call waits behind a long kernel, one on another stream does not: it has the weights all the same."""
+    h, g, runs, call = merged_after_gathered(lib, orc, cuda, [32, 32])
+
+    def both():
+        with torch.cuda.stream(runs[0][4]):
+            torch.cuda._sleep(200_000_000)
+        for run in runs:
+            call(run)
+
+    assert_ran(kernels_of(both), "conv_rbm_tile_kernel")
+    for B, _, dY, want, _ in runs:
+        assert_bit_equal(dY.cpu().numpy(), want, f"batch {B}")
+
+
+@chosen
+def test_merged_weights_for_several_threads(lib, orc, cuda):
+    """A handle's first merged calls, made by eight threads on streams of their own at once."""
+    for _ in range(4):
+        h, g, runs, call = merged_after_gathered(lib, orc, cuda, [32, 64, 36, 32, 40, 32, 64, 32])
+        start, errors = threading.Barrier(len(runs)), []
+
+        def work(run):
+            try:
+                start.wait()
+                for _ in range(3):
+                    call(run)
+            except Exception as e:      # noqa: BLE001
+                errors.append(e)
+
+        threads = [threading.Thread(target=work, args=(run,)) for run in runs]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        torch.cuda.synchronize()
+        assert not errors, errors
+        for B, _, dY, want, _ in runs:
+            assert_bit_equal(dY.cpu().numpy(), want, f"batch {B}")
+
+
+@chosen
+def test_recording_a_merged_call_waits_for_no_other_work(lib, orc, cuda):
+    """Recording a call that lacks the merged weights builds them at once, beside what other streams do: that kernel is no part
+    of the graph."""
+    h, g, runs, call = merged_after_gathered(lib, orc, cuda, [32])
+    (B, _, dY, want, stream), graph = runs[0], ctypes.c_void_p()
+    assert not waits_for_the_device(lambda: None)           # (makes the stream)
+
+    def record():
+        lib.spx_graph_capture_begin(stream.cuda_stream)
+        call(runs[0])
+        lib.spx_graph_capture_end(stream.cuda_stream, ctypes.byref(graph))
+
+    before = lib.spx_launch_count()
+    assert not waits_for_the_device(record)
+    assert lib.spx_launch_count() == before + 1
+    for _ in range(2):
+        lib.spx_graph_launch(graph, stream.cuda_stream)
+    torch.cuda.synchronize()
+    assert lib.spx_launch_count() == before + 3
+    assert_bit_equal(dY.cpu().numpy(), want, "replayed")
+    lib.spx_graph_destroy(graph)
 
 
 def test_forced_kernel():
