@@ -704,14 +704,29 @@ conv_rbm_tile_kernel(const uint2* __restrict__ hdr, const float4* __restrict__ w
 
 namespace spx {
 
-static int ensure_taps(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s)
+ConvTables* new_conv_tables() { return new (std::nothrow) ConvTables(); }
+void free_conv_tables(spx_ell* e) { delete e->conv; e->conv = nullptr; }
+
+// What a handle's convolutions share is built on a stream beside the call's, which is waited for: the calls of other threads and
+// streams find it complete, and where the call's stream is being recorded it is there before the graph runs.  (A handle's
+// arrays are complete when it is handed out, so there is nothing to wait for before.)
+
+// Builds (once per handle and kernel shape) the tap table.
+static int ensure_taps(spx_ell* e, uint32_t kH, uint32_t kW)
 {
-    if (e->taps && e->taps_kH == kH && e->taps_kW == kW) return SPX_OK;
     if (e->r == 0) return SPX_OK;
+    std::lock_guard<std::mutex> lk(e->conv->mu);
+    if (e->taps && e->taps_kH == kH && e->taps_kW == kW) return SPX_OK;
+    RelaxedCapture relaxed;                     // allocations and waits below end no capture
+    cudaStream_t side = nullptr;
+    if (int rc = side_stream(e->device, &side)) return rc;
+    if (e->taps) wait_for_device();             // another kernel shape's, which calls may still be using
     if (!e->taps)
-        if (int rc = pool_alloc_now(reinterpret_cast<void**>(&e->taps), (size_t)e->m * e->pitch * sizeof(uint32_t), e->device)) return rc;
-    build_taps_kernel<<<e->m, 128, 0, s>>>(e->idx, e->nnz, e->m, e->pitch, kH, kW, e->taps);
-    SPX_LAUNCH_CHECK("build_taps_kernel");
+        if (int rc = pool_alloc(reinterpret_cast<void**>(&e->taps), (size_t)e->m * e->pitch * sizeof(uint32_t), e->device, side)) return rc;
+    build_taps_kernel<<<e->m, 128, 0, side>>>(e->idx, e->nnz, e->m, e->pitch, kH, kW, e->taps);
+    SPX_CUDA(cudaGetLastError());
+    count_launch_beside();
+    SPX_CUDA(cudaStreamSynchronize(side));
     e->taps_kH = kH;
     e->taps_kW = kW;
     return SPX_OK;
@@ -766,12 +781,7 @@ static bool rbm_fits(const ConvParams& p, uint32_t qb, int nb, int g)
     return THin * TWin * qb * 4 * sizeof(float) <= rbm_budget(nb) / (nb == 16 ? 1 : 2);
 }
 
-ConvTables* new_conv_tables() { return new (std::nothrow) ConvTables(); }
-void free_conv_tables(spx_ell* e) { delete e->conv; e->conv = nullptr; }
-
-// Builds (once per handle and kernel shape) the row-block-merged weights.  On a stream beside the call's, which is waited for:
-// the calls of other threads and streams find them complete, and where the call's stream is being recorded they are there
-// before the graph runs.  (A handle's arrays are complete when it is handed out, so there is nothing to wait for before.)
+// Builds (once per handle and kernel shape) the row-block-merged weights, as ensure_taps does.
 int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW)
 {
     std::lock_guard<std::mutex> lk(e->conv->mu);
@@ -1255,7 +1265,7 @@ int launch_conv2d(spx_ell* e, const spx_conv_geom* g, int layout, const float* i
             return SPX_OK;
         }
     }
-    int rc = ensure_taps(e, g->kH, g->kW, s);
+    int rc = ensure_taps(e, g->kH, g->kW);
     if (rc != SPX_OK) return rc;
     ConvParams p{g->Cin, g->Cout, g->kH, g->kW, g->sH, g->sW, g->pH, g->pW, g->dH, g->dW,
                  g->H, g->W, g->Ho, g->Wo, B};

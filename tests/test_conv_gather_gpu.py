@@ -196,6 +196,32 @@ def test_merged_weights_for_several_threads(lib, orc, cuda):
 
 
 @chosen
+@pytest.mark.parametrize("B", [1, 3, 32])
+def test_eager_call_between_recording_and_replay(lib, orc, cuda, B):
+    """A handle's very first call is recorded; an eager one before the graph has run finds what it needs all the same, and so
+    does one on another stream behind which a long kernel is queued."""
+    rng, C, H = np.random.default_rng(16), 64, 28
+    E = orc.encode(sparse(rng, C, C * 9, 0.3))
+    src = as_layout(rng.standard_normal((B, C, H, H)).astype(np.float32), sx.LAYOUT_PF)
+    want = orc.conv2d(E, dict(Cin=C, kH=3, kW=3, sH=2, sW=2, pH=1, pW=1, dH=1, dW=1, H=H, W=H), sx.LAYOUT_PF, src, B, None, 0)
+    h, g, dX = gpu_ell(lib, E), sx.conv_geom(C, C, 3, 3, H, H, 2, 2, 1, 1), dev(src, cuda)
+    Y = [torch.full(want.shape, float("nan"), device=cuda) for _ in range(4)]
+    other, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    call = lambda y, stream=0: h.conv2d(g, sx.LAYOUT_PF, ptr(dX), B, None, 0, ptr(y), stream)
+    with torch.cuda.graph(graph):
+        call(Y[0], torch.cuda.current_stream().cuda_stream)
+    call(Y[1])
+    with torch.cuda.stream(other):
+        torch.cuda._sleep(100_000_000)
+    call(Y[2], other.cuda_stream)
+    call(Y[3])
+    graph.replay()
+    torch.cuda.synchronize()
+    for k, y in enumerate(Y):
+        assert_bit_equal(y.cpu().numpy(), want, f"call {k}")
+
+
+@chosen
 def test_recording_a_merged_call_waits_for_no_other_work(lib, orc, cuda):
     """Recording a call that lacks the merged weights builds them at once, beside what other streams do: that kernel is no part
     of the graph."""
