@@ -426,12 +426,7 @@ int spx_ell_destroy(spx_ell* e)
     pool_free(e->idx, (size_t)e->m * e->pitch * 4, nullptr);
     pool_free(e->nnz, (size_t)e->m * 4, nullptr);
     pool_free(e->rows, (size_t)e->m * 8, nullptr);
-    pool_free(e->taps, (size_t)e->m * e->pitch * 4, nullptr);
     pool_free(e->spmv_split, e->spmv_split_bytes, nullptr);
-    const size_t blocks4 = (e->m + 3) / 4, slots4 = blocks4 * e->rbm_cap;       // rbm_cap means nothing without the arrays
-    pool_free(e->rbm_ncols, blocks4 * 4, nullptr);
-    pool_free(e->rbm_w, slots4 * 16, nullptr);
-    pool_free(e->rbm_hdr, slots4 * sizeof(uint2), nullptr);
     pool_free(e->stage_dev, e->stage_dev_bytes, nullptr);
     pool_free(e->conv_scratch, e->conv_scratch_bytes, nullptr);
     pool_free(e->tma_failed_dev, sizeof(int), nullptr);

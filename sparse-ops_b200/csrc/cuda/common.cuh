@@ -37,22 +37,10 @@ struct spx_ell {
     // id so that a warp needs one load, not two dependent ones, before it can ask for its slab.
     uint2* rows = nullptr;           // m entries
     uint32_t long_rows = 0;          // rows with at least 512 stored entries (a prefix of rows)
-    // Lazily built, cached conv tap table: idx decoded to packed (cin, kh, kw) for one
-    // kernel shape (conv.cu); keyed by (kH, kW).
-    uint32_t* taps = nullptr;
-    uint32_t taps_kH = 0, taps_kW = 0;
     // True when every row's stored column ids are strictly ascending (always so for handles made
     // from CSR, from a dense matrix or by the encoders; checked at upload for raw arrays).  The
     // tiled convolution kernels rely on it; without it the convolution takes the general kernel.
     bool cols_ascending = true;
-    // Lazily built row-block-merged form of the weights for the convolution (conv.cu): per block
-    // of 4 rows the ascending union of their column ids; per union column a header
-    // (packed tap, 4-bit row mask) and the 4 rows' weights (0.0f where a row has no entry).
-    // Block b owns entries [b * rbm_cap, b * rbm_cap + rbm_ncols[b]).
-    uint2* rbm_hdr = nullptr;
-    float* rbm_w = nullptr;
-    uint32_t* rbm_ncols = nullptr;
-    uint32_t rbm_cap = 0, rbm_kH = 0, rbm_kW = 0;
     // Raised by a convolution kernel whose bounded wait for a bulk tensor copy ran out: a word in
     // device memory (read by the kernel's later CTAs) and a word in pinned host memory (its device
     // alias is tma_failed_mapped; read by the next convolution call on the handle).
@@ -67,7 +55,7 @@ struct spx_ell {
     // counted, 2 not to be counted (no memory).
     int conv_loads_state = 0;
     double conv_loads[3][4] = {};
-    // Lock of what the convolution builds (conv.cuh).
+    // Tap tables and merged weights of the convolution (conv.cuh).
     spx::ConvTables* conv = nullptr;
     // The convolution's entries for conv_tmem.cu, built on the first call that uses them.
     void* conv_tmem = nullptr;
@@ -224,7 +212,7 @@ struct RelaxedCapture {
 };
 
 // Device memory from the library's pool of the given device, stream-ordered (mem.cu).
-int pool_alloc(void** p, size_t bytes, int device, cudaStream_t s);
+int pool_alloc(void** p, size_t bytes, int device, cudaStream_t s, bool optional = false);   // optional: as below
 void pool_free(void* p, size_t bytes, cudaStream_t s);      // bytes as allocated; p may be null
 int scratch_alloc(void** p, size_t bytes, int device, cudaStream_t s, bool optional = false);   // for one call: allocated and freed in stream order
 void scratch_free(void* p, cudaStream_t s);

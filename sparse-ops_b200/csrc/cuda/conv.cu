@@ -51,8 +51,9 @@ __global__ void build_taps_kernel(const uint32_t* __restrict__ idx, const uint32
 
 // General kernel: one thread per output element, any layout, any geometry.  Threads of a warp
 // are adjacent along the fastest output dimension (batch for PF, width for NCHW), so input
-// reads of a tap are coalesced and the row's (w, tap) reads are warp-uniform.
-template <int LAYOUT>
+// reads of a tap are coalesced and the row's (w, tap) reads are warp-uniform.  RAW: `taps` are the
+// column ids themselves, for a handle without memory for the table.
+template <int LAYOUT, bool RAW = false>
 __global__ void __launch_bounds__(256)
 conv_direct_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ taps,
                    const uint32_t* __restrict__ nnz, uint32_t pitch, ConvParams p,
@@ -87,7 +88,8 @@ conv_direct_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ ta
     const uint32_t nn = __ldg(nnz + mo);
     float acc = bias ? __ldg(bias + mo) : 0.0f;
     for (uint32_t j = 0; j < nn; ++j) {
-        const uint32_t t = __ldg(tp + j);
+        uint32_t t = __ldg(tp + j);
+        if (RAW) t = t / (p.kW * p.kH) << 16 | t / p.kW % p.kH << 8 | t % p.kW;
         const uint32_t cin = t >> 16;
         const int ih = ih0 + (int)(((t >> 8) & 0xffu) * p.dH);
         const int iw = iw0 + (int)((t & 0xffu) * p.dW);
@@ -356,7 +358,8 @@ conv_pf_tile_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ t
 //   w[(b*cap + c)*4 + r] = that row's weight, 0.0f where the bit is clear (never multiplied)
 //   ncols[b] = number of union columns.
 // One CTA per block: a K-bit set in shared memory collects the columns, a scan over its words
-// ranks them, a second pass over the rows scatters taps, masks and weights.
+// ranks them, a second pass over the rows scatters taps, masks and weights.  (w4 null: the headers alone, for a
+// further kernel shape; weights and counts are the same for all.)
 // ---------------------------------------------------------------------------------------------
 constexpr uint32_t kRbmRows = 4;
 constexpr uint32_t kRbmMaxK = 1u << 17;         // 2 x 16 KB of shared memory for the set and its ranks
@@ -396,13 +399,16 @@ build_rbm_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ idx,
             if (i < words) rank[i] = run + inc - c;
             run += __shfl_sync(0xffffffffu, inc, 31);
         }
-        if (threadIdx.x == 0) { total_s = run; ncols[blk] = run; }
+        if (threadIdx.x == 0) {
+            total_s = run;
+            if (w4) ncols[blk] = run;
+        }
     }
     __syncthreads();
     const uint32_t total = total_s;
     const size_t base = (size_t)blk * cap;
     for (uint32_t c = threadIdx.x; c < total; c += blockDim.x) hdr[base + c] = make_uint2(0u, 0u);
-    for (uint32_t c = threadIdx.x; c < total * kRbmRows; c += blockDim.x) w4[base * kRbmRows + c] = 0.0f;
+    for (uint32_t c = threadIdx.x; w4 && c < total * kRbmRows; c += blockDim.x) w4[base * kRbmRows + c] = 0.0f;
     __syncthreads();
     for (uint32_t r = 0; r < kRbmRows && r0 + r < m; ++r) {
         const uint32_t row = r0 + r, nn = nnz[row];
@@ -412,7 +418,7 @@ build_rbm_kernel(const float* __restrict__ Wd, const uint32_t* __restrict__ idx,
             const uint32_t kw = k % kW, kh = (k / kW) % kH, cin = k / (kW * kH);
             hdr[base + c].x = (cin << 16) | (kh << 8) | kw;      // the same value from every row
             atomicOr(&hdr[base + c].y, 1u << r);
-            w4[(base + c) * kRbmRows + r] = Wd[(size_t)row * pitch + j];
+            if (w4) w4[(base + c) * kRbmRows + r] = Wd[(size_t)row * pitch + j];
         }
     }
 }
@@ -705,39 +711,80 @@ conv_rbm_tile_kernel(const uint2* __restrict__ hdr, const float4* __restrict__ w
 namespace spx {
 
 ConvTables* new_conv_tables() { return new (std::nothrow) ConvTables(); }
-void free_conv_tables(spx_ell* e) { delete e->conv; e->conv = nullptr; }
 
-// What a handle's convolutions share is built on a stream beside the call's, which is waited for: the calls of other threads and
-// streams find it complete, and where the call's stream is being recorded it is there before the graph runs.  (A handle's
-// arrays are complete when it is handed out, so there is nothing to wait for before.)
+static size_t merged_slots(const spx_ell* e) { return (size_t)((e->m + kRbmRows - 1) / kRbmRows) * e->conv->cap; }
 
-// Builds (once per handle and kernel shape) the tap table.
-static int ensure_taps(spx_ell* e, uint32_t kH, uint32_t kW)
+void free_conv_tables(spx_ell* e)
 {
-    if (e->r == 0) return SPX_OK;
+    ConvTables* t = e->conv;
+    if (!t) return;
+    for (ConvTables::Shape* s = t->shapes; s;) {
+        pool_free(s->taps, (size_t)e->m * e->pitch * sizeof(uint32_t), nullptr);
+        pool_free(s->hdr, merged_slots(e) * sizeof(uint2), nullptr);
+        ConvTables::Shape* next = s->next;
+        delete s;
+        s = next;
+    }
+    pool_free(t->w, merged_slots(e) * kRbmRows * sizeof(float), nullptr);
+    pool_free(t->ncols, (size_t)((e->m + kRbmRows - 1) / kRbmRows) * sizeof(uint32_t), nullptr);
+    delete t;
+    e->conv = nullptr;
+}
+
+// A kernel shape's tables, empty where it is new; null without host memory.  Under the lock.
+static ConvTables::Shape* shape_tables(ConvTables* t, uint32_t kH, uint32_t kW)
+{
+    for (ConvTables::Shape* s = t->shapes; s; s = s->next)
+        if (s->kH == kH && s->kW == kW) return s;
+    ConvTables::Shape* s = new (std::nothrow) ConvTables::Shape();
+    if (!s) return nullptr;
+    s->kH = kH;
+    s->kW = kW;
+    s->next = t->shapes;
+    return t->shapes = s;
+}
+
+// Tables are built on a stream beside the call's, which is waited for: the calls of other threads and streams find them
+// complete, and where the call's stream is being recorded they are there before the graph runs.  (A handle's arrays are
+// complete when it is handed out, so there is nothing to wait for before.)
+
+// The tap table of a kernel shape, built once per handle; null where there is no memory for it.
+static int ensure_taps(spx_ell* e, uint32_t kH, uint32_t kW, const uint32_t** taps)
+{
     std::lock_guard<std::mutex> lk(e->conv->mu);
-    if (e->taps && e->taps_kH == kH && e->taps_kW == kW) return SPX_OK;
+    ConvTables::Shape* t = shape_tables(e->conv, kH, kW);
+    if (!t) return fail(SPX_ERR_OOM, "out of host memory");
+    *taps = t->taps;
+    if (t->taps || e->r == 0) return SPX_OK;
     RelaxedCapture relaxed;                     // allocations and waits below end no capture
     cudaStream_t side = nullptr;
     if (int rc = side_stream(e->device, &side)) return rc;
-    if (e->taps) wait_for_device();             // another kernel shape's, which calls may still be using
-    if (!e->taps)
-        if (int rc = pool_alloc(reinterpret_cast<void**>(&e->taps), (size_t)e->m * e->pitch * sizeof(uint32_t), e->device, side)) return rc;
-    build_taps_kernel<<<e->m, 128, 0, side>>>(e->idx, e->nnz, e->m, e->pitch, kH, kW, e->taps);
-    SPX_CUDA(cudaGetLastError());
-    count_launch_beside();
-    SPX_CUDA(cudaStreamSynchronize(side));
-    e->taps_kH = kH;
-    e->taps_kW = kW;
+    const size_t bytes = (size_t)e->m * e->pitch * sizeof(uint32_t);
+    void* made = nullptr;
+    if (int rc = pool_alloc(&made, bytes, e->device, side, t->no_taps)) {
+        t->no_taps = rc == SPX_ERR_OOM;
+        return t->no_taps ? SPX_OK : rc;
+    }
+    build_taps_kernel<<<e->m, 128, 0, side>>>(e->idx, e->nnz, e->m, e->pitch, kH, kW, static_cast<uint32_t*>(made));
+    cudaError_t err = cudaGetLastError();
+    if (err == cudaSuccess) {
+        count_launch_beside();
+        err = cudaStreamSynchronize(side);
+    }
+    if (err != cudaSuccess) {
+        pool_free(made, bytes, side);
+        return fail(SPX_ERR_CUDA, "conv2d: building the tap table failed: %s", cudaGetErrorString(err));
+    }
+    *taps = t->taps = static_cast<uint32_t*>(made);
     return SPX_OK;
 }
 
 template <int QB, int G, int WARPS, int MINB>
-static int launch_tile_qb(const spx_ell* e, const TileParams& tp, dim3 grid, size_t smem, const float* in,
+static int launch_tile_qb(const spx_ell* e, const uint32_t* taps, const TileParams& tp, dim3 grid, size_t smem, const float* in,
                           const float* bias, int act, float* out, cudaStream_t s)
 {
     if (int rc = allow_smem<conv_pf_tile_kernel<QB, G, WARPS, MINB>>(e->device)) return rc;
-    conv_pf_tile_kernel<QB, G, WARPS, MINB><<<grid, WARPS * 32, smem, s>>>(e->Wd, e->taps, e->nnz, e->pitch, tp, in, bias, act, out);
+    conv_pf_tile_kernel<QB, G, WARPS, MINB><<<grid, WARPS * 32, smem, s>>>(e->Wd, taps, e->nnz, e->pitch, tp, in, bias, act, out);
     SPX_LAUNCH_CHECK("conv_pf_tile_kernel");
     return SPX_OK;
 }
@@ -781,49 +828,61 @@ static bool rbm_fits(const ConvParams& p, uint32_t qb, int nb, int g)
     return THin * TWin * qb * 4 * sizeof(float) <= rbm_budget(nb) / (nb == 16 ? 1 : 2);
 }
 
-// Builds (once per handle and kernel shape) the row-block-merged weights, as ensure_taps does.
-int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW)
+// The row-block-merged weights, built once per handle, and the headers of a kernel shape, built as ensure_taps does.
+int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, const uint2** hdr)
 {
-    std::lock_guard<std::mutex> lk(e->conv->mu);
-    if (e->rbm_hdr && e->rbm_kH == kH && e->rbm_kW == kW) return SPX_OK;
+    ConvTables* t = e->conv;
+    std::lock_guard<std::mutex> lk(t->mu);
+    ConvTables::Shape* shape = shape_tables(t, kH, kW);
+    if (!shape) return fail(SPX_ERR_OOM, "out of host memory");
+    if (hdr) *hdr = shape->hdr;
+    if (shape->hdr) return SPX_OK;
+    if (t->no_merged || shape->no_hdr) return -1;
     RelaxedCapture relaxed;                     // allocations and waits below end no capture
     cudaStream_t side = nullptr;
     if (int rc = side_stream(e->device, &side)) return rc;
     const uint32_t nblocks = (e->m + kRbmRows - 1) / kRbmRows;
-    if (e->rbm_hdr) wait_for_device();          // another kernel shape's, which calls may still be using
-    if (!e->rbm_hdr) {
-        // Up to three times the ELLPACK slab (24 bytes per union column, at most 4 * max_nnz columns
-        // per block of 4 rows).  Without room for it the per-row kernel is used instead.
-        if (e->rbm_cap == UINT32_MAX) return -1;        // an earlier attempt ran out of memory
-        const uint32_t cap = (uint32_t)std::min<uint64_t>((uint64_t)kRbmRows * e->max_nnz, e->n);
-        const size_t slots = (size_t)nblocks * cap;
-        if (pool_alloc_now(reinterpret_cast<void**>(&e->rbm_ncols), (size_t)nblocks * sizeof(uint32_t), e->device) != SPX_OK ||
-            pool_alloc_now(reinterpret_cast<void**>(&e->rbm_w), slots * kRbmRows * sizeof(float), e->device) != SPX_OK ||
-            pool_alloc_now(reinterpret_cast<void**>(&e->rbm_hdr), slots * sizeof(uint2), e->device) != SPX_OK) {
-            pool_free(e->rbm_ncols, (size_t)nblocks * sizeof(uint32_t), side);
-            pool_free(e->rbm_w, slots * kRbmRows * sizeof(float), side);
-            pool_free(e->rbm_hdr, slots * sizeof(uint2), side);
-            e->rbm_ncols = nullptr; e->rbm_w = nullptr; e->rbm_hdr = nullptr;
-            e->rbm_cap = UINT32_MAX;
-            return -1;
-        }
-        e->rbm_cap = cap;
+    // Up to three times the ELLPACK slab (24 bytes per union column, at most 4 * max_nnz columns
+    // per block of 4 rows).  Without room for it the per-row kernel is used instead.
+    const bool first = !t->w;
+    if (first) t->cap = (uint32_t)std::min<uint64_t>((uint64_t)kRbmRows * e->max_nnz, e->n);
+    const size_t slots = merged_slots(e);
+    void *w = nullptr, *ncols = nullptr, *made = nullptr;
+    int rc = pool_alloc(&made, slots * sizeof(uint2), e->device, side);
+    if (rc == SPX_OK && first) rc = pool_alloc(&w, slots * kRbmRows * sizeof(float), e->device, side);
+    if (rc == SPX_OK && first) rc = pool_alloc(&ncols, nblocks * sizeof(uint32_t), e->device, side);
+    cudaError_t err = cudaSuccess;
+    if (rc == SPX_OK) {
         ensure_tma_words(e);
         (void)cudaGetLastError();
+        const size_t smem = (size_t)((e->n + 31) / 32) * 2 * sizeof(uint32_t);
+        build_rbm_kernel<<<nblocks, 256, smem, side>>>(e->Wd, e->idx, e->nnz, e->m, e->n, e->pitch, kH, kW, t->cap,
+                                                       static_cast<uint2*>(made), static_cast<float*>(w), static_cast<uint32_t*>(ncols));
+        err = cudaGetLastError();
+        if (err == cudaSuccess) {
+            count_launch_beside();
+            err = cudaStreamSynchronize(side);
+        }
     }
-    const size_t smem = (size_t)((e->n + 31) / 32) * 2 * sizeof(uint32_t);
-    build_rbm_kernel<<<nblocks, 256, smem, side>>>(e->Wd, e->idx, e->nnz, e->m, e->n, e->pitch, kH, kW, e->rbm_cap,
-                                                   e->rbm_hdr, e->rbm_w, e->rbm_ncols);
-    SPX_CUDA(cudaGetLastError());
-    count_launch_beside();
-    SPX_CUDA(cudaStreamSynchronize(side));
-    e->rbm_kH = kH;
-    e->rbm_kW = kW;
+    if (rc != SPX_OK || err != cudaSuccess) {
+        pool_free(made, slots * sizeof(uint2), side);
+        pool_free(w, slots * kRbmRows * sizeof(float), side);
+        pool_free(ncols, nblocks * sizeof(uint32_t), side);
+        if (err != cudaSuccess) return fail(SPX_ERR_CUDA, "conv2d: merging the weights failed: %s", cudaGetErrorString(err));
+        (first ? t->no_merged : shape->no_hdr) = true;
+        return -1;
+    }
+    if (first) {
+        t->w = static_cast<float*>(w);
+        t->ncols = static_cast<uint32_t*>(ncols);
+    }
+    shape->hdr = static_cast<uint2*>(made);
+    if (hdr) *hdr = shape->hdr;
     return SPX_OK;
 }
 
 template <int QB, int NB, int G>
-static int launch_rbm_units(const spx_ell* e, TileParams tp, RbmUnits un, uint32_t ctas, const float* in, const float* bias,
+static int launch_rbm_units(const spx_ell* e, const uint2* hdr, TileParams tp, RbmUnits un, uint32_t ctas, const float* in, const float* bias,
                             int act, float* out, cudaStream_t s, uint32_t b_avail)
 {
     const ConvParams& p = tp.c;
@@ -864,8 +923,8 @@ static int launch_rbm_units(const spx_ell* e, TileParams tp, RbmUnits un, uint32
     }
     const size_t smem = use_tma ? (size_t)tp.stage * (p.Cin > tp.CC ? 2 : 1) * sizeof(float) : chanBytes * tp.CC;
     if (int rc = allow_smem<conv_rbm_tile_kernel<QB, NB, G>>(e->device)) return rc;
-    const cudaError_t err = launch_pdl(conv_rbm_tile_kernel<QB, NB, G>, dim3(ctas), dim3(NB * 32), smem, s, e->rbm_hdr, reinterpret_cast<const float4*>(e->rbm_w), e->rbm_ncols,
-                     e->rbm_cap, tp, un, in, bias, act, out, map, use_tma, e->tma_failed_dev, e->tma_failed_mapped);
+    const cudaError_t err = launch_pdl(conv_rbm_tile_kernel<QB, NB, G>, dim3(ctas), dim3(NB * 32), smem, s, hdr, reinterpret_cast<const float4*>(e->conv->w), e->conv->ncols,
+                     e->conv->cap, tp, un, in, bias, act, out, map, use_tma, e->tma_failed_dev, e->tma_failed_mapped);
     if (err != cudaSuccess) return fail(SPX_ERR_CUDA, "launch of conv_rbm_tile_kernel failed: %s", cudaGetErrorString(err));
     count_launch();
     return SPX_OK;
@@ -962,13 +1021,14 @@ static int launch_rbm_qb(spx_ell* e, TileParams tp, const float* in, const float
     const uint32_t groups = (nblocks + cut.nb - 1) / cut.nb;
     const uint64_t units = tiles * groups * (b_len / (QB * 4));
     if (units > 0x3fffffffull) return -1;
-    const int rc = ensure_rbm(e, p.kH, p.kW);
+    const uint2* hdr = nullptr;
+    const int rc = ensure_rbm(e, p.kH, p.kW, &hdr);
     if (rc != SPX_OK) return rc;                        // -1: no memory for the merged weights
     RbmUnits un{0u, (uint32_t)tiles, groups, 0u};
-    if (cut.nb == 8 && cut.g == 4) return launch_rbm_units<QB, 8, 4>(e, tp, un, (uint32_t)units, in, bias, act, out, s, b_avail);
-    if (cut.nb == 8) return launch_rbm_units<QB, 8, 2>(e, tp, un, (uint32_t)units, in, bias, act, out, s, b_avail);
-    if (cut.nb == 4 && cut.g == 2) return launch_rbm_units<QB, 4, 2>(e, tp, un, (uint32_t)units, in, bias, act, out, s, b_avail);
-    if (cut.nb == 4) return launch_rbm_units<QB, 4, 1>(e, tp, un, (uint32_t)units, in, bias, act, out, s, b_avail);
+    if (cut.nb == 8 && cut.g == 4) return launch_rbm_units<QB, 8, 4>(e, hdr, tp, un, (uint32_t)units, in, bias, act, out, s, b_avail);
+    if (cut.nb == 8) return launch_rbm_units<QB, 8, 2>(e, hdr, tp, un, (uint32_t)units, in, bias, act, out, s, b_avail);
+    if (cut.nb == 4 && cut.g == 2) return launch_rbm_units<QB, 4, 2>(e, hdr, tp, un, (uint32_t)units, in, bias, act, out, s, b_avail);
+    if (cut.nb == 4) return launch_rbm_units<QB, 4, 1>(e, hdr, tp, un, (uint32_t)units, in, bias, act, out, s, b_avail);
     // One CTA per SM, all units equally long: the launch runs in waves of sm_count units.  A last
     // wave that fills less than half of the SMs is issued as a second launch of half-height tiles
     // (twice the CTAs, each about 0.6 of a full unit's time): 784 units on 148 SMs are 5 full waves
@@ -977,13 +1037,13 @@ static int launch_rbm_qb(spx_ell* e, TileParams tp, const float* in, const float
     const uint32_t sms = (uint32_t)sm_count(e->device);
     const uint32_t rem = (uint32_t)(units % sms);
     if (split_tail && units > sms && rem && rem * 2 <= sms) {
-        const int rc1 = launch_rbm_units<QB, 16, kRbmG>(e, tp, un, (uint32_t)(units - rem), in, bias, act, out, s, b_avail);
+        const int rc1 = launch_rbm_units<QB, 16, kRbmG>(e, hdr, tp, un, (uint32_t)(units - rem), in, bias, act, out, s, b_avail);
         if (rc1 != SPX_OK) return rc1;
         un.unit0 = (uint32_t)(units - rem);
         un.half = 1;
-        return launch_rbm_units<QB, 16, kRbmG / 2>(e, tp, un, rem * 2, in, bias, act, out, s, b_avail);
+        return launch_rbm_units<QB, 16, kRbmG / 2>(e, hdr, tp, un, rem * 2, in, bias, act, out, s, b_avail);
     }
-    return launch_rbm_units<QB, 16, kRbmG>(e, tp, un, (uint32_t)units, in, bias, act, out, s, b_avail);
+    return launch_rbm_units<QB, 16, kRbmG>(e, hdr, tp, un, (uint32_t)units, in, bias, act, out, s, b_avail);
 }
 
 // Row-block-merged path.  Taken whenever K fits the builder's set and the batch is a multiple of 4:
@@ -1048,7 +1108,7 @@ static int launch_conv_rbm_tile(spx_ell* e, const ConvParams& p, const ConvViews
 }
 
 // Returns -1 when the shape is not covered (caller falls back to the direct kernel).
-static int launch_conv_pf_tile(spx_ell* e, const ConvParams& p, const ConvViews& v, const float* in, const float* bias, int act,
+static int launch_conv_pf_tile(spx_ell* e, const uint32_t* taps, const ConvParams& p, const ConvViews& v, const float* in, const float* bias, int act,
                                float* out, cudaStream_t s)
 {
     if (!e->cols_ascending || !pf_tile_covers(p)) return -1;
@@ -1098,11 +1158,11 @@ static int launch_conv_pf_tile(spx_ell* e, const ConvParams& p, const ConvViews&
     if (tiles > 0x7fffffffull || gy > 65535 || gz > 65535) return -1;
     dim3 grid((unsigned)tiles, gy, gz);
     const size_t smem = chanBytes * tp.CC;
-    if (small) return launch_tile_qb<8, 4, 32, 1>(e, tp, grid, smem, in, bias, act, out, s);
-    if (Gv != QBv) return launch_tile_qb<2, 4, kTileWarps, 2>(e, tp, grid, smem, in, bias, act, out, s);
+    if (small) return launch_tile_qb<8, 4, 32, 1>(e, taps, tp, grid, smem, in, bias, act, out, s);
+    if (Gv != QBv) return launch_tile_qb<2, 4, kTileWarps, 2>(e, taps, tp, grid, smem, in, bias, act, out, s);
 #define SPX_TILE_CASE(Q)                                                                                           \
-    case Q: return per_sm == 2 ? launch_tile_qb<Q, Q, kTileWarps, 2>(e, tp, grid, smem, in, bias, act, out, s)     \
-                               : launch_tile_qb<Q, Q, kTileWarps, 1>(e, tp, grid, smem, in, bias, act, out, s);
+    case Q: return per_sm == 2 ? launch_tile_qb<Q, Q, kTileWarps, 2>(e, taps, tp, grid, smem, in, bias, act, out, s)     \
+                               : launch_tile_qb<Q, Q, kTileWarps, 1>(e, taps, tp, grid, smem, in, bias, act, out, s);
     switch (BT / 4) {
         SPX_TILE_CASE(1) SPX_TILE_CASE(2) SPX_TILE_CASE(3) SPX_TILE_CASE(4)
         SPX_TILE_CASE(5) SPX_TILE_CASE(6) SPX_TILE_CASE(7) SPX_TILE_CASE(8)
@@ -1265,8 +1325,8 @@ int launch_conv2d(spx_ell* e, const spx_conv_geom* g, int layout, const float* i
             return SPX_OK;
         }
     }
-    int rc = ensure_taps(e, g->kH, g->kW);
-    if (rc != SPX_OK) return rc;
+    const uint32_t* taps = nullptr;
+    if (int rc = ensure_taps(e, g->kH, g->kW, &taps)) return rc;
     ConvParams p{g->Cin, g->Cout, g->kH, g->kW, g->sH, g->sW, g->pH, g->pW, g->dH, g->dW,
                  g->H, g->W, g->Ho, g->Wo, B};
     // The tiled kernels read the batch as the innermost dimension, in multiples of 4 and of 16 bytes, and
@@ -1278,10 +1338,10 @@ int launch_conv2d(spx_ell* e, const spx_conv_geom* g, int layout, const float* i
     const uint32_t B4 = padded_batch(B, merged_kernel_takes(e));
     ConvParams p4 = p;
     p4.B = B4;
-    const bool tiled = e->r && e->cols_ascending && pf_tile_covers(p4);
+    const bool tiled = taps && e->cols_ascending && pf_tile_covers(p4);
     ConvGatherPlan gather;
-    const bool gathers = e->r && plan_conv_gather(e, p, layout, in, out, gather);
-    if (gathers && !tiled) return launch_conv_gather(e, p, layout, in, bias, act, out, gather, s);
+    const bool gathers = taps && plan_conv_gather(e, p, layout, in, out, gather);
+    if (gathers && !tiled) return launch_conv_gather(e, taps, p, layout, in, bias, act, out, gather, s);
     if (tiled) {
         const uint64_t H = g->H, W = g->W, Ho = g->Ho, Wo = g->Wo;
         ConvViews v{};
@@ -1300,7 +1360,7 @@ int launch_conv2d(spx_ell* e, const spx_conv_geom* g, int layout, const float* i
         v.vec_out = v.oB == 1 && B4 == B && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
         const float* src = in;
         const bool copies = iB != 1 || B4 != B || (reinterpret_cast<uintptr_t>(in) & 15);
-        if (gathers && gather_pays(e, p4, v, copies, B, gather, s)) return launch_conv_gather(e, p, layout, in, bias, act, out, gather, s);
+        if (gathers && gather_pays(e, p4, v, copies, B, gather, s)) return launch_conv_gather(e, taps, p, layout, in, bias, act, out, gather, s);
         if (copies) {
             const uint64_t positions = g->Cin * H * W;
             const size_t need = positions * B4 * sizeof(float);
@@ -1323,7 +1383,7 @@ int launch_conv2d(spx_ell* e, const spx_conv_geom* g, int layout, const float* i
             v.iC = H * W * B4; v.iH = W * B4; v.iW = B4;
             src = dst;
         }
-        rc = launch_conv_pf_tile(e, p4, v, src, bias, act, out, s);
+        const int rc = launch_conv_pf_tile(e, taps, p4, v, src, bias, act, out, s);
         if (rc != -1) return rc;                 // -1: shape not covered by the tiled kernels
     }
     const uint64_t per_m = (uint64_t)g->Ho * g->Wo * B;
@@ -1331,12 +1391,11 @@ int launch_conv2d(spx_ell* e, const spx_conv_geom* g, int layout, const float* i
     if (gx > 0x7fffffffull || e->m > 65535)
         return fail(SPX_ERR_LIMIT, "conv2d: output too large for one launch");
     dim3 grid((unsigned)gx, e->m);
-    if (layout == SPX_LAYOUT_PF)
-        conv_direct_kernel<SPX_LAYOUT_PF><<<grid, 256, 0, s>>>(e->Wd, e->taps, e->nnz, e->pitch, p, in, bias, act, out);
-    else if (layout == SPX_LAYOUT_FMAJOR)
-        conv_direct_kernel<SPX_LAYOUT_FMAJOR><<<grid, 256, 0, s>>>(e->Wd, e->taps, e->nnz, e->pitch, p, in, bias, act, out);
-    else
-        conv_direct_kernel<SPX_LAYOUT_NCHW><<<grid, 256, 0, s>>>(e->Wd, e->taps, e->nnz, e->pitch, p, in, bias, act, out);
+    const bool raw = !taps;
+    const auto direct = layout == SPX_LAYOUT_PF       ? (raw ? conv_direct_kernel<SPX_LAYOUT_PF, true> : conv_direct_kernel<SPX_LAYOUT_PF>)
+                        : layout == SPX_LAYOUT_FMAJOR ? (raw ? conv_direct_kernel<SPX_LAYOUT_FMAJOR, true> : conv_direct_kernel<SPX_LAYOUT_FMAJOR>)
+                                                      : (raw ? conv_direct_kernel<SPX_LAYOUT_NCHW, true> : conv_direct_kernel<SPX_LAYOUT_NCHW>);
+    direct<<<grid, 256, 0, s>>>(e->Wd, raw ? e->idx : taps, e->nnz, e->pitch, p, in, bias, act, out);
     SPX_LAUNCH_CHECK("conv_direct_kernel");
     return SPX_OK;
 }

@@ -41,17 +41,32 @@ struct ConvGatherPlan {
     double us = 0.0;
 };
 bool plan_conv_gather(const spx_ell* e, const ConvParams& p, int layout, const float* in, const float* out, ConvGatherPlan& plan);
-int launch_conv_gather(const spx_ell* e, const ConvParams& p, int layout, const float* in, const float* bias, int act, float* out,
+int launch_conv_gather(const spx_ell* e, const uint32_t* taps, const ConvParams& p, int layout, const float* in, const float* bias, int act, float* out,
                        const ConvGatherPlan& plan, cudaStream_t s);
-// What a handle's convolutions share is built by whichever call first needs it, on any thread and stream: under this lock, and
-// complete for every stream when it is let go.
+// What a handle's convolutions share.  Built by whichever call first needs it, on any thread and stream: under the lock, and
+// complete for every stream when that is let go.  Nothing is changed or given back before the handle is: calls in flight
+// and recorded graphs may be using it.
 struct ConvTables {
+    struct Shape {                  // of a kernel
+        uint32_t kH = 0, kW = 0;
+        uint32_t* taps = nullptr;   // per slot of the slab: the column as cin << 16 | kh << 8 | kw
+        uint2* hdr = nullptr;       // per merged column: (the same, bit r set when row r of the block stores it)
+        bool no_taps = false, no_hdr = false;   // an earlier call found no memory for them
+        Shape* next = nullptr;
+    };
     std::mutex mu;
+    Shape* shapes = nullptr;        // as many as the handle is used with: divisors of its columns
+    // Row-block-merged weights (conv.cu): per block of 4 rows the ascending union of their column ids.  Block b owns entries
+    // [b * cap, b * cap + ncols[b]): the 4 rows' weights, 0.0f where a row has none, and the headers above.
+    float* w = nullptr;
+    uint32_t* ncols = nullptr;
+    uint32_t cap = 0;
+    bool no_merged = false;         // an earlier call found no memory for them
 };
 ConvTables* new_conv_tables();
 void free_conv_tables(spx_ell* e);
-// conv.cu: the merged weights of conv_rbm_tile_kernel; -1 where there is no memory for them.
-int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW);
+// conv.cu: the merged weights of conv_rbm_tile_kernel, and (hdr may be null) their headers; -1 where there is no memory for them.
+int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, const uint2** hdr);
 void* new_conv_tmem();
 void free_conv_tmem(spx_ell* e);
 

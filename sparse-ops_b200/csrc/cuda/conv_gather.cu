@@ -292,12 +292,12 @@ bool plan_conv_gather(const spx_ell* e, const ConvParams& p, int layout, const f
     return true;
 }
 
-int launch_conv_gather(const spx_ell* e, const ConvParams& p, int layout, const float* in, const float* bias, int act, float* out,
+int launch_conv_gather(const spx_ell* e, const uint32_t* taps, const ConvParams& p, int layout, const float* in, const float* bias, int act, float* out,
                        const ConvGatherPlan& plan, cudaStream_t s)
 {
     const uint32_t H = p.H, W = p.W, Ho = p.Ho, Wo = p.Wo, B = p.B;
     GatherArgs a{};
-    a.Wd = e->Wd; a.taps = e->taps; a.rows = e->rows; a.m = e->m; a.pitch = e->pitch;
+    a.Wd = e->Wd; a.taps = taps; a.rows = e->rows; a.m = e->m; a.pitch = e->pitch;
     a.in = in; a.bias = bias; a.out = out; a.act = act;
     a.kH = p.kH; a.kW = p.kW; a.sH = p.sH; a.sW = p.sW; a.pH = p.pH; a.pW = p.pW; a.dH = p.dH; a.dW = p.dW; a.H = H; a.W = W;
     a.positions = Ho * Wo * B;

@@ -580,7 +580,7 @@ static int find_form(spx_ell* e, const FormShape& f, uint32_t chunks, uint32_t p
     }
     RelaxedCapture relaxed;                     // s is not being captured; another stream may be, by this thread
     // The other kernel's weights, which a later call may take (another batch, say); how many columns they have is counted below.
-    const int merged = ensure_rbm(e, f.kH, f.kW);
+    const int merged = ensure_rbm(e, f.kH, f.kW, nullptr);
     if (merged > 0) return merged;
     ensure_tma_words(e);
     if (!e->tma_failed_dev || !e->tma_failed_mapped) {
@@ -616,7 +616,7 @@ static int find_form(spx_ell* e, const FormShape& f, uint32_t chunks, uint32_t p
     cudaError_t err = cudaGetLastError();
     if (err == cudaSuccess) count_launch();
     if (err == cudaSuccess && loads) {
-        conv_load_kernel<<<groups, 128, 0, s>>>(static_cast<uint32_t*>(entries), e->rbm_ncols, e->nnz, e->m, chunks, per_group, f.chunk_cols,
+        conv_load_kernel<<<groups, 128, 0, s>>>(static_cast<uint32_t*>(entries), e->conv->ncols, e->nnz, e->m, chunks, per_group, f.chunk_cols,
                                                 static_cast<CtaClocks*>(found), reinterpret_cast<uint2*>(static_cast<CtaClocks*>(found) + groups));
         err = cudaGetLastError();
         if (err == cudaSuccess) count_launch();

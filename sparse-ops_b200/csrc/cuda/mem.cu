@@ -77,10 +77,10 @@ static int allocate(void** p, size_t bytes, int device, cudaStream_t s, bool poo
     return SPX_OK;
 }
 
-int pool_alloc(void** p, size_t bytes, int device, cudaStream_t s) { return allocate(p, bytes, device, s, bytes <= kPoolBlock); }
+// optional: the caller can do without, and is told at once; to give memory back first would wait for the whole device.
+int pool_alloc(void** p, size_t bytes, int device, cudaStream_t s, bool optional) { return allocate(p, bytes, device, s, bytes <= kPoolBlock, !optional); }
 
 // Scratch of one call, whatever its size: mapping and freeing memory directly would make the call wait for the device.
-// optional: the caller can do without, and is told at once; to give memory back first would wait for the whole device.
 int scratch_alloc(void** p, size_t bytes, int device, cudaStream_t s, bool optional) { return allocate(p, bytes, device, s, true, !optional); }
 void scratch_free(void* p, cudaStream_t s) { if (p) (void)cudaFreeAsync(p, s); }
 

@@ -11,7 +11,7 @@ import torch
 
 import spx_ctypes as sx
 from conftest import assert_bit_equal
-from test_conv_tmem_gpu import assert_ran, child, kernels_of, waits_for_the_device
+from test_conv_tmem_gpu import assert_ran, child, fill_device, kernels_of, waits_for_the_device
 from test_parity_gpu import as_layout, dev, gpu_ell, ptr, sparse
 
 pytestmark = pytest.mark.gpu
@@ -219,6 +219,82 @@ def test_eager_call_between_recording_and_replay(lib, orc, cuda, B):
     torch.cuda.synchronize()
     for k, y in enumerate(Y):
         assert_bit_equal(y.cpu().numpy(), want, f"call {k}")
+
+
+def two_kernel_shapes(lib, orc, cuda, Cin, Cout, H, B, density, full_row=False):
+    """A handle, and what a 3 x 3 and a 1 x 9 kernel over its columns give: (geometry, batch, input, result) each."""
+    rng = np.random.default_rng(17)
+    wt = sparse(rng, Cout, Cin * 9, density)
+    if full_row:
+        wt[0] = 1
+    E = orc.encode(wt)
+    x = rng.standard_normal((max(B), Cin, H, H)).astype(np.float32)
+    runs = []
+    for b in B:
+        for kH, kW in ((3, 3), (1, 9)):
+            src = as_layout(x[:b], sx.LAYOUT_PF)
+            gd = dict(Cin=Cin, kH=kH, kW=kW, sH=2, sW=2, pH=kH // 2, pW=kW // 2, dH=1, dW=1, H=H, W=H)
+            runs.append((sx.conv_geom(Cin, Cout, kH, kW, H, H, 2, 2, kH // 2, kW // 2), b, dev(src, cuda), orc.conv2d(E, gd, sx.LAYOUT_PF, src, b, None, 0)))
+    return gpu_ell(lib, E), runs
+
+
+@chosen
+def test_two_kernel_shapes_of_a_handle(lib, orc, cuda):
+    """Graphs of one kernel shape keep theirs when another one is recorded and called; calls of both alternate on two streams,
+    one of which is held up."""
+    h, runs = two_kernel_shapes(lib, orc, cuda, 64, 64, 28, [1, 32], 0.3)
+    graphs, outs = [], [torch.full(want.shape, float("nan"), device=cuda) for *_, want in runs]
+    for (g, B, dX, want), dY in zip(runs, outs):
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1]):
+            h.conv2d(g, sx.LAYOUT_PF, ptr(dX), B, None, 0, ptr(dY), torch.cuda.current_stream().cuda_stream)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    with torch.cuda.stream(streams[0]):
+        torch.cuda._sleep(100_000_000)
+    eager = []
+    for _ in range(2):
+        for k, (g, B, dX, want) in enumerate(runs):
+            eager.append((torch.full(want.shape, float("nan"), device=cuda), want))
+            torch.cuda.current_stream().synchronize()
+            h.conv2d(g, sx.LAYOUT_PF, ptr(dX), B, None, 0, ptr(eager[-1][0]), streams[k % 2].cuda_stream)
+    torch.cuda.synchronize()
+    for graph in graphs:
+        graph.replay()
+    torch.cuda.synchronize()
+    for dY, want in eager + [(dY, run[3]) for dY, run in zip(outs, runs)]:
+        assert_bit_equal(dY.cpu().numpy(), want, "two kernel shapes")
+
+
+no_memory = pytest.mark.skipif(os.environ.get("SPX_TEST_NO_MEMORY") != "1", reason="runs in a child process")
+
+
+@no_memory
+def test_second_kernel_shape_without_memory(lib, orc, cuda):
+    """There is no room for another kernel shape's tables: the ids are decoded by the general kernel, and no call waits for the
+    device to look for memory again."""
+    h, runs = two_kernel_shapes(lib, orc, cuda, 512, 2048, 4, [4], 0.01, full_row=True)     # a tap table is 38 MB
+    outs = [torch.full(want.shape, float("nan"), device=cuda) for *_, want in runs]
+    call = lambda k: h.conv2d(runs[k][0], sx.LAYOUT_PF, ptr(runs[k][2]), runs[k][1], None, 0, ptr(outs[k]))
+    call(0)
+    assert not waits_for_the_device(lambda: None)           # (makes the stream while there is room)
+    held = fill_device(lib, 4 << 20, 16 << 20)
+    try:
+        for again in (False, True):
+            outs[1].fill_(float("nan"))
+            waited = waits_for_the_device(lambda: call(1))
+            assert not (again and waited), "waited for another stream's work"
+            assert_bit_equal(outs[1].cpu().numpy(), runs[1][3], "no room")
+            call(0)
+            assert_bit_equal(outs[0].cpu().numpy(), runs[0][3], "the first kernel shape")
+    finally:
+        for p in held:
+            lib.spx_free(p)
+    call(1)
+    assert_bit_equal(outs[1].cpu().numpy(), runs[1][3], "room again")
+
+
+def test_without_memory():
+    child(["test_conv_gather_gpu.py"], "second_kernel_shape_without", {"SPX_TEST_NO_MEMORY": "1"})
 
 
 @chosen
