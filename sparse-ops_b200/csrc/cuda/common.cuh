@@ -51,11 +51,7 @@ struct spx_ell {
     bool tma_off = false;
     // Tiled form of the matrix for spmm_tile.cu, built on the second SpMM call that can use it.
     void* tiles = nullptr;
-    // How the entries lie for the merged kernel (conv.cu, MergedLoad of CTAs of 16, 8 and 4 row blocks): 0 not counted yet, 1
-    // counted, 2 not to be counted (no memory).
-    int conv_loads_state = 0;
-    double conv_loads[3][4] = {};
-    // Tap tables and merged weights of the convolution (conv.cuh).
+    // Tap tables and merged weights of the convolution, and how the entries lie for it (conv.cuh).
     spx::ConvTables* conv = nullptr;
     // The convolution's entries for conv_tmem.cu, built on the first call that uses them.
     void* conv_tmem = nullptr;

@@ -1203,33 +1203,33 @@ union_count_kernel(const uint32_t* __restrict__ idx, const uint32_t* __restrict_
     if (threadIdx.x == 0) blocks[blockIdx.x] = make_uint2(s_fresh, all);
 }
 
-// Counts once per handle; the call then waits for its stream.  Not while a graph is recorded on it.
+// Counts once per handle, beside the call like the tables.  Not for a call that is recorded.
 static void count_loads(spx_ell* e, cudaStream_t s)
 {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) { (void)cudaGetLastError(); return; }
+    ConvTables* t = e->conv;
+    std::lock_guard<std::mutex> lk(t->mu);
+    if (t->loads_state.load(std::memory_order_relaxed) != ConvTables::unknown) return;
     RelaxedCapture relaxed;                     // s is not being captured; another stream may be, by this thread
-    e->conv_loads_state = 2;
     const uint32_t nblocks = (e->m + kRbmRows - 1) / kRbmRows;
     const size_t bytes = (size_t)nblocks * sizeof(uint2);
     PinnedBlock host;
     void* blocks = nullptr;
-    if (scratch_alloc(&blocks, bytes, e->device, s, true) == SPX_OK && pinned_acquire(bytes, &host) == SPX_OK) {
-        union_count_kernel<<<nblocks, 256, std::min(kCountWords, (e->n + 31) / 32) * 4, s>>>(e->idx, e->nnz, e->m, e->n, e->pitch, static_cast<uint2*>(blocks));
-        count_launch();
-        if (cudaGetLastError() == cudaSuccess && cudaMemcpyAsync(host.host, blocks, bytes, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-            cudaStreamSynchronize(s) == cudaSuccess) {
-            MergedLoad load[3];
-            merged_loads(static_cast<const uint2*>(host.host), nblocks, load);
-            for (int k = 0; k < 3; ++k) {
-                const double v[4] = {load[k].longest, load[k].work, load[k].longest_worst, load[k].work_worst};
-                std::copy(v, v + 4, e->conv_loads[k]);
-            }
-            e->conv_loads_state = 1;
+    cudaStream_t side = nullptr;
+    int state = ConvTables::no_memory;
+    if (side_stream(e->device, &side) == SPX_OK && scratch_alloc(&blocks, bytes, e->device, side, true) == SPX_OK && pinned_acquire(bytes, &host) == SPX_OK) {
+        union_count_kernel<<<nblocks, 256, std::min(kCountWords, (e->n + 31) / 32) * 4, side>>>(e->idx, e->nnz, e->m, e->n, e->pitch, static_cast<uint2*>(blocks));
+        count_launch_beside();
+        if (cudaGetLastError() == cudaSuccess && cudaMemcpyAsync(host.host, blocks, bytes, cudaMemcpyDeviceToHost, side) == cudaSuccess &&
+            cudaStreamSynchronize(side) == cudaSuccess) {
+            merged_loads(static_cast<const uint2*>(host.host), nblocks, t->loads);
+            state = ConvTables::counted;
         }
     }
     pinned_release(host);
-    scratch_free(blocks, s);
+    scratch_free(blocks, side);
+    t->loads_state.store(state, std::memory_order_release);
 }
 
 // What the tiled kernels are expected to take: the merged kernel, the one in tensor memory, and the copy of an input that is
@@ -1247,10 +1247,8 @@ static double tiled_us(const spx_ell* e, const ConvParams& p4, const ConvViews& 
             const double work = std::min(16u >> k, (p4.Cout + kRbmRows - 1) / kRbmRows) * (0.7 + 0.2 * kRbmRows) * len;
             load[k] = MergedLoad{len, work, len, work};
         }
-    } else if (by == Loads::counted) {
-        for (int k = 0; k < 3; ++k) load[k] = MergedLoad{e->conv_loads[k][0], e->conv_loads[k][1], e->conv_loads[k][2], e->conv_loads[k][3]};
     }
-    double us = conv_rbm_us(e, p4, by == Loads::density ? nullptr : load);
+    double us = conv_rbm_us(e, p4, by == Loads::density ? nullptr : by == Loads::counted ? e->conv->loads : load);
     if (e->m >= 8 * kRbmRows - 3) us = std::min(us, conv_tmem_expected(e, p4, v, conv_rbm_us));
     if (copies) us += 2.5 + 4e-6 / 3 * (double)p4.Cin * p4.H * p4.W * (p4.B + B);
     return us < 1e20 ? us : 0.0;                // (a patch that no cut of the merged kernel stages)
@@ -1267,12 +1265,14 @@ static bool gather_pays(spx_ell* e, const ConvParams& p4, const ConvViews& v, bo
 {
     const double us = plan.us / (plan.form >= 2 ? 0.85 : 0.9);
     if (e->m < 8 * kRbmRows - 3) return us <= tiled_us(e, p4, v, copies, B, Loads::density);
-    if (e->conv_loads_state == 0) {
+    const std::atomic<int>& state = e->conv->loads_state;
+    if (state.load(std::memory_order_acquire) != ConvTables::counted) {
         if (us <= tiled_us(e, p4, v, copies, B, Loads::least)) return true;
-        if (us > 1.05 * tiled_us(e, p4, v, copies, B, Loads::density)) return false;
+        if (state.load(std::memory_order_relaxed) == ConvTables::no_memory || us > 1.05 * tiled_us(e, p4, v, copies, B, Loads::density)) return false;
         count_loads(e, s);
+        if (state.load(std::memory_order_acquire) != ConvTables::counted) return false;
     }
-    return e->conv_loads_state == 1 && us <= tiled_us(e, p4, v, copies, B, Loads::counted);
+    return us <= tiled_us(e, p4, v, copies, B, Loads::counted);
 }
 
 // Batch size the tiled kernels run at: B rounded up to a multiple of 4, or further up to a multiple

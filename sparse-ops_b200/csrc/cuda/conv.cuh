@@ -62,6 +62,10 @@ struct ConvTables {
     uint32_t* ncols = nullptr;
     uint32_t cap = 0;
     bool no_merged = false;         // an earlier call found no memory for them
+    // How the entries lie for the merged kernel's CTAs of 16, 8 and 4 row blocks: read once they are counted.
+    enum { unknown, counted, no_memory };
+    std::atomic<int> loads_state{unknown};
+    MergedLoad loads[3];
 };
 ConvTables* new_conv_tables();
 void free_conv_tables(spx_ell* e);

@@ -293,8 +293,64 @@ def test_second_kernel_shape_without_memory(lib, orc, cuda):
     assert_bit_equal(outs[1].cpu().numpy(), runs[1][3], "room again")
 
 
+def exhaust(lib):
+    """Takes all device memory, what the library's pool has left included."""
+    held, handles = fill_device(lib, 0, 2 << 20), []
+    for m in (1 << 20, 1 << 16, 1 << 12, 1 << 8, 1 << 6):   # 12 bytes a row
+        nnz = np.zeros(m, np.uint32)
+        try:
+            while True:
+                handles.append(lib.ell_create(np.zeros((m, 0), np.float32), np.zeros((m, 0), np.uint32), nnz, 1))
+        except sx.SpxError as e:
+            assert e.status == 3, e
+    return held, handles
+
+
+@no_memory
+def test_calls_that_are_sure_to_gain_without_memory(lib, orc, cuda):
+    """A call that would count the shared columns finds no memory for it: from then on the calls that depend on the count take
+    the tiled kernels, and those that are faster gathered whatever it says still are."""
+    rng, C, H = np.random.default_rng(18), 1024, 14         # the count takes 2 KB
+    E = orc.encode(sparse(rng, C, 64 * 9, 0.3))
+    g, outs = sx.conv_geom(64, C, 3, 3, H, H, 2, 2, 1, 1), {}
+    gd = dict(Cin=64, kH=3, kW=3, sH=2, sW=2, pH=1, pW=1, dH=1, dW=1, H=H, W=H)
+    x = rng.standard_normal((32, 64, H, H)).astype(np.float32)
+    for B in (1, 32):
+        src = as_layout(x[:B], sx.LAYOUT_PF)
+        want = orc.conv2d(E, gd, sx.LAYOUT_PF, src, B, None, 0)
+        outs[B] = dev(src, cuda), torch.full(want.shape, float("nan"), device=cuda), want
+
+    def call(h, B, stream=0):
+        h.conv2d(g, sx.LAYOUT_PF, ptr(outs[B][0]), B, None, 0, ptr(outs[B][1]), stream)
+
+    def check(B):
+        assert_bit_equal(outs[B][1].cpu().numpy(), outs[B][2], f"batch {B}")
+        outs[B][1].fill_(float("nan"))
+
+    other, h = gpu_ell(lib, E), gpu_ell(lib, E)             # (the other one: kernels are loaded while there is room)
+    assert_ran(kernels_of(lambda: call(other, 1)), "conv_gather_kernel")
+    assert_ran(kernels_of(lambda: call(other, 32)), "union_count_kernel")
+    call(h, 1)
+    with torch.cuda.graph(torch.cuda.CUDAGraph()):          # builds the merged weights without a count
+        call(h, 32, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    before = lib.spx_launch_count()
+    held, handles = exhaust(lib)
+    try:
+        call(h, 32)
+        assert lib.spx_launch_count() == before + 1, "there was memory for the count"
+        check(32)
+    finally:
+        for p in held:
+            lib.spx_free(p)
+        handles.clear()
+    for B, kernel in ((1, "conv_gather_kernel"), (32, "conv_rbm_tile_kernel")):
+        assert_ran(kernels_of(lambda: call(h, B)), kernel)
+        check(B)
+
+
 def test_without_memory():
-    child(["test_conv_gather_gpu.py"], "second_kernel_shape_without", {"SPX_TEST_NO_MEMORY": "1"})
+    child(["test_conv_gather_gpu.py"], "second_kernel_shape_without or sure_to_gain_without", {"SPX_TEST_NO_MEMORY": "1"})
 
 
 @chosen
