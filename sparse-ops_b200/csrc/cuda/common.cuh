@@ -44,11 +44,11 @@ struct spx_ell {
     // Raised by a convolution kernel whose bounded wait for a bulk tensor copy ran out: a word in
     // device memory (read by the kernel's later CTAs) and a word in pinned host memory (its device
     // alias is tma_failed_mapped; read by the next convolution call on the handle).
-    int* tma_failed_host = nullptr;
+    std::atomic<int*> tma_failed_host{nullptr};     // set last: the others are there when it is seen
     spx::PinnedBlock tma_failed_block;
     int* tma_failed_mapped = nullptr;
     int* tma_failed_dev = nullptr;
-    bool tma_off = false;
+    std::atomic<bool> tma_off{false};
     // Tiled form of the matrix for spmm_tile.cu, built on the second SpMM call that can use it.
     void* tiles = nullptr;
     // Tap tables and merged weights of the convolution, and how the entries lie for it (conv.cuh).

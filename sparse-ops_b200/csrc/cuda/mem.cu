@@ -218,13 +218,17 @@ int allow_smem(const void* kernel, int device, std::atomic<uint64_t>& done)
     return SPX_OK;
 }
 
+// Any of a handle's calls may be the first to need them, on any thread.
 void ensure_tma_words(spx_ell* e)
 {
-    if (e->tma_failed_host || pinned_acquire(sizeof(int), &e->tma_failed_block) != SPX_OK) return;
-    e->tma_failed_host = static_cast<int*>(e->tma_failed_block.host);
-    *e->tma_failed_host = 0;
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    PinnedBlock block;
+    if (e->tma_failed_host.load(std::memory_order_relaxed) || pinned_acquire(sizeof(int), &block) != SPX_OK) return;
+    int* host = static_cast<int*>(block.host);
+    *host = 0;                                  // (the block may have served before)
     cudaStream_t side = nullptr;
-    if (cudaHostGetDevicePointer(reinterpret_cast<void**>(&e->tma_failed_mapped), e->tma_failed_host, 0) != cudaSuccess ||
+    if (cudaHostGetDevicePointer(reinterpret_cast<void**>(&e->tma_failed_mapped), host, 0) != cudaSuccess ||
         side_stream(e->device, &side) != SPX_OK ||
         pool_alloc(reinterpret_cast<void**>(&e->tma_failed_dev), sizeof(int), e->device, side) != SPX_OK ||
         cudaMemsetAsync(e->tma_failed_dev, 0, sizeof(int), side) != cudaSuccess || cudaStreamSynchronize(side) != cudaSuccess) {
@@ -233,12 +237,15 @@ void ensure_tma_words(spx_ell* e)
         e->tma_failed_dev = nullptr;
         (void)cudaGetLastError();
     }
+    e->tma_failed_block = block;
+    e->tma_failed_host.store(host, std::memory_order_release);
 }
 
 int check_tma_words(spx_ell* e, const char* what)
 {
-    if (!e->tma_failed_host || !*e->tma_failed_host) return SPX_OK;
-    *e->tma_failed_host = 0;
+    volatile int* failed = e->tma_failed_host.load(std::memory_order_acquire);
+    if (!failed || !*failed) return SPX_OK;
+    *failed = 0;
     e->tma_off = true;
     return fail(SPX_ERR_CUDA, "%s: a bulk tensor copy of a call on this handle did not complete; that call's output is invalid", what);
 }
