@@ -428,7 +428,6 @@ int spx_ell_destroy(spx_ell* e)
     pool_free(e->rows, (size_t)e->m * 8, nullptr);
     pool_free(e->spmv_split, e->spmv_split_bytes, nullptr);
     pool_free(e->stage_dev, e->stage_dev_bytes, nullptr);
-    pool_free(e->conv_scratch, e->conv_scratch_bytes, nullptr);
     pool_free(e->tma_failed_dev, sizeof(int), nullptr);
     pinned_release(e->tma_failed_block);
     for (cudaStream_t st : e->pipe_streams) if (st) cudaStreamDestroy(st);

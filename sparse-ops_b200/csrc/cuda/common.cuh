@@ -63,9 +63,6 @@ struct spx_ell {
     // Pinned + device staging for the host-buffer entry points (abi.cu), grown on demand.
     void* stage_dev = nullptr;
     size_t stage_dev_bytes = 0;
-    // Scratch of the convolution: an input brought into [C,H,W,B4] order (conv.cu).
-    void* conv_scratch = nullptr;
-    size_t conv_scratch_bytes = 0;
     // Streams of the pipelined host-buffer SpMM (copy in, exchange, multiply, copy out) and the events
     // that chain and time its stages, created on first use and kept.
     cudaStream_t pipe_streams[4] = {nullptr, nullptr, nullptr, nullptr};

@@ -725,6 +725,13 @@ void free_conv_tables(spx_ell* e)
         delete s;
         s = next;
     }
+    pool_free(t->scratch.p, t->scratch.bytes, nullptr);
+    for (ConvTables::Block* b = t->scratch.next; b;) {
+        pool_free(b->p, b->bytes, nullptr);
+        ConvTables::Block* next = b->next;
+        delete b;
+        b = next;
+    }
     pool_free(t->w, merged_slots(e) * kRbmRows * sizeof(float), nullptr);
     pool_free(t->ncols, (size_t)((e->m + kRbmRows - 1) / kRbmRows) * sizeof(uint32_t), nullptr);
     delete t;
@@ -776,6 +783,28 @@ static int ensure_taps(spx_ell* e, uint32_t kH, uint32_t kW, const uint32_t** ta
         return fail(SPX_ERR_CUDA, "conv2d: building the tap table failed: %s", cudaGetErrorString(err));
     }
     *taps = t->taps = static_cast<uint32_t*>(made);
+    return SPX_OK;
+}
+
+// Scratch for a call's input, kept with the handle and grown as needed, by a call that is recorded too: calls before it may
+// all have gathered.  A block that a recorded call uses stays when a larger one takes its place.
+static int input_scratch(spx_ell* e, size_t need, cudaStream_t s, float** out)
+{
+    ConvTables* t = e->conv;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    const bool recorded = cudaStreamIsCapturing(s, &status) == cudaSuccess && status != cudaStreamCaptureStatusNone;
+    if (t->scratch.bytes < need) {
+        RelaxedCapture relaxed;                 // allocations and waits below end no capture
+        if (t->scratch_recorded) {
+            ConvTables::Block* kept = new (std::nothrow) ConvTables::Block(t->scratch);
+            if (!kept) return fail(SPX_ERR_OOM, "out of host memory");
+            t->scratch = ConvTables::Block{nullptr, 0, kept};
+            t->scratch_recorded = false;
+        }
+        if (int rc = grow_scratch(e, &t->scratch.p, &t->scratch.bytes, need)) return rc;
+    }
+    t->scratch_recorded = t->scratch_recorded || recorded;
+    *out = static_cast<float*>(t->scratch.p);
     return SPX_OK;
 }
 
@@ -1363,10 +1392,8 @@ int launch_conv2d(spx_ell* e, const spx_conv_geom* g, int layout, const float* i
         if (gathers && gather_pays(e, p4, v, copies, B, gather, s)) return launch_conv_gather(e, taps, p, layout, in, bias, act, out, gather, s);
         if (copies) {
             const uint64_t positions = g->Cin * H * W;
-            const size_t need = positions * B4 * sizeof(float);
-            if (e->conv_scratch_bytes < need)
-                if (int rs = grow_scratch(e, &e->conv_scratch, &e->conv_scratch_bytes, need)) return rs;
-            float* dst = static_cast<float*>(e->conv_scratch);
+            float* dst = nullptr;
+            if (int rs = input_scratch(e, positions * B4 * sizeof(float), s, &dst)) return rs;
             if (iB != 1 && B >= 16 && B4 == B) {        // wide transpose through shared memory: both sides in whole lines
                 if (int rt = transpose2d(in, B, positions, dst, s)) return rt;
             } else {

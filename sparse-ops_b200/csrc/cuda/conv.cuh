@@ -66,6 +66,14 @@ struct ConvTables {
     enum { unknown, counted, no_memory };
     std::atomic<int> loads_state{unknown};
     MergedLoad loads[3];
+    // An input brought into [C,H,W,B4] order.  Calls that use it do not run side by side.
+    struct Block {
+        void* p = nullptr;
+        size_t bytes = 0;
+        Block* next = nullptr;
+    };
+    Block scratch;                  // next: smaller ones that recorded graphs use
+    bool scratch_recorded = false;
 };
 ConvTables* new_conv_tables();
 void free_conv_tables(spx_ell* e);

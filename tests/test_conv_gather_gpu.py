@@ -354,6 +354,33 @@ def test_without_memory():
 
 
 @chosen
+@pytest.mark.parametrize("first", [1, 16])
+def test_recorded_calls_that_need_more_scratch(lib, orc, cuda, first):
+    """NCHW calls copy their input: one that is recorded after smaller ones (gathered, or with less scratch) gets what it needs, and
+    its graph keeps that when a later call needs more."""
+    rng, C, H = np.random.default_rng(19), 128, 14
+    E = orc.encode(sparse(rng, C, C * 9, 0.5))
+    h, g, x = gpu_ell(lib, E), sx.conv_geom(C, C, 3, 3, H, H, 1, 1, 1, 1), rng.standard_normal((64, C, H, H)).astype(np.float32)
+    runs = {}
+    for B in (first, 32, 48, 64):
+        want = orc.conv2d(E, dict(Cin=C, kH=3, kW=3, sH=1, sW=1, pH=1, pW=1, dH=1, dW=1, H=H, W=H), sx.LAYOUT_NCHW, x[:B], B, None, 0)
+        runs[B] = dev(x[:B], cuda), torch.full(want.shape, float("nan"), device=cuda), want
+    call = lambda B: h.conv2d(g, sx.LAYOUT_NCHW, ptr(runs[B][0]), B, None, 0, ptr(runs[B][1]), torch.cuda.current_stream().cuda_stream)
+    call(first)
+    graphs = []
+    for B in (32, 48):
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1]):
+            call(B)
+    assert_ran(kernels_of(lambda: call(64)), "transpose2d_kernel")
+    for graph in graphs * 2:
+        graph.replay()
+    torch.cuda.synchronize()
+    for B, (_, dY, want) in runs.items():
+        assert_bit_equal(dY.cpu().numpy(), want, f"batch {B}")
+
+
+@chosen
 def test_recording_a_merged_call_waits_for_no_other_work(lib, orc, cuda):
     """Recording a call that lacks the merged weights builds them at once, beside what other streams do: that kernel is no part
     of the graph."""
