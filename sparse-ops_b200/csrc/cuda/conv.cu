@@ -898,7 +898,8 @@ int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, const uint2** hdr)
         pool_free(w, slots * kRbmRows * sizeof(float), side);
         pool_free(ncols, nblocks * sizeof(uint32_t), side);
         if (err != cudaSuccess) return fail(SPX_ERR_CUDA, "conv2d: merging the weights failed: %s", cudaGetErrorString(err));
-        (first ? t->no_merged : shape->no_hdr) = true;
+        if (first) t->no_merged = true;
+        else shape->no_hdr = true;
         return -1;
     }
     if (first) {
@@ -908,6 +909,14 @@ int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, const uint2** hdr)
     shape->hdr = static_cast<uint2*>(made);
     if (hdr) *hdr = shape->hdr;
     return SPX_OK;
+}
+
+// Whether every segment of the batch does in the merged kernel's largest cut.
+static bool merged_fits(const ConvParams& p)
+{
+    const uint32_t n16 = p.B / 16 * 16, rest = p.B - n16;
+    const auto fits = [&](uint32_t qb) { return rbm_fits(p, qb, 16, kRbmG); };
+    return (!n16 || fits(4)) && (rest < 8 || fits(2)) && (rest % 8 != 4 || fits(1));
 }
 
 template <int QB, int NB, int G>
@@ -1108,9 +1117,7 @@ static int launch_conv_rbm_tile(spx_ell* e, const ConvParams& p, const ConvViews
     const uint32_t n16 = p.B / 16 * 16, rest = p.B - n16;
     if (!segments && n16 && rest) return -1;
     if (!segments && !n16 && rest == 12) return -1;
-    // every segment's staged patch must fit shared memory (checked before any launch)
-    const auto fits = [&](uint32_t qb) { return rbm_fits(p, qb, 16, kRbmG); };
-    if ((n16 && !fits(4)) || (rest >= 8 && !fits(2)) || (rest % 8 == 4 && !fits(1))) return -1;
+    if (!merged_fits(p)) return -1;             // checked before any launch
     {
         const int rc = launch_conv_tmem(e, p, v, in, bias, act, out, conv_rbm_us, s);
         if (rc != -1) return rc;
@@ -1136,19 +1143,20 @@ static int launch_conv_rbm_tile(spx_ell* e, const ConvParams& p, const ConvViews
     return SPX_OK;
 }
 
-// Returns -1 when the shape is not covered (caller falls back to the direct kernel).
-static int launch_conv_pf_tile(spx_ell* e, const uint32_t* taps, const ConvParams& p, const ConvViews& v, const float* in, const float* bias, int act,
-                               float* out, cudaStream_t s)
+// How the per-row kernel is cut: batch entries, float4 groups a lane, rows of positions and channels (warps) of a CTA.
+struct PfTile {
+    uint32_t BT, G, TH, warps;
+    int per_sm;
+    uint32_t THin, TWin;
+    size_t chan_bytes, budget;
+    bool small;
+};
+static bool pf_tile(const ConvParams& p, PfTile& t)
 {
-    if (!e->cols_ascending || !pf_tile_covers(p)) return -1;
     // batch entries per CTA: the largest multiple of 4 that divides B and is <= 32
-    uint32_t BT = 0;
-    for (uint32_t c = 32; c >= 4; c -= 4) if (p.B % c == 0) { BT = c; break; }
-    if (!BT) return -1;
-    {
-        const int rc = launch_conv_rbm_tile(e, p, v, in, bias, act, out, s);
-        if (rc != -1) return rc;
-    }
+    t.BT = 0;
+    for (uint32_t c = 32; c >= 4; c -= 4) if (p.B % c == 0) { t.BT = c; break; }
+    if (!t.BT) return false;
     static const int ctas = [] { const char* v = getenv("SPX_CONV_CTAS"); return v ? atoi(v) : 0; }();
     static const int small_tile = [] { const char* v = getenv("SPX_CONV_SMALL_TILE"); return v ? atoi(v) : -1; }();
     // Full batch tile (32 entries): 2 x 8 positions per warp and 32 warps (= output channels) per
@@ -1156,43 +1164,59 @@ static int launch_conv_pf_tile(spx_ell* e, const uint32_t* taps, const ConvParam
     // the shared-memory latency, half the staging traffic per output channel.  Measured on
     // 256 -> 256 channels, 56 x 56, batch 32: 1.89 ms against 2.03 ms.  SPX_CONV_SMALL_TILE=0 selects
     // the larger tile.
-    const bool small = BT == 32 && small_tile != 0;
+    t.small = t.BT == 32 && small_tile != 0;
     // Batch tile of 8 entries: a 4 x 8 tile would leave a lane two float4 per nonzero, so the warp
     // takes 8 x 8 positions instead and the two broadcast shuffles per nonzero are amortised over 4
     // shared-memory loads (0.571 ms against 0.593 ms on 256 -> 256 channels, 56 x 56, batch 8; a
     // 16 x 8 tile for 4 entries measured slower than 4 x 8).  SPX_CONV_WIDE_TILE=0 turns it off.
     static const int wide_env = [] { const char* v = getenv("SPX_CONV_WIDE_TILE"); return v ? atoi(v) : 1; }();
-    const uint32_t QBv = BT / 4;
-    const uint32_t Gv = (wide_env && QBv == 2) ? 4 : (small ? 4 : QBv);
-    const uint32_t TH = 32 * Gv / QBv / kTileW;
-    const uint32_t warps = small ? 32 : kTileWarps;
+    const uint32_t QB = t.BT / 4;
+    t.G = (wide_env && QB == 2) ? 4 : (t.small ? 4 : QB);
+    t.TH = 32 * t.G / QB / kTileW;
+    t.warps = t.small ? 32 : kTileWarps;
+    t.THin = (t.TH - 1) * p.sH + (p.kH - 1) * p.dH + 1;
+    t.TWin = (kTileW - 1) * p.sW + (p.kW - 1) * p.dW + 1;
+    t.chan_bytes = (size_t)t.THin * t.TWin * t.BT * sizeof(float);
+    // Two CTAs per SM overlap one CTA's staging with the other's FMAs; with 8 float4 groups per
+    // lane (batch 32) the accumulators need more than the 64 registers that allows.
+    t.per_sm = t.small ? 1 : (ctas == 1 || ctas == 2 ? ctas : (QB > 4 ? 1 : 2));
+    t.budget = t.per_sm == 2 ? 100 * 1024 : 200 * 1024;
+    return t.chan_bytes <= t.budget;
+}
+
+// Returns -1 when the shape is not covered (caller falls back to the direct kernel).
+static int launch_conv_pf_tile(spx_ell* e, const uint32_t* taps, const ConvParams& p, const ConvViews& v, const float* in, const float* bias, int act,
+                               float* out, cudaStream_t s)
+{
+    if (!e->cols_ascending || !pf_tile_covers(p)) return -1;
+    {
+        const int rc = launch_conv_rbm_tile(e, p, v, in, bias, act, out, s);
+        if (rc != -1) return rc;
+    }
+    PfTile t;
+    if (!pf_tile(p, t)) return -1;
     TileParams tp{};
     tp.c = p;
     tp.v = v;
-    tp.BT = BT;
-    tp.THin = (TH - 1) * p.sH + (p.kH - 1) * p.dH + 1;
-    tp.TWin = (kTileW - 1) * p.sW + (p.kW - 1) * p.dW + 1;
-    const size_t chanBytes = (size_t)tp.THin * tp.TWin * BT * sizeof(float);
-    // Two CTAs per SM overlap one CTA's staging with the other's FMAs; with 8 float4 groups per
-    // lane (batch 32) the accumulators need more than the 64 registers that allows.
-    const int per_sm = small ? 1 : (ctas == 1 || ctas == 2 ? ctas : (BT / 4 > 4 ? 1 : 2));
-    const size_t budget = per_sm == 2 ? 100 * 1024 : 200 * 1024;
-    if (chanBytes > budget) return -1;
-    tp.CC = (uint32_t)std::min<size_t>(p.Cin, budget / chanBytes);
+    tp.BT = t.BT;
+    tp.THin = t.THin;
+    tp.TWin = t.TWin;
+    tp.CC = (uint32_t)std::min<size_t>(p.Cin, t.budget / t.chan_bytes);
     // the per-nonzero shared-memory offset must fit 32 bits (it does: <= budget / 4)
     tp.tilesX = (p.Wo + kTileW - 1) / kTileW;
-    const uint32_t tilesY = (p.Ho + TH - 1) / TH;
+    const uint32_t tilesY = (p.Ho + t.TH - 1) / t.TH;
     const uint64_t tiles = (uint64_t)tp.tilesX * tilesY;
-    const uint32_t gy = (p.Cout + warps - 1) / warps, gz = p.B / BT;
+    const uint32_t gy = (p.Cout + t.warps - 1) / t.warps, gz = p.B / t.BT;
     if (tiles > 0x7fffffffull || gy > 65535 || gz > 65535) return -1;
     dim3 grid((unsigned)tiles, gy, gz);
-    const size_t smem = chanBytes * tp.CC;
-    if (small) return launch_tile_qb<8, 4, 32, 1>(e, taps, tp, grid, smem, in, bias, act, out, s);
-    if (Gv != QBv) return launch_tile_qb<2, 4, kTileWarps, 2>(e, taps, tp, grid, smem, in, bias, act, out, s);
+    const size_t smem = t.chan_bytes * tp.CC;
+    const int per_sm = t.per_sm;
+    if (t.small) return launch_tile_qb<8, 4, 32, 1>(e, taps, tp, grid, smem, in, bias, act, out, s);
+    if (t.G != t.BT / 4) return launch_tile_qb<2, 4, kTileWarps, 2>(e, taps, tp, grid, smem, in, bias, act, out, s);
 #define SPX_TILE_CASE(Q)                                                                                           \
     case Q: return per_sm == 2 ? launch_tile_qb<Q, Q, kTileWarps, 2>(e, taps, tp, grid, smem, in, bias, act, out, s)     \
                                : launch_tile_qb<Q, Q, kTileWarps, 1>(e, taps, tp, grid, smem, in, bias, act, out, s);
-    switch (BT / 4) {
+    switch (t.BT / 4) {
         SPX_TILE_CASE(1) SPX_TILE_CASE(2) SPX_TILE_CASE(3) SPX_TILE_CASE(4)
         SPX_TILE_CASE(5) SPX_TILE_CASE(6) SPX_TILE_CASE(7) SPX_TILE_CASE(8)
     }
@@ -1202,28 +1226,23 @@ static int launch_conv_pf_tile(spx_ell* e, const uint32_t* taps, const ConvParam
 
 // CTA per block of 4 rows: its union columns and its entries.  A column counts where its bit is set first.  (A warp per block
 // that looked each column up in the rows before took 370 us for 120 rows of 1830 entries, as long as the convolution behind it.)
-constexpr uint32_t kCountWords = 8192;          // of columns at a time: up to 32 KB
 __global__ void __launch_bounds__(256)
 union_count_kernel(const uint32_t* __restrict__ idx, const uint32_t* __restrict__ nnz, uint32_t m, uint32_t n, uint32_t pitch, uint2* __restrict__ blocks)
 {
-    extern __shared__ uint32_t s_seen[];
+    extern __shared__ uint32_t s_seen[];        // (n + 31) / 32 words
     __shared__ uint32_t s_fresh;
-    const uint32_t row0 = blockIdx.x * kRbmRows, rows = min(kRbmRows, m - row0), words = min(kCountWords, (n + 31) / 32);
+    const uint32_t row0 = blockIdx.x * kRbmRows, rows = min(kRbmRows, m - row0), words = (n + 31) / 32;
     if (threadIdx.x == 0) s_fresh = 0;
+    for (uint32_t w = threadIdx.x; w < words; w += blockDim.x) s_seen[w] = 0;
+    __syncthreads();
     uint32_t fresh = 0, all = 0;
-    for (uint32_t from = 0; from < n; from += words * 32) {
-        __syncthreads();
-        for (uint32_t w = threadIdx.x; w < words; w += blockDim.x) s_seen[w] = 0;
-        __syncthreads();
-        all = 0;
-        for (uint32_t r = 0; r < rows; ++r) {
-            const uint32_t len = __ldg(nnz + row0 + r);
-            const uint32_t* __restrict__ k = idx + (size_t)(row0 + r) * pitch;
-            all += len;
-            for (uint32_t j = threadIdx.x; j < len; j += blockDim.x) {
-                const uint32_t col = __ldg(k + j) - from, bit = 1u << (col & 31);
-                if (col < words * 32) fresh += (atomicOr(s_seen + col / 32, bit) & bit) == 0;
-            }
+    for (uint32_t r = 0; r < rows; ++r) {
+        const uint32_t len = __ldg(nnz + row0 + r);
+        const uint32_t* __restrict__ k = idx + (size_t)(row0 + r) * pitch;
+        all += len;
+        for (uint32_t j = threadIdx.x; j < len; j += blockDim.x) {
+            const uint32_t col = __ldg(k + j), bit = 1u << (col & 31);
+            fresh += (atomicOr(s_seen + col / 32, bit) & bit) == 0;
         }
     }
     fresh = __reduce_add_sync(0xffffffffu, fresh);
@@ -1248,7 +1267,7 @@ static void count_loads(spx_ell* e, cudaStream_t s)
     cudaStream_t side = nullptr;
     int state = ConvTables::no_memory;
     if (side_stream(e->device, &side) == SPX_OK && scratch_alloc(&blocks, bytes, e->device, side, true) == SPX_OK && pinned_acquire(bytes, &host) == SPX_OK) {
-        union_count_kernel<<<nblocks, 256, std::min(kCountWords, (e->n + 31) / 32) * 4, side>>>(e->idx, e->nnz, e->m, e->n, e->pitch, static_cast<uint2*>(blocks));
+        union_count_kernel<<<nblocks, 256, (e->n + 31) / 32 * 4, side>>>(e->idx, e->nnz, e->m, e->n, e->pitch, static_cast<uint2*>(blocks));
         count_launch_beside();
         if (cudaGetLastError() == cudaSuccess && cudaMemcpyAsync(host.host, blocks, bytes, cudaMemcpyDeviceToHost, side) == cudaSuccess &&
             cudaStreamSynchronize(side) == cudaSuccess) {
@@ -1265,7 +1284,7 @@ static void count_loads(spx_ell* e, cudaStream_t s)
 // not as they read it.  How the merged kernel fares depends on the columns that the rows of a block share: by the
 // density, by the counted loads, or as if every block's rows shared all of them, which is the least it can take.  Rows of
 // fewer than 29 channels are not merged: the estimate is by the density there, and on the low side (0.7 of the
-// time in the middle).  0 where it is not known.
+// time in the middle).
 enum class Loads { least, density, counted };
 static double tiled_us(const spx_ell* e, const ConvParams& p4, const ConvViews& v, bool copies, uint32_t B, Loads by)
 {
@@ -1280,7 +1299,21 @@ static double tiled_us(const spx_ell* e, const ConvParams& p4, const ConvViews& 
     double us = conv_rbm_us(e, p4, by == Loads::density ? nullptr : by == Loads::counted ? e->conv->loads : load);
     if (e->m >= 8 * kRbmRows - 3) us = std::min(us, conv_tmem_expected(e, p4, v, conv_rbm_us));
     if (copies) us += 2.5 + 4e-6 / 3 * (double)p4.Cin * p4.H * p4.W * (p4.B + B);
-    return us < 1e20 ? us : 0.0;                // (a patch that no cut of the merged kernel stages)
+    return us;
+}
+
+// The least that the per-row kernel can take, where the merged one does not take the call: an operand a clock and bank from
+// shared memory, or the staging, a byte a clock and warp.  0.1 to 1.02 of the time on 312 shapes (more than 131072 columns, strides
+// of 10 to 20, and the ranges below with the merged kernel turned off), 0.4 in the middle.
+static double per_row_least_us(const spx_ell* e, const ConvParams& p, bool copies, uint32_t B)
+{
+    PfTile t;
+    if (!pf_tile(p, t)) return 0.0;
+    const double sms = sm_count(e->device), tiles = (double)((p.Wo + kTileW - 1) / kTileW) * ((p.Ho + t.TH - 1) / t.TH) * (p.B / t.BT);
+    const double units = tiles * ((p.Cout + t.warps - 1) / t.warps);
+    const double operands = (double)e->nnz_total * tiles * t.G * 4 / sms;
+    const double staging = (double)p.Cin * t.chan_bytes / t.warps * std::max(1.0, units / (sms * t.per_sm));
+    return 2.0 + std::max(operands, staging) / 1900.0 + (copies ? 2.5 + 4e-6 / 3 * (double)p.Cin * p.H * p.W * (p.B + B) : 0.0);
 }
 
 // Whether gathering is expected to be faster than the tiled kernels: below 0.9 of their time, 0.85 where it takes four batch
@@ -1293,7 +1326,14 @@ static double tiled_us(const spx_ell* e, const ConvParams& p4, const ConvViews& 
 static bool gather_pays(spx_ell* e, const ConvParams& p4, const ConvViews& v, bool copies, uint32_t B, const ConvGatherPlan& plan, cudaStream_t s)
 {
     const double us = plan.us / (plan.form >= 2 ? 0.85 : 0.9);
-    if (e->m < 8 * kRbmRows - 3) return us <= tiled_us(e, p4, v, copies, B, Loads::density);
+    const bool few = e->m < 8 * kRbmRows - 3, no_merged = e->conv->no_merged;
+    if (!merged_fits(p4) || (!few && (e->n > kRbmMaxK || no_merged))) {
+        // 1.5 times the least: of those 312 shapes gathering is slower for 18 (up to 1.9), none of them among the 179 it takes
+        double other = 1.5 * per_row_least_us(e, p4, copies, B);
+        if (no_merged) other = std::min(other, conv_tmem_expected(e, p4, v, conv_rbm_us));
+        return us <= other;
+    }
+    if (few) return us <= tiled_us(e, p4, v, copies, B, Loads::density);
     const std::atomic<int>& state = e->conv->loads_state;
     if (state.load(std::memory_order_acquire) != ConvTables::counted) {
         if (us <= tiled_us(e, p4, v, copies, B, Loads::least)) return true;

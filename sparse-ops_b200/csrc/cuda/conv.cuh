@@ -61,7 +61,7 @@ struct ConvTables {
     float* w = nullptr;
     uint32_t* ncols = nullptr;
     uint32_t cap = 0;
-    bool no_merged = false;         // an earlier call found no memory for them
+    std::atomic<bool> no_merged{false};     // an earlier call found no memory for them
     // How the entries lie for the merged kernel's CTAs of 16, 8 and 4 row blocks: read once they are counted.
     enum { unknown, counted, no_memory };
     std::atomic<int> loads_state{unknown};

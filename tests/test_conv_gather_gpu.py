@@ -110,6 +110,23 @@ def test_choice_of_gathering(lib, orc, cuda, shared, kernel):
 
 
 @chosen
+@pytest.mark.parametrize("B,Cin,Cout,H,k,s,density", [(4, 19, 70, 84, 3, 12, 0.05), (1, 28, 158, 61, 4, 14, 0.23),      # 39 and 80 us against 4 and 7
+                                                      (3, 14700, 40, 6, 3, 1, 0.004), (16, 5300, 33, 5, 5, 2, 0.004)])  # 132300 columns and more
+def test_choice_where_nothing_is_merged(lib, orc, cuda, B, Cin, Cout, H, k, s, density):
+    """Strides that leave no patch to the merged kernel, and more columns than it takes: the call is compared with the per-row kernel,
+    and no columns are counted."""
+    rng = np.random.default_rng([B, Cin])
+    E = orc.encode(sparse(rng, Cout, Cin * k * k, density))
+    src = as_layout(rng.standard_normal((B, Cin, H, H)).astype(np.float32), sx.LAYOUT_PF)
+    want = orc.conv2d(E, dict(Cin=Cin, kH=k, kW=k, sH=s, sW=s, pH=k // 2, pW=k // 2, dH=1, dW=1, H=H, W=H), sx.LAYOUT_PF, src, B, None, 0)
+    h, g, dX, dY = gpu_ell(lib, E), sx.conv_geom(Cin, Cout, k, k, H, H, s, s, k // 2, k // 2), dev(src, cuda), torch.empty(want.shape, device=cuda)
+    names = kernels_of(lambda: h.conv2d(g, sx.LAYOUT_PF, ptr(dX), B, None, 0, ptr(dY)))
+    assert_ran(names, "conv_gather_kernel")
+    assert names is None or "union_count_kernel" not in names
+    assert_bit_equal(dY.cpu().numpy(), want, "gathered")
+
+
+@chosen
 def test_tiled_call_recorded_after_gathered_ones(lib, orc, cuda):
     """Calls that gather need no merged weights; a later one that is recorded does, and has them: in the graph, and in an
     eager call before the graph is launched."""
