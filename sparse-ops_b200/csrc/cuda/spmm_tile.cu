@@ -646,9 +646,10 @@ int launch_spmm_tile(spx_ell* e, const float* X, uint32_t C, uint64_t ldx, const
     const bool sectors = !vec_x || (ldx % 8 == 0 && reinterpret_cast<uintptr_t>(X) % 32 == 0);
     Plan p = plan_tiles(e, C, 1, sms, vec_x, sectors);
     uint32_t NV = 1;
-    if (C > 32) {
+    static const int slices_env = [] { const char* v = getenv("SPX_SPMM_SLICES"); return v ? atoi(v) : 0; }();      // 32 or 64, for tests
+    if (slices_env ? slices_env == 64 : C > 32) {
         const Plan wide = plan_tiles(e, C, 2, sms, vec_x, sectors);
-        if (p.us > wide.us) {
+        if (slices_env || p.us > wide.us) {
             p = wide;
             NV = 2;
         }

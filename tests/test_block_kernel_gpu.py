@@ -10,6 +10,7 @@ import torch
 
 import spx_ctypes as sx
 from conftest import assert_bit_equal
+from test_conv_tmem_gpu import kernels_of
 
 pytestmark = pytest.mark.gpu
 
@@ -62,30 +63,52 @@ def test_stage_refills_forced():
     in_child("test_stage_refills", SPX_SPMM_TILE="2")
 
 
-@pytest.mark.parametrize("C", [32, 33, 63, 64, 65, 95, 96, 97, 128, 130, 352])
-@pytest.mark.parametrize("m", [5, 300, 1300])
-def test_slices(lib, orc, cuda, m, C):
-    """Slices of 32 and of 64 columns, whole, cut short and with a single column, of aligned rows and of a copy."""
-    if os.environ.get("SPX_SPMM_TILE") != "2":
-        pytest.skip("runs in a child process of test_slices_forced")
+def check_slices(lib, orc, cuda, m, n, C, p, kernel):
     rng = np.random.default_rng([m, C])
-    n = 700
-    W = sparse(rng, m, n, 0.2)
-    E = orc.encode(W)
+    E = orc.encode(sparse(rng, m, n, p))
     b = rng.standard_normal(m).astype(np.float32)
     X = rng.uniform(-1, 1, (n, C)).astype(np.float32)
     want = orc.spmm(E, X, b, act=1)
     h = lib.ell_create(E.Wd, E.idx, E.nnz, E.n)
     dX, dB = torch.from_numpy(X).to(cuda), torch.from_numpy(b).to(cuda)
-    for call in range(3):                   # the first one gathers
-        dY = torch.full((m, C), float("nan"), device=cuda)
-        h.spmm(dX.data_ptr(), C, C, dB.data_ptr(), sx.ACT_RELU, dY.data_ptr(), C)
-        torch.cuda.synchronize()
-        assert_bit_equal(dY.cpu().numpy(), want, f"call {call}")
+    dY = torch.full((m, C), float("nan"), device=cuda)
+    call = lambda: h.spmm(dX.data_ptr(), C, C, dB.data_ptr(), sx.ACT_RELU, dY.data_ptr(), C)
+    for k in range(3):                      # the first one gathers
+        dY.fill_(float("nan"))
+        names = kernels_of(call)
+        assert names is None or (kernel in names) == (k > 0), names
+        assert_bit_equal(dY.cpu().numpy(), want, f"call {k}")
 
 
-def test_slices_forced():
-    in_child("test_slices", SPX_SPMM_TILE="2")
+slices = pytest.mark.skipif(os.environ.get("SPX_SPMM_SLICES") not in ("32", "64"), reason="runs in a child process of test_slices_forced")
+
+
+@slices
+@pytest.mark.parametrize("C", [9, 32, 33, 63, 64, 65, 95, 96, 97, 128, 130, 352])
+@pytest.mark.parametrize("m", [5, 300, 1300])
+def test_slices(lib, orc, cuda, m, C):
+    """Slices of 32 and of 64 columns, whole, cut short and with a single column, of aligned rows and of a copy.  (X is larger than
+    shared memory: the kernels that hold it whole do not take these.)"""
+    nv = int(os.environ["SPX_SPMM_SLICES"]) // 32
+    n = 1900 if C > 30 else 6500
+    check_slices(lib, orc, cuda, m, n, C, 0.2 if n < 2000 else 0.06, f"spmm_tile_kernel<{nv}, ")
+
+
+@slices
+@pytest.mark.parametrize("width,m,C,kernel", [
+    (32, 1300, 130, "<1, 20>"), (32, 2604, 130, "<1, 24>"), (32, 3197, 130, "<1, 28>"), (32, 3196, 131, "<1, 28>"),
+    (64, 1300, 130, "<2, 16>"), (64, 4200, 130, "<2, 28>"), (64, 4201, 131, "<2, 28>")])
+def test_slices_of_each_kernel(lib, orc, cuda, width, m, C, kernel):
+    """Several slices, the last one of two and three columns, in the kernels for few and for many warps."""
+    if os.environ["SPX_SPMM_SLICES"] != str(width):
+        pytest.skip("in the other child")
+    check_slices(lib, orc, cuda, m, 1900, C, 0.1, "spmm_tile_kernel" + kernel)
+
+
+@pytest.mark.parametrize("width", [32, 64])
+def test_slices_forced(width):
+    in_child("test_slices", SPX_SPMM_TILE="2", SPX_SPMM_SLICES=str(width))
+    in_child("test_slices_of_each_kernel", SPX_SPMM_TILE="2", SPX_SPMM_SLICES=str(width))
 
 
 # ---- a bounded wait that runs out -----------------------------------------------------------------
