@@ -142,7 +142,7 @@ struct TileArgs {
     const uint32_t* off;
     const uint32_t* cnt;
     const uint2* rows;
-    uint32_t m, groups, chunks, row_blocks, C, ring_blocks;
+    uint32_t m, groups, chunks, row_blocks, C;
     int vec_out;                // 16-byte stores: C % 4 == 0 and aligned destinations
     const float* bias;
     int act;
@@ -218,6 +218,8 @@ align_rows_kernel(const float* __restrict__ X, uint64_t ldx, uint32_t n, uint32_
     }
 }
 
+template <int WARPS> constexpr uint32_t kRingBlocks = WARPS < (int)kMaxWarps ? 4 : 2;       // of four steps, per warp
+
 // For CTAs of up to WARPS warps.  kMaxWarps of them pass their gathers at the rate of shared memory with one step's operands
 // in registers; fewer wait for their own latencies, and have registers for two steps (kDeep below).  2048 x 2048, 30 %,
 // C = 32 16.6 -> 11.2 us, 640 x 1955, 35 %, C = 35 18.9 -> 14.0; 4096 x 4096, 10 %, C = 64 24.7 -> 19.3; 3001 x 4999, 6 %,
@@ -228,6 +230,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
 spmm_tile_kernel(const __grid_constant__ TileArgs a, const __grid_constant__ CUtensorMap tmap)
 {
     constexpr bool kDeep = WARPS < (int)kMaxWarps;
+    constexpr uint32_t kRing = kRingBlocks<WARPS>;
     constexpr uint32_t kPitch = NV * 128u;                  // bytes of a staged row of X
     constexpr uint32_t kBox = kChunk * kPitch;              // bytes of a staged chunk
     extern __shared__ __align__(128) unsigned char s_mem[]; // [kStages] chunks of X, a row of zeros, a ring per warp
@@ -243,15 +246,18 @@ spmm_tile_kernel(const __grid_constant__ TileArgs a, const __grid_constant__ CUt
     const uint32_t nactive = (a.groups - rb + a.row_blocks - 1) / a.row_blocks;    // at least warp 0: row_blocks <= groups
 
     // the warp's steps and counts do not depend on the predecessor kernel
-    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(s_mem) + kStages * kBox + kPitch + warp * (a.ring_blocks * 512u);
-    const uint32_t ring_mask = a.ring_blocks - 1;          // a power of two
+    // Known to the compiler it goes into the addresses, and CTAs of up to 20 warps take 0.7 % longer (51 shapes).
+    uint32_t ring_blocks = kRing;
+    if (kDeep) asm volatile("" : "+r"(ring_blocks));
+    const uint32_t ring_mask = ring_blocks - 1;
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(s_mem) + kStages * kBox + kPitch + warp * (ring_blocks * 512u);
     const uint32_t first = active ? __ldg(a.off + group) : 0u, n_steps = active ? __ldg(a.off + group + 1) - first : 0u;
     const unsigned char* src = reinterpret_cast<const unsigned char*>(a.steps) + (size_t)first * 128 + lane * 16;
     auto fill = [&](uint32_t blk) {             // block blk of 4 steps; the array ends with room for a whole block
         if (blk < (n_steps + 3) / 4) cp_async16(ring + (blk & ring_mask) * 512u + lane * 16, src + (size_t)blk * 512);
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    for (uint32_t b = 0; b < 3; ++b) fill(b < ring_mask ? b : 0xffffffu);     // three groups, whatever the ring holds
+    for (uint32_t b = 0; b + 1 < kRing; ++b) fill(b);
     const uint32_t slot = group * kGroupRows + lane / 8;
     const uint2 ri = active && slot < a.m ? __ldg(a.rows + slot) : make_uint2(0u, 0u);
     uint32_t my_cnt = active && lane < a.chunks ? __ldg(a.cnt + (size_t)group * a.chunks + lane) : 0u;
@@ -297,7 +303,7 @@ spmm_tile_kernel(const __grid_constant__ TileArgs a, const __grid_constant__ CUt
     // one is multiplied.  Operands only within a phase: the next chunk may not have landed (looking across it, with the wait
     // in the step, made every case slower, 11.2 to 14.2 us at 2048 x 2048, 30 %, C = 32).
     float4 w0, w1, k0, k1, x0[4][NV], x1[4][NV];
-    auto place = [&](uint32_t st) { return ring + ((st & 15u) * 128u) + r * 16; };
+    auto place = [&](uint32_t st) { return ring + ((st % (4 * kRing)) * 128u) + r * 16; };
     auto next_block = [&](uint32_t blk) {       // entering it: it has landed, and the one before the last is free
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncwarp();
@@ -387,12 +393,11 @@ spmm_tile_kernel(const __grid_constant__ TileArgs a, const __grid_constant__ CUt
             for (uint32_t s = 0; s < all;) {
                 const uint32_t in_block = step & 3u, n = min(4u - in_block, all - s);
                 if (in_block == 0) {                // entering a block of the ring: it has landed, and the one before is free
-                    if (ring_mask == 1) asm volatile("cp.async.wait_group 0;" ::: "memory");
-                    else asm volatile("cp.async.wait_group 2;" ::: "memory");
+                    asm volatile("cp.async.wait_group 0;" ::: "memory");
                     __syncwarp();
-                    fill(step / 4 + ring_mask);
+                    fill(step / 4 + 1);
                 }
-                const uint32_t at = ring + ((step & (4 * ring_mask + 3)) * 128u) + r * 16;
+                const uint32_t at = place(step);
                 switch (n) {                        // unrolled: the hand-off and the gathers of a step run ahead of its FMAs
                 case 1: tile_steps<NV, 1>(acc, at, xbase); break;
                 case 2: tile_steps<NV, 2>(acc, at, xbase); break;
@@ -542,8 +547,7 @@ template <int NV, int WARPS>
 static int launch_tile_nv(const spx_ell* e, TileArgs a, const CUtensorMap& map, uint32_t warps, uint32_t slices, cudaStream_t s)
 {
     a.row_blocks = (a.groups + warps - 1) / warps;
-    a.ring_blocks = WARPS < (int)kMaxWarps ? 4 : 2;
-    size_t smem = (size_t)(kStages * kChunk + 1) * NV * 128 + (size_t)warps * a.ring_blocks * 512;
+    size_t smem = (size_t)(kStages * kChunk + 1) * NV * 128 + (size_t)warps * kRingBlocks<WARPS> * 512;
     // One CTA to an SM where the grid is one wave: started while the kernel before still fills some of the SMs, two small ones
     // share one and take twice as long (435 x 3968, 35 %, C = 274, behind the copy of X: 61 us against 34).
     if (a.row_blocks * slices <= sm_count(e->device)) smem = std::max<size_t>(smem, 116 * 1024);
