@@ -618,8 +618,12 @@ double gather_us(const spx_ell* e, uint32_t C, uint32_t V, bool half)
     const bool brief = e->nnz_total < 100ull * e->m;
     const double load = V == 4 ? 3.15e-3 : V == 2 ? 1.7e-3 : 1.34e-3, off_lines = V == 4 ? 0.47e-3 : V == 2 ? 0.5e-3 : 0.39e-3;
     double loads = e->nnz_total / sms * panels * (load * NV / RW + (C % 32 ? off_lines : 0.0)) + (brief ? 0.037 : 0.10) * per_sm;
-    if (V == 4 && NV == 2 && per_sm >= 12 && !brief)        // 16 warps reside: a last round of a few takes as long as a full one
+    // Two CTAs of 8 warps reside: a last round of a few takes as long as a full one.  From the second CTA on: by the average, matrices
+    // with 8 to 12 warps per SM were expected in 0.8 of what gathering them takes (41 shapes).
+    if (V == 4 && NV == 2 && per_sm > 8 && !brief)
         loads = e->nnz_total / sms * panels * (5.5e-3 + (C % 32 ? off_lines : 0.0)) * std::ceil(per_sm / 16.0) * 16.0 / per_sm;
+    else if (V == 4 && NV == 2 && per_sm > 8 && per_sm < 12)
+        loads *= 1.25;
     if (V == 4 && RW > 1 && !brief) {           // long rows side by side in a warp: half as if each took a power of two of lanes
         uint32_t lanes = 1;
         while (lanes < q) lanes *= 2;
