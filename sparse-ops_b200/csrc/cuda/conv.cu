@@ -721,6 +721,8 @@ void free_conv_tables(spx_ell* e)
     for (ConvTables::Shape* s = t->shapes; s;) {
         pool_free(s->taps, (size_t)e->m * e->pitch * sizeof(uint32_t), nullptr);
         pool_free(s->hdr, merged_slots(e) * sizeof(uint2), nullptr);
+        for (cudaEvent_t ev : {s->taps_built.done, s->hdr_built.done})
+            if (ev) (void)cudaEventDestroy(ev);
         ConvTables::Shape* next = s->next;
         delete s;
         s = next;
@@ -751,18 +753,48 @@ static ConvTables::Shape* shape_tables(ConvTables* t, uint32_t kH, uint32_t kW)
     return t->shapes = s;
 }
 
-// Tables are built on a stream beside the call's, which is waited for: the calls of other threads and streams find them
-// complete, and where the call's stream is being recorded they are there before the graph runs.  (A handle's arrays are
-// complete when it is handed out, so there is nothing to wait for before.)
+// Tables are built on a stream beside the call's, not behind what the caller has queued.  (A handle's arrays are complete when it is
+// handed out, so there is nothing to wait for before.)  The call's stream waits for the event behind the build, and so does
+// any other call's until it has passed; where the call is being recorded, the call itself does: the table is there before
+// the graph runs and before eager calls.  (Waiting for every build on the host made a handle's first call 12 to 20 us longer.)
+static int table_queued(ConvTables::Built& b, cudaStream_t side)
+{
+    cudaError_t err = cudaGetLastError();
+    if (err != cudaSuccess) return fail(SPX_ERR_CUDA, "conv2d: building a table failed: %s", cudaGetErrorString(err));
+    count_launch_beside();
+    if (cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming) == cudaSuccess && cudaEventRecord(b.done, side) == cudaSuccess) {
+        b.pending = true;
+        return SPX_OK;
+    }
+    (void)cudaGetLastError();
+    SPX_CUDA(cudaStreamSynchronize(side));
+    return SPX_OK;
+}
+static int table_behind(ConvTables::Built& b, cudaStream_t s)
+{
+    if (!b.pending) return SPX_OK;
+    RelaxedCapture relaxed;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool recorded = cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+    (void)cudaGetLastError();
+    cudaError_t err = recorded ? cudaEventSynchronize(b.done) : cudaEventQuery(b.done);
+    b.pending = err == cudaErrorNotReady;
+    if (b.pending) {
+        (void)cudaGetLastError();
+        err = cudaStreamWaitEvent(s, b.done, 0);
+    }
+    SPX_CUDA(err);
+    return SPX_OK;
+}
 
 // The tap table of a kernel shape, built once per handle; null where there is no memory for it.
-static int ensure_taps(spx_ell* e, uint32_t kH, uint32_t kW, const uint32_t** taps)
+static int ensure_taps(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s, const uint32_t** taps)
 {
     std::lock_guard<std::mutex> lk(e->conv->mu);
     ConvTables::Shape* t = shape_tables(e->conv, kH, kW);
     if (!t) return fail(SPX_ERR_OOM, "out of host memory");
     *taps = t->taps;
-    if (t->taps || e->r == 0) return SPX_OK;
+    if (t->taps || e->r == 0) return table_behind(t->taps_built, s);
     RelaxedCapture relaxed;                     // allocations and waits below end no capture
     cudaStream_t side = nullptr;
     if (int rc = side_stream(e->device, &side)) return rc;
@@ -773,17 +805,12 @@ static int ensure_taps(spx_ell* e, uint32_t kH, uint32_t kW, const uint32_t** ta
         return t->no_taps ? SPX_OK : rc;
     }
     build_taps_kernel<<<e->m, 128, 0, side>>>(e->idx, e->nnz, e->m, e->pitch, kH, kW, static_cast<uint32_t*>(made));
-    cudaError_t err = cudaGetLastError();
-    if (err == cudaSuccess) {
-        count_launch_beside();
-        err = cudaStreamSynchronize(side);
-    }
-    if (err != cudaSuccess) {
+    if (int rc = table_queued(t->taps_built, side)) {
         pool_free(made, bytes, side);
-        return fail(SPX_ERR_CUDA, "conv2d: building the tap table failed: %s", cudaGetErrorString(err));
+        return rc;
     }
     *taps = t->taps = static_cast<uint32_t*>(made);
-    return SPX_OK;
+    return table_behind(t->taps_built, s);
 }
 
 // Scratch for a call's input, kept with the handle and grown as needed, by a call that is recorded too: calls before it may
@@ -858,14 +885,14 @@ static bool rbm_fits(const ConvParams& p, uint32_t qb, int nb, int g)
 }
 
 // The row-block-merged weights, built once per handle, and the headers of a kernel shape, built as ensure_taps does.
-int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, const uint2** hdr)
+int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s, const uint2** hdr)
 {
     ConvTables* t = e->conv;
     std::lock_guard<std::mutex> lk(t->mu);
     ConvTables::Shape* shape = shape_tables(t, kH, kW);
     if (!shape) return fail(SPX_ERR_OOM, "out of host memory");
     if (hdr) *hdr = shape->hdr;
-    if (shape->hdr) return SPX_OK;
+    if (shape->hdr) return table_behind(shape->hdr_built, s);
     if (t->no_merged || shape->no_hdr) return -1;
     RelaxedCapture relaxed;                     // allocations and waits below end no capture
     cudaStream_t side = nullptr;
@@ -880,24 +907,19 @@ int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, const uint2** hdr)
     int rc = pool_alloc(&made, slots * sizeof(uint2), e->device, side);
     if (rc == SPX_OK && first) rc = pool_alloc(&w, slots * kRbmRows * sizeof(float), e->device, side);
     if (rc == SPX_OK && first) rc = pool_alloc(&ncols, nblocks * sizeof(uint32_t), e->device, side);
-    cudaError_t err = cudaSuccess;
     if (rc == SPX_OK) {
         ensure_tma_words(e);
         (void)cudaGetLastError();
         const size_t smem = (size_t)((e->n + 31) / 32) * 2 * sizeof(uint32_t);
         build_rbm_kernel<<<nblocks, 256, smem, side>>>(e->Wd, e->idx, e->nnz, e->m, e->n, e->pitch, kH, kW, t->cap,
                                                        static_cast<uint2*>(made), static_cast<float*>(w), static_cast<uint32_t*>(ncols));
-        err = cudaGetLastError();
-        if (err == cudaSuccess) {
-            count_launch_beside();
-            err = cudaStreamSynchronize(side);
-        }
+        rc = table_queued(shape->hdr_built, side);
     }
-    if (rc != SPX_OK || err != cudaSuccess) {
+    if (rc != SPX_OK) {
         pool_free(made, slots * sizeof(uint2), side);
         pool_free(w, slots * kRbmRows * sizeof(float), side);
         pool_free(ncols, nblocks * sizeof(uint32_t), side);
-        if (err != cudaSuccess) return fail(SPX_ERR_CUDA, "conv2d: merging the weights failed: %s", cudaGetErrorString(err));
+        if (rc != SPX_ERR_OOM) return rc;
         if (first) t->no_merged = true;
         else shape->no_hdr = true;
         return -1;
@@ -908,7 +930,7 @@ int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, const uint2** hdr)
     }
     shape->hdr = static_cast<uint2*>(made);
     if (hdr) *hdr = shape->hdr;
-    return SPX_OK;
+    return table_behind(shape->hdr_built, s);
 }
 
 // Whether every segment of the batch does in the merged kernel's largest cut.
@@ -1060,7 +1082,7 @@ static int launch_rbm_qb(spx_ell* e, TileParams tp, const float* in, const float
     const uint64_t units = tiles * groups * (b_len / (QB * 4));
     if (units > 0x3fffffffull) return -1;
     const uint2* hdr = nullptr;
-    const int rc = ensure_rbm(e, p.kH, p.kW, &hdr);
+    const int rc = ensure_rbm(e, p.kH, p.kW, s, &hdr);
     if (rc != SPX_OK) return rc;                        // -1: no memory for the merged weights
     RbmUnits un{0u, (uint32_t)tiles, groups, 0u};
     if (cut.nb == 8 && cut.g == 4) return launch_rbm_units<QB, 8, 4>(e, hdr, tp, un, (uint32_t)units, in, bias, act, out, s, b_avail);
@@ -1395,7 +1417,7 @@ int launch_conv2d(spx_ell* e, const spx_conv_geom* g, int layout, const float* i
         }
     }
     const uint32_t* taps = nullptr;
-    if (int rc = ensure_taps(e, g->kH, g->kW, &taps)) return rc;
+    if (int rc = ensure_taps(e, g->kH, g->kW, s, &taps)) return rc;
     ConvParams p{g->Cin, g->Cout, g->kH, g->kW, g->sH, g->sW, g->pH, g->pW, g->dH, g->dW,
                  g->H, g->W, g->Ho, g->Wo, B};
     // The tiled kernels read the batch as the innermost dimension, in multiples of 4 and of 16 bytes, and

@@ -43,14 +43,19 @@ struct ConvGatherPlan {
 bool plan_conv_gather(const spx_ell* e, const ConvParams& p, int layout, const float* in, const float* out, ConvGatherPlan& plan);
 int launch_conv_gather(const spx_ell* e, const uint32_t* taps, const ConvParams& p, int layout, const float* in, const float* bias, int act, float* out,
                        const ConvGatherPlan& plan, cudaStream_t s);
-// What a handle's convolutions share.  Built by whichever call first needs it, on any thread and stream: under the lock, and
-// complete for every stream when that is let go.  Nothing is changed or given back before the handle is: calls in flight
-// and recorded graphs may be using it.
+// What a handle's convolutions share.  Built under the lock by whichever call first needs it, on any thread and stream; every
+// call's stream is behind that, and a recorded call's table complete, before it is used.  Nothing is changed or given back before
+// the handle is: calls in flight and recorded graphs may be using it.
 struct ConvTables {
+    struct Built {
+        cudaEvent_t done = nullptr;
+        bool pending = false;       // not known to be complete
+    };
     struct Shape {                  // of a kernel
         uint32_t kH = 0, kW = 0;
         uint32_t* taps = nullptr;   // per slot of the slab: the column as cin << 16 | kh << 8 | kw
         uint2* hdr = nullptr;       // per merged column: (the same, bit r set when row r of the block stores it)
+        Built taps_built, hdr_built;
         bool no_taps = false, no_hdr = false;   // an earlier call found no memory for them
         Shape* next = nullptr;
     };
@@ -77,8 +82,9 @@ struct ConvTables {
 };
 ConvTables* new_conv_tables();
 void free_conv_tables(spx_ell* e);
-// conv.cu: the merged weights of conv_rbm_tile_kernel, and (hdr may be null) their headers; -1 where there is no memory for them.
-int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, const uint2** hdr);
+// conv.cu: the merged weights of conv_rbm_tile_kernel, for use on s, and (hdr may be null) their headers; -1 where there is no
+// memory for them.
+int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s, const uint2** hdr);
 void* new_conv_tmem();
 void free_conv_tmem(spx_ell* e);
 

@@ -580,7 +580,7 @@ static int find_form(spx_ell* e, const FormShape& f, uint32_t chunks, uint32_t p
     }
     RelaxedCapture relaxed;                     // s is not being captured; another stream may be, by this thread
     // The other kernel's weights, which a later call may take (another batch, say); how many columns they have is counted below.
-    const int merged = ensure_rbm(e, f.kH, f.kW, nullptr);
+    const int merged = ensure_rbm(e, f.kH, f.kW, s, nullptr);
     if (merged > 0) return merged;
     ensure_tma_words(e);
     if (!e->tma_failed_dev || !e->tma_failed_mapped) {
