@@ -753,31 +753,35 @@ static ConvTables::Shape* shape_tables(ConvTables* t, uint32_t kH, uint32_t kW)
     return t->shapes = s;
 }
 
-// Tables are built on a stream beside the call's, not behind what the caller has queued.  (A handle's arrays are complete when it is
-// handed out, so there is nothing to wait for before.)  The call's stream waits for the event behind the build, and so does
-// any other call's until it has passed; where the call is being recorded, the call itself does: the table is there before
-// the graph runs and before eager calls.  (Waiting for every build on the host made a handle's first call 12 to 20 us longer.)
-static int table_queued(ConvTables::Built& b, cudaStream_t side)
+// Tables are built on the call's stream, and other calls' streams wait for the event behind that until it has passed.  A call that
+// is being recorded builds them on a stream beside it and waits itself: they are there before the graph runs and before
+// eager calls.  (A handle's arrays are complete when it is handed out, so there is nothing to wait for before.  Waiting on the
+// host every time made a handle's first call 12 to 20 us longer; kernels on the side stream, every later wait for the device 9.)
+static bool is_recorded(cudaStream_t s)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) == cudaSuccess) return cap != cudaStreamCaptureStatusNone;
+    (void)cudaGetLastError();                   // the default stream while another one is being recorded
+    return true;
+}
+static int table_queued(ConvTables::Built& b, cudaStream_t on, bool recorded)
 {
     cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return fail(SPX_ERR_CUDA, "conv2d: building a table failed: %s", cudaGetErrorString(err));
-    count_launch_beside();
-    if (cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming) == cudaSuccess && cudaEventRecord(b.done, side) == cudaSuccess) {
+    recorded ? count_launch_beside() : count_launch();
+    if (!recorded && cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming) == cudaSuccess && cudaEventRecord(b.done, on) == cudaSuccess) {
         b.pending = true;
         return SPX_OK;
     }
     (void)cudaGetLastError();
-    SPX_CUDA(cudaStreamSynchronize(side));
+    SPX_CUDA(cudaStreamSynchronize(on));
     return SPX_OK;
 }
 static int table_behind(ConvTables::Built& b, cudaStream_t s)
 {
     if (!b.pending) return SPX_OK;
     RelaxedCapture relaxed;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    const bool recorded = cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
-    (void)cudaGetLastError();
-    cudaError_t err = recorded ? cudaEventSynchronize(b.done) : cudaEventQuery(b.done);
+    cudaError_t err = is_recorded(s) ? cudaEventSynchronize(b.done) : cudaEventQuery(b.done);
     b.pending = err == cudaErrorNotReady;
     if (b.pending) {
         (void)cudaGetLastError();
@@ -796,21 +800,22 @@ static int ensure_taps(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s, con
     *taps = t->taps;
     if (t->taps || e->r == 0) return table_behind(t->taps_built, s);
     RelaxedCapture relaxed;                     // allocations and waits below end no capture
-    cudaStream_t side = nullptr;
-    if (int rc = side_stream(e->device, &side)) return rc;
+    const bool recorded = is_recorded(s);
+    if (recorded)
+        if (int rc = side_stream(e->device, &s)) return rc;
     const size_t bytes = (size_t)e->m * e->pitch * sizeof(uint32_t);
     void* made = nullptr;
-    if (int rc = pool_alloc(&made, bytes, e->device, side, t->no_taps)) {
+    if (int rc = pool_alloc(&made, bytes, e->device, s, t->no_taps)) {
         t->no_taps = rc == SPX_ERR_OOM;
         return t->no_taps ? SPX_OK : rc;
     }
-    build_taps_kernel<<<e->m, 128, 0, side>>>(e->idx, e->nnz, e->m, e->pitch, kH, kW, static_cast<uint32_t*>(made));
-    if (int rc = table_queued(t->taps_built, side)) {
-        pool_free(made, bytes, side);
+    build_taps_kernel<<<e->m, 128, 0, s>>>(e->idx, e->nnz, e->m, e->pitch, kH, kW, static_cast<uint32_t*>(made));
+    if (int rc = table_queued(t->taps_built, s, recorded)) {
+        pool_free(made, bytes, s);
         return rc;
     }
     *taps = t->taps = static_cast<uint32_t*>(made);
-    return table_behind(t->taps_built, s);
+    return SPX_OK;
 }
 
 // Scratch for a call's input, kept with the handle and grown as needed, by a call that is recorded too: calls before it may
@@ -818,8 +823,7 @@ static int ensure_taps(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s, con
 static int input_scratch(spx_ell* e, size_t need, cudaStream_t s, float** out)
 {
     ConvTables* t = e->conv;
-    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    const bool recorded = cudaStreamIsCapturing(s, &status) == cudaSuccess && status != cudaStreamCaptureStatusNone;
+    const bool recorded = is_recorded(s);
     if (t->scratch.bytes < need) {
         RelaxedCapture relaxed;                 // allocations and waits below end no capture
         if (t->scratch_recorded) {
@@ -892,33 +896,36 @@ int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s, const uint2
     ConvTables::Shape* shape = shape_tables(t, kH, kW);
     if (!shape) return fail(SPX_ERR_OOM, "out of host memory");
     if (hdr) *hdr = shape->hdr;
+    if (t->first)
+        if (int rc = table_behind(t->first->hdr_built, s)) return rc;
     if (shape->hdr) return table_behind(shape->hdr_built, s);
     if (t->no_merged || shape->no_hdr) return -1;
     RelaxedCapture relaxed;                     // allocations and waits below end no capture
-    cudaStream_t side = nullptr;
-    if (int rc = side_stream(e->device, &side)) return rc;
+    const bool recorded = is_recorded(s);
+    if (recorded)
+        if (int rc = side_stream(e->device, &s)) return rc;
     const uint32_t nblocks = (e->m + kRbmRows - 1) / kRbmRows;
     // Up to three times the ELLPACK slab (24 bytes per union column, at most 4 * max_nnz columns
     // per block of 4 rows).  Without room for it the per-row kernel is used instead.
-    const bool first = !t->w;
+    const bool first = !t->first;
     if (first) t->cap = (uint32_t)std::min<uint64_t>((uint64_t)kRbmRows * e->max_nnz, e->n);
     const size_t slots = merged_slots(e);
     void *w = nullptr, *ncols = nullptr, *made = nullptr;
-    int rc = pool_alloc(&made, slots * sizeof(uint2), e->device, side);
-    if (rc == SPX_OK && first) rc = pool_alloc(&w, slots * kRbmRows * sizeof(float), e->device, side);
-    if (rc == SPX_OK && first) rc = pool_alloc(&ncols, nblocks * sizeof(uint32_t), e->device, side);
+    int rc = pool_alloc(&made, slots * sizeof(uint2), e->device, s);
+    if (rc == SPX_OK && first) rc = pool_alloc(&w, slots * kRbmRows * sizeof(float), e->device, s);
+    if (rc == SPX_OK && first) rc = pool_alloc(&ncols, nblocks * sizeof(uint32_t), e->device, s);
     if (rc == SPX_OK) {
         ensure_tma_words(e);
         (void)cudaGetLastError();
         const size_t smem = (size_t)((e->n + 31) / 32) * 2 * sizeof(uint32_t);
-        build_rbm_kernel<<<nblocks, 256, smem, side>>>(e->Wd, e->idx, e->nnz, e->m, e->n, e->pitch, kH, kW, t->cap,
+        build_rbm_kernel<<<nblocks, 256, smem, s>>>(e->Wd, e->idx, e->nnz, e->m, e->n, e->pitch, kH, kW, t->cap,
                                                        static_cast<uint2*>(made), static_cast<float*>(w), static_cast<uint32_t*>(ncols));
-        rc = table_queued(shape->hdr_built, side);
+        rc = table_queued(shape->hdr_built, s, recorded);
     }
     if (rc != SPX_OK) {
-        pool_free(made, slots * sizeof(uint2), side);
-        pool_free(w, slots * kRbmRows * sizeof(float), side);
-        pool_free(ncols, nblocks * sizeof(uint32_t), side);
+        pool_free(made, slots * sizeof(uint2), s);
+        pool_free(w, slots * kRbmRows * sizeof(float), s);
+        pool_free(ncols, nblocks * sizeof(uint32_t), s);
         if (rc != SPX_ERR_OOM) return rc;
         if (first) t->no_merged = true;
         else shape->no_hdr = true;
@@ -927,10 +934,11 @@ int ensure_rbm(spx_ell* e, uint32_t kH, uint32_t kW, cudaStream_t s, const uint2
     if (first) {
         t->w = static_cast<float*>(w);
         t->ncols = static_cast<uint32_t*>(ncols);
+        t->first = shape;
     }
     shape->hdr = static_cast<uint2*>(made);
     if (hdr) *hdr = shape->hdr;
-    return table_behind(shape->hdr_built, s);
+    return SPX_OK;
 }
 
 // Whether every segment of the batch does in the merged kernel's largest cut.
@@ -1273,11 +1281,10 @@ union_count_kernel(const uint32_t* __restrict__ idx, const uint32_t* __restrict_
     if (threadIdx.x == 0) blocks[blockIdx.x] = make_uint2(s_fresh, all);
 }
 
-// Counts once per handle, beside the call like the tables.  Not for a call that is recorded.
+// Counts once per handle; the call then waits for its stream.  Not for a call that is recorded.
 static void count_loads(spx_ell* e, cudaStream_t s)
 {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) { (void)cudaGetLastError(); return; }
+    if (is_recorded(s)) return;
     ConvTables* t = e->conv;
     std::lock_guard<std::mutex> lk(t->mu);
     if (t->loads_state.load(std::memory_order_relaxed) != ConvTables::unknown) return;
@@ -1286,19 +1293,18 @@ static void count_loads(spx_ell* e, cudaStream_t s)
     const size_t bytes = (size_t)nblocks * sizeof(uint2);
     PinnedBlock host;
     void* blocks = nullptr;
-    cudaStream_t side = nullptr;
     int state = ConvTables::no_memory;
-    if (side_stream(e->device, &side) == SPX_OK && scratch_alloc(&blocks, bytes, e->device, side, true) == SPX_OK && pinned_acquire(bytes, &host) == SPX_OK) {
-        union_count_kernel<<<nblocks, 256, (e->n + 31) / 32 * 4, side>>>(e->idx, e->nnz, e->m, e->n, e->pitch, static_cast<uint2*>(blocks));
-        count_launch_beside();
-        if (cudaGetLastError() == cudaSuccess && cudaMemcpyAsync(host.host, blocks, bytes, cudaMemcpyDeviceToHost, side) == cudaSuccess &&
-            cudaStreamSynchronize(side) == cudaSuccess) {
+    if (scratch_alloc(&blocks, bytes, e->device, s, true) == SPX_OK && pinned_acquire(bytes, &host) == SPX_OK) {
+        union_count_kernel<<<nblocks, 256, (e->n + 31) / 32 * 4, s>>>(e->idx, e->nnz, e->m, e->n, e->pitch, static_cast<uint2*>(blocks));
+        count_launch();
+        if (cudaGetLastError() == cudaSuccess && cudaMemcpyAsync(host.host, blocks, bytes, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
+            cudaStreamSynchronize(s) == cudaSuccess) {
             merged_loads(static_cast<const uint2*>(host.host), nblocks, t->loads);
             state = ConvTables::counted;
         }
     }
     pinned_release(host);
-    scratch_free(blocks, side);
+    scratch_free(blocks, s);
     t->loads_state.store(state, std::memory_order_release);
 }
 

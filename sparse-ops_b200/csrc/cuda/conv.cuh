@@ -63,7 +63,8 @@ struct ConvTables {
     Shape* shapes = nullptr;        // as many as the handle is used with: divisors of its columns
     // Row-block-merged weights (conv.cu): per block of 4 rows the ascending union of their column ids.  Block b owns entries
     // [b * cap, b * cap + ncols[b]): the 4 rows' weights, 0.0f where a row has none, and the headers above.
-    float* w = nullptr;
+    float* w = nullptr;             // built with the first shape's headers
+    Shape* first = nullptr;
     uint32_t* ncols = nullptr;
     uint32_t cap = 0;
     std::atomic<bool> no_merged{false};     // an earlier call found no memory for them
