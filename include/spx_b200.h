@@ -10,8 +10,8 @@
  *   - `stream` is a cudaStream_t passed as void* (NULL = the default stream).  Kernel
  *     entry points only enqueue work; they do not synchronise.
  *   - A handle may be used from several host threads for kernel launches, but entry points
- *     that grow per-handle scratch (spx_conv2d's first call per kernel shape, its NCHW and
- *     F-major layouts and batch sizes that are not a multiple of 4,
+ *     that grow per-handle scratch (spx_conv2d in its NCHW and F-major layouts, with batch
+ *     sizes that are not a multiple of 4 and with inputs off 16 bytes,
  *     the first spx_spmv of a handle with n > 51200, the *_host calls) must not run concurrently
  *     on the same handle.
  *   - There is no CPU fallback: without a usable CUDA device every compute entry point
@@ -163,16 +163,19 @@ int spx_spmv_reference_order(const spx_ell* e, const float* x, const float* bias
  * [Cout x Cin*kH*kW].  Replaces conv2d_patchmajor_tiled / conv2d_tiled_im2col_cmajor /
  * conv2d_tiled_im2col_fmajor / conv2d_rbm_fmajor_implicit (src/layers/conv_kernels.cpp:66-470)
  * and, on the device, build_rbm_from_ellpack (src/layers/rbm_conv.cpp:7-73): the first call per
- * handle and kernel shape builds and caches a tap table (4 bytes a slot of the slab), where the
- * batch size and weight density favour it, the row-block-merged form of the weights (up to three
- * slabs) and, for larger calls, a second form for the kernel that keeps its input in tensor memory
- * (about a slab per kernel shape, dilation and row stride, at most four), beside which it builds
- * the first as well: the two are compared.  (Device allocations, and a wait for `stream`; make
- * that call outside a stream capture: a captured call uses the forms that are there.)  Small calls gather
- * their input and use the tap table alone; a handle's first one may wait for `stream` to count the columns that
- * its rows share.  A form that
- * finds no memory is gone without from then on.  Results do not depend on which kernel is chosen.  Both of those kernels fetch their
- * input with bulk tensor copies: see spx_ell_status. */
+ * handle and kernel shape builds and caches a tap table (4 bytes a slot of the slab), and where they
+ * favour it by batch size, density and where the entries lie, calls build the row-block-merged form of the
+ * weights (up to three slabs; one for each further kernel shape) and, for larger calls, another one for the
+ * kernel that keeps its input in tensor memory (about a slab per kernel shape, dilation and row stride, at
+ * most four), beside which the merged one is built as well: the two are compared.  Small calls gather their
+ * input and use the tap table alone.  Any call may be the first to need a form, on any stream and thread; what is built
+ * stays as it is until the handle is destroyed, so graphs and calls of several kernel shapes go side by side.
+ * Building allocates device memory.  The form for tensor memory, and a count of the columns that rows share (once per handle,
+ * where the choice depends on it), also wait for `stream`.  A call that is being captured builds the tap table and the
+ * merged form where they are missing, at once and beside the capture, and waits for them; it builds and counts nothing
+ * else, so make a first call outside.  Without memory a form is done without from then on (without a tap table the
+ * general kernel decodes the columns, and later calls try again).  Results do not depend on which kernel is chosen.  The merged and the tensor-memory
+ * kernel fetch their input with bulk tensor copies: see spx_ell_status. */
 int spx_conv2d(const spx_ell* e, const spx_conv_geom* g, int layout, const float* in, uint32_t B,
                const float* bias, int act, float* out, void* stream);
 /* spx_conv2d for callers that must not allocate device memory (no counterpart in the

@@ -1349,8 +1349,9 @@ static double per_row_least_us(const spx_ell* e, const ConvParams& p, bool copie
 // longer).  Sure if it is so for the least that these can take, and not worth a count if it is not so by the density;
 // else the columns that rows share are counted, which the density does not tell.  Measured on 173 drawn shapes of 8 us and
 // more that were not fitted to, the calls take 0.65 of the time they took before there was this kernel, none of them 5 % longer;
-// on 500 shapes with weights of eleven kinds (iid, rows of different density, channels, kernels or patterns removed) 0.73, 4 of
-// them more than 10 % longer.  By the density alone some structured kinds had calls 1.3 to 1.5 times as long.
+// on 866 shapes with weights of eleven kinds (iid, rows of different density, channels, kernels or patterns removed) 0.68, 12
+// of them more than 10 % longer (up to 1.34, uneven rows).  By the density alone some structured kinds had calls 1.3 to 1.5
+// times as long; a penalty for uneven rows gave away more than it saved.
 static bool gather_pays(spx_ell* e, const ConvParams& p4, const ConvViews& v, bool copies, uint32_t B, const ConvGatherPlan& plan, cudaStream_t s)
 {
     const double us = plan.us / (plan.form >= 2 ? 0.85 : 0.9);

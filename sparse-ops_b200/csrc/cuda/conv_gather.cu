@@ -6,7 +6,7 @@
 // stride, the last three of four batch entries are padding, and NCHW images are copied first.  Here a warp takes one output
 // channel at 32 V positions and loads each operand when it needs it: no staging, no copy, no padding, any batch and layout.
 //
-// Bound by issue slots (65 to 70 % used; 6 to 9 an operand, 200 to 400 a warp for its ends), L1 wavefronts (50 %; a stride
+// Bound by issue slots (63 % used; 6 to 9 an operand, 200 to 400 a warp for its ends), L1 wavefronts (48 %; a stride
 // of two or positions that are not neighbours in memory take two to 32 a load) and, with few warps, by the round trips of a
 // row's entries, 8 at a time.  Measured against the tiled kernels: 64 -> 128 channels, 3 x 3, stride 2, 57 x 57, batch 3,
 // NCHW 28 -> 15 us; 219 -> 32, 3 x 3, stride 2, 104 x 104, batch 1 100 -> 17; 384 -> 25, 3 x 3, 9 x 9, batch 27 300 -> 44; 96 -> 214,

@@ -19,7 +19,7 @@
 // Bound by shared-memory wavefronts (16 NV + 4 per step and warp) with many warps per SM, by the latency
 // of a warp's steps (0.04 us each, 0.05 with slices of 64) and the phases with few; chunks of 128 columns, six of them staged, lose 1 to 60 % to
 // the phases' fixed cost, 192 x 4 up to 4 %.  Measured against gathering: 4096 x 4096, 10 %, C = 64 / 128 / 256 / 512
-// 19.5 / 32.7 / 61.5 / 121.7 us against 26.1 / 43.5 / 72.5 / 141.6; 8192 x 8192, 10 %, C = 64 62.9 against 103;
+// 18.9 / 32.7 / 60.8 / 121 us against 25.3 / 43.5 / 72.6 / 142; 8192 x 8192, 10 %, C = 64 62.9 against 103;
 // 3512 x 3227, 19 %, C = 160 59.5 against 106; 4927 x 3082, 21 %, C = 160 86.8 against 159.
 #include "common.cuh"
 #include "tma.cuh"
@@ -222,8 +222,8 @@ template <int WARPS> constexpr uint32_t kRingBlocks = WARPS < (int)kMaxWarps ? 4
 
 // For CTAs of up to WARPS warps.  kMaxWarps of them pass their gathers at the rate of shared memory with one step's operands
 // in registers; fewer wait for their own latencies, and have registers for two steps (kDeep below).  2048 x 2048, 30 %,
-// C = 32 16.6 -> 11.2 us, 640 x 1955, 35 %, C = 35 18.9 -> 14.0; 4096 x 4096, 10 %, C = 64 24.7 -> 19.3; 3001 x 4999, 6 %,
-// C = 64 19.0 -> 15.5.  The steps' places in their blocks are known to the compiler: with one loop of steps, whose next block
+// C = 32 16.6 -> 11.1 us, 640 x 1955, 35 %, C = 35 18.9 -> 14.0; 4096 x 4096, 10 %, C = 64 24.7 -> 18.9; 3001 x 4999, 6 %,
+// C = 64 19.0 -> 15.4.  The steps' places in their blocks are known to the compiler: with one loop of steps, whose next block
 // and register set are found at run time, these were 16.1, -, 21.6 and 16.6.
 template <int NV, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 1)
@@ -413,9 +413,8 @@ spmm_tile_kernel(const __grid_constant__ TileArgs a, const __grid_constant__ CUt
         // No later phase reads chunk c + 1 - kWindow: the last warp to get here asks for the chunk that takes its
         // place.  The arrival tells whether it is the last (one pending before it) and releases this warp's reads;
         // the test of the phase it has just completed acquires the other warps' arrivals, so that all reads of the
-        // stage come before the copy unit's writes (3001 x 4999, 6 %, C = 77: 28.2 us without it, 28.8 so, 29.6 with the
-        // whole bounded wait).  A fence and an atomic instead would wait for the warp's cp.async in flight, 1500 cycles
-        // per chunk.
+        // stage come before the copy unit's writes (3001 x 4999, 6 %, C = 77: 21.5 us; 24.6 with the whole bounded wait in its
+        // place).  A fence and an atomic instead would wait for the warp's cp.async in flight, 1500 cycles per chunk.
         const uint32_t out = c + 1 - kWindow, st = out % kStages;
         if (lane == 0 && spx::mbar_arrive_pending(&s_free[st]) == 1u && landed && out + kStages < a.chunks) {
             spx::mbar_acquire(&s_free[st], (out / kStages) & 1u);

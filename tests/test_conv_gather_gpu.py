@@ -312,8 +312,8 @@ def test_second_kernel_shape_without_memory(lib, orc, cuda):
 
 def exhaust(lib):
     """Takes all device memory, what the library's pool has left included."""
-    held, handles = fill_device(lib, 0, 2 << 20), []
-    for m in (1 << 20, 1 << 16, 1 << 12, 1 << 8, 1 << 6):   # 12 bytes a row
+    held, handles = fill_device(lib, 64 << 20, 16 << 20), []
+    for m in (1 << 22, 1 << 20, 1 << 16, 1 << 12, 1 << 8, 1 << 6):   # 12 bytes a row
         nnz = np.zeros(m, np.uint32)
         try:
             while True:
