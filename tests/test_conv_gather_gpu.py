@@ -398,6 +398,38 @@ def test_recorded_calls_that_need_more_scratch(lib, orc, cuda, first):
 
 
 @chosen
+def test_recording_while_a_table_is_being_built(lib, orc, cuda):
+    """The build of the tables is queued behind a long kernel when the same stream begins to record calls that need them: those
+    wait for it, and calls on another stream come behind it."""
+    rng, C, H = np.random.default_rng(20), 64, 28
+    E = orc.encode(sparse(rng, C, C * 9, 0.3))
+    h, g, x = gpu_ell(lib, E), sx.conv_geom(C, C, 3, 3, H, H, 2, 2, 1, 1), rng.standard_normal((32, C, H, H)).astype(np.float32)
+    stream, other, graph, runs = torch.cuda.Stream(), torch.cuda.Stream(), ctypes.c_void_p(), []
+    for B in (1, 32):
+        src = as_layout(x[:B], sx.LAYOUT_PF)
+        want = orc.conv2d(E, dict(Cin=C, kH=3, kW=3, sH=2, sW=2, pH=1, pW=1, dH=1, dW=1, H=H, W=H), sx.LAYOUT_PF, src, B, None, 0)
+        runs.append((B, dev(src, cuda), want, [torch.full(want.shape, float("nan"), device=cuda) for _ in range(3)]))
+    call = lambda run, k, st: h.conv2d(g, sx.LAYOUT_PF, ptr(run[1]), run[0], None, 0, ptr(run[3][k]), st.cuda_stream)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(200_000_000)
+    call(runs[0], 0, stream)                                # batch 1: the tap table alone
+    call(runs[0], 1, other)
+    lib.spx_graph_capture_begin(stream.cuda_stream)
+    for run in runs:
+        call(run, 2, stream)
+    lib.spx_graph_capture_end(stream.cuda_stream, ctypes.byref(graph))
+    call(runs[1], 0, other)
+    call(runs[1], 1, stream)
+    lib.spx_graph_launch(graph, stream.cuda_stream)
+    torch.cuda.synchronize()
+    for B, _, want, outs in runs:
+        for k, y in enumerate(outs):
+            assert_bit_equal(y.cpu().numpy(), want, f"batch {B}, call {k}")
+    lib.spx_graph_destroy(graph)
+
+
+@chosen
 def test_recording_a_merged_call_waits_for_no_other_work(lib, orc, cuda):
     """Recording a call that lacks the merged weights builds them at once, beside what other streams do: that kernel is no part
     of the graph."""
